@@ -7,12 +7,11 @@
 // (plate/Constraints.h:54-119, 341-436), Meshless::assembleSystem* (plate/Meshless.h:102-127)
 // and the energies (plate/Meshless.h:197-220, Constraints.h:310-339).
 //
-// One warp per Gauss point. Lanes first reduce the kinematic sums (r0,a and r0,ab over
-// the neighbours) with shuffles, every lane then holds the point's frame a1, a2, b,
-// C0^-1 and the resultants N, M. Per neighbour (lane-strided) the FP64 residual
-// contribution is formed and scattered, and a record of the neighbour's factors is
-// staged in shared memory. The pair loop then spreads the n(n+1)/2 blocks over the
-// lanes. Each block is written in the rank-3 form
+// A step runs as two kernels: the residual (one Gauss point per thread, FP64: kinematics,
+// resultants, nodal forces, and the point's state for the tangent) and the tangent, which forms
+// the n(n+1)/2 blocks of every point: per group of points with merged contributions in FP32
+// (face_tangent_merged_kernel), or per (point, neighbour) entry (tangent_entry.cuh: FP64, and
+// FP32 supports too wide to merge). The merged kernel writes each block in the rank-3 form
 //     K_IJ = a1 (x) Y1 + a2 (x) Y2 + b (x) Y3 + geo I,
 // which follows from Bm_I = a1 (x) (dx, 0, dy) + a2 (x) (0, dy, dx) in strain space,
 // Bb_I = beta_I (x) b, Db_J = -(a1 c_J0 + a2 c_J1) (x) b with c_J = C0^-1 grad Phi_J:
@@ -227,6 +226,12 @@ __device__ __forceinline__ void store_contrib(void* cbuf, int64_t q, bool flip, 
 constexpr int kState = 32;
 enum : int { S_A1 = 0, S_A2 = 3, S_B = 6, S_RXX = 9, S_RYY = 12, S_RXY = 15, S_CI = 18, S_N = 22,
              S_M = 25, S_P = 28, S_BV = 30, S_W = 31 };
+// The FP64 tangent's state: a1(3) a2(3) b(3), the dual basis a^1(3) a^2(3), r_k . a^1 and
+// r_k . a^2 for r_k = r0XX, r0YY, 2 r0XY, C0^-1 (00 01 11), N(3) M(3) pXY(2) bv W. The dual
+// basis and its products cost 30 FMA once per point here instead of once per neighbour.
+constexpr int kState64 = 34;
+enum : int { D_A1 = 0, D_A2 = 3, D_B = 6, D_AX = 9, D_AY = 12, D_BX = 15, D_BY = 18, D_CI = 21, D_N = 24,
+             D_M = 27, D_P = 30, D_BV = 32, D_W = 33 };
 
 // TIN: element type of the grad / Hessian Phi arrays the pair phase reads (TK, or FP64
 // read and rounded in the kernel). POS_MAP: map_slot holds the reference's csrMapping
@@ -281,7 +286,28 @@ __device__ __forceinline__ void phase1_point(const FaceArgs& a, int g0, int lane
       const double W = a.weight[g];
       // The state the tangent needs goes out first, so that only the residual's coefficients
       // stay live through the neighbour loop.
-      if (st) {
+      if constexpr (sizeof(TK) == 8) {
+        if (st) {
+          auto put = [&](int f, double v) { st[f * st_stride + st_idx] = v; };
+          double Ax[3], Ay[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            Ax[c] = P.Ci[0] * P.a1[c] + P.Ci[1] * P.a2[c];
+            Ay[c] = P.Ci[2] * P.a1[c] + P.Ci[3] * P.a2[c];
+            put(D_A1 + c, P.a1[c]); put(D_A2 + c, P.a2[c]); put(D_B + c, P.b[c]);
+            put(D_AX + c, Ax[c]); put(D_AY + c, Ay[c]);
+            put(D_N + c, P.N[c]); put(D_M + c, P.M[c]);
+          }
+          put(D_BX, P.rxx[0] * Ax[0] + P.rxx[1] * Ax[1] + P.rxx[2] * Ax[2]);
+          put(D_BX + 1, P.ryy[0] * Ax[0] + P.ryy[1] * Ax[1] + P.ryy[2] * Ax[2]);
+          put(D_BX + 2, 2.0 * (P.rxy[0] * Ax[0] + P.rxy[1] * Ax[1] + P.rxy[2] * Ax[2]));
+          put(D_BY, P.rxx[0] * Ay[0] + P.rxx[1] * Ay[1] + P.rxx[2] * Ay[2]);
+          put(D_BY + 1, P.ryy[0] * Ay[0] + P.ryy[1] * Ay[1] + P.ryy[2] * Ay[2]);
+          put(D_BY + 2, 2.0 * (P.rxy[0] * Ay[0] + P.rxy[1] * Ay[1] + P.rxy[2] * Ay[2]));
+          put(D_CI, P.Ci[0]); put(D_CI + 1, P.Ci[1]); put(D_CI + 2, P.Ci[3]);
+          put(D_P, P.pXY[0]); put(D_P + 1, P.pXY[1]); put(D_BV, P.bv); put(D_W, W);
+        }
+      } else if (st) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           st[(S_A1 + c) * st_stride + st_idx] = static_cast<TK>(P.a1[c]);
@@ -559,26 +585,7 @@ __global__ void __launch_bounds__(256) face_residual_kernel(FaceArgs a, TK* gsta
   }
 }
 
-constexpr int kTanWarps = 4;
-
-template <typename TK, bool DET, bool BZERO>
-__global__ void __launch_bounds__(32 * kTanWarps) face_tangent_kernel(FaceArgs a, const TK* __restrict__ gstate) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nmax = a.nmax;
-  TK* base_w = reinterpret_cast<TK*>(smem_raw) + static_cast<size_t>(w) * (kState * 32 + kRec * nmax);
-  TK* st = base_w;
-  TK* rec = base_w + kState * 32;
-  int* nid = reinterpret_cast<int*>(reinterpret_cast<TK*>(smem_raw) +
-                                    static_cast<size_t>(kTanWarps) * (kState * 32 + kRec * nmax)) + w * nmax;
-  for (int g0 = a.g_begin + (blockIdx.x * kTanWarps + w) * 32; g0 < a.g_end; g0 += gridDim.x * kTanWarps * 32) {
-    const int g = g0 + lane;
-#pragma unroll 4
-    for (int f = 0; f < kState; ++f) st[f * 32 + lane] = g < a.g_end ? gstate[static_cast<int64_t>(f) * a.n_gp + g] : TK(0);
-    __syncwarp();
-    phase2_group<TK, DET, TK, false, BZERO>(a, g0, lane, st, rec, nid);
-  }
-}
+#include "tangent_entry.cuh"
 
 // ---- hinge (FP64) -----------------------------------------------------------------
 
@@ -1440,6 +1447,21 @@ __global__ void fill_sell(int n_gp, const int64_t* __restrict__ ptr, const int32
   }
 }
 
+// The point of every face entry (made once per assembler: it depends on the lists only).
+__global__ void entry_points(int n_gp, const int64_t* __restrict__ ptr, int32_t* __restrict__ ent_point) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n_gp) return;
+  for (int64_t e = ptr[g]; e < ptr[g + 1]; ++e) ent_point[e] = g;
+}
+
+void ensure_entry_points(cgb_assembler* a) {
+  if (a->ent_point.p) return;
+  const cgb_shape* S = a->faces;
+  a->ent_point.alloc(S->nnz);
+  if (S->n_gp) entry_points<<<nb(S->n_gp, 128), 128, 0, a->ctx->stream>>>(S->n_gp, S->nbr_ptr.p, a->ent_point.p);
+  CGB_CUDA(cudaGetLastError());
+}
+
 void ensure_sell(cgb_assembler* a) {
   if (a->sell_ptr.p) return;
   const cgb_shape* S = a->faces;
@@ -1594,9 +1616,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   fa.Fc = a->fcontrib.p;
   fa.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
   fa.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
-  const size_t tk = mixed ? sizeof(float) : sizeof(double);
-  const size_t smem = want_K ? static_cast<size_t>(kFaceWarps) * ((kState * 32 + kRec * fa.nmax) * tk +
-                                                                 fa.nmax * sizeof(int)) : 0;
+  if (want_K && !merged) ensure_entry_points(a);
   if (mixed && want_K) {
     ensure_fp32_shapes(a);
     fa.dpsi_t = a->dpsi32.p;
@@ -1605,16 +1625,16 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     fa.dpsi_t = S->dpsi.p;
     fa.ddpsi_t = S->ddpsi.p;
   }
-  if (smem > 200 * 1024)
+  // The entry point's limit on the neighbours per point (about 165 in FP64, 340 in mixed mode).
+  const size_t tk = mixed ? sizeof(float) : sizeof(double);
+  if (want_K && kFaceWarps * ((kState * 32 + kRec * static_cast<size_t>(fa.nmax)) * tk + fa.nmax * sizeof(int)) > 200 * 1024)
     throw Error(CGB_ERR_CAPACITY, "assemble: " + std::to_string(S->max_n) + " neighbours per Gauss point exceed the shared-memory staging");
   const int sms = sm_count(ctx->device);
-  const unsigned grid = std::max(1u, std::min(nb(S->n_gp, 32 * kFaceWarps), static_cast<unsigned>(sms * 8)));
-  (void)grid;
   // Residual kernel (phase 1) then tangent kernel (phase 2), each at its own occupancy.
-  const size_t state_bytes = static_cast<size_t>(kState) * std::max(S->n_gp, 1) * tk;
+  const size_t state_vals = static_cast<size_t>(mixed ? kState : kState64) * std::max(S->n_gp, 1);
   if (want_K) {
-    if (mixed) a->state32.ensure(state_bytes / sizeof(float));
-    else a->state64.ensure(state_bytes / sizeof(double));
+    if (mixed) a->state32.ensure(state_vals);
+    else a->state64.ensure(state_vals);
   }
   float* st32 = a->state32.p;
   double* st64 = a->state64.p;
@@ -1635,7 +1655,6 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     return static_cast<int>(std::min<int64_t>(b, S->n_gp));
   };
   int nface = 0;
-  const size_t tsm = static_cast<size_t>(kTanWarps) * ((kState * 32 + kRec * fa.nmax) * tk + fa.nmax * sizeof(int));
   // Work counters of the chunks' residual launches.
   a->work_ctr.ensure(kMaxChunks);
   CGB_CUDA(cudaMemsetAsync(a->work_ctr.p, 0, kMaxChunks * sizeof(int), st));
@@ -1669,11 +1688,9 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     CGB_CUDA(cudaEventRecord(a->ev_chunk[c], st));
     CGB_CUDA(cudaStreamWaitEvent(a->side, a->ev_chunk[c], 0));
     prof_begin(ctx, CGB_PHASE_TANGENT, a->side);
-    const unsigned tgrid = std::max(1u, std::min(nb(ncg, 32 * kTanWarps), static_cast<unsigned>(sms * 16)));
-    auto tl = [&](auto kern, auto* stp) {
-      if (tsm > 48 * 1024) CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tsm)));
-      kern<<<tgrid, 32 * kTanWarps, tsm, a->side>>>(fa, stp);
-    };
+    // One thread per entry of the chunk (at most max_n per point; the surplus CTAs leave).
+    const unsigned egrid = std::max(1u, nb(std::min(S->nnz, static_cast<int64_t>(ncg) * fa.nmax), kEntryThreads));
+    auto tl = [&](auto kern, auto* stp) { kern<<<egrid, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p); };
     int ntan = 1;
     if (merged) {
       MergeArgs mg{a->mrg_ent_ptr.p, a->mrg_ent_slot.p, a->mrg_ent_cstart.p, a->mrg_direct.p, a->mrg_code.p,
@@ -1723,11 +1740,11 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
         kern<<<mgrid, kMrgThreads, msm, a->side>>>(fa, st32, mg);
       }
     } else if (mixed) {
-      if (det) { if (bzero) tl(face_tangent_kernel<float, true, true>, st32); else tl(face_tangent_kernel<float, true, false>, st32); }
-      else { if (bzero) tl(face_tangent_kernel<float, false, true>, st32); else tl(face_tangent_kernel<float, false, false>, st32); }
+      if (det) { if (bzero) tl(face_tangent_entry_kernel<float, true, true>, st32); else tl(face_tangent_entry_kernel<float, true, false>, st32); }
+      else { if (bzero) tl(face_tangent_entry_kernel<float, false, true>, st32); else tl(face_tangent_entry_kernel<float, false, false>, st32); }
     } else {
-      if (det) { if (bzero) tl(face_tangent_kernel<double, true, true>, st64); else tl(face_tangent_kernel<double, true, false>, st64); }
-      else { if (bzero) tl(face_tangent_kernel<double, false, true>, st64); else tl(face_tangent_kernel<double, false, false>, st64); }
+      if (det) { if (bzero) tl(face_tangent_entry_kernel<double, true, true>, st64); else tl(face_tangent_entry_kernel<double, true, false>, st64); }
+      else { if (bzero) tl(face_tangent_entry_kernel<double, false, true>, st64); else tl(face_tangent_entry_kernel<double, false, false>, st64); }
     }
     ++nface;
     prof_end(ctx, CGB_PHASE_TANGENT, ntan, a->side);

@@ -217,6 +217,7 @@ struct cgb_assembler {
   cudaEvent_t ev_start = nullptr, ev_done = nullptr, ev_chunk[kMaxChunks] = {nullptr};
   cgb::DevBuf<float> state32;         // per-point state between the residual and tangent kernels
   cgb::DevBuf<double> state64;
+  cgb::DevBuf<int32_t> ent_point;     // the point of every face entry (per-entry tangent)
   cgb::DevBuf<int64_t> sell_ptr;      // sliced-ELL copy for the FP64 phase (groups of 32 points)
   cgb::DevBuf<int32_t> sidx;
   cgb::DevBuf<double> sdpsi, sddpsi;
