@@ -21,9 +21,9 @@
 // Bound: the FP64 pipe (2 FMA per cycle and SM). Taking threads per entry and not a warp per
 // point fills the chip on small plates and needs no shared-memory records (at 113 neighbours
 // they had left one CTA of four warps per SM); 36 FMA per pair replace about 90. Measured on
-// one GB300, whole assembly, before and after: 15 x 15 nodes (1,764 points) 1516 -> 249 us;
-// 61 x 61 nodes with the cubic basis (32,400 points, 113 neighbours) 39.1 -> 18.7 ms;
-// 97 x 97 nodes, 4x4 rule, rho = 3.5h (147,456 points) 32.0 -> 11.8 ms.
+// one GB300, this kernel alone: 15 x 15 nodes (1,764 points) 1,340 -> 86 us; 61 x 61 nodes with
+// the cubic basis (32,400 points, 113 neighbours) 37 -> 13.2 ms; 97 x 97 nodes, 4x4 rule,
+// rho = 3.5h (147,456 points) 31 -> 9.2 ms.
 
 // Per-point quantities of the tangent. Bx, By: k = XX, YY, XY (the last doubled).
 template <typename TK>
@@ -149,22 +149,27 @@ __device__ __forceinline__ void column_record(const Frame<TK>& f, const Material
     }
 }
 
-// The block (row i, column j) from phi_i and T_j, added to K.
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+
+// The block (row i, column j) from phi_i and T_j. Written as chains of FMA: a sum that starts
+// from a zeroed K costs a DADD per value on top (20 % of the FP64 instructions of a pair).
 template <typename TK, bool BZERO>
-__device__ __forceinline__ void add_block(const ColumnRecord<TK, BZERO>& R, const TK* b, TK dx, TK dy, TK dxx, TK dyy,
-                                          TK dxy, TK K[9]) {
+__device__ __forceinline__ void form_block(const ColumnRecord<TK, BZERO>& R, const TK* b, TK dx, TK dy, TK dxx, TK dyy,
+                                           TK dxy, TK K[9]) {
   TK l[3];
   if constexpr (!BZERO) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) l[c] = dxx * R.w[c] + dyy * R.w[3 + c] + dxy * R.w[6 + c];
+    for (int c = 0; c < 3; ++c) l[c] = fma_t(dxy, R.w[6 + c], fma_t(dyy, R.w[3 + c], dxx * R.w[c]));
   }
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    const TK s = dxx * R.v[r] + dyy * R.v[3 + r] + dxy * R.v[6 + r];
+    const TK s = fma_t(dxy, R.v[6 + r], fma_t(dyy, R.v[3 + r], dxx * R.v[r]));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      K[3 * r + c] += dx * R.Tx[3 * r + c] + dy * R.Ty[3 * r + c] + s * b[c];
-      if constexpr (!BZERO) K[3 * r + c] += b[r] * l[c];
+      TK k = fma_t(s, b[c], fma_t(dy, R.Ty[3 * r + c], dx * R.Tx[3 * r + c]));
+      if constexpr (!BZERO) k = fma_t(b[r], l[c], k);
+      K[3 * r + c] = k;
     }
   }
 }
@@ -221,9 +226,7 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
       const int64_t q = m0 + static_cast<int64_t>(lo) * n - (static_cast<int64_t>(lo) * (lo - 1)) / 2 + (hi - lo);
       at = kStride * (DET ? q : static_cast<int64_t>(a.map_slot[q]));
       TK K[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) K[k] = TK(0);
-      add_block<TK, BZERO>(R, b, D1[2 * ei], D1[2 * ei + 1], D2[3 * ei], D2[3 * ei + 1], D2[3 * ei + 2], K);
+      form_block<TK, BZERO>(R, b, D1[2 * ei], D1[2 * ei + 1], D2[3 * ei], D2[3 * ei + 1], D2[3 * ei + 2], K);
       const bool flip = a.idx[ei] > nj;   // the stored block's row is the lower node
 #pragma unroll
       for (int r = 0; r < 3; ++r)
