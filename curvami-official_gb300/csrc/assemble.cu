@@ -32,6 +32,7 @@
 #include <atomic>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
@@ -50,6 +51,7 @@ constexpr int kErrIndex = 8;
 
 struct Material {
   double A[9], B[9], D[9];
+  bool bzero;   // B == 0: its products are left out
   // FP32 copies for the FP32 tangent: a double -> float conversion issues on the FP64 pipe,
   // which the records loop would otherwise pay for 9-27 times per record.
   float Af[9], Bf[9], Df[9];
@@ -60,7 +62,9 @@ struct Material {
 
 inline Material make_material(const double* A, const double* B, const double* D) {
   Material m;
+  m.bzero = true;
   for (int i = 0; i < 9; ++i) {
+    m.bzero = m.bzero && B[i] == 0.0;
     m.A[i] = A[i]; m.B[i] = B[i]; m.D[i] = D[i];
     m.Af[i] = static_cast<float>(A[i]); m.Bf[i] = static_cast<float>(B[i]); m.Df[i] = static_cast<float>(D[i]);
   }
@@ -136,7 +140,7 @@ __device__ __forceinline__ void point_state(const double s[15], const Material& 
   P.Ci[0] = C11 * id; P.Ci[1] = -C01 * id; P.Ci[2] = -C01 * id; P.Ci[3] = C00 * id;
   double n[3] = {P.a1[1] * P.a2[2] - P.a1[2] * P.a2[1], P.a1[2] * P.a2[0] - P.a1[0] * P.a2[2],
                  P.a1[0] * P.a2[1] - P.a1[1] * P.a2[0]};
-  const double inv_area = 1.0 / sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);   // one division, not three
+  const double inv_area = rsqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
 #pragma unroll
   for (int c = 0; c < 3; ++c) P.b[c] = n[c] * inv_area;
   P.e0[0] = 0.5 * (C00 - 1.0);
@@ -148,10 +152,15 @@ __device__ __forceinline__ void point_state(const double s[15], const Material& 
   P.e1el[0] = P.e1[0] + kbar; P.e1el[1] = P.e1[1]; P.e1el[2] = P.e1[2];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    P.N[r] = m.A[3 * r] * P.e0[0] + m.A[3 * r + 1] * P.e0[1] + m.A[3 * r + 2] * P.e0[2] +
-             (m.B[3 * r] * P.e1el[0] + m.B[3 * r + 1] * P.e1el[1] + m.B[3 * r + 2] * P.e1el[2]);
-    P.M[r] = m.B[r] * P.e0[0] + m.B[3 + r] * P.e0[1] + m.B[6 + r] * P.e0[2] +
-             (m.D[3 * r] * P.e1el[0] + m.D[3 * r + 1] * P.e1el[1] + m.D[3 * r + 2] * P.e1el[2]);
+    P.N[r] = m.A[3 * r] * P.e0[0] + m.A[3 * r + 1] * P.e0[1] + m.A[3 * r + 2] * P.e0[2];
+    P.M[r] = m.D[3 * r] * P.e1el[0] + m.D[3 * r + 1] * P.e1el[1] + m.D[3 * r + 2] * P.e1el[2];
+  }
+  if (!m.bzero) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      P.N[r] += m.B[3 * r] * P.e1el[0] + m.B[3 * r + 1] * P.e1el[1] + m.B[3 * r + 2] * P.e1el[2];
+      P.M[r] += m.B[r] * P.e0[0] + m.B[3 + r] * P.e0[1] + m.B[6 + r] * P.e0[2];
+    }
   }
   double vc[3];
 #pragma unroll
@@ -240,23 +249,26 @@ enum : int { D_A1 = 0, D_A2 = 3, D_B = 6, D_AX = 9, D_AY = 12, D_BX = 15, D_BY =
 // single isotropic ply of the reference's app, whose B = Q (z1^2 - z0^2) / 2 is exactly
 // 0). Then P = A Bm = a1 (x) pa + a2 (x) pb and Q = D Bb = b (x) qc, and the J-side
 // record shrinks from 23 to 14 values.
-// Phase 1 for the Gauss point g0 + lane (g0 a multiple of 32): FP64 kinematics,
+// Phase 1 for one Gauss point: FP64 kinematics,
 // resultants and residual (F atomics, or per-entry contributions when DET); when st is
 // not null the point's state goes to st[field * st_stride + st_idx] in TK.
 // CHECK (caller-owned arrays only): a neighbour id outside [0, n_nodes) is flagged in the
 // error word and the neighbour is left out.
-template <typename TK, bool DET, bool CHECK = false>
-__device__ __forceinline__ void phase1_point(const FaceArgs& a, int g0, int lane, TK* st, int64_t st_stride,
+// L lanes share a point (g: this lane's point, sub: its number among them): the neighbours are
+// dealt to them in turn, their sums added by shuffles, and lane 0 of them stores the state.
+template <typename TK, bool DET, bool CHECK = false, int L = 1>
+__device__ __forceinline__ void phase1_point(const FaceArgs& a, int g, int sub, TK* st, int64_t st_stride,
                                              int64_t st_idx) {
   const Material& m = a.mat;
-  const int g = g0 + lane;
-  if (g < a.g_end) {
+  const bool here = g < a.g_end;
+  if (!here) g = a.g_end - 1;   // lanes past the end keep their warp's shuffles whole and write nothing
+  if (here || L > 1) {
       const int64_t p0 = a.ptr[g];
       const int n = static_cast<int>(a.ptr[g + 1] - p0);
       // Entry q of this lane's point: CSR p0 + q, or sliced-ELL sb + 32 q (coalesced
       // across the warp: the 32 lanes read 32 consecutive entries per q).
       const bool sell = a.sell_ptr != nullptr;
-      const int64_t sb = sell ? a.sell_ptr[g0 >> 5] + lane : p0;
+      const int64_t sb = sell ? a.sell_ptr[g >> 5] + (g & 31) : p0;
       const int64_t stride = sell ? 32 : 1;
       const int32_t* Ix = sell ? a.sidx : a.idx;
       const double* Dp = sell ? a.sdpsi : a.dpsi;
@@ -265,7 +277,7 @@ __device__ __forceinline__ void phase1_point(const FaceArgs& a, int g0, int lane
 #pragma unroll
       for (int k = 0; k < 15; ++k) s[k] = 0.0;
 #pragma unroll 4
-      for (int q = 0; q < n; ++q) {
+      for (int q = sub; q < n; q += L) {
         const int64_t e = sb + q * stride;
         const int64_t j = Ix[e];
         if (CHECK && (j < 0 || j >= a.n_nodes)) {
@@ -281,9 +293,14 @@ __device__ __forceinline__ void phase1_point(const FaceArgs& a, int g0, int lane
         s[9] += u0 * dyy; s[10] += u1 * dyy; s[11] += u2 * dyy;
         s[12] += u0 * dxy; s[13] += u1 * dxy; s[14] += u2 * dxy;
       }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 15; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
       PointState P;
       point_state(s, m, P, a.gp_xy ? natcurv_kappa(a.nc, a.gp_xy[2 * static_cast<int64_t>(g)]) : 0.0);
       const double W = a.weight[g];
+      if (L > 1 && (!here || sub != 0)) st = nullptr;
       // The state the tangent needs goes out first, so that only the residual's coefficients
       // stay live through the neighbour loop.
       if constexpr (sizeof(TK) == 8) {
@@ -341,9 +358,9 @@ __device__ __forceinline__ void phase1_point(const FaceArgs& a, int g0, int lane
         Hyy[c] = -W * P.b[c] * P.M[1];
         Hxy[c] = -2.0 * W * P.b[c] * P.M[2];
       }
-      if (n > 0) {
+      if (here) {
 #pragma unroll 2
-        for (int q = 0; q < n; ++q) {
+        for (int q = sub; q < n; q += L) {
           const int64_t es = sb + q * stride;
           const int64_t e = p0 + q;
           const double2 d = reinterpret_cast<const double2*>(Dp)[es];
@@ -556,7 +573,7 @@ __global__ void __launch_bounds__(32 * kFaceWarps, sizeof(TK) == 4 ? 5 : 3) face
     // Phase 1: one Gauss point per lane, FP64. Every lane does distinct work, so no FP64
     // issue slot is spent on a redundant or masked copy (on GB300 an FP64 warp
     // instruction costs the same with 1 or 32 lanes).
-    phase1_point<TK, DET, POS_MAP>(a, g0, lane, WANT_K ? st : static_cast<TK*>(nullptr), 32, lane);
+    phase1_point<TK, DET, POS_MAP>(a, g0 + lane, 0, WANT_K ? st : static_cast<TK*>(nullptr), 32, lane);
     if (!WANT_K) continue;
     __syncwarp();
     phase2_group<TK, DET, TIN, POS_MAP, BZERO>(a, g0, lane, st, rec, nid);
@@ -567,22 +584,36 @@ __global__ void __launch_bounds__(32 * kFaceWarps, sizeof(TK) == 4 ? 5 : 3) face
 // (phase 1, one Gauss point per thread, FP64 bound) writes the per-point state to
 // global memory ([field][n_gp]); the tangent kernel (phase 2) stages 32 points' states
 // in shared memory and runs the pair loop.
-// Work is handed out 32 points at a time from a counter (zeroed per assembly), so the
+// Work is handed out a warp's points at a time from a counter (zeroed per assembly), so the
 // warps of a launch finish together whatever the grid: when the tangent kernel of the
 // previous chunk holds most of each SM, only one residual CTA fits beside it, and a
 // fixed split into CTAs would leave a partial last wave.
-template <typename TK, bool DET, bool STORE>
+// LANES per point: each SM quarter issues one FP64 warp instruction in 64 cycles, and a point
+// takes about 30 per neighbour and 200 by itself, so a launch that does not fill the quarters
+// is as long as one warp's work; splitting the points' neighbours over lanes shortens it
+// (residual_lanes).
+template <typename TK, bool DET, bool STORE, int LANES>
 __global__ void __launch_bounds__(256) face_residual_kernel(FaceArgs a, TK* gstate, int* __restrict__ work) {
+  constexpr int PTS = 32 / LANES;
   const int lane = threadIdx.x & 31;
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(work, 1);
     unit = __shfl_sync(0xffffffffu, unit, 0);
-    const int64_t g0 = a.g_begin + 32 * static_cast<int64_t>(unit);
+    const int64_t g0 = a.g_begin + PTS * static_cast<int64_t>(unit);
     if (g0 >= a.g_end) break;
-    phase1_point<TK, DET>(a, static_cast<int>(g0), lane, STORE ? gstate : static_cast<TK*>(nullptr), a.n_gp,
-                          g0 + lane);
+    const int g = static_cast<int>(g0) + lane / LANES;
+    phase1_point<TK, DET, false, LANES>(a, g, lane % LANES, STORE ? gstate : static_cast<TK*>(nullptr), a.n_gp, g);
   }
+}
+
+// Lanes per point of a residual launch over n points: as many as still leave every warp an SM
+// quarter of its own. At 28 neighbours one warp's work is 1070 FP64 instructions with one lane
+// per point, 665 with two, 470 with four and 380 with eight; once two warps share a quarter the
+// fewer lanes win again (the point's own part is repeated by each).
+inline int residual_lanes(int n, int sms) {
+  const int64_t lanes = 32LL * 4 * sms;
+  return n * 8LL <= lanes ? 8 : n * 4LL <= lanes ? 4 : n * 2LL <= lanes ? 2 : 1;
 }
 
 #include "tangent_entry.cuh"
@@ -602,6 +633,7 @@ struct HingeArgs {
   const double* x;
   int exact;
   int want_K;
+  int parts;         // warps per crease point
   int tk_float;      // accumulator type
   double* F; void* Kacc;              // atomic mode
   double* Fc; void* Kc;               // deterministic mode
@@ -615,69 +647,53 @@ __device__ __forceinline__ void cross(const double* a, const double* b, double* 
 }
 __device__ __forceinline__ double dot(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
-// Constraints::foldAngleAndGrad (plate/Constraints.h:54-119).
+// Constraints::foldAngleAndGrad (plate/Constraints.h:54-119): theta = atan2(-s, c) with
+// c = bL . bR, s = (bL x bR) . t. The gradient is taken backwards: w_L, w_R, w_t are the
+// cofactors of dbL, dbR, dt in dtheta = -(c ds - s dc) / (c^2 + s^2); through b = n / |n| and
+// n = a1 x a2 a cofactor w of db becomes m = (w - (w . b) b) / |n| and then a2 x m on a1 and
+// m x a1 on a2. About 150 FP64 operations, a sixth of forming the 3x6 derivative matrices
+// (one warp's latency, which is what a hinge launch of a few crease points is made of).
 __device__ double fold_angle(const double* F, double tx, double ty, double* grad) {
   const double *a1L = F, *a2L = F + 3, *a1R = F + 6, *a2R = F + 9;
   double nL[3], nR[3];
   cross(a1L, a2L, nL); cross(a1R, a2R, nR);
-  const double normL = sqrt(dot(nL, nL)), normR = sqrt(dot(nR, nR));
+  const double iL = rsqrt(dot(nL, nL)), iR = rsqrt(dot(nR, nR));
   double bL[3], bR[3], aT[3], t[3];
-  for (int c = 0; c < 3; ++c) { bL[c] = nL[c] / normL; bR[c] = nR[c] / normR; aT[c] = a1L[c] * tx + a2L[c] * ty; }
-  const double naT = sqrt(dot(aT, aT));
-  for (int c = 0; c < 3; ++c) t[c] = aT[c] / naT;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { bL[c] = nL[c] * iL; bR[c] = nR[c] * iR; aT[c] = a1L[c] * tx + a2L[c] * ty; }
+  const double iT = rsqrt(dot(aT, aT));
+#pragma unroll
+  for (int c = 0; c < 3; ++c) t[c] = aT[c] * iT;
   const double cth = dot(bL, bR);
   double bxb[3];
   cross(bL, bR, bxb);
   const double sth = dot(bxb, t);
-  const double theta = atan2(-sth, cth);
   if (grad) {
-    double dbL[3][6], dbR[3][6];
-    for (int side = 0; side < 2; ++side) {
-      const double* a1 = side ? a1R : a1L;
-      const double* a2 = side ? a2R : a2L;
-      const double* b = side ? bR : bL;
-      const double nn = side ? normR : normL;
-      double (*out)[6] = side ? dbR : dbL;
-      double dn[3][6];
-      for (int i = 0; i < 3; ++i) {
-        double e[3] = {0, 0, 0};
-        e[i] = 1.0;
-        double c1[3], c2[3];
-        cross(e, a2, c1); cross(a1, e, c2);
-        for (int r = 0; r < 3; ++r) { dn[r][i] = c1[r]; dn[r][i + 3] = c2[r]; }
-      }
-      for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 6; ++c) {
-          double acc = 0.0;
-          for (int k = 0; k < 3; ++k) acc += (((r == k) ? 1.0 : 0.0) - b[r] * b[k]) / nn * dn[k][c];
-          out[r][c] = acc;
-        }
-    }
-    double dt[3][6];
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 6; ++c) {
-        double acc = 0.0;
-        for (int k = 0; k < 3; ++k) {
-          const double daT = (c < 3) ? ((c == k) ? tx : 0.0) : ((c - 3 == k) ? ty : 0.0);
-          acc += (((r == k) ? 1.0 : 0.0) - t[r] * t[k]) / naT * daT;
-        }
-        dt[r][c] = acc;
-      }
     double bRxt[3], txbL[3];
     cross(bR, t, bRxt); cross(t, bL, txbL);
     const double denom = cth * cth + sth * sth;
     const double inv = (denom > 1e-14) ? 1.0 / denom : 0.0;
-    for (int c = 0; c < 6; ++c) {
-      const double dcL = bR[0] * dbL[0][c] + bR[1] * dbL[1][c] + bR[2] * dbL[2][c];
-      const double dcR = bL[0] * dbR[0][c] + bL[1] * dbR[1][c] + bL[2] * dbR[2][c];
-      const double dsL = (bRxt[0] * dbL[0][c] + bRxt[1] * dbL[1][c] + bRxt[2] * dbL[2][c]) +
-                         (bxb[0] * dt[0][c] + bxb[1] * dt[1][c] + bxb[2] * dt[2][c]);
-      const double dsR = txbL[0] * dbR[0][c] + txbL[1] * dbR[1][c] + txbL[2] * dbR[2][c];
-      grad[c] = -(cth * dsL - sth * dcL) * inv;
-      grad[6 + c] = -(cth * dsR - sth * dcR) * inv;
+    const double ci = -cth * inv, si = sth * inv;
+    double mL[3], mR[3], mT[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      mL[c] = ci * bRxt[c] + si * bR[c];
+      mR[c] = ci * txbL[c] + si * bL[c];
+      mT[c] = ci * bxb[c];
     }
+    const double pL = dot(mL, bL), pR = dot(mR, bR), pT = dot(mT, t);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      mL[c] = (mL[c] - pL * bL[c]) * iL;
+      mR[c] = (mR[c] - pR * bR[c]) * iR;
+      mT[c] = (mT[c] - pT * t[c]) * iT;
+    }
+    cross(a2L, mL, grad); cross(mL, a1L, grad + 3);
+    cross(a2R, mR, grad + 6); cross(mR, a1R, grad + 9);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) { grad[c] += tx * mT[c]; grad[3 + c] += ty * mT[c]; }
   }
-  return theta;
+  return atan2(-sth, cth);
 }
 
 constexpr int kHingeWarps = 2;
@@ -685,7 +701,9 @@ constexpr int kHingeWarps = 2;
 // One warp per crease Gauss point (Constraints.h:349-435). The left and right
 // entries are merged per node: with G_u = sum of the dof gradients of node u over both
 // sides, the reference's triplets (all k, m with node_k <= node_m) sum to
-// W Kt G_P (x) G_Q (+ W moment B_P^T H B_Q) on block (P, Q) of the merged list.
+// W Kt G_P (x) G_Q (+ W moment B_P^T H B_Q) on block (P, Q) of the merged list. a.parts warps
+// share a point's pairs (each repeats the angle): a crease has few points, and with one warp
+// each a merged list of 160 nodes is 400 rounds of about 200 FP64 instructions.
 __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -694,8 +712,10 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
   double* G = base;
   double* Bs = base + 3 * a.max_u;
   double* H = base + 7 * a.max_u;
-  for (int g = blockIdx.x * kHingeWarps + w; g < a.n_gp; g += gridDim.x * kHingeWarps) {
-    if (a.active && a.active[g] == 0) continue;  // Constraints.h:350
+  const int gw = blockIdx.x * kHingeWarps + w;
+  const int g = gw / a.parts, part = gw - g * a.parts;
+  if (g < a.n_gp) {
+    if (a.active && a.active[g] == 0) return;  // Constraints.h:350
     double sL[6] = {0, 0, 0, 0, 0, 0}, sR[6] = {0, 0, 0, 0, 0, 0};
     for (int64_t e = a.lptr[g] + lane; e < a.lptr[g + 1]; e += 32) {
       const int64_t j = a.lidx[e];
@@ -768,7 +788,7 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
       Bs[4 * u + 2] += dX; Bs[4 * u + 3] += dY;
     }
     __syncwarp();
-    for (int u = lane; u < mu; u += 32) {
+    for (int u = part == 0 ? lane : mu; u < mu; u += 32) {
       const int node = a.u_node[u0 + u];
       for (int d = 0; d < 3; ++d) {
         const double f = G[3 * u + d] * Wm;
@@ -779,9 +799,9 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
     if (a.want_K) {
       const int64_t np = static_cast<int64_t>(mu) * (mu + 1) / 2;
       const int64_t q0 = a.pair_ptr[g];
-      int P = 0, off = lane;
+      int P = 0, off = 32 * part + lane;
       while (P < mu && off >= mu - P) { off -= mu - P; ++P; }
-      for (int64_t p = lane; p < np; p += 32) {
+      for (int64_t p = 32 * part + lane; p < np; p += 32 * a.parts) {
         const int Q = P + off;
         double v[9];
         for (int dk = 0; dk < 3; ++dk)
@@ -809,11 +829,10 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
           if (a.tk_float) { float t[9]; for (int k = 0; k < 9; ++k) t[k] = static_cast<float>(v[k]); scatter_atomic<float>(a.Kacc, slot, false, t); }
           else scatter_atomic<double>(a.Kacc, slot, false, v);
         }
-        off += 32;
+        off += 32 * a.parts;
         while (P < mu && off >= mu - P) { off -= mu - P; ++P; }
       }
     }
-    __syncwarp();
   }
 }
 
@@ -1641,7 +1660,8 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   // The residual kernel of chunk c + 1 (FP64 pipe) runs beside the tangent kernel of
   // chunk c (FP32 pipe, L2 atomics) on a second stream; chunks are multiples of 32 points.
   ensure_side_stream(a);
-  const int n_chunks = a->tuning.n_chunks > 0 ? a->tuning.n_chunks : (S->n_gp >= 65536 ? kChunks : 1);
+  // Only the FP32 tangent has another pipe to overlap with; without one, chunks are just tails.
+  const int n_chunks = a->tuning.n_chunks > 0 ? a->tuning.n_chunks : (mixed && want_K && S->n_gp >= 65536 ? kChunks : 1);
   const int rthreads = a->tuning.residual_threads > 0 ? a->tuning.residual_threads : 256;
   const int chunk = ((S->n_gp + n_chunks - 1) / n_chunks + 31) / 32 * 32;
   // Chunk c covers [cb(c), cb(c + 1)). The first chunk is a quarter of the others: the
@@ -1658,29 +1678,73 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   // Work counters of the chunks' residual launches.
   a->work_ctr.ensure(kMaxChunks);
   CGB_CUDA(cudaMemsetAsync(a->work_ctr.p, 0, kMaxChunks * sizeof(int), st));
-  if (want_K) {
+  // Hinge: it reads x, its shape sets and the fold state and adds into F and the block
+  // accumulator with atomics (or into its own contribution slots in deterministic mode), none
+  // of which the face kernels read, so it runs beside them: on the side stream when the residual
+  // is all there is (a hinge launch is mostly the latency of one warp), else on the context
+  // stream beside the last tangent chunks.
+  auto launch_hinge = [&](cudaStream_t hst) {
+    prof_begin(ctx, CGB_PHASE_HINGE, hst);
+    int nl = 0;
+    int64_t kb = k_face_units, fb = a->hinge_f_base;
+    for (auto& f : a->folds) {
+      if (f.n_gp == 0) continue;
+      HingeArgs h = hinge_args(a, f, d_x, flags);
+      h.F = d_F;
+      h.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
+      if (det) {
+        h.Fc = a->fcontrib.p;
+        h.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
+        h.f_base = fb; h.k_base = kb;
+      }
+      // Warps per point: two per SM quarter over the launch, each with at least 4 rounds of pairs.
+      const int64_t rounds = static_cast<int64_t>(h.max_u) * (h.max_u + 1) / 2 / 128;
+      h.parts = want_K ? static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(rounds, 8 * sms / f.n_gp))) : 1;
+      const size_t hs = static_cast<size_t>(kHingeWarps) * (7 * h.max_u + 144 + 16) * sizeof(double);
+      if (hs > 48 * 1024) CGB_CUDA(cudaFuncSetAttribute(hinge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(hs)));
+      hinge_kernel<<<nb(static_cast<int64_t>(f.n_gp) * h.parts, kHingeWarps), 32 * kHingeWarps, hs, hst>>>(h);
+      CGB_CUDA(cudaGetLastError());
+      ++nl;
+      kb += f.n_pairs;
+      fb += f.n_u;
+    }
+    prof_end(ctx, CGB_PHASE_HINGE, nl, hst);
+  };
+  const bool hinge_first = hinge && !want_K;
+  const bool use_side = want_K || hinge_first;
+  if (use_side) {
     CGB_CUDA(cudaEventRecord(a->ev_start, st));
     CGB_CUDA(cudaStreamWaitEvent(a->side, a->ev_start, 0));
   }
+  if (hinge_first) launch_hinge(a->side);
   for (int c = 0; c < n_chunks && S->n_gp > 0; ++c) {
     int* work = a->work_ctr.p + c;
     fa.g_begin = cb(c);
     fa.g_end = cb(c + 1);
     if (fa.g_begin >= fa.g_end) break;
     const int ncg = fa.g_end - fa.g_begin;
-    const unsigned rgrid = std::max(1u, std::min(nb(ncg, rthreads), static_cast<unsigned>(sms * 16 * (256 / rthreads))));
     prof_begin(ctx, CGB_PHASE_FACE);
-    if (mixed) {
-      if (det) { if (want_K) face_residual_kernel<float, true, true><<<rgrid, rthreads, 0, st>>>(fa, st32, work);
-                 else face_residual_kernel<float, true, false><<<rgrid, rthreads, 0, st>>>(fa, st32, work); }
-      else { if (want_K) face_residual_kernel<float, false, true><<<rgrid, rthreads, 0, st>>>(fa, st32, work);
-             else face_residual_kernel<float, false, false><<<rgrid, rthreads, 0, st>>>(fa, st32, work); }
-    } else {
-      if (det) { if (want_K) face_residual_kernel<double, true, true><<<rgrid, rthreads, 0, st>>>(fa, st64, work);
-                 else face_residual_kernel<double, true, false><<<rgrid, rthreads, 0, st>>>(fa, st64, work); }
-      else { if (want_K) face_residual_kernel<double, false, true><<<rgrid, rthreads, 0, st>>>(fa, st64, work);
-             else face_residual_kernel<double, false, false><<<rgrid, rthreads, 0, st>>>(fa, st64, work); }
-    }
+    auto rl = [&](auto lanes, auto* stp) {
+      constexpr int L = decltype(lanes)::value;
+      using TK = std::remove_pointer_t<decltype(stp)>;
+      auto kern = det ? (want_K ? face_residual_kernel<TK, true, true, L> : face_residual_kernel<TK, true, false, L>)
+                      : (want_K ? face_residual_kernel<TK, false, true, L> : face_residual_kernel<TK, false, false, L>);
+      // Few points: small blocks, so that every SM gets a share (25,600 points are only 100
+      // blocks of 256 threads).
+      const int rt = L > 1 ? 32 : (a->tuning.residual_threads == 0 && ncg < 256 * 4 * sms ? 64 : rthreads);
+      const int64_t pts = rt / L;
+      kern<<<std::max(1u, std::min(nb(ncg, static_cast<int>(pts)), static_cast<unsigned>(sms * 16 * (256 / rt)))), rt, 0, st>>>(fa, stp, work);
+    };
+    auto rk = [&](auto* stp) {
+      switch (residual_lanes(ncg, sms)) {
+        case 8: rl(std::integral_constant<int, 8>{}, stp); break;
+        case 4: rl(std::integral_constant<int, 4>{}, stp); break;
+        case 2: rl(std::integral_constant<int, 2>{}, stp); break;
+        default: rl(std::integral_constant<int, 1>{}, stp); break;
+      }
+    };
+    if (mixed) rk(st32);
+    else rk(st64);
     ++nface;
     prof_end(ctx, CGB_PHASE_FACE, 1);
     CGB_CUDA(cudaGetLastError());
@@ -1752,34 +1816,8 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   }
   (void)nface;
 
-  // Hinge, on the context stream beside the last tangent chunks: it reads x, its shape sets
-  // and the fold state and adds into F and the block accumulator with atomics (or into its
-  // own contribution slots in deterministic mode), none of which the tangent reads.
-  if (hinge) {
-    prof_begin(ctx, CGB_PHASE_HINGE);
-    int nl = 0;
-    int64_t kb = k_face_units, fb = a->hinge_f_base;
-    for (auto& f : a->folds) {
-      if (f.n_gp == 0) continue;
-      HingeArgs h = hinge_args(a, f, d_x, flags);
-      h.F = d_F;
-      h.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
-      if (det) {
-        h.Fc = a->fcontrib.p;
-        h.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
-        h.f_base = fb; h.k_base = kb;
-      }
-      const size_t hs = static_cast<size_t>(kHingeWarps) * (7 * h.max_u + 144 + 16) * sizeof(double);
-      if (hs > 48 * 1024) CGB_CUDA(cudaFuncSetAttribute(hinge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(hs)));
-      hinge_kernel<<<nb(f.n_gp, kHingeWarps), 32 * kHingeWarps, hs, st>>>(h);
-      CGB_CUDA(cudaGetLastError());
-      ++nl;
-      kb += f.n_pairs;
-      fb += f.n_u;
-    }
-    prof_end(ctx, CGB_PHASE_HINGE, nl);
-  }
-  if (want_K) {
+  if (hinge && !hinge_first) launch_hinge(st);
+  if (use_side) {
     CGB_CUDA(cudaEventRecord(a->ev_done, a->side));
     CGB_CUDA(cudaStreamWaitEvent(st, a->ev_done, 0));
   }
