@@ -610,8 +610,10 @@ __global__ void __launch_bounds__(256) face_residual_kernel(FaceArgs a, TK* gsta
 // Lanes per point of a residual launch over n points: as many as still leave every warp an SM
 // quarter of its own. At 28 neighbours one warp's work is 1070 FP64 instructions with one lane
 // per point, 665 with two, 470 with four and 380 with eight; once two warps share a quarter the
-// fewer lanes win again (the point's own part is repeated by each).
-inline int residual_lanes(int n, int sms) {
+// fewer lanes win again (the point's own part is repeated by each). One in deterministic mode: a
+// point's sums then do not depend on how many points the launch has.
+inline int residual_lanes(int n, int sms, bool det) {
+  if (det) return 1;
   const int64_t lanes = 32LL * 4 * sms;
   return n * 8LL <= lanes ? 8 : n * 4LL <= lanes ? 4 : n * 2LL <= lanes ? 2 : 1;
 }
@@ -1736,7 +1738,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       kern<<<std::max(1u, std::min(nb(ncg, static_cast<int>(pts)), static_cast<unsigned>(sms * 16 * (256 / rt)))), rt, 0, st>>>(fa, stp, work);
     };
     auto rk = [&](auto* stp) {
-      switch (residual_lanes(ncg, sms)) {
+      switch (residual_lanes(ncg, sms, det)) {
         case 8: rl(std::integral_constant<int, 8>{}, stp); break;
         case 4: rl(std::integral_constant<int, 4>{}, stp); break;
         case 2: rl(std::integral_constant<int, 2>{}, stp); break;
