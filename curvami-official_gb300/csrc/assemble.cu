@@ -9,9 +9,10 @@
 //
 // A step runs as two kernels: the residual (one Gauss point per thread, FP64: kinematics,
 // resultants, nodal forces, and the point's state for the tangent) and the tangent, which forms
-// the n(n+1)/2 blocks of every point: per group of points with merged contributions in FP32
-// (face_tangent_merged_kernel), or per (point, neighbour) entry (tangent_entry.cuh: FP64, and
-// FP32 supports too wide to merge). The merged kernel writes each block in the rank-3 form
+// the n(n+1)/2 blocks of every point: per cell of 16 points with the contributions to
+// a block summed first (tangent_tile.cuh, FP32), or per (point, neighbour) entry (tangent_entry.cuh:
+// FP64, and FP32 supports too wide for a cell). They form each block of
+//
 //     K_IJ = a1 (x) Y1 + a2 (x) Y2 + b (x) Y3 + geo I,
 // which follows from Bm_I = a1 (x) (dx, 0, dy) + a2 (x) (0, dy, dx) in strain space,
 // Bb_I = beta_I (x) b, Db_J = -(a1 c_J0 + a2 c_J1) (x) b with c_J = C0^-1 grad Phi_J:
@@ -618,6 +619,8 @@ inline int residual_lanes(int n, int sms, bool det) {
   return n * 8LL <= lanes ? 8 : n * 4LL <= lanes ? 4 : n * 2LL <= lanes ? 2 : 1;
 }
 
+constexpr int kMG = 16;   // points per cell of the FP32 tangent (the set-up kernel uses the same)
+
 #include "tangent_entry.cuh"
 
 // ---- hinge (FP64) -----------------------------------------------------------------
@@ -1008,31 +1011,6 @@ __global__ void hinge_energy_kernel(HingeArgs a, double* out) {
   atomicAdd(out, a.weight[g] * (0.5 * a.Kt * (d * d)));
 }
 
-// ---- FP32 tangent with merged contributions ------------------------------------------
-// One CTA per group of kMG consecutive Gauss points. The CTA builds the group's
-// per-neighbour records (AoS, 16-byte rows) and point frames in shared memory, then each
-// thread takes distinct blocks ("entries") of the group, sums every contribution to its
-// block in registers (in a fixed order: point, then local pair) and scatters it once with
-// three 16-byte vector atomics. On GB300 a scattered 48-byte block costs ~14 ns of L2
-// atomic throughput per SM-slot (~70 G blocks/s for the chip); merging the ~7.5
-// contributions per block of a 4x4 quadrature cell divides that traffic accordingly.
-constexpr int kMG = 16;          // points per group (the setup kernel uses the same)
-constexpr int kMrgThreads = 256;
-
-struct MergeArgs {
-  const int64_t* ent_ptr;
-  const int32_t* ent_slot;
-  const int32_t* ent_cstart;  // (count << 16) | first contribution
-  const int8_t* direct;
-  const uint16_t* code;       // point (4) | i (6) | j (6)
-  int* err;                   // set to kErrStage when a staging copy never completes
-  uint32_t extra_tx;          // 0; the failure-detection test expects bytes that never arrive
-  // The merged kernel's groups: glist[0 .. gcount) when glist is set (the groups the tensor
-  // tangent does not take), else every group of [g_begin, g_end).
-  const int32_t* glist;
-  int gcount;
-};
-
 // ---- bulk-copy (TMA) staging --------------------------------------------------------
 // One elected thread copies a group's contiguous ranges of grad / Hessian Phi and ids
 // into shared memory with cp.async.bulk, completing on an mbarrier the CTA waits on.
@@ -1089,296 +1067,7 @@ __device__ __forceinline__ StageWin stage_window(int64_t q0, int64_t q1, int es)
   return w;
 }
 
-// The block of the local pair (i, j) of one point from the frame (fr[0..1]: a1 | b.v,
-// a2), the I-side record (ri[0..1]) and the J-side record (rj), as in phase2_group, added
-// to v (the three rank-1 terms of each entry as one FMA chain onto it). The unit normal
-// b = a1 x a2 / |a1 x a2| and g_I = a1 c0_I + a2 c1_I are rebuilt from the frame here
-// rather than read: the kernel is bound by shared-memory wavefronts, not FMAs.
-template <bool BZERO>
-__device__ __forceinline__ void merged_pair(const float4* fr, const float4* ri, const float4* rj, float v[9]) {
-  const float4 f0 = fr[0], f1 = fr[1];
-  const float a1t[3] = {f0.x, f0.y, f0.z}, a2t[3] = {f1.x, f1.y, f1.z};
-  float bt[3] = {a1t[1] * a2t[2] - a1t[2] * a2t[1], a1t[2] * a2t[0] - a1t[0] * a2t[2],
-                 a1t[0] * a2t[1] - a1t[1] * a2t[0]};
-  const float rn = rsqrtf(bt[0] * bt[0] + bt[1] * bt[1] + bt[2] * bt[2]);
-  bt[0] *= rn; bt[1] *= rn; bt[2] *= rn;
-  const float bv = f0.w;
-  const float4 i0 = ri[0], i1 = ri[1];
-  const float dxi = i0.x, dyi = i0.y, be0 = i0.z, be1 = i0.w, be2 = i1.x, Tui = i1.y;
-  const float gi[3] = {a1t[0] * i1.z + a2t[0] * i1.w, a1t[1] * i1.z + a2t[1] * i1.w, a1t[2] * i1.z + a2t[2] * i1.w};
-  float Y1[3], Y2[3], Y3[3], geo;
-  if constexpr (BZERO) {
-    const float4 j0 = rj[0], j1 = rj[1], j2 = rj[2], j3 = rj[3];
-    const float pa0 = j0.x, pa1 = j0.y, pa2 = j0.z, pb0 = j0.w, pb1 = j1.x, pb2 = j1.y;
-    const float qc0 = j1.z, qc1 = j1.w, qc2 = j2.x, cj0 = j2.y, cj1 = j2.z, nj0 = j2.w, nj1 = j3.x, TuWj = j3.y;
-    const float s1 = Tui * cj0, s2 = Tui * cj1;
-    geo = dxi * nj0 + dyi * nj1;
-    const float z11 = dxi * pa0 + dyi * pa2, z12 = dxi * pb0 + dyi * pb2;
-    const float z21 = dyi * pa1 + dxi * pa2, z22 = dyi * pb1 + dxi * pb2;
-    const float z33 = be0 * qc0 + be1 * qc1 + be2 * qc2 + bv * (dxi * cj0 + dyi * cj1);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      Y1[c] = a1t[c] * z11 + a2t[c] * z12 - s1 * bt[c];
-      Y2[c] = a1t[c] * z21 + a2t[c] * z22 - s2 * bt[c];
-      Y3[c] = bt[c] * z33 - TuWj * gi[c];
-    }
-  } else {
-    float J[24];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const float4 t = rj[q];
-      J[4 * q] = t.x; J[4 * q + 1] = t.y; J[4 * q + 2] = t.z; J[4 * q + 3] = t.w;
-    }
-    const float cj0 = J[18], cj1 = J[19], nj0 = J[20], nj1 = J[21], TuWj = J[22];
-    const float s1 = Tui * cj0, s2 = Tui * cj1;
-    const float t3 = bv * (dxi * cj0 + dyi * cj1);
-    geo = dxi * nj0 + dyi * nj1;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      Y1[c] = dxi * J[c] + dyi * J[6 + c] - s1 * bt[c];
-      Y2[c] = dyi * J[3 + c] + dxi * J[6 + c] - s2 * bt[c];
-      Y3[c] = be0 * J[9 + c] + be1 * J[12 + c] + be2 * J[15 + c] + t3 * bt[c] - TuWj * gi[c];
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      v[3 * r + c] = fmaf(bt[r], Y3[c], fmaf(a2t[r], Y2[c], fmaf(a1t[r], Y1[c], v[3 * r + c])));
-    v[4 * r] += geo;
-  }
-}
-
-// DET: every entry's sum is stored (9 floats at unit e0 + e of a.Kc) for the ordered
-// per-block reduction instead of being added atomically; it needs no direct group.
-template <bool BZERO, bool DET>
-__global__ void __launch_bounds__(kMrgThreads, 4) face_tangent_merged_kernel(FaceArgs a, const float* __restrict__ gstate,
-                                                                            MergeArgs mg) {
-  // One record per (point, neighbour): the I side (2 float4) then the J side (4 float4, 6
-  // when B != 0), with an odd stride RW in float4. A warp reads the records of 32
-  // different (point, neighbour) pairs at once, and with an even stride of 2^m float4
-  // those addresses fall into only 8 / 2^m of the 8 four-bank groups (a stride of 4
-  // serialises a float4 load into ~16 wavefronts instead of ~4).
-  constexpr int RW = BZERO ? 7 : 9;  // float4 rows of a record (6 or 8 used)
-  constexpr int FW = 3;              // float4 rows of a point frame (2 used)
-  extern __shared__ __align__(16) float msm[];
-  __shared__ uint64_t stage_bar;
-  __shared__ int64_t sptr[kMG + 1];
-  const int nmax = a.nmax;
-  const int E = kMG * nmax;                                 // most entries of a group
-  float* st = msm;                                          // [kState][kMG]
-  float4* fr = reinterpret_cast<float4*>(st + kState * kMG); // [kMG][FW]
-  float4* rec = fr + FW * kMG;                              // [kMG * nmax][RW]
-  // Staging windows (16-byte aligned): grad Phi, Hessian Phi of the group's entries.
-  unsigned char* s_d = reinterpret_cast<unsigned char*>(rec + RW * E);
-  unsigned char* s_dd = s_d + 8 * E + 32;
-  const unsigned char* dpsi_b = static_cast<const unsigned char*>(a.dpsi_t);
-  const unsigned char* ddpsi_b = static_cast<const unsigned char*>(a.ddpsi_t);
-  const Material& m = a.mat;
-  // Groups of this launch: [g_begin, g_end) are multiples of kMG apart (chunk bounds are
-  // multiples of 32), so a group never straddles two launches.
-  const int G0 = a.g_begin / kMG;
-  const int nG = mg.glist ? mg.gcount : (a.g_end + kMG - 1) / kMG - G0;
-  auto group = [&](int gi) { return mg.glist ? mg.glist[gi] : G0 + gi; };
-  // Thread 0 starts the copies of group G's ranges; every thread later waits on the phase.
-  auto stage = [&](int G) {
-    const int g0 = G * kMG, g1 = min(g0 + kMG, a.g_end);
-    const int64_t q0 = a.ptr[g0], q1 = a.ptr[g1];
-    const StageWin wd = stage_window(q0, q1, 8), wdd = stage_window(q0, q1, 12);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect(&stage_bar, wd.len + wdd.len + mg.extra_tx);
-    if (wd.len) bulk_load(s_d, dpsi_b + wd.lo, wd.len, &stage_bar);
-    if (wdd.len) bulk_load(s_dd, ddpsi_b + wdd.lo, wdd.len, &stage_bar);
-    // The group's pair codes and entry tables are read once per step from DRAM, one code per
-    // contribution: bring them into L2 now, a group ahead of their use.
-    l2_prefetch(mg.code, 2 * a.map_ptr[g0], 2 * a.map_ptr[g1]);
-    const int64_t e0 = mg.ent_ptr[G], e1 = mg.ent_ptr[G + 1];
-    l2_prefetch(mg.ent_cstart, 4 * e0, 4 * e1);
-    l2_prefetch(mg.ent_slot, 4 * e0, 4 * e1);
-  };
-  if (threadIdx.x == 0) {
-    mbar_init(&stage_bar);
-    if (static_cast<int>(blockIdx.x) < nG) stage(group(blockIdx.x));
-  }
-  __syncthreads();
-  uint32_t phase = 0;
-  for (int gi = blockIdx.x; gi < nG; gi += gridDim.x) {
-    const int G = group(gi);
-    const int g0 = G * kMG;
-    const int kn = min(kMG, a.g_end - g0);
-    for (int t = threadIdx.x; t < kState * kMG; t += blockDim.x) {
-      const int f = t / kMG, k = t - f * kMG;
-      st[t] = k < kn ? gstate[static_cast<int64_t>(f) * a.n_gp + g0 + k] : 0.0f;
-    }
-    if (threadIdx.x <= kn) sptr[threadIdx.x] = a.ptr[g0 + threadIdx.x];
-    // Every thread waits on the copies of this group, then the CTA agrees on the outcome
-    // so that no thread leaves while another waits at a barrier.
-    const bool ok = mbar_wait(&stage_bar, phase);
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) {
-        atomicOr(mg.err, kErrStage);
-        mbar_wait(&stage_bar, phase);   // let copies still in flight land before leaving
-      }
-      return;
-    }
-    phase ^= 1u;
-    const int64_t q0 = sptr[0];
-    const float* sdp = reinterpret_cast<const float*>(s_d + (q0 * 8 - ((q0 * 8) & ~static_cast<int64_t>(15))));
-    const float* sddp = reinterpret_cast<const float*>(s_dd + (q0 * 12 - ((q0 * 12) & ~static_cast<int64_t>(15))));
-    if (threadIdx.x < kn) {
-      const int k = threadIdx.x;
-      fr[FW * k] = make_float4(st[(S_A1) * kMG + k], st[(S_A1 + 1) * kMG + k], st[(S_A1 + 2) * kMG + k], st[S_BV * kMG + k]);
-      fr[FW * k + 1] = make_float4(st[(S_A2) * kMG + k], st[(S_A2 + 1) * kMG + k], st[(S_A2 + 2) * kMG + k], 0.0f);
-    }
-    // Records of every (point, neighbour) of the group (the same formulas as phase2_group),
-    // from the staged copies.
-    for (int t = threadIdx.x; t < kMG * nmax; t += blockDim.x) {
-      const int k = t / nmax, i = t - k * nmax;
-      if (k >= kn) continue;
-      const int64_t p0 = sptr[k];
-      if (i >= sptr[k + 1] - p0) continue;
-      const int64_t e = p0 + i - q0;   // entry within the group's staged range
-      const float a1t[3] = {st[S_A1 * kMG + k], st[(S_A1 + 1) * kMG + k], st[(S_A1 + 2) * kMG + k]};
-      const float a2t[3] = {st[S_A2 * kMG + k], st[(S_A2 + 1) * kMG + k], st[(S_A2 + 2) * kMG + k]};
-      const float bt[3] = {st[S_B * kMG + k], st[(S_B + 1) * kMG + k], st[(S_B + 2) * kMG + k]};
-      float rxx[3], ryy[3], rxy[3], Nt[3], Mt[3], Ci[4];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        rxx[c] = st[(S_RXX + c) * kMG + k]; ryy[c] = st[(S_RYY + c) * kMG + k]; rxy[c] = st[(S_RXY + c) * kMG + k];
-        Nt[c] = st[(S_N + c) * kMG + k]; Mt[c] = st[(S_M + c) * kMG + k];
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) Ci[c] = st[(S_CI + c) * kMG + k];
-      const float pX = st[S_P * kMG + k], pY = st[(S_P + 1) * kMG + k], Wt = st[S_W * kMG + k];
-      const float dx = sdp[2 * e], dy = sdp[2 * e + 1];
-      const float dxx = sddp[3 * e], dyy = sddp[3 * e + 1], dxy = sddp[3 * e + 2];
-      const float c0 = Ci[0] * dx + Ci[1] * dy, c1 = Ci[2] * dx + Ci[3] * dy;
-      float gI[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) gI[r] = a1t[r] * c0 + a2t[r] * c1;
-      const float b0 = -dxx + (rxx[0] * gI[0] + rxx[1] * gI[1] + rxx[2] * gI[2]);
-      const float b1 = -dyy + (ryy[0] * gI[0] + ryy[1] * gI[1] + ryy[2] * gI[2]);
-      const float b2 = 2.0f * (-dxy + (rxy[0] * gI[0] + rxy[1] * gI[1] + rxy[2] * gI[2]));
-      const float Tu = dx * pX + dy * pY - (dxx * Mt[0] + 2.0f * dxy * Mt[2] + dyy * Mt[1]);
-      float4* RI = rec + RW * t;
-      RI[0] = make_float4(dx, dy, b0, b1);
-      RI[1] = make_float4(b2, Tu, c0, c1);
-      float4* RJ = rec + RW * t + 2;
-      if constexpr (BZERO) {
-        float pa[3], pb[3], qc[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          pa[r] = (m.Ai<float>(3 * r) * dx + m.Ai<float>(3 * r + 2) * dy) * Wt;
-          pb[r] = (m.Ai<float>(3 * r + 1) * dy + m.Ai<float>(3 * r + 2) * dx) * Wt;
-          qc[r] = (m.Di<float>(3 * r) * b0 + m.Di<float>(3 * r + 1) * b1 +
-                   m.Di<float>(3 * r + 2) * b2) * Wt;
-        }
-        RJ[0] = make_float4(pa[0], pa[1], pa[2], pb[0]);
-        RJ[1] = make_float4(pb[1], pb[2], qc[0], qc[1]);
-        RJ[2] = make_float4(qc[2], c0 * Wt, c1 * Wt, (Nt[0] * dx + Nt[2] * dy) * Wt);
-        RJ[3] = make_float4((Nt[2] * dx + Nt[1] * dy) * Wt, Tu * Wt, 0.0f, 0.0f);
-      } else {
-        float J[24];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          const float Ar0 = m.Ai<float>(3 * r), Ar1 = m.Ai<float>(3 * r + 1), Ar2 = m.Ai<float>(3 * r + 2);
-          const float Br0 = m.Bi<float>(3 * r), Br1 = m.Bi<float>(3 * r + 1), Br2 = m.Bi<float>(3 * r + 2);
-          const float Dr0 = m.Di<float>(3 * r), Dr1 = m.Di<float>(3 * r + 1), Dr2 = m.Di<float>(3 * r + 2);
-          const float pa = (Ar0 * dx + Ar2 * dy) * Wt, pb = (Ar1 * dy + Ar2 * dx) * Wt, pc = (Br0 * b0 + Br1 * b1 + Br2 * b2) * Wt;
-          const float qa = (Br0 * dx + Br2 * dy) * Wt, qb = (Br1 * dy + Br2 * dx) * Wt, qc = (Dr0 * b0 + Dr1 * b1 + Dr2 * b2) * Wt;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            J[3 * r + c] = a1t[c] * pa + a2t[c] * pb + bt[c] * pc;
-            J[9 + 3 * r + c] = a1t[c] * qa + a2t[c] * qb + bt[c] * qc;
-          }
-        }
-        J[18] = c0 * Wt; J[19] = c1 * Wt;
-        J[20] = (Nt[0] * dx + Nt[2] * dy) * Wt; J[21] = (Nt[2] * dx + Nt[1] * dy) * Wt;
-        J[22] = Tu * Wt; J[23] = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) RJ[q] = make_float4(J[4 * q], J[4 * q + 1], J[4 * q + 2], J[4 * q + 3]);
-      }
-    }
-    __syncthreads();
-    // The staging buffers are free again: start the next group's copies, which land while
-    // this group's entries are summed.
-    if (threadIdx.x == 0 && gi + static_cast<int>(gridDim.x) < nG) stage(group(gi + gridDim.x));
-    float4* acc4 = static_cast<float4*>(a.Kacc);
-    const int64_t cbase = a.map_ptr[g0];
-    if (!DET && mg.direct[G]) {
-      // Too many pairs for the setup's shared-memory sort: scatter pair by pair.
-      for (int k = 0; k < kn; ++k) {
-        const int64_t p0k = a.ptr[g0 + k];
-        const int n = static_cast<int>(a.ptr[g0 + k + 1] - p0k);
-        const int np = n * (n + 1) / 2;
-        const int64_t m0 = a.map_ptr[g0 + k];
-        for (int p = threadIdx.x; p < np; p += blockDim.x) {
-          int i = 0, off = p;
-          while (off >= n - i) { off -= n - i; ++i; }
-          const int j = i + off;
-          float v[9] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-          merged_pair<BZERO>(fr + FW * k, rec + RW * (k * nmax + i), rec + RW * (k * nmax + j) + 2, v);
-          scatter_atomic<float>(a.Kacc, a.map_slot[m0 + p], a.idx[p0k + i] > a.idx[p0k + j], v);
-        }
-      }
-    } else {
-      const int64_t e0 = mg.ent_ptr[G];
-      const int ne = static_cast<int>(mg.ent_ptr[G + 1] - e0);
-      // Entries are count-descending; thread t takes one entry per round of blockDim.x, in
-      // ascending order on even rounds and descending on odd ones, so that every warp's
-      // rounds add up to about the same work before the group's closing barrier. Each
-      // thread's entries are software-pipelined: the next entry's (count, first) word and its
-      // first code are fetched while this entry's contributions are summed, so that no entry
-      // starts on two dependent global loads.
-      const int step = static_cast<int>(blockDim.x);
-      const int t = threadIdx.x;
-      auto entry_of = [&](int r) {
-        const int base = r * step, rem = min(step, ne - base);
-        return t < rem ? base + ((r & 1) ? rem - 1 - t : t) : ne;
-      };
-      const uint16_t* gcodes = mg.code + cbase;
-      int r = 0;
-      int e = entry_of(0);
-      int cs = e < ne ? mg.ent_cstart[e0 + e] : 0;
-      unsigned first = (e < ne && (cs >> 16) > 0) ? gcodes[cs & 0xffff] : 0u;
-      for (; e < ne; e = entry_of(++r)) {
-        const int cnt = cs >> 16, c0 = cs & 0xffff;
-        const int en = entry_of(r + 1);
-        const int cs_n = en < ne ? mg.ent_cstart[e0 + en] : 0;
-        const int32_t slot = DET ? 0 : mg.ent_slot[e0 + e];
-        float acc[9];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) acc[q] = 0.0f;
-        // Codes are in the block's stored orientation (row node first); the next code (after
-        // the last one, the next entry's first) is fetched while the current contribution is
-        // computed.
-        const uint16_t* codes = gcodes + c0;
-        unsigned next = first;
-        for (int c = 0; c < cnt; ++c) {
-          const unsigned code = next;
-          if (c + 1 < cnt) next = codes[c + 1];
-          else next = (cs_n >> 16) > 0 ? gcodes[cs_n & 0xffff] : 0u;
-          const int k = code >> 12, i = (code >> 6) & 63, j = code & 63;
-          merged_pair<BZERO>(fr + FW * k, rec + RW * (k * nmax + i), rec + RW * (k * nmax + j) + 2, acc);
-        }
-        first = cnt > 0 ? next : ((cs_n >> 16) > 0 ? gcodes[cs_n & 0xffff] : 0u);
-        cs = cs_n;
-        if constexpr (DET) {
-          float* d = static_cast<float*>(a.Kc) + 9 * (e0 + e);
-#pragma unroll
-          for (int q = 0; q < 9; ++q) d[q] = acc[q];
-        } else {
-          float4* d = acc4 + 3 * static_cast<int64_t>(slot);
-          atomicAdd(d, make_float4(acc[0], acc[1], acc[2], acc[3]));
-          atomicAdd(d + 1, make_float4(acc[4], acc[5], acc[6], acc[7]));
-          atomicAdd(d + 2, make_float4(acc[8], 0.0f, 0.0f, 0.0f));
-        }
-      }
-    }
-    __syncthreads();
-  }
-}
-
+#include "tangent_tile.cuh"
 #include "tangent_tc.cuh"
 
 inline unsigned nb(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
@@ -1542,15 +1231,7 @@ void ensure_side_stream(cgb_assembler* a) {
 
 }  // namespace
 
-// Dynamic shared memory of the merged FP32 tangent for neighbour lists of up to nmax
-// entries: per-point state and frames of the 16 points, one record per (point, neighbour)
-// (RW float4, odd), and the staging windows of grad / Hessian Phi (20 bytes per entry + 64).
-constexpr size_t kMergedSmemMax = 220 * 1024;
-size_t merged_smem_bytes(int nmax, bool bzero) {
-  const size_t RW = bzero ? 7 : 9, FW = 3;
-  const size_t E = static_cast<size_t>(kMG) * nmax;
-  return (static_cast<size_t>(kState) * kMG + 4 * FW * kMG + 4 * RW * E) * sizeof(float) + (20 * E + 64);
-}
+constexpr size_t kTangentSmemMax = 220 * 1024;
 
 void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d_F, int flags) {
   cgb_context* ctx = a->ctx;
@@ -1566,27 +1247,24 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   if (det) deterministic_prepare(a);
   bool bzero = true;
   for (double v : a->B) bzero = bzero && (v == 0.0);
-  // The FP32 tangent merges each group's contributions per block; in deterministic mode the
-  // merged sums become the K units, unless a group is too large to merge. The merged kernel
-  // stages a group's records in shared memory: supports too wide for that (the reference
-  // app's cubic basis at rho = 6h has over 100 neighbours) take the per-point FP32 tangent.
-  const size_t msm = merged_smem_bytes(std::max(S->max_n, 1), bzero);
+  // The FP32 tangent sums each cell's contributions per block; in deterministic mode those sums
+  // become the K units, unless a cell is direct. Supports too wide for a cell's lists (the
+  // reference app's cubic basis at rho = 6h has over 100 neighbours) take the per-entry tangent.
   bool merged = false;
-  if (mixed && want_K && msm <= kMergedSmemMax) {
-    merge_prepare(a);
-    merged = !det || a->mrg_n_direct == 0;
+  if (mixed && want_K && S->max_n <= kTileMaxList) {
+    tile_prepare(a);
+    merged = (!det || a->direct_h.empty()) && a->n_items > 0;
   }
-  // The tensor-core tangent takes the merged path's cells whose node union fits one
-  // 128-row tile (its entries are the merged entries, so the deterministic lists are the
-  // same).
+  const size_t msm = merged ? tile_smem_bytes(a->cell_max_e, a->cell_max_u, bzero) : 0;
+  // The tensor-core tangent takes the cells whose node union fits one 128-row tile (its blocks
+  // are the items' slots too, so the deterministic lists are the same).
   const size_t tcsm = tc_smem_bytes(std::max(S->max_n, 1), bzero);
-  const bool use_tc = merged && a->tuning.tangent_kind == CGB_TANGENT_TENSOR && tcsm <= kMergedSmemMax;
-  if (use_tc) tc_prepare(a);
+  const bool use_tc = merged && a->tuning.tangent_kind == CGB_TANGENT_TENSOR && tcsm <= kTangentSmemMax;
   if (det && want_K) {
     if (merged) deterministic_entry_lists(a);
     else deterministic_pair_lists(a);
   }
-  const int64_t k_face_units = merged ? a->mrg_n_ent : a->n_pairs;
+  const int64_t k_face_units = merged ? 4 * a->n_items : a->n_pairs;
 
   const int64_t ndof = 3 * static_cast<int64_t>(a->n_nodes);
   // Accumulators.
@@ -1637,7 +1315,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   fa.Fc = a->fcontrib.p;
   fa.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
   fa.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
-  if (want_K && !merged) ensure_entry_points(a);
+  if (want_K && (!merged || !a->direct_h.empty())) ensure_entry_points(a);
   if (mixed && want_K) {
     ensure_fp32_shapes(a);
     fa.dpsi_t = a->dpsi32.p;
@@ -1754,25 +1432,36 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     CGB_CUDA(cudaEventRecord(a->ev_chunk[c], st));
     CGB_CUDA(cudaStreamWaitEvent(a->side, a->ev_chunk[c], 0));
     prof_begin(ctx, CGB_PHASE_TANGENT, a->side);
-    // One thread per entry of the chunk (at most max_n per point; the surplus CTAs leave).
-    const unsigned egrid = std::max(1u, nb(std::min(S->nnz, static_cast<int64_t>(ncg) * fa.nmax), kEntryThreads));
-    auto tl = [&](auto kern, auto* stp) { kern<<<egrid, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p); };
+    // One thread per entry of the chunk (at most max_n per point; the surplus CTAs leave), or of
+    // the chunk's direct cells.
+    auto tl = [&](auto kern, auto* stp, const int32_t* glist = nullptr, int gcount = 0) {
+      const int per_cell = glist ? static_cast<int>(nb(static_cast<int64_t>(kMG) * fa.nmax, kEntryThreads)) : 0;
+      const unsigned egrid = glist ? static_cast<unsigned>(gcount) * per_cell
+                                   : std::max(1u, nb(std::min(S->nnz, static_cast<int64_t>(ncg) * fa.nmax), kEntryThreads));
+      kern<<<egrid, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p, glist, per_cell);
+    };
     int ntan = 1;
     if (merged) {
-      MergeArgs mg{a->mrg_ent_ptr.p, a->mrg_ent_slot.p, a->mrg_ent_cstart.p, a->mrg_direct.p, a->mrg_code.p,
-                   ctx->dev_err.p, a->test_stage_extra_tx, nullptr, 0};
-      auto kern = det ? (bzero ? face_tangent_merged_kernel<true, true> : face_tangent_merged_kernel<false, true>)
-                      : (bzero ? face_tangent_merged_kernel<true, false> : face_tangent_merged_kernel<false, false>);
+      TileArgs tg{a->item_ptr.p, a->item_code.p, reinterpret_cast<const int4*>(a->item_slot.p), a->nbr_u.p, a->cell_U.p,
+                  a->cell_max_e, a->cell_max_u, ctx->dev_err.p, a->test_stage_extra_tx, nullptr, 0};
+      auto kern = det ? (bzero ? face_tangent_tile_kernel<true, true> : face_tangent_tile_kernel<false, true>)
+                      : (bzero ? face_tangent_tile_kernel<true, false> : face_tangent_tile_kernel<false, false>);
       CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(msm)));
       int per_sm = 0;
-      CGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMrgThreads, msm));
+      CGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileThreads, msm));
       const int Gb = fa.g_begin / kMG, Ge = (fa.g_end + kMG - 1) / kMG;
       const int groups = Ge - Gb;
       if (a->tuning.tangent_ctas_per_sm > 0) per_sm = std::min(per_sm, a->tuning.tangent_ctas_per_sm);
+      per_sm = std::max(per_sm, 1);
+      // The part of a sorted cell list that lies in this chunk.
+      auto part = [&](const std::vector<int32_t>& v) {
+        const auto lo = std::lower_bound(v.begin(), v.end(), Gb), hi = std::lower_bound(lo, v.end(), Ge);
+        return std::make_pair(static_cast<int>(lo - v.begin()), static_cast<int>(hi - lo));
+      };
       if (use_tc) {
         // Cells whose node union fits one 128-row tile: one tensor-core product each; the
-        // others (sorted group list, this chunk's part) on the CUDA cores.
-        TcArgs tca{a->tc_nbr_u.p, a->tc_cell_U.p, a->tc_ent_uv.p};
+        // others on the CUDA cores.
+        TcArgs tca{a->nbr_u.p, a->cell_U.p};
         auto tk = det ? (bzero ? face_tangent_tc_kernel<true, true> : face_tangent_tc_kernel<false, true>)
                       : (bzero ? face_tangent_tc_kernel<true, false> : face_tangent_tc_kernel<false, false>);
         CGB_CUDA(cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tcsm)));
@@ -1788,22 +1477,22 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
         if (a->tuning.tangent_ctas_per_sm > 0) tc_per_sm = std::min(tc_per_sm, a->tuning.tangent_ctas_per_sm);
         a->tc_last_per_sm = tc_per_sm;
         const unsigned tgrid2 = static_cast<unsigned>(std::max(1, std::min(groups, tc_per_sm * sms)));
-        tk<<<tgrid2, kTcThreads, tcsm, a->side>>>(fa, st32, mg, tca);
-        const auto& fb = a->tc_fallback_h;
-        const int lo = static_cast<int>(std::lower_bound(fb.begin(), fb.end(), Gb) - fb.begin());
-        const int hi = static_cast<int>(std::lower_bound(fb.begin(), fb.end(), Ge) - fb.begin());
-        ntan = 1;
-        if (hi > lo) {
-          MergeArgs mf = mg;
-          mf.glist = a->tc_fallback.p + lo;
-          mf.gcount = hi - lo;
-          const unsigned fgrid = static_cast<unsigned>(std::max(1, std::min(hi - lo, std::max(per_sm, 1) * sms)));
-          kern<<<fgrid, kMrgThreads, msm, a->side>>>(fa, st32, mf);
-          ntan = 2;
+        tk<<<tgrid2, kTcThreads, tcsm, a->side>>>(fa, st32, tg, tca);
+        const auto [at, count] = part(a->tc_rest_h);
+        if (count > 0) {
+          tg.glist = a->tc_rest.p + at;
+          tg.gcount = count;
+          kern<<<static_cast<unsigned>(std::min(count, per_sm * sms)), kTileThreads, msm, a->side>>>(fa, st32, tg);
+          ++ntan;
         }
       } else {
-        const unsigned mgrid = static_cast<unsigned>(std::max(1, std::min(groups, std::max(per_sm, 1) * sms)));
-        kern<<<mgrid, kMrgThreads, msm, a->side>>>(fa, st32, mg);
+        kern<<<static_cast<unsigned>(std::max(1, std::min(groups, per_sm * sms))), kTileThreads, msm, a->side>>>(fa, st32, tg);
+      }
+      const auto [at, count] = part(a->direct_h);
+      if (count > 0) {
+        if (bzero) tl(face_tangent_entry_kernel<float, false, true>, st32, a->direct.p + at, count);
+        else tl(face_tangent_entry_kernel<float, false, false>, st32, a->direct.p + at, count);
+        ++ntan;
       }
     } else if (mixed) {
       if (det) { if (bzero) tl(face_tangent_entry_kernel<float, true, true>, st32); else tl(face_tangent_entry_kernel<float, true, false>, st32); }

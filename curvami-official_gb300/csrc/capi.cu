@@ -538,11 +538,11 @@ int cgb_assembler_stats(cgb_assembler* a, int64_t out[4]) {
   return guarded(a->ctx, [&] {
     need(out != nullptr, "cgb_assembler_stats: out is NULL");
     bind_device(a->ctx);
-    cgb::merge_prepare(a);
+    cgb::tile_prepare(a);
     out[0] = a->n_pairs;
     out[1] = a->n_blocks;
-    out[2] = a->mrg_n_ent;
-    out[3] = a->mrg_n_direct;
+    out[2] = a->n_entries;
+    out[3] = static_cast<int64_t>(a->direct_h.size());
   });
 }
 
@@ -551,9 +551,9 @@ int cgb_assembler_tensor_stats(cgb_assembler* a, int64_t out[4]) {
   return guarded(a->ctx, [&] {
     need(out != nullptr, "cgb_assembler_tensor_stats: out is NULL");
     bind_device(a->ctx);
-    cgb::tc_prepare(a);
+    cgb::tile_prepare(a);
     out[0] = a->tc_n_groups;
-    out[1] = static_cast<int64_t>(a->tc_fallback_h.size());
+    out[1] = static_cast<int64_t>(a->tc_rest_h.size() + a->direct_h.size());
     out[2] = a->tc_point_cols;
     out[3] = a->tc_last_per_sm;
   });

@@ -185,33 +185,30 @@ struct cgb_assembler {
   cgb::DevBuf<double> x;            // 3 n_nodes
   cgb::DevBuf<float> dpsi32, ddpsi32; // FP32 copies of the face shape derivatives (mixed mode)
   uint64_t faces_version = 0;       // faces->version the copies (FP32, sliced-ELL) were made from
-  // Merged contributions of the FP32 tangent: per group of 16 consecutive Gauss points the
-  // distinct blocks ("entries", count-descending) and every pair's code in entry order.
-  bool mrg_ready = false;
-  cgb::DevBuf<int64_t> mrg_ent_ptr;   // n_groups + 1
-  cgb::DevBuf<int32_t> mrg_ent_slot;  // block slot of each entry
-  cgb::DevBuf<int32_t> mrg_ent_cstart;// (count << 16) | first contribution within its group
-  cgb::DevBuf<int8_t> mrg_direct;     // 1: group too large, scatter directly
-  cgb::DevBuf<uint16_t> mrg_code;     // per pair: point | i | j, grouped by entry
-  // Tensor-core tangent: per face entry the index of its node in its group's sorted node
-  // union, per group the union's size, per merged entry the union indices of its block's
-  // row and column nodes, and the groups the tensor path does not take (union above 42
-  // nodes, or too large to merge) on the device and on the host.
-  bool tc_ready = false;
-  cgb::DevBuf<uint8_t> tc_nbr_u;
-  cgb::DevBuf<int16_t> tc_cell_U;
-  cgb::DevBuf<uint16_t> tc_ent_uv;
-  cgb::DevBuf<int32_t> tc_fallback;
-  std::vector<int32_t> tc_fallback_h;
-  int64_t tc_n_groups = 0;            // groups on the tensor path
+  // Tables of the FP32 tangent (tile_prepare): per face entry the index of its node in its
+  // cell's sorted node union (a cell: 16 consecutive Gauss points), per cell the union's size,
+  // and the cell's items, each a node J and four nodes I <= J: the mask of the points they
+  // share | tile << 16 | J << 24, and the four block slots (-1: none). Cells with too many pairs
+  // or nodes are "direct" (the per-entry tangent); tc_rest: the others that the tensor-core
+  // tangent does not take (union above 42 nodes).
+  bool tile_ready = false;
+  cgb::DevBuf<uint8_t> nbr_u;
+  cgb::DevBuf<int16_t> cell_U;
+  cgb::DevBuf<int64_t> item_ptr;      // n_cells + 1
+  cgb::DevBuf<uint32_t> item_code;
+  cgb::DevBuf<int32_t> item_slot;     // 4 per item
+  cgb::DevBuf<int32_t> direct, tc_rest;
+  std::vector<int32_t> direct_h, tc_rest_h;
+  int64_t n_items = 0;
+  int64_t n_entries = 0;              // blocks over all cells (slots that are not -1)
+  int cell_max_e = 0, cell_max_u = 0; // most entries and nodes of a cell that is not direct
+  int64_t tc_n_groups = 0;            // cells on the tensor path
   int64_t tc_point_cols = 0;          // sum over them of points x MMA columns (N)
   int tc_last_per_sm = 0;             // CTAs per SM of the last tensor-core tangent launch
   cgb_tuning tuning{};                // launch shape (0 = library default)
   cgb::DevBuf<int> work_ctr;          // per-chunk work counters of the residual kernel
   uint32_t test_stage_extra_tx = 0;   // failure-detection test only: bytes the staging never gets
   int n_graphs = 0;                   // live cgb_graph objects on this assembler
-  int64_t mrg_n_ent = 0;              // entries over all groups
-  int mrg_n_direct = 0;               // groups scattered pair by pair
   // Second stream of the chunked face launch (tangent of chunk c beside residual of c+1).
   cudaStream_t side = nullptr;
   cudaEvent_t ev_start = nullptr, ev_done = nullptr, ev_chunk[kMaxChunks] = {nullptr};
@@ -222,11 +219,11 @@ struct cgb_assembler {
   cgb::DevBuf<int32_t> sidx;
   cgb::DevBuf<double> sdpsi, sddpsi;
   // Deterministic scatter: contributions ("units") and per-block / per-node ordered lists.
-  // K units are either every pair (FP64, or groups the merge cannot take) or, for the FP32
-  // tangent, every merged entry (one fixed-order sum per group and block); hinge pairs follow.
+  // K units are either every pair (FP64, or with direct cells) or, for the FP32 tangent, the
+  // slots of the cells' items (one fixed-order sum per cell and block); hinge pairs follow.
   bool det_ready = false;             // F lists
   bool det_pairs_ready = false;       // K lists over pairs
-  bool det_entries_ready = false;     // K lists over merged entries
+  bool det_entries_ready = false;     // K lists over the items' slots
   cgb::DevBuf<int64_t> blk_list_ptr;  // n_blocks + 1 (pair units)
   cgb::DevBuf<int64_t> blk_list;      // pair unit ids, ascending
   cgb::DevBuf<int64_t> ent_list_ptr;  // n_blocks + 1 (entry units)
@@ -265,14 +262,15 @@ void pattern_build(cgb_assembler* a);
 void deterministic_prepare(cgb_assembler* a);
 void shape_concat(cgb_context* ctx, const cgb_shape* const* sets, const int32_t* node_offset, int n_sets,
                   cgb_shape* out);
-// Per-block lists of K units: pairs (units [0, n_pairs) then hinge pairs) or merged entries
-// (units [0, mrg_n_ent) then hinge pairs; needs merge_prepare and no direct group).
+// Per-block lists of K units: pairs (units [0, n_pairs) then hinge pairs) or the slots of the
+// cells' items (units [0, 4 n_items) then hinge pairs; needs tile_prepare and no direct cell).
 void deterministic_pair_lists(cgb_assembler* a);
 void deterministic_entry_lists(cgb_assembler* a);
-void merge_prepare(cgb_assembler* a);
-// The tensor-core tangent's tables (needs merge_prepare; made once per assembler).
+// The tables of the FP32 tangent, made once per assembler.
 constexpr int kTcMaxUnion = 42;
-void tc_prepare(cgb_assembler* a);
+constexpr int kTileMaxU = 128;
+constexpr int kTileMaxList = 110;  // lists above this take the per-entry tangent throughout
+void tile_prepare(cgb_assembler* a);
 // assemble.cu
 void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d_F, int flags);
 // Re-derive the assembler's copies of the face shape derivatives after a rebuild of the

@@ -150,15 +150,15 @@ __global__ void slot_map_kernel(int n_gp, const int64_t* __restrict__ ptr, const
   }
 }
 
-// CSR fill of the deterministic lists: one thread per contribution id.
+// CSR fill of the deterministic lists: one thread per contribution id (a negative key: no unit).
 __global__ void count_slots(int64_t n, const int32_t* __restrict__ key, int64_t* __restrict__ cnt) {
   const int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (q < n) atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[key[q]]), 1ULL);
+  if (q < n && key[q] >= 0) atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[key[q]]), 1ULL);
 }
 __global__ void fill_slots(int64_t n, int64_t base, const int32_t* __restrict__ key, int64_t* __restrict__ cursor,
                            int64_t* __restrict__ list) {
   const int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (q < n) {
+  if (q < n && key[q] >= 0) {
     const int64_t at = atomicAdd(reinterpret_cast<unsigned long long*>(&cursor[key[q]]), 1ULL);
     list[at] = base + q;
   }
@@ -176,127 +176,151 @@ __global__ void sort_lists(int64_t n, const int64_t* __restrict__ lptr, int64_t*
   }
 }
 
-// ---- merged contributions for the FP32 tangent ---------------------------------------
-// A group is kMergeGroup consecutive face Gauss points (one quadrature cell with a 4x4 rule).
-// Its pairs are sorted by (block slot, point, i, j); each distinct slot is an entry whose
-// contributions are summed in registers before one scatter. Entries are ordered by
-// contribution count, descending (stable), so the threads of a warp get similar loops.
-// Contribution code: point k (4 bits) | local i (6 bits) | local j (6 bits).
+// ---- tables of the FP32 tangent ---------------------------------------------------------
+// A cell is kMergeGroup consecutive face Gauss points (one quadrature cell with a 4x4 rule). Its
+// node union, ascending, numbers the cell's nodes u; a block (I, J), I <= J, of the cell is then in
+// its stored orientation (row: the lower node). The tangent's work item is a node J and a tile of
+// four consecutive nodes I <= J, with the mask of the points that have J and at least one of them
+// as neighbours: one CTA per cell finds the union, every entry's index in it, and the items, their
+// block slots (-1 where no point has both nodes) and their order: most points first, so the lanes
+// of a warp have loops of about one length, then by J, so that they share J's records.
+// A cell with more than kMergePairs pairs, a list above 64 or with a node twice, or a union above
+// kTileMaxU is left to the per-entry tangent ("direct").
 constexpr int kMergeGroup = 16;
-constexpr int kMergeItems = 16384;  // sortable pairs per group (8-byte keys, 128 KB)
+constexpr int kMergePairs = 16384;
+constexpr int kCellEntries = 64 * kMergeGroup;
+constexpr int kCellItems = kTileMaxU * (kTileMaxU / 4 + 1) / 2 + kTileMaxU;  // above sum_J (J / 4 + 1)
+constexpr int kCellThreads = 128;
 
-__global__ void __launch_bounds__(256) merge_groups_kernel(int n_gp, const int64_t* __restrict__ ptr,
-                                                          const int32_t* __restrict__ idx,
-                                                          const int64_t* __restrict__ map_ptr,
-                                                          const int32_t* __restrict__ map_slot, int phase,
-                                                          int32_t* __restrict__ ent_count,
-                                                          const int64_t* __restrict__ ent_ptr,
-                                                          int32_t* __restrict__ ent_slot,
-                                                          int32_t* __restrict__ ent_cstart,
-                                                          uint16_t* __restrict__ con_code) {
-  extern __shared__ unsigned long long mkeys[];
-  __shared__ int hist[kMergeGroup + 2];
-  __shared__ int n_ent;
-  const int G = blockIdx.x;
+__global__ void __launch_bounds__(kCellThreads) tile_cells_kernel(
+    int n_gp, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const int64_t* __restrict__ map_ptr,
+    const int64_t* __restrict__ col_ptr, const int32_t* __restrict__ col_nodes, int phase, uint8_t* __restrict__ nbr_u,
+    int16_t* __restrict__ cell_U, int32_t* __restrict__ n_items, const int64_t* __restrict__ item_ptr,
+    uint32_t* __restrict__ item_code, int32_t* __restrict__ item_slot, unsigned long long* __restrict__ n_entries) {
+  __shared__ int ids[kCellEntries];
+  __shared__ unsigned mask[kTileMaxU];
+  __shared__ uint8_t weight[kCellItems];   // points of every (J, tile), J-major
+  __shared__ uint16_t order[kCellItems];
+  __shared__ int s_n, s_bad;
+  const int G = blockIdx.x, t = threadIdx.x;
   const int g0 = G * kMergeGroup, g1 = min(n_gp, g0 + kMergeGroup);
-  const int64_t q0 = map_ptr[g0], q1 = map_ptr[g1];
+  const int64_t q0 = ptr[g0], q1 = ptr[g1];
   const int items = static_cast<int>(q1 - q0);
-  bool ok = items <= kMergeItems;
-  for (int k = 0; k < g1 - g0; ++k) ok = ok && (ptr[g0 + k + 1] - ptr[g0 + k] <= 64);
-  if (!ok) {  // the group scatters directly (count -1)
-    if (phase == 0 && threadIdx.x == 0) ent_count[G] = -1;
-    return;
-  }
-  // Keys: slot (high 32 bits) | k i j (low 16 bits); pairs walked point by point. The
-  // local pair is written row node first (i and j swapped when node(i) > node(j)), so the
-  // tangent evaluates the block in its stored orientation, K_{min,max}, and needs no
-  // transpose (the pair blocks are symmetric: K_ji = K_ij^T).
-  for (int k = 0; k < g1 - g0; ++k) {
-    const int64_t p0 = ptr[g0 + k];
-    const int n = static_cast<int>(ptr[g0 + k + 1] - p0);
-    const int64_t m0 = map_ptr[g0 + k] - q0;
-    const int np = n * (n + 1) / 2;
-    for (int p = threadIdx.x; p < np; p += blockDim.x) {
-      int i = 0, off = p;
-      while (off >= n - i) { off -= n - i; ++i; }
-      int j = i + off;
-      int ii = i;
-      if (idx[p0 + i] > idx[p0 + j]) { ii = j; j = i; }
-      const unsigned code = (static_cast<unsigned>(k) << 12) | (static_cast<unsigned>(ii) << 6) | static_cast<unsigned>(j);
-      mkeys[m0 + p] = (static_cast<unsigned long long>(static_cast<unsigned>(map_slot[q0 + m0 + p])) << 16) | code;
-    }
-  }
-  int n2 = 1;
-  while (n2 < items) n2 <<= 1;
-  for (int t = items + threadIdx.x; t < n2; t += blockDim.x) mkeys[t] = ~0ULL;
+  if (t == 0) s_bad = 0;
   __syncthreads();
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-        const int u = t ^ j;
-        if (u > t) {
-          const bool up = (t & k) == 0;
-          const unsigned long long a = mkeys[t], b = mkeys[u];
-          if ((a > b) == up) { mkeys[t] = b; mkeys[u] = a; }
+  if (t < g1 - g0 && ptr[g0 + t + 1] - ptr[g0 + t] > 64) s_bad = 1;
+  if (t == 0 && map_ptr[g1] - map_ptr[g0] > kMergePairs) s_bad = 1;
+  __syncthreads();
+  int U = 0;
+  if (!s_bad) {
+    int n2 = 1;
+    while (n2 < items) n2 <<= 1;
+    for (int i = t; i < n2; i += kCellThreads) ids[i] = i < items ? idx[q0 + i] : 0x7fffffff;
+    __syncthreads();
+    for (int k = 2; k <= n2; k <<= 1) {
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = t; i < n2; i += kCellThreads) {
+          const int u = i ^ j;
+          if (u > i) {
+            const bool up = (i & k) == 0;
+            const int x = ids[i], y = ids[u];
+            if ((x > y) == up) { ids[i] = y; ids[u] = x; }
+          }
         }
+        __syncthreads();
       }
-      __syncthreads();
     }
+    if (t == 0) {  // unique, in place
+      int m = 0;
+      for (int i = 0; i < items; ++i)
+        if (m == 0 || ids[i] != ids[m - 1]) ids[m++] = ids[i];
+      s_n = m;
+    }
+    __syncthreads();
+    U = s_n;
   }
-  // Entry heads: position t starts an entry when its slot differs from t - 1.
-  if (threadIdx.x == 0) n_ent = 0;
-  __syncthreads();
-  for (int t = threadIdx.x; t < items; t += blockDim.x)
-    if (t == 0 || (mkeys[t] >> 16) != (mkeys[t - 1] >> 16)) atomicAdd(&n_ent, 1);
-  __syncthreads();
-  const int m = n_ent;
-  if (phase == 0) {
-    if (threadIdx.x == 0) ent_count[G] = m;
+  if (s_bad || U > kTileMaxU) {
+    if (phase == 0) {
+      if (t == 0) { n_items[G] = -1; cell_U[G] = 32767; }
+      for (int64_t e = q0 + t; e < q1; e += kCellThreads) nbr_u[e] = 255;
+    }
     return;
   }
-  if (ent_ptr[G + 1] - ent_ptr[G] != m) return;
-  // Per entry: start (rank among heads, by a serial scan over the sorted keys is avoided:
-  // each head counts the heads before it with a parallel prefix over positions).
-  // Reuse the key array's tail (beyond n2) is not possible in general, so write the codes
-  // in sorted order first, then the entry table.
-  const int64_t c0 = q0;  // contribution base of this group
-  for (int t = threadIdx.x; t < items; t += blockDim.x) con_code[c0 + t] = static_cast<uint16_t>(mkeys[t] & 0xffff);
-  // Entry start positions and counts, then a stable counting sort of the entries by count.
-  // Thread 0 walks the sorted keys (items <= 16384): the entry table is small.
-  if (threadIdx.x == 0) {
-    for (int c = 0; c < kMergeGroup + 2; ++c) hist[c] = 0;
-    int e = 0, start = 0;
-    for (int t = 1; t <= items; ++t) {
-      if (t == items || (mkeys[t] >> 16) != (mkeys[t - 1] >> 16)) {
-        const int cnt = t - start;
-        hist[cnt > kMergeGroup ? kMergeGroup : cnt]++;  // counts <= points per group
-        // temporarily store (start, slot) at the entry's unsorted index
-        ent_cstart[ent_ptr[G] + e] = start;
-        ent_slot[ent_ptr[G] + e] = static_cast<int32_t>(mkeys[start] >> 16);
-        ++e;
-        start = t;
+  for (int u = t; u < U; u += kCellThreads) mask[u] = 0;
+  __syncthreads();
+  for (int k = 0; k < g1 - g0; ++k)
+    for (int64_t e = ptr[g0 + k] + t; e < ptr[g0 + k + 1]; e += kCellThreads) {
+      const int node = idx[e];
+      int lo = 0, hi = U;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ids[mid] < node) lo = mid + 1; else hi = mid;
       }
+      if (phase == 0) nbr_u[e] = static_cast<uint8_t>(lo);
+      if (atomicOr(&mask[lo], 1u << k) & (1u << k)) s_bad = 1;   // a node twice in one list
     }
+  __syncthreads();
+  if (s_bad) {
+    if (phase == 0) {
+      if (t == 0) { n_items[G] = -1; cell_U[G] = 32767; }
+      for (int64_t e = q0 + t; e < q1; e += kCellThreads) nbr_u[e] = 255;
+    }
+    return;
+  }
+  auto tile_mask = [&](int J, int tile) {
+    unsigned m = 0;
+    for (int I = 4 * tile; I < 4 * tile + 4 && I <= J; ++I) m |= mask[I];
+    return m & mask[J];
+  };
+  for (int J = t; J < U; J += kCellThreads) {
+    const int h = J >> 2, first = 2 * h * (h + 1) + (J & 3) * (h + 1);   // sum of (j / 4 + 1), j < J
+    for (int tile = 0; tile <= h; ++tile) weight[first + tile] = static_cast<uint8_t>(__popc(tile_mask(J, tile)));
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    // Descending count order: offsets for count = 16, 15, ..., 1.
-    int acc = 0;
-    int off[kMergeGroup + 1];
-    for (int c = kMergeGroup; c >= 1; --c) { off[c] = acc; acc += hist[c]; }
-    // Stable placement needs the unsorted table; copy it through the key array (no longer used).
-    int* tmp = reinterpret_cast<int*>(mkeys);
-    for (int e = 0; e < m; ++e) { tmp[2 * e] = ent_cstart[ent_ptr[G] + e]; tmp[2 * e + 1] = ent_slot[ent_ptr[G] + e]; }
-    for (int e = 0; e < m; ++e) {
-      const int start = tmp[2 * e];
-      const int end = (e + 1 < m) ? tmp[2 * e + 2] : items;
-      int cnt = end - start;
-      if (cnt > kMergeGroup) cnt = kMergeGroup;
-      const int at = off[cnt]++;
-      ent_cstart[ent_ptr[G] + at] = (cnt << 16) | start;  // count in the high half
-      ent_slot[ent_ptr[G] + at] = tmp[2 * e + 1];
+  const int hU = U >> 2, total = 2 * hU * (hU + 1) + (U & 3) * (hU + 1);
+  if (t == 0) {  // stable counting sort, most points first; at most a few thousand items
+    int at[kMergeGroup + 1], n = 0;
+    for (int c = 0; c <= kMergeGroup; ++c) at[c] = 0;
+    for (int i = 0; i < total; ++i) ++at[weight[i]];
+    for (int c = kMergeGroup; c >= 1; --c) { const int v = at[c]; at[c] = n; n += v; }
+    for (int i = 0; i < total; ++i)
+      if (weight[i]) order[at[weight[i]]++] = static_cast<uint16_t>(i);
+    s_n = n;
+  }
+  __syncthreads();
+  const int n = s_n;
+  if (phase == 0) {
+    if (t == 0) { n_items[G] = n; cell_U[G] = static_cast<int16_t>(U); }
+    return;
+  }
+  const int64_t base = item_ptr[G];
+  int found = 0;
+  for (int i = t; i < n; i += kCellThreads) {
+    const int c = order[i];
+    int J = 0;   // the last J whose first item is at or below c
+    for (int step = 64; step > 0; step >>= 1) {
+      const int K = J + step, h = K >> 2;
+      if (K < U && 2 * h * (h + 1) + (K & 3) * (h + 1) <= c) J = K;
+    }
+    const int h = J >> 2, tile = c - (2 * h * (h + 1) + (J & 3) * (h + 1));
+    item_code[base + i] = tile_mask(J, tile) | (static_cast<unsigned>(tile) << 16) | (static_cast<unsigned>(J) << 24);
+    const int64_t c0 = col_ptr[ids[J]], c1 = col_ptr[ids[J] + 1];
+    for (int q = 0; q < 4; ++q) {
+      const int I = 4 * tile + q;
+      int32_t slot = -1;
+      if (I <= J && (mask[I] & mask[J])) {
+        int64_t lo = c0, hi = c1;
+        while (lo < hi) {
+          const int64_t mid = (lo + hi) >> 1;
+          if (col_nodes[mid] < ids[I]) lo = mid + 1; else hi = mid;
+        }
+        slot = static_cast<int32_t>(lo);
+        ++found;
+      }
+      item_slot[4 * (base + i) + q] = slot;
     }
   }
+  if (found) atomicAdd(n_entries, static_cast<unsigned long long>(found));
 }
 
 inline unsigned nb(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
@@ -468,154 +492,62 @@ void pattern_build(cgb_assembler* a) {
   CGB_CUDA(cudaStreamSynchronize(st));
 }
 
-// ---- tables of the tensor-core tangent --------------------------------------------------
-// One CTA per group of kMergeGroup points: the group's neighbour ids sorted and made unique
-// (the group's node union, ascending ids), every face entry's index in it, the union's size,
-// and for every merged entry (from its first contribution code, written row node first) the
-// union indices of the block's row and column nodes. Groups with more than kTcItems entries
-// get the size 32767 (not on the tensor path).
-constexpr int kTcItems = 1024;
-
-__global__ void __launch_bounds__(128) tc_cells_kernel(int n_gp, const int64_t* __restrict__ ptr,
-                                                       const int32_t* __restrict__ idx,
-                                                       const int64_t* __restrict__ map_ptr,
-                                                       const int64_t* __restrict__ ent_ptr,
-                                                       const int32_t* __restrict__ ent_cstart,
-                                                       const uint16_t* __restrict__ code, uint8_t* __restrict__ nbr_u,
-                                                       int16_t* __restrict__ cell_U, uint16_t* __restrict__ ent_uv) {
-  __shared__ int ids[kTcItems];
-  __shared__ int s_nu;
-  const int G = blockIdx.x, t = threadIdx.x;
-  const int g0 = G * kMergeGroup, g1 = min(n_gp, g0 + kMergeGroup);
-  const int64_t q0 = ptr[g0], q1 = ptr[g1];
-  const int items = static_cast<int>(q1 - q0);
-  if (items > kTcItems) {
-    for (int64_t e = q0 + t; e < q1; e += blockDim.x) nbr_u[e] = 255;
-    if (t == 0) cell_U[G] = 32767;
-    return;
-  }
-  int n2 = 1;
-  while (n2 < items) n2 <<= 1;
-  for (int i = t; i < n2; i += blockDim.x) ids[i] = i < items ? idx[q0 + i] : 0x7fffffff;
-  __syncthreads();
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = t; i < n2; i += blockDim.x) {
-        const int u = i ^ j;
-        if (u > i) {
-          const bool up = (i & k) == 0;
-          const int x = ids[i], y = ids[u];
-          if ((x > y) == up) { ids[i] = y; ids[u] = x; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (t == 0) {  // unique, in place (items <= 1024)
-    int m = 0;
-    for (int i = 0; i < items; ++i)
-      if (m == 0 || ids[i] != ids[m - 1]) ids[m++] = ids[i];
-    s_nu = m;
-  }
-  __syncthreads();
-  const int U = s_nu;
-  if (t == 0) cell_U[G] = static_cast<int16_t>(U);
-  auto find = [&](int node) {
-    int lo = 0, hi = U;  // first position with ids[pos] >= node
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (ids[mid] < node) lo = mid + 1; else hi = mid;
-    }
-    return lo < 255 ? lo : 255;
-  };
-  for (int64_t e = q0 + t; e < q1; e += blockDim.x) nbr_u[e] = static_cast<uint8_t>(find(idx[e]));
-  const int64_t e0 = ent_ptr[G], e1 = ent_ptr[G + 1];
-  const int64_t cbase = map_ptr[g0];
-  for (int64_t e = e0 + t; e < e1; e += blockDim.x) {
-    const unsigned cd = code[cbase + (ent_cstart[e] & 0xffff)];
-    const int k = cd >> 12, i = (cd >> 6) & 63, j = cd & 63;
-    const int64_t p0 = ptr[g0 + k];
-    ent_uv[e] = static_cast<uint16_t>(find(idx[p0 + i]) | (find(idx[p0 + j]) << 8));
-  }
-}
-
-void tc_prepare(cgb_assembler* a) {
-  if (a->tc_ready) return;
-  merge_prepare(a);
+void tile_prepare(cgb_assembler* a) {
+  if (a->tile_ready) return;
   cudaStream_t st = a->ctx->stream;
   const cgb_shape* S = a->faces;
   const int n_gp = S->n_gp;
   const int ng = (n_gp + kMergeGroup - 1) / kMergeGroup;
-  a->tc_nbr_u.alloc(std::max<int64_t>(S->nnz, 1));
-  a->tc_cell_U.alloc(std::max(ng, 1));
-  a->tc_ent_uv.alloc(std::max<int64_t>(a->mrg_n_ent, 1));
-  if (ng > 0)
-    tc_cells_kernel<<<ng, 128, 0, st>>>(n_gp, S->nbr_ptr.p, S->nbr_idx.p, a->map_ptr.p, a->mrg_ent_ptr.p,
-                                        a->mrg_ent_cstart.p, a->mrg_code.p, a->tc_nbr_u.p, a->tc_cell_U.p,
-                                        a->tc_ent_uv.p);
-  CGB_CUDA(cudaGetLastError());
+  a->nbr_u.alloc(S->nnz + 32);   // the tangent stages it with bulk copies widened to 16 bytes
+  a->cell_U.alloc(ng);
+  DevBuf<int32_t> counts(ng);
+  DevBuf<unsigned long long> entries(1);
+  CGB_CUDA(cudaMemsetAsync(entries.p, 0, entries.bytes(), st));
+  auto cells = [&](int phase) {
+    if (ng > 0)
+      tile_cells_kernel<<<ng, kCellThreads, 0, st>>>(n_gp, S->nbr_ptr.p, S->nbr_idx.p, a->map_ptr.p, a->col_ptr.p,
+                                                     a->col_nodes.p, phase, a->nbr_u.p, a->cell_U.p, counts.p,
+                                                     a->item_ptr.p, a->item_code.p, a->item_slot.p, entries.p);
+    CGB_CUDA(cudaGetLastError());
+  };
+  cells(0);
+  std::vector<int32_t> hc(std::max(ng, 1));
   std::vector<int16_t> cu(std::max(ng, 1));
-  std::vector<int8_t> direct(std::max(ng, 1));
+  std::vector<int64_t> ptr(n_gp + 1);
   if (ng > 0) {
-    CGB_CUDA(cudaMemcpyAsync(cu.data(), a->tc_cell_U.p, ng * sizeof(int16_t), cudaMemcpyDeviceToHost, st));
-    CGB_CUDA(cudaMemcpyAsync(direct.data(), a->mrg_direct.p, ng * sizeof(int8_t), cudaMemcpyDeviceToHost, st));
+    CGB_CUDA(cudaMemcpyAsync(hc.data(), counts.p, ng * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    CGB_CUDA(cudaMemcpyAsync(cu.data(), a->cell_U.p, ng * sizeof(int16_t), cudaMemcpyDeviceToHost, st));
+    CGB_CUDA(cudaMemcpyAsync(ptr.data(), S->nbr_ptr.p, ptr.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   }
   CGB_CUDA(cudaStreamSynchronize(st));
-  a->tc_fallback_h.clear();
+  std::vector<int64_t> ip(ng + 1, 0);
+  a->direct_h.clear();
+  a->tc_rest_h.clear();
   a->tc_n_groups = 0;
   a->tc_point_cols = 0;
+  a->cell_max_e = a->cell_max_u = 0;
   for (int G = 0; G < ng; ++G) {
-    if (direct[G] || cu[G] > kTcMaxUnion) {
-      a->tc_fallback_h.push_back(G);
-    } else {
-      const int n_cols = std::max(16, (3 * cu[G] + 15) & ~15);
-      ++a->tc_n_groups;
-      a->tc_point_cols += static_cast<int64_t>(std::min(kMergeGroup, n_gp - G * kMergeGroup)) * n_cols;
-    }
+    ip[G + 1] = ip[G] + std::max(hc[G], 0);
+    if (hc[G] < 0) { a->direct_h.push_back(G); continue; }
+    const int g1 = std::min(n_gp, (G + 1) * kMergeGroup);
+    a->cell_max_e = std::max<int>(a->cell_max_e, static_cast<int>(ptr[g1] - ptr[G * kMergeGroup]));
+    a->cell_max_u = std::max<int>(a->cell_max_u, cu[G]);
+    if (cu[G] > kTcMaxUnion) { a->tc_rest_h.push_back(G); continue; }
+    ++a->tc_n_groups;
+    a->tc_point_cols += static_cast<int64_t>(g1 - G * kMergeGroup) * std::max(16, (3 * cu[G] + 15) & ~15);
   }
-  upload(a->tc_fallback, a->tc_fallback_h.data(), a->tc_fallback_h.size(), st);
+  upload(a->direct, a->direct_h.data(), a->direct_h.size(), st);
+  upload(a->tc_rest, a->tc_rest_h.data(), a->tc_rest_h.size(), st);
+  upload(a->item_ptr, ip.data(), ip.size(), st);
+  a->n_items = ip[ng];
+  a->item_code.alloc(a->n_items);
+  a->item_slot.alloc(4 * a->n_items);
+  cells(1);
+  unsigned long long n_ent = 0;
+  CGB_CUDA(cudaMemcpyAsync(&n_ent, entries.p, sizeof(n_ent), cudaMemcpyDeviceToHost, st));
   CGB_CUDA(cudaStreamSynchronize(st));
-  a->tc_ready = true;
-}
-
-void merge_prepare(cgb_assembler* a) {
-  if (a->mrg_ready) return;
-  cudaStream_t st = a->ctx->stream;
-  const cgb_shape* S = a->faces;
-  const int n_gp = S->n_gp;
-  const int ng = (n_gp + kMergeGroup - 1) / kMergeGroup;
-  const size_t smem = kMergeItems * sizeof(unsigned long long);
-  CGB_CUDA(cudaFuncSetAttribute(merge_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  DevBuf<int32_t> counts(ng);
-  if (ng > 0)
-    merge_groups_kernel<<<ng, 256, smem, st>>>(n_gp, S->nbr_ptr.p, S->nbr_idx.p, a->map_ptr.p, a->map_slot.p, 0, counts.p,
-                                               nullptr, nullptr, nullptr, nullptr);
-  CGB_CUDA(cudaGetLastError());
-  std::vector<int32_t> hc(std::max(ng, 1));
-  if (ng > 0) CGB_CUDA(cudaMemcpyAsync(hc.data(), counts.p, ng * 4, cudaMemcpyDeviceToHost, st));
-  CGB_CUDA(cudaStreamSynchronize(st));
-  std::vector<int64_t> ep(ng + 1, 0);
-  std::vector<int8_t> direct(std::max(ng, 1), 0);
-  for (int G = 0; G < ng; ++G) {
-    if (hc[G] < 0) { direct[G] = 1; ep[G + 1] = ep[G]; }
-    else ep[G + 1] = ep[G] + hc[G];
-  }
-  upload(a->mrg_ent_ptr, ep.data(), ep.size(), st);
-  upload(a->mrg_direct, direct.data(), direct.size(), st);
-  a->mrg_ent_slot.alloc(ep[ng]);
-  a->mrg_ent_cstart.alloc(ep[ng]);
-  a->mrg_code.alloc(a->n_pairs);
-  a->mrg_n_ent = ep[ng];
-  a->mrg_n_direct = 0;
-  for (int G = 0; G < ng; ++G) a->mrg_n_direct += direct[G];
-  if (ng > 0)
-    merge_groups_kernel<<<ng, 256, smem, st>>>(n_gp, S->nbr_ptr.p, S->nbr_idx.p, a->map_ptr.p, a->map_slot.p, 1, nullptr,
-                                               a->mrg_ent_ptr.p, a->mrg_ent_slot.p, a->mrg_ent_cstart.p,
-                                               a->mrg_code.p);
-  CGB_CUDA(cudaGetLastError());
-  CGB_CUDA(cudaStreamSynchronize(st));
-  a->mrg_ready = true;
+  a->n_entries = static_cast<int64_t>(n_ent);
+  a->tile_ready = true;
 }
 
 // Ordered lists for the deterministic scatter. F contribution ids: face entries
@@ -667,9 +599,9 @@ void deterministic_pair_lists(cgb_assembler* a) {
 
 void deterministic_entry_lists(cgb_assembler* a) {
   if (a->det_entries_ready) return;
-  merge_prepare(a);
-  if (a->mrg_n_direct) throw Error(CGB_ERR_INVALID, "deterministic entry lists need every group merged");
-  block_lists(a, a->mrg_n_ent, a->mrg_ent_slot.p, a->ent_list_ptr, a->ent_list);
+  tile_prepare(a);
+  if (!a->direct_h.empty()) throw Error(CGB_ERR_INVALID, "deterministic entry lists need every group merged");
+  block_lists(a, 4 * a->n_items, a->item_slot.p, a->ent_list_ptr, a->ent_list);
   a->det_entries_ready = true;
 }
 

@@ -176,18 +176,26 @@ __device__ __forceinline__ void form_block(const ColumnRecord<TK, BZERO>& R, con
 
 constexpr int kEntryThreads = 128;
 
-// Entries [ptr[g_begin], ptr[g_end]) of the launch, one per thread; ent_point: the point of
+// Entries [ptr[g_begin], ptr[g_end]) of the launch, one per thread, or those of the cells
+// glist[0 .. gcount) of 16 points, each with `per_cell` thread blocks; ent_point: the point of
 // every entry. A warp's 32 blocks of one step are turned through shared memory, so that a
 // block's nine values leave on neighbouring lanes (72 consecutive bytes: 3 sectors instead of
 // the 9 of one value per lane and instruction).
 template <typename TK, bool DET, bool BZERO>
 __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceArgs a, const TK* __restrict__ gstate,
-                                                                         const int32_t* __restrict__ ent_point) {
+                                                                         const int32_t* __restrict__ ent_point,
+                                                                         const int32_t* __restrict__ glist, int per_cell) {
   __shared__ TK s_val[kEntryThreads / 32][32 * 9];
   __shared__ int64_t s_at[kEntryThreads / 32][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t e_end = a.ptr[a.g_end];
-  const int64_t ew = a.ptr[a.g_begin] + static_cast<int64_t>(blockIdx.x) * kEntryThreads + 32 * w;  // the warp's first
+  int gb = a.g_begin, ge = a.g_end, blk = blockIdx.x;
+  if (glist) {
+    gb = kMG * glist[blockIdx.x / per_cell];
+    ge = min(gb + kMG, a.g_end);
+    blk = blockIdx.x % per_cell;
+  }
+  const int64_t e_end = a.ptr[ge];
+  const int64_t ew = a.ptr[gb] + static_cast<int64_t>(blk) * kEntryThreads + 32 * w;  // the warp's first
   if (ew >= e_end) return;
   const int64_t e = ew + lane;
   const bool live = e < e_end;
@@ -227,7 +235,8 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
       at = kStride * (DET ? q : static_cast<int64_t>(a.map_slot[q]));
       TK K[9];
       form_block<TK, BZERO>(R, b, D1[2 * ei], D1[2 * ei + 1], D2[3 * ei], D2[3 * ei + 1], D2[3 * ei + 2], K);
-      const bool flip = a.idx[ei] > nj;   // the stored block's row is the lower node
+      const int ni = a.idx[ei];
+      const bool flip = ni != nj ? ni > nj : i > j;   // the stored block's row is the lower node
 #pragma unroll
       for (int r = 0; r < 3; ++r)
 #pragma unroll

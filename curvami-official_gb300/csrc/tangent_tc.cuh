@@ -1,7 +1,7 @@
 // tangent_tc.cuh — the FP32-class tangent of one quadrature cell (16 consecutive Gauss
 // points) as one tensor-core product on sm_103a (tcgen05, 3xTF32 with FP32 accumulation
-// in tensor memory). Included by assemble.cu after the merged CUDA-core tangent, whose
-// per-point state, staging and merge tables it shares.
+// in tensor memory). Included by assemble.cu after the CUDA-core tile tangent, whose
+// per-point state, staging and tables it shares.
 //
 // The pair loop of NonLinearAssembler::updateStiffness (plate/Assembly.h:282-324) gives,
 // per Gauss point and local pair (i, j), the 3x3 block
@@ -29,8 +29,8 @@
 //    thread issues the five MMAs (A from tensor memory, B from shared memory) and commits
 //    them to the stage's mbarrier; the stage is rewritten two points later, after it;
 //  - after the last point: the accumulator (128 lanes x 3U columns of tensor memory) goes to
-//    a dense matrix in shared memory (over the B stages and the records), and each merged
-//    entry of the cell (a distinct 3x3 block of K, from the merge tables) is read from it and
+//    a dense matrix in shared memory (over the B stages and the records), and each distinct
+//    3x3 block of the cell (the slots of its items, tile_prepare) is read from it and
 //    scattered with three 16-byte FP32 vector atomics (or stored, deterministic mode).
 // Every wait is bounded (about one second of SM clock); a CTA that gives up records bit 16
 // (or bit 4 for the staging copy) in the device error word, lets its copies and MMAs land
@@ -52,7 +52,6 @@ constexpr uint32_t kTcACol = 128;
 struct TcArgs {
   const uint8_t* nbr_u;    // per face entry: its node's index in the cell's sorted union
   const int16_t* cell_U;   // per group: union size (above kTcMaxU: not on this path)
-  const uint16_t* ent_uv;  // per merged entry: union index of its row node | its column node << 8
 };
 
 // Floats of one neighbour record: the I side (dx dy Tu c0 c1 beta0 beta1 beta2) and the
@@ -193,7 +192,7 @@ __device__ __forceinline__ void tc_b_values(const float* R, float a1r, float a2r
 
 template <bool BZERO, bool DET>
 __global__ void __launch_bounds__(kTcThreads, 2) face_tangent_tc_kernel(FaceArgs a, const float* __restrict__ gstate,
-                                                                       MergeArgs mg, TcArgs tc) {
+                                                                       TileArgs mg, TcArgs tc) {
   constexpr int RS = tc_rec_floats(BZERO);
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ __align__(8) uint64_t stage_bar;
@@ -219,7 +218,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) face_tangent_tc_kernel(FaceArgs
   const Material& m = a.mat;
   const int G1 = (a.g_end + kMG - 1) / kMG;
   const int stride = static_cast<int>(gridDim.x);
-  auto eligible = [&](int G) { return !mg.direct[G] && tc.cell_U[G] <= kTcMaxU; };
+  auto eligible = [&](int G) { return tc.cell_U[G] <= kTcMaxU; };
   auto next_from = [&](int G) {
     while (G < G1 && !eligible(G)) G += stride;
     return G;
@@ -392,13 +391,17 @@ __global__ void __launch_bounds__(kTcThreads, 2) face_tangent_tc_kernel(FaceArgs
     }
     umma::fence_before_sync();
     __syncthreads();
-    // Merged entries: block (row node, column node) = D[3 ul + r][3 uh + c].
-    const int64_t e0 = mg.ent_ptr[G];
-    const int ne = static_cast<int>(mg.ent_ptr[G + 1] - e0);
+    // The cell's blocks (the slots of its items): block (row node, column node) =
+    // D[3 ul + r][3 uh + c].
+    const int64_t e0 = 4 * mg.item_ptr[G];
+    const int ne = static_cast<int>(4 * mg.item_ptr[G + 1] - e0);
+    const int32_t* slots = reinterpret_cast<const int32_t*>(mg.item_slot);
     float4* acc4 = static_cast<float4*>(a.Kacc);
     for (int e = t; e < ne; e += kTcThreads) {
-      const unsigned uv = tc.ent_uv[e0 + e];
-      const int ul = uv & 255u, uh = uv >> 8;
+      const int32_t slot = slots[e0 + e];
+      if (slot < 0) continue;
+      const uint32_t code = mg.item_code[(e0 + e) >> 2];
+      const int ul = static_cast<int>(4 * ((code >> 16) & 255u) + (e & 3)), uh = static_cast<int>(code >> 24);
       const float* d0p = Dm + (3 * ul) * kTcDStride + 3 * uh;
       float v[9];
 #pragma unroll
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) face_tangent_tc_kernel(FaceArgs
 #pragma unroll
         for (int q = 0; q < 9; ++q) d[q] = v[q];
       } else {
-        float4* d = acc4 + 3 * static_cast<int64_t>(mg.ent_slot[e0 + e]);
+        float4* d = acc4 + 3 * static_cast<int64_t>(slot);
         atomicAdd(d, make_float4(v[0], v[1], v[2], v[3]));
         atomicAdd(d + 1, make_float4(v[4], v[5], v[6], v[7]));
         atomicAdd(d + 2, make_float4(v[8], 0.0f, 0.0f, 0.0f));
