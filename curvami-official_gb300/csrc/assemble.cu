@@ -1255,7 +1255,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     tile_prepare(a);
     merged = (!det || a->direct_h.empty()) && a->n_items > 0;
   }
-  const size_t msm = merged ? tile_smem_bytes(a->cell_max_e, a->cell_max_u, bzero) : 0;
+  const size_t msm = merged ? tile_smem_bytes(a->cell_max_e, a->cell_max_u, a->cell_max_i, bzero) : 0;
   // The tensor-core tangent takes the cells whose node union fits one 128-row tile (its blocks
   // are the items' slots too, so the deterministic lists are the same).
   const size_t tcsm = tc_smem_bytes(std::max(S->max_n, 1), bzero);
@@ -1409,6 +1409,10 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       using TK = std::remove_pointer_t<decltype(stp)>;
       auto kern = det ? (want_K ? face_residual_kernel<TK, true, true, L> : face_residual_kernel<TK, true, false, L>)
                       : (want_K ? face_residual_kernel<TK, false, true, L> : face_residual_kernel<TK, false, false, L>);
+      // Beside the FP32 tangent the SMs must stay set up for its shared memory: an SM drains before
+      // it changes the split between L1 and shared memory, so a residual that asks for none (and
+      // gets the largest L1) and the tangent would never share one.
+      if (merged) CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
       // Few points: small blocks, so that every SM gets a share (25,600 points are only 100
       // blocks of 256 threads).
       const int rt = L > 1 ? 32 : (a->tuning.residual_threads == 0 && ncg < 256 * 4 * sms ? 64 : rthreads);
@@ -1442,11 +1446,12 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     };
     int ntan = 1;
     if (merged) {
-      TileArgs tg{a->item_ptr.p, a->item_code.p, reinterpret_cast<const int4*>(a->item_slot.p), a->nbr_u.p, a->cell_U.p,
-                  a->cell_max_e, a->cell_max_u, ctx->dev_err.p, a->test_stage_extra_tx, nullptr, 0};
+      TileArgs tg{a->cells.p, a->item_code.p, reinterpret_cast<const int4*>(a->item_slot.p), a->nbr_u.p,
+                  a->cell_max_e, a->cell_max_u, a->cell_max_i, ctx->dev_err.p, a->test_stage_extra_tx, nullptr, 0};
       auto kern = det ? (bzero ? face_tangent_tile_kernel<true, true> : face_tangent_tile_kernel<false, true>)
                       : (bzero ? face_tangent_tile_kernel<true, false> : face_tangent_tile_kernel<false, false>);
       CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(msm)));
+      CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
       int per_sm = 0;
       CGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileThreads, msm));
       const int Gb = fa.g_begin / kMG, Ge = (fa.g_end + kMG - 1) / kMG;
@@ -1461,7 +1466,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       if (use_tc) {
         // Cells whose node union fits one 128-row tile: one tensor-core product each; the
         // others on the CUDA cores.
-        TcArgs tca{a->nbr_u.p, a->cell_U.p};
+        TcArgs tca{a->nbr_u.p, a->cell_U.p, a->item_ptr.p};
         auto tk = det ? (bzero ? face_tangent_tc_kernel<true, true> : face_tangent_tc_kernel<false, true>)
                       : (bzero ? face_tangent_tc_kernel<true, false> : face_tangent_tc_kernel<false, false>);
         CGB_CUDA(cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tcsm)));

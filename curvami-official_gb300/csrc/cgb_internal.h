@@ -74,6 +74,13 @@ struct NatCurv {
   double x0 = 0.0, width = 1.0, amp = 0.0;
 };
 
+// One cell of the FP32 tangent: its first entry and item, how many it has, and its node union's
+// size (32767: direct).
+struct TileCell {
+  int64_t q0, i0;
+  int32_t n_ent, n_items, U, pad;
+};
+
 }  // namespace cgb
 
 // Opaque handles of the C ABI.
@@ -195,13 +202,14 @@ struct cgb_assembler {
   cgb::DevBuf<uint8_t> nbr_u;
   cgb::DevBuf<int16_t> cell_U;
   cgb::DevBuf<int64_t> item_ptr;      // n_cells + 1
+  cgb::DevBuf<cgb::TileCell> cells;   // the same per cell, with its entries, in one record
   cgb::DevBuf<uint32_t> item_code;
   cgb::DevBuf<int32_t> item_slot;     // 4 per item
   cgb::DevBuf<int32_t> direct, tc_rest;
   std::vector<int32_t> direct_h, tc_rest_h;
   int64_t n_items = 0;
   int64_t n_entries = 0;              // blocks over all cells (slots that are not -1)
-  int cell_max_e = 0, cell_max_u = 0; // most entries and nodes of a cell that is not direct
+  int cell_max_e = 0, cell_max_u = 0, cell_max_i = 0;  // most entries, nodes, items of a cell that is not direct
   int64_t tc_n_groups = 0;            // cells on the tensor path
   int64_t tc_point_cols = 0;          // sum over them of points x MMA columns (N)
   int tc_last_per_sm = 0;             // CTAs per SM of the last tensor-core tangent launch

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kCellThreads) tile_cells_kernel(
     uint32_t* __restrict__ item_code, int32_t* __restrict__ item_slot, unsigned long long* __restrict__ n_entries) {
   __shared__ int ids[kCellEntries];
   __shared__ unsigned mask[kTileMaxU];
-  __shared__ uint8_t weight[kCellItems];   // points of every (J, tile), J-major
+  __shared__ uint8_t weight[kCellItems];   // points of every item (0: no shared point), J-major
   __shared__ uint16_t order[kCellItems];
   __shared__ int s_n, s_bad;
   const int G = blockIdx.x, t = threadIdx.x;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kCellThreads) tile_cells_kernel(
   auto tile_mask = [&](int J, int tile) {
     unsigned m = 0;
     for (int I = 4 * tile; I < 4 * tile + 4 && I <= J; ++I) m |= mask[I];
-    return m & mask[J];
+    return (m & mask[J]) ? mask[J] : 0u;
   };
   for (int J = t; J < U; J += kCellThreads) {
     const int h = J >> 2, first = 2 * h * (h + 1) + (J & 3) * (h + 1);   // sum of (j / 4 + 1), j < J
@@ -521,17 +521,22 @@ void tile_prepare(cgb_assembler* a) {
   }
   CGB_CUDA(cudaStreamSynchronize(st));
   std::vector<int64_t> ip(ng + 1, 0);
+  std::vector<TileCell> cells_h(ng);
   a->direct_h.clear();
   a->tc_rest_h.clear();
   a->tc_n_groups = 0;
   a->tc_point_cols = 0;
-  a->cell_max_e = a->cell_max_u = 0;
+  a->cell_max_e = a->cell_max_u = a->cell_max_i = 0;
   for (int G = 0; G < ng; ++G) {
     ip[G + 1] = ip[G] + std::max(hc[G], 0);
+    cells_h[G] = TileCell{ptr[G * kMergeGroup], ip[G],
+                          static_cast<int32_t>(ptr[std::min(n_gp, (G + 1) * kMergeGroup)] - ptr[G * kMergeGroup]),
+                          std::max(hc[G], 0), cu[G], 0};
     if (hc[G] < 0) { a->direct_h.push_back(G); continue; }
     const int g1 = std::min(n_gp, (G + 1) * kMergeGroup);
     a->cell_max_e = std::max<int>(a->cell_max_e, static_cast<int>(ptr[g1] - ptr[G * kMergeGroup]));
     a->cell_max_u = std::max<int>(a->cell_max_u, cu[G]);
+    a->cell_max_i = std::max<int>(a->cell_max_i, hc[G]);
     if (cu[G] > kTcMaxUnion) { a->tc_rest_h.push_back(G); continue; }
     ++a->tc_n_groups;
     a->tc_point_cols += static_cast<int64_t>(g1 - G * kMergeGroup) * std::max(16, (3 * cu[G] + 15) & ~15);
@@ -539,8 +544,9 @@ void tile_prepare(cgb_assembler* a) {
   upload(a->direct, a->direct_h.data(), a->direct_h.size(), st);
   upload(a->tc_rest, a->tc_rest_h.data(), a->tc_rest_h.size(), st);
   upload(a->item_ptr, ip.data(), ip.size(), st);
+  upload(a->cells, cells_h.data(), cells_h.size(), st);
   a->n_items = ip[ng];
-  a->item_code.alloc(a->n_items);
+  a->item_code.alloc(a->n_items + 8);  // staged with bulk copies widened to 16 bytes
   a->item_slot.alloc(4 * a->n_items);
   cells(1);
   unsigned long long n_ent = 0;

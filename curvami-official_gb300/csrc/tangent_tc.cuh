@@ -52,6 +52,7 @@ constexpr uint32_t kTcACol = 128;
 struct TcArgs {
   const uint8_t* nbr_u;    // per face entry: its node's index in the cell's sorted union
   const int16_t* cell_U;   // per group: union size (above kTcMaxU: not on this path)
+  const int64_t* item_ptr; // per group: its first item
 };
 
 // Floats of one neighbour record: the I side (dx dy Tu c0 c1 beta0 beta1 beta2) and the
@@ -393,8 +394,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) face_tangent_tc_kernel(FaceArgs
     __syncthreads();
     // The cell's blocks (the slots of its items): block (row node, column node) =
     // D[3 ul + r][3 uh + c].
-    const int64_t e0 = 4 * mg.item_ptr[G];
-    const int ne = static_cast<int>(4 * mg.item_ptr[G + 1] - e0);
+    const int64_t e0 = 4 * tc.item_ptr[G];
+    const int ne = static_cast<int>(4 * tc.item_ptr[G + 1] - e0);
     const int32_t* slots = reinterpret_cast<const int32_t*>(mg.item_slot);
     float4* acc4 = static_cast<float4*>(a.Kacc);
     for (int e = t; e < ne; e += kTcThreads) {
