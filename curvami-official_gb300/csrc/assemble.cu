@@ -251,136 +251,148 @@ enum : int { D_A1 = 0, D_A2 = 3, D_B = 6, D_AX = 9, D_AY = 12, D_BX = 15, D_BY =
 // 0). Then P = A Bm = a1 (x) pa + a2 (x) pb and Q = D Bb = b (x) qc, and the J-side
 // record shrinks from 23 to 14 values.
 // Phase 1 for one Gauss point: FP64 kinematics,
-// resultants and residual (F atomics, or per-entry contributions when DET); when st is
-// not null the point's state goes to st[field * st_stride + st_idx] in TK.
+// resultants and residual (F atomics, or per-entry contributions when DET).
 // CHECK (caller-owned arrays only): a neighbour id outside [0, n_nodes) is flagged in the
 // error word and the neighbour is left out.
 // L lanes share a point (g: this lane's point, sub: its number among them): the neighbours are
-// dealt to them in turn, their sums added by shuffles, and lane 0 of them stores the state.
-template <typename TK, bool DET, bool CHECK = false, int L = 1>
-__device__ __forceinline__ void phase1_point(const FaceArgs& a, int g, int sub, TK* st, int64_t st_stride,
-                                             int64_t st_idx) {
+// dealt to them in turn, their sums added by shuffles, and put(state, weight) is called by lane 0 of
+// them as soon as the point's state is known, before the nodal forces.
+// Both neighbour loops hold the next neighbour's loads in flight (and its node's index two ahead)
+// while the current one is summed: its 15 FMA take 960 cycles of a quarter's FP64 pipe, about a
+// load's latency, so one or two warps per quarter keep the pipe busy.
+template <bool DET, bool CHECK, int L, class Put>
+__device__ __forceinline__ void phase1_point(const FaceArgs& a, int g, int sub, Put&& put) {
   const Material& m = a.mat;
   const bool here = g < a.g_end;
   if (!here) g = a.g_end - 1;   // lanes past the end keep their warp's shuffles whole and write nothing
-  if (here || L > 1) {
-      const int64_t p0 = a.ptr[g];
-      const int n = static_cast<int>(a.ptr[g + 1] - p0);
-      // Entry q of this lane's point: CSR p0 + q, or sliced-ELL sb + 32 q (coalesced
-      // across the warp: the 32 lanes read 32 consecutive entries per q).
-      const bool sell = a.sell_ptr != nullptr;
-      const int64_t sb = sell ? a.sell_ptr[g >> 5] + (g & 31) : p0;
-      const int64_t stride = sell ? 32 : 1;
-      const int32_t* Ix = sell ? a.sidx : a.idx;
-      const double* Dp = sell ? a.sdpsi : a.dpsi;
-      const double* Ddp = sell ? a.sddpsi : a.ddpsi;
-      double s[15];
+  if (!here && L == 1) return;
+  const int64_t p0 = a.ptr[g];
+  const int n = static_cast<int>(a.ptr[g + 1] - p0);
+  // Entry q of this lane's point: CSR p0 + q, or sliced-ELL sb + 32 q (coalesced
+  // across the warp: the 32 lanes read 32 consecutive entries per q).
+  const bool sell = a.sell_ptr != nullptr;
+  const int64_t sb = sell ? a.sell_ptr[g >> 5] + (g & 31) : p0;
+  const int64_t stride = sell ? 32 : 1;
+  const int32_t* Ix = sell ? a.sidx : a.idx;
+  const double* Dp = sell ? a.sdpsi : a.dpsi;
+  const double* Ddp = sell ? a.sddpsi : a.ddpsi;
+  struct Derivs { double x, y, xx, yy, xy; };
+  auto derivs = [&](int q) {
+    const int64_t e = sb + q * stride;
+    const double2 d = reinterpret_cast<const double2*>(Dp)[e];
+    return Derivs{d.x, d.y, Ddp[3 * e], Ddp[3 * e + 1], Ddp[3 * e + 2]};
+  };
+  auto node = [&](int q) -> int64_t { return q < n ? Ix[sb + q * stride] : 0; };
+  auto inside = [&](int64_t j) {   // caller-owned arrays: an index out of range is flagged and skipped
+    if (!CHECK || (j >= 0 && j < a.n_nodes)) return true;
+    atomicOr(a.err, kErrIndex);
+    return false;
+  };
+  double s[15];
 #pragma unroll
-      for (int k = 0; k < 15; ++k) s[k] = 0.0;
-#pragma unroll 4
-      for (int q = sub; q < n; q += L) {
-        const int64_t e = sb + q * stride;
-        const int64_t j = Ix[e];
-        if (CHECK && (j < 0 || j >= a.n_nodes)) {
-          atomicOr(a.err, kErrIndex);
-          continue;
-        }
-        const double u0 = a.x[3 * j], u1 = a.x[3 * j + 1], u2 = a.x[3 * j + 2];
-        const double2 d = reinterpret_cast<const double2*>(Dp)[e];
-        const double dxx = Ddp[3 * e], dyy = Ddp[3 * e + 1], dxy = Ddp[3 * e + 2];
-        s[0] += u0 * d.x; s[1] += u1 * d.x; s[2] += u2 * d.x;
-        s[3] += u0 * d.y; s[4] += u1 * d.y; s[5] += u2 * d.y;
-        s[6] += u0 * dxx; s[7] += u1 * dxx; s[8] += u2 * dxx;
-        s[9] += u0 * dyy; s[10] += u1 * dyy; s[11] += u2 * dyy;
-        s[12] += u0 * dxy; s[13] += u1 * dxy; s[14] += u2 * dxy;
+  for (int k = 0; k < 15; ++k) s[k] = 0.0;
+  {
+    struct Nb { Derivs d; double u0, u1, u2; };
+    auto load = [&](int q, int64_t j) {
+      Nb v{};
+      if (q < n && inside(j)) {
+        v.d = derivs(q);
+        v.u0 = a.x[3 * j]; v.u1 = a.x[3 * j + 1]; v.u2 = a.x[3 * j + 2];
       }
-#pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < 15; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-      PointState P;
-      point_state(s, m, P, a.gp_xy ? natcurv_kappa(a.nc, a.gp_xy[2 * static_cast<int64_t>(g)]) : 0.0);
-      const double W = a.weight[g];
-      if (L > 1 && (!here || sub != 0)) st = nullptr;
-      // The state the tangent needs goes out first, so that only the residual's coefficients
-      // stay live through the neighbour loop.
-      if constexpr (sizeof(TK) == 8) {
-        if (st) {
-          auto put = [&](int f, double v) { st[f * st_stride + st_idx] = v; };
-          double Ax[3], Ay[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            Ax[c] = P.Ci[0] * P.a1[c] + P.Ci[1] * P.a2[c];
-            Ay[c] = P.Ci[2] * P.a1[c] + P.Ci[3] * P.a2[c];
-            put(D_A1 + c, P.a1[c]); put(D_A2 + c, P.a2[c]); put(D_B + c, P.b[c]);
-            put(D_AX + c, Ax[c]); put(D_AY + c, Ay[c]);
-            put(D_N + c, P.N[c]); put(D_M + c, P.M[c]);
-          }
-          put(D_BX, P.rxx[0] * Ax[0] + P.rxx[1] * Ax[1] + P.rxx[2] * Ax[2]);
-          put(D_BX + 1, P.ryy[0] * Ax[0] + P.ryy[1] * Ax[1] + P.ryy[2] * Ax[2]);
-          put(D_BX + 2, 2.0 * (P.rxy[0] * Ax[0] + P.rxy[1] * Ax[1] + P.rxy[2] * Ax[2]));
-          put(D_BY, P.rxx[0] * Ay[0] + P.rxx[1] * Ay[1] + P.rxx[2] * Ay[2]);
-          put(D_BY + 1, P.ryy[0] * Ay[0] + P.ryy[1] * Ay[1] + P.ryy[2] * Ay[2]);
-          put(D_BY + 2, 2.0 * (P.rxy[0] * Ay[0] + P.rxy[1] * Ay[1] + P.rxy[2] * Ay[2]));
-          put(D_CI, P.Ci[0]); put(D_CI + 1, P.Ci[1]); put(D_CI + 2, P.Ci[3]);
-          put(D_P, P.pXY[0]); put(D_P + 1, P.pXY[1]); put(D_BV, P.bv); put(D_W, W);
-        }
-      } else if (st) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          st[(S_A1 + c) * st_stride + st_idx] = static_cast<TK>(P.a1[c]);
-          st[(S_A2 + c) * st_stride + st_idx] = static_cast<TK>(P.a2[c]);
-          st[(S_B + c) * st_stride + st_idx] = static_cast<TK>(P.b[c]);
-          st[(S_RXX + c) * st_stride + st_idx] = static_cast<TK>(P.rxx[c]);
-          st[(S_RYY + c) * st_stride + st_idx] = static_cast<TK>(P.ryy[c]);
-          st[(S_RXY + c) * st_stride + st_idx] = static_cast<TK>(P.rxy[c]);
-          st[(S_N + c) * st_stride + st_idx] = static_cast<TK>(P.N[c]);
-          st[(S_M + c) * st_stride + st_idx] = static_cast<TK>(P.M[c]);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) st[(S_CI + c) * st_stride + st_idx] = static_cast<TK>(P.Ci[c]);
-        st[(S_P + 0) * st_stride + st_idx] = static_cast<TK>(P.pXY[0]);
-        st[(S_P + 1) * st_stride + st_idx] = static_cast<TK>(P.pXY[1]);
-        st[S_BV * st_stride + st_idx] = static_cast<TK>(P.bv);
-        st[S_W * st_stride + st_idx] = static_cast<TK>(W);
-      }
-      // f_I = W (Bm_I^T N + Bb_I^T M) (Assembly.h:249) = W (a1 u1 + a2 u2 + b Tu_I), since
-      // beta_I . M = dPhi_I . pXY - (Phi_XX M0 + 2 Phi_XY M2 + Phi_YY M1) = Tu_I, with
-      // u1 = Phi_X N0 + Phi_Y N2 and u2 = Phi_Y N1 + Phi_X N2. It is linear in the five
-      // derivatives of Phi_I, so per point f_I[c] = Gx[c] Phi_X + Gy[c] Phi_Y + Hxx[c] Phi_XX +
-      // Hyy[c] Phi_YY + Hxy[c] Phi_XY: five FP64 FMAs per component and neighbour (GB300's
-      // FP64 pipe bounds this kernel).
-      double Gx[3], Gy[3], Hxx[3], Hyy[3], Hxy[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        Gx[c] = W * (P.a1[c] * P.N[0] + P.a2[c] * P.N[2] + P.b[c] * P.pXY[0]);
-        Gy[c] = W * (P.a1[c] * P.N[2] + P.a2[c] * P.N[1] + P.b[c] * P.pXY[1]);
-        Hxx[c] = -W * P.b[c] * P.M[0];
-        Hyy[c] = -W * P.b[c] * P.M[1];
-        Hxy[c] = -2.0 * W * P.b[c] * P.M[2];
-      }
-      if (here) {
-#pragma unroll 2
-        for (int q = sub; q < n; q += L) {
-          const int64_t es = sb + q * stride;
-          const int64_t e = p0 + q;
-          const double2 d = reinterpret_cast<const double2*>(Dp)[es];
-          const double dxx = Ddp[3 * es], dyy = Ddp[3 * es + 1], dxy = Ddp[3 * es + 2];
-          double f[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) f[c] = Gx[c] * d.x + Gy[c] * d.y + Hxx[c] * dxx + Hyy[c] * dyy + Hxy[c] * dxy;
-          if (DET) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) a.Fc[3 * e + c] = f[c];
-          } else {
-            const int64_t node = Ix[es];
-            if (CHECK && (node < 0 || node >= a.n_nodes)) continue;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) atomicAdd(a.F + 3 * node + c, f[c]);
-          }
-        }
-      }
+      return v;
+    };
+    int64_t j = node(sub);
+    Nb A = load(sub, j);
+    j = node(sub + L);
+    for (int q = sub; q < n; q += L) {
+      const Nb B = load(q + L, j);
+      j = node(q + 2 * L);
+      s[0] += A.u0 * A.d.x; s[1] += A.u1 * A.d.x; s[2] += A.u2 * A.d.x;
+      s[3] += A.u0 * A.d.y; s[4] += A.u1 * A.d.y; s[5] += A.u2 * A.d.y;
+      s[6] += A.u0 * A.d.xx; s[7] += A.u1 * A.d.xx; s[8] += A.u2 * A.d.xx;
+      s[9] += A.u0 * A.d.yy; s[10] += A.u1 * A.d.yy; s[11] += A.u2 * A.d.yy;
+      s[12] += A.u0 * A.d.xy; s[13] += A.u1 * A.d.xy; s[14] += A.u2 * A.d.xy;
+      A = B;
     }
+  }
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 15; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+  PointState P;
+  point_state(s, m, P, a.gp_xy ? natcurv_kappa(a.nc, a.gp_xy[2 * static_cast<int64_t>(g)]) : 0.0);
+  const double W = a.weight[g];
+  if (here && sub == 0) put(P, W);
+  // f_I = W (Bm_I^T N + Bb_I^T M) (Assembly.h:249) = W (a1 u1 + a2 u2 + b Tu_I), since
+  // beta_I . M = dPhi_I . pXY - (Phi_XX M0 + 2 Phi_XY M2 + Phi_YY M1) = Tu_I, with
+  // u1 = Phi_X N0 + Phi_Y N2 and u2 = Phi_Y N1 + Phi_X N2. It is linear in the five
+  // derivatives of Phi_I, so per point f_I[c] = Gx[c] Phi_X + Gy[c] Phi_Y + Hxx[c] Phi_XX +
+  // Hyy[c] Phi_YY + Hxy[c] Phi_XY: five FP64 FMAs per component and neighbour (GB300's
+  // FP64 pipe bounds this kernel).
+  double Gx[3], Gy[3], Hxx[3], Hyy[3], Hxy[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    Gx[c] = W * (P.a1[c] * P.N[0] + P.a2[c] * P.N[2] + P.b[c] * P.pXY[0]);
+    Gy[c] = W * (P.a1[c] * P.N[2] + P.a2[c] * P.N[1] + P.b[c] * P.pXY[1]);
+    Hxx[c] = -W * P.b[c] * P.M[0];
+    Hyy[c] = -W * P.b[c] * P.M[1];
+    Hxy[c] = -2.0 * W * P.b[c] * P.M[2];
+  }
+  if (!here) return;
+  Derivs A{};
+  int64_t jA = node(sub);
+  if (sub < n) A = derivs(sub);
+  for (int q = sub; q < n; q += L) {
+    Derivs B{};
+    const int64_t jB = node(q + L);
+    if (q + L < n) B = derivs(q + L);
+    double f[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = Gx[c] * A.x + Gy[c] * A.y + Hxx[c] * A.xx + Hyy[c] * A.yy + Hxy[c] * A.xy;
+    if (DET) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a.Fc[3 * (p0 + q) + c] = f[c];
+    } else if (inside(jA)) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) atomicAdd(a.F + 3 * jA + c, f[c]);
+    }
+    A = B;
+    jA = jB;
+  }
+}
+
+// The state of one point for a tangent kernel, st[field * stride + idx] in its precision.
+__device__ __forceinline__ void store_state(const PointState& P, double W, double* st, int64_t stride, int64_t idx) {
+  auto put = [&](int f, double v) { st[f * stride + idx] = v; };
+  double Ax[3], Ay[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    Ax[c] = P.Ci[0] * P.a1[c] + P.Ci[1] * P.a2[c];
+    Ay[c] = P.Ci[2] * P.a1[c] + P.Ci[3] * P.a2[c];
+    put(D_A1 + c, P.a1[c]); put(D_A2 + c, P.a2[c]); put(D_B + c, P.b[c]);
+    put(D_AX + c, Ax[c]); put(D_AY + c, Ay[c]);
+    put(D_N + c, P.N[c]); put(D_M + c, P.M[c]);
+  }
+  put(D_BX, P.rxx[0] * Ax[0] + P.rxx[1] * Ax[1] + P.rxx[2] * Ax[2]);
+  put(D_BX + 1, P.ryy[0] * Ax[0] + P.ryy[1] * Ax[1] + P.ryy[2] * Ax[2]);
+  put(D_BX + 2, 2.0 * (P.rxy[0] * Ax[0] + P.rxy[1] * Ax[1] + P.rxy[2] * Ax[2]));
+  put(D_BY, P.rxx[0] * Ay[0] + P.rxx[1] * Ay[1] + P.rxx[2] * Ay[2]);
+  put(D_BY + 1, P.ryy[0] * Ay[0] + P.ryy[1] * Ay[1] + P.ryy[2] * Ay[2]);
+  put(D_BY + 2, 2.0 * (P.rxy[0] * Ay[0] + P.rxy[1] * Ay[1] + P.rxy[2] * Ay[2]));
+  put(D_CI, P.Ci[0]); put(D_CI + 1, P.Ci[1]); put(D_CI + 2, P.Ci[3]);
+  put(D_P, P.pXY[0]); put(D_P + 1, P.pXY[1]); put(D_BV, P.bv); put(D_W, W);
+}
+__device__ __forceinline__ void store_state(const PointState& P, double W, float* st, int64_t stride, int64_t idx) {
+  auto put = [&](int f, double v) { st[f * stride + idx] = static_cast<float>(v); };
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    put(S_A1 + c, P.a1[c]); put(S_A2 + c, P.a2[c]); put(S_B + c, P.b[c]);
+    put(S_RXX + c, P.rxx[c]); put(S_RYY + c, P.ryy[c]); put(S_RXY + c, P.rxy[c]);
+    put(S_N + c, P.N[c]); put(S_M + c, P.M[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) put(S_CI + c, P.Ci[c]);
+  put(S_P, P.pXY[0]); put(S_P + 1, P.pXY[1]); put(S_BV, P.bv); put(S_W, W);
 }
 
 // Phase 2 for the Gauss points g0 .. g0 + 31 across the warp, in the tangent's precision:
@@ -574,7 +586,9 @@ __global__ void __launch_bounds__(32 * kFaceWarps, sizeof(TK) == 4 ? 5 : 3) face
     // Phase 1: one Gauss point per lane, FP64. Every lane does distinct work, so no FP64
     // issue slot is spent on a redundant or masked copy (on GB300 an FP64 warp
     // instruction costs the same with 1 or 32 lanes).
-    phase1_point<TK, DET, POS_MAP>(a, g0 + lane, 0, WANT_K ? st : static_cast<TK*>(nullptr), 32, lane);
+    phase1_point<DET, POS_MAP, 1>(a, g0 + lane, 0, [&](const PointState& P, double W) {
+      if (WANT_K) store_state(P, W, st, 32, lane);
+    });
     if (!WANT_K) continue;
     __syncwarp();
     phase2_group<TK, DET, TIN, POS_MAP, BZERO>(a, g0, lane, st, rec, nid);
@@ -604,7 +618,9 @@ __global__ void __launch_bounds__(256) face_residual_kernel(FaceArgs a, TK* gsta
     const int64_t g0 = a.g_begin + PTS * static_cast<int64_t>(unit);
     if (g0 >= a.g_end) break;
     const int g = static_cast<int>(g0) + lane / LANES;
-    phase1_point<TK, DET, false, LANES>(a, g, lane % LANES, STORE ? gstate : static_cast<TK*>(nullptr), a.n_gp, g);
+    phase1_point<DET, false, LANES>(a, g, lane % LANES, [&](const PointState& P, double W) {
+      if (STORE) store_state(P, W, gstate, a.n_gp, g);
+    });
   }
 }
 
@@ -1217,7 +1233,10 @@ void refresh_face_copies(cgb_assembler* a) {
 
 namespace {
 
+// Chunks of the mixed step with the library's choice. Measured, one against four: 66,564 points
+// 657 / 694 us, 118,336 points 560 / 525 us, 193,600 points 853 / 832 us, 640,000 points 2.70 / 2.24 ms.
 constexpr int kChunks = 4;
+constexpr int kChunkPoints = 98304;
 
 // The second stream and the events of the chunked face launch (created once per
 // assembler; the stream is non-blocking and joined back into the context stream).
@@ -1341,7 +1360,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   // chunk c (FP32 pipe, L2 atomics) on a second stream; chunks are multiples of 32 points.
   ensure_side_stream(a);
   // Only the FP32 tangent has another pipe to overlap with; without one, chunks are just tails.
-  const int n_chunks = a->tuning.n_chunks > 0 ? a->tuning.n_chunks : (mixed && want_K && S->n_gp >= 65536 ? kChunks : 1);
+  const int n_chunks = a->tuning.n_chunks > 0 ? a->tuning.n_chunks : (mixed && want_K && S->n_gp >= kChunkPoints ? kChunks : 1);
   const int rthreads = a->tuning.residual_threads > 0 ? a->tuning.residual_threads : 256;
   const int chunk = ((S->n_gp + n_chunks - 1) / n_chunks + 31) / 32 * 32;
   // Chunk c covers [cb(c), cb(c + 1)). The first chunk is a quarter of the others: the
@@ -1414,10 +1433,14 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       // gets the largest L1) and the tangent would never share one.
       if (merged) CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
       // Few points: small blocks, so that every SM gets a share (25,600 points are only 100
-      // blocks of 256 threads).
-      const int rt = L > 1 ? 32 : (a->tuning.residual_threads == 0 && ncg < 256 * 4 * sms ? 64 : rthreads);
+      // blocks of 256 threads). Beside the previous chunk's tangent: small blocks too, and as many
+      // warps per SM as leave the tangent's blocks their registers (8: 640,000 points in 4 chunks
+      // take 2.22 ms, against 2.40 with 16 and 2.88 with 4).
+      const bool beside = merged && c > 0;
+      const int rt = L > 1 ? 32 : (a->tuning.residual_threads == 0 && (beside || ncg < 256 * 4 * sms) ? 64 : rthreads);
       const int64_t pts = rt / L;
-      kern<<<std::max(1u, std::min(nb(ncg, static_cast<int>(pts)), static_cast<unsigned>(sms * 16 * (256 / rt)))), rt, 0, st>>>(fa, stp, work);
+      const unsigned most = static_cast<unsigned>(beside ? sms * std::max(1, 256 / rt) : sms * 16 * (256 / rt));
+      kern<<<std::max(1u, std::min(nb(ncg, static_cast<int>(pts)), most)), rt, 0, st>>>(fa, stp, work);
     };
     auto rk = [&](auto* stp) {
       switch (residual_lanes(ncg, sms, det)) {

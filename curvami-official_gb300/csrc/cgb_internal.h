@@ -139,6 +139,10 @@ struct cgb_shape {
   cgb::DevBuf<int8_t> scr_side;   // n_creases * n_nodes
   cgb::DevBuf<double> scr_gind;   // n_creases * 6 * n_gp
   cgb::DevBuf<int8_t> scr_bad;    // n_gp
+  cgb::DevBuf<int> scr_guard;     // 4: flagged points
+  cgb::DevBuf<int8_t> scr_tip;        // n_gp, FP64
+  cgb::DevBuf<double> scr_fac;        // n_nodes, FP64 with per-node radius
+  cgb::DevBuf<double> scr_mom, scr_coef;  // FP64: moment sums and polynomials of a chunk of points
   cgb::DevBuf<float4> scr_node_pair;  // 2 * n_nodes, mixed precision only
   cgb::DevBuf<float> scr_point_rec;   // point records of the mixed RKPM, n_gp x record floats
 };

@@ -292,9 +292,9 @@ int cgb_shape_concat(cgb_context* ctx, const cgb_shape* const* sets, const int32
                      cgb_shape** out);
 
 /* Launch shape of an assembly; 0 keeps the library's choice. n_chunks (1..16): Gauss-point
- * chunks whose residual and tangent kernels overlap on two streams (default 4 from 65,536
- * points, else 1); residual_threads (64, 128, 256): block size of the residual kernel
- * (default 256); tangent_ctas_per_sm (1..4): resident CTAs per SM of the merged FP32
+ * chunks whose residual and tangent kernels overlap on two streams (default 4 for the mixed
+ * step from 98,304 points, else 1); residual_threads (64, 128, 256): block size of the residual kernel
+ * (default by size; small launches split points over lanes instead); tangent_ctas_per_sm (1..4): resident CTAs per SM of the merged FP32
  * tangent (default: as many as fit); tangent_kind, the mixed-precision tangent:
  * CGB_TANGENT_CORES (the default) every cell on the CUDA cores (FP32, merged
  * contributions); CGB_TANGENT_TENSOR forms each quadrature cell's blocks as one
