@@ -18,6 +18,7 @@
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
@@ -54,8 +55,7 @@ struct FrnnPre {
 __global__ void frnn_kernel(int n_gp, const double* __restrict__ gp_xy,
                             const double* __restrict__ node_xy, const double* __restrict__ rho_node,
                             double rho, double rho2, GridDev G, FrnnPre pre, const int64_t* __restrict__ ptr,
-                            int32_t* __restrict__ count, int32_t* __restrict__ out_idx,
-                            double* __restrict__ out_s) {
+                            int32_t* __restrict__ count, int32_t* __restrict__ out_idx) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n_gp) return;
   const double gx = gp_xy[2 * g], gy = gp_xy[2 * g + 1];
@@ -77,21 +77,16 @@ __global__ void frnn_kernel(int n_gp, const double* __restrict__ gp_xy,
         const float r2f = pre.r2n32 ? pre.r2n32[j] : pre.r2f;
         if (d2f > r2f + pre.margin) continue;          // outside, whatever FP64 gives
         bool inside = d2f < r2f - pre.margin;          // inside, whatever FP64 gives
-        double dist2 = 0.0, r = rho;
-        if (!inside || out_s) {
+        if (!inside) {
           const double ddx = __dsub_rn(node_xy[2 * j], gx);
           const double ddy = __dsub_rn(node_xy[2 * j + 1], gy);
-          dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
+          const double dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
           double r2 = rho2;
-          if (rho_node) { r = rho_node[j]; r2 = __dmul_rn(r, r); }
-          if (!inside) inside = dist2 <= r2;
+          if (rho_node) { const double r = rho_node[j]; r2 = __dmul_rn(r, r); }
+          inside = dist2 <= r2;
         }
         if (inside) {
-          if (out_idx) {
-            out_idx[pos] = j;
-            if (out_s) out_s[pos] = __ddiv_rn(__dsqrt_rn(dist2), r);
-            ++pos;
-          }
+          if (out_idx) out_idx[pos++] = j;
           ++cnt;
         }
       }
@@ -100,23 +95,50 @@ __global__ void frnn_kernel(int n_gp, const double* __restrict__ gp_xy,
   if (!out_idx) count[g] = cnt;
 }
 
-// Normalised distances s of an existing neighbour list, with the FRNN's own rounded
-// operations (so bitwise equal to what frnn_kernel writes); sets built in mixed
-// precision skip s in the FRNN and compute it here when a caller downloads it.
+// The point of entry e of the points [g0, g1): lane 0 of each warp finds it for the warp's first
+// entry by bisection, the other lanes step forward from there. Every lane of the warp calls it.
+__device__ __forceinline__ int point_of(const int64_t* __restrict__ ptr, int g0, int g1, int64_t e, int64_t e_end) {
+  int lo = g0;
+  if ((threadIdx.x & 31) == 0) {
+    const int64_t ef = e < e_end ? e : e_end - 1;
+    int hi = g1;                       // ptr[lo] <= ef < ptr[hi]
+    while (hi - lo > 1) {
+      const int mid = lo + (hi - lo) / 2;
+      if (__ldg(ptr + mid) <= ef) lo = mid; else hi = mid;
+    }
+  }
+  int g = __shfl_sync(0xffffffffu, lo, 0);
+  if (e < e_end)
+    while (__ldg(ptr + g + 1) <= e) ++g;
+  return g;
+}
+
+// Normalised distances s of the neighbour lists, with explicitly rounded operations (bitwise the
+// FRNN's own). One entry per thread: the square root and the division, about 30 FP64 operations, on
+// full warps; inside the FRNN's candidate loop a third of the lanes had work (300,000 points:
+// 1.15 ms of its 1.79 ms). Sets built in mixed precision, whose RKPM does not read s, get it when a
+// caller downloads it.
 __global__ void distance_kernel(int n_gp, const double* __restrict__ gp_xy, const double* __restrict__ node_xy,
                                 const double* __restrict__ rho_node, double rho, const int64_t* __restrict__ ptr,
-                                const int32_t* __restrict__ idx, double* __restrict__ out_s) {
+                                const int32_t* __restrict__ idx, int64_t nnz, double* __restrict__ out_s) {
+  const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int g = point_of(ptr, 0, n_gp, e, nnz);
+  if (e >= nnz) return;
+  const int j = idx[e];
+  const double ddx = __dsub_rn(node_xy[2 * j], gp_xy[2 * g]);
+  const double ddy = __dsub_rn(node_xy[2 * j + 1], gp_xy[2 * g + 1]);
+  const double dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
+  out_s[e] = __ddiv_rn(__dsqrt_rn(dist2), rho_node ? rho_node[j] : rho);
+}
+
+// The reference's guards over the points: out = {singular points, first of them, collapsed
+// pivots, first of them}, preset to {0, n, 0, n}.
+__global__ void guard_kernel(int n, const int8_t* __restrict__ bad, int* __restrict__ out) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_gp) return;
-  const double gx = gp_xy[2 * g], gy = gp_xy[2 * g + 1];
-  for (int64_t e = ptr[g]; e < ptr[g + 1]; ++e) {
-    const int j = idx[e];
-    const double ddx = __dsub_rn(node_xy[2 * j], gx);
-    const double ddy = __dsub_rn(node_xy[2 * j + 1], gy);
-    const double dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
-    const double r = rho_node ? rho_node[j] : rho;
-    out_s[e] = __ddiv_rn(__dsqrt_rn(dist2), r);
-  }
+  const int b = g < n ? bad[g] : 0;
+  if (b != 1 && b != 2) return;
+  atomicAdd(out + 2 * (b - 1), 1);
+  atomicMin(out + 2 * (b - 1) + 1, g);
 }
 
 // Neighbour counts -> CSR offsets on the device: ptr[g + 1] = sum of cnt[0..g], plus the
@@ -191,103 +213,6 @@ __global__ void gp_indicator_kernel(int n_gp, const double* __restrict__ gp_xy, 
   o[0] = I.f; o[1] = I.gx; o[2] = I.gy; o[3] = I.hxx; o[4] = I.hyy; o[5] = I.hxy;
 }
 
-__device__ __forceinline__ void window(int kernel, double s, double& w, double& dw, double& d2w) {
-  if (kernel == 0) {  // quartic spline, GlobalRKPM.h:15-17
-    if (s >= 1.0) { w = 0.0; } else { const double s2 = s * s; w = 1.0 - 6.0 * s2 + 8.0 * s2 * s - 3.0 * s2 * s2; }
-    dw = (s >= 1.0 || s < 1e-14) ? 0.0 : -12.0 * s + 24.0 * s * s - 12.0 * s * s * s;
-    d2w = (s >= 1.0) ? 0.0 : -12.0 + 48.0 * s - 36.0 * s * s;
-  } else {  // cubic B-spline (extension), same cut-offs
-    if (s >= 1.0) { w = 0.0; dw = 0.0; d2w = 0.0; return; }
-    if (s <= 0.5) {
-      w = 2.0 / 3.0 - 4.0 * s * s + 4.0 * s * s * s;
-      dw = (s < 1e-14) ? 0.0 : -8.0 * s + 12.0 * s * s;
-      d2w = -8.0 + 24.0 * s;
-    } else {
-      const double r = 1.0 - s;
-      w = 4.0 / 3.0 * r * r * r;
-      dw = -4.0 * r * r;
-      d2w = 8.0 * r;
-    }
-  }
-}
-
-struct Jets { double w, x, y, xx, yy, xy; };
-
-// Weight jets with crease visibility for one (Gauss point, neighbour) entry:
-// GlobalRKPM.h:59-84 (including the reference's d2x = xi^2/s^3, d2y = eta^2/s^3) and
-// the visibility product of GlobalRKPM.h:87-112.
-__device__ __forceinline__ Jets weight_jets(int kernel, double xi, double eta, double si, double fac,
-                                            int n_creases, const double* gind,
-                                            const int8_t* node_side, int n_nodes, int j,
-                                            double rho) {
-  const double zx = xi * fac, zy = eta * fac;
-  double wi, d, dd;
-  window(kernel, si, wi, d, dd);
-  const double dx = (si == 0.0) ? 0.0 : zx / si;
-  const double dy = (si == 0.0) ? 0.0 : zy / si;
-  Jets J;
-  J.w = wi;
-  J.x = d * dx;
-  J.y = d * dy;
-  const double si3 = si * si * si;
-  const double d2x = (si == 0.0) ? dd : (zx * zx) / si3;
-  const double d2y = (si == 0.0) ? dd : (zy * zy) / si3;
-  J.xx = dd * dx * dx + d * d2x;
-  J.yy = dd * dy * dy + d * d2y;
-  J.xy = (si == 0.0) ? 0.0 : dd * dx * dy + d * (-(zx * zy) / si3);
-  if (fac != 1.0) {
-    const double f2 = fac * fac;
-    J.x *= fac; J.y *= fac; J.xx *= f2; J.yy *= f2; J.xy *= f2;
-  }
-  for (int c = 0; c < n_creases; ++c) {
-    const double* I = gind + 6 * c;
-    const double sn = static_cast<double>(node_side[static_cast<int64_t>(c) * n_nodes + j]);
-    const double W = 0.5 * (1.0 + sn * I[0]);
-    const double dWx = 0.5 * sn * I[1] * rho, dWy = 0.5 * sn * I[2] * rho;
-    const double ddWxx = 0.5 * sn * I[3] * rho * rho;
-    const double ddWyy = 0.5 * sn * I[4] * rho * rho;
-    const double ddWxy = 0.5 * sn * I[5] * rho * rho;
-    const Jets o = J;
-    J.w = o.w * W;
-    J.x = o.x * W + o.w * dWx;
-    J.y = o.y * W + o.w * dWy;
-    J.xx = o.xx * W + 2.0 * o.x * dWx + o.w * ddWxx;
-    J.yy = o.yy * W + 2.0 * o.y * dWy + o.w * ddWyy;
-    J.xy = o.xy * W + o.x * dWy + o.y * dWx + o.w * ddWxy;
-  }
-  return J;
-}
-
-// Monomial basis jets (GlobalRKPM.h:114-152): degree-major, p_y ascending.
-template <int ORDER>
-struct Basis {
-  static constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  double p[NP], px[NP], py[NP], pxx[NP], pyy[NP], pxy[NP];
-  __device__ __forceinline__ explicit Basis(double x, double y) {
-    double xp[ORDER + 1], yp[ORDER + 1];
-    xp[0] = 1.0; yp[0] = 1.0;
-#pragma unroll
-    for (int q = 1; q <= ORDER; ++q) { xp[q] = xp[q - 1] * x; yp[q] = yp[q - 1] * y; }
-    int idx = 0;
-#pragma unroll
-    for (int d = 0; d <= ORDER; ++d) {
-#pragma unroll
-      for (int qy = 0; qy <= d; ++qy) {
-        const int qx = d - qy;
-        p[idx] = xp[qx] * yp[qy];
-        px[idx] = qx > 0 ? static_cast<double>(qx) * xp[qx > 0 ? qx - 1 : 0] * yp[qy] : 0.0;
-        py[idx] = qy > 0 ? static_cast<double>(qy) * xp[qx] * yp[qy > 0 ? qy - 1 : 0] : 0.0;
-        pxx[idx] = qx > 1 ? static_cast<double>(qx * (qx - 1)) * xp[qx > 1 ? qx - 2 : 0] * yp[qy] : 0.0;
-        pyy[idx] = qy > 1 ? static_cast<double>(qy * (qy - 1)) * xp[qx] * yp[qy > 1 ? qy - 2 : 0] : 0.0;
-        pxy[idx] = (qx > 0 && qy > 0)
-                       ? static_cast<double>(qx * qy) * xp[qx > 0 ? qx - 1 : 0] * yp[qy > 0 ? qy - 1 : 0]
-                       : 0.0;
-        ++idx;
-      }
-    }
-  }
-};
-
 template <int NP>
 struct PackedIdx {
   // K[i][j] of GlobalRKPM.h:29-36, row-major over i <= j.
@@ -352,17 +277,16 @@ struct RowJets {
 //   D_x mu_ab = S^x_ab + a S_{a-1,b},   D_xx mu_ab = S^xx_ab + 2a S^x_{a-1,b} + a(a-1) S_{a-2,b},
 //   D_xy mu_ab = S^xy_ab + b S^x_{a,b-1} + a S^y_{a-1,b} + ab S_{a-1,b-1}   (y alike),
 // with S^g_ab = sum_I (D^g w_I) xi^a eta^b.
-template <int ORDER>
-__device__ __forceinline__ int point_solve(const double* S0, const double* Sx, const double* Sy,
-                                           const double* Sxx, const double* Syy, const double* Sxy,
-                                           RowJets<ORDER>& R) {
+// at(g, a, b): S^g_ab for g = 0 (w), 1 (x), 2 (y), 3 (xx), 4 (yy), 5 (xy).
+template <int ORDER, class Sums>
+__device__ __forceinline__ int point_solve(const Sums& sums, RowJets<ORDER>& R) {
   constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
   constexpr int NM = NP * (NP + 1) / 2;
   using PI = PackedIdx<NP>;
   using RI = RawIdx<ORDER>;
   double M[NM], Mx[NM], My[NM], Mxx[NM], Myy[NM], Mxy[NM];
   {
-    auto at = [](const double* S, int aa, int bb) { return (aa < 0 || bb < 0) ? 0.0 : S[RI::r(aa, bb)]; };
+    auto at = [&](int g, int aa, int bb) { return (aa < 0 || bb < 0) ? 0.0 : sums(g, aa, bb); };
 #pragma unroll
     for (int ip = 0; ip < NP; ++ip) {
 #pragma unroll
@@ -370,12 +294,12 @@ __device__ __forceinline__ int point_solve(const double* S0, const double* Sx, c
         const int k = PI::k(ip, jp);
         const int A = RI::bx(ip) + RI::bx(jp), Bq = RI::by(ip) + RI::by(jp);
         const double fa = static_cast<double>(A), fb = static_cast<double>(Bq);
-        M[k] = at(S0, A, Bq);
-        Mx[k] = at(Sx, A, Bq) + fa * at(S0, A - 1, Bq);
-        My[k] = at(Sy, A, Bq) + fb * at(S0, A, Bq - 1);
-        Mxx[k] = at(Sxx, A, Bq) + 2.0 * fa * at(Sx, A - 1, Bq) + fa * (fa - 1.0) * at(S0, A - 2, Bq);
-        Myy[k] = at(Syy, A, Bq) + 2.0 * fb * at(Sy, A, Bq - 1) + fb * (fb - 1.0) * at(S0, A, Bq - 2);
-        Mxy[k] = at(Sxy, A, Bq) + fb * at(Sx, A, Bq - 1) + fa * at(Sy, A - 1, Bq) + fa * fb * at(S0, A - 1, Bq - 1);
+        M[k] = at(0, A, Bq);
+        Mx[k] = at(1, A, Bq) + fa * at(0, A - 1, Bq);
+        My[k] = at(2, A, Bq) + fb * at(0, A, Bq - 1);
+        Mxx[k] = at(3, A, Bq) + 2.0 * fa * at(1, A - 1, Bq) + fa * (fa - 1.0) * at(0, A - 2, Bq);
+        Myy[k] = at(4, A, Bq) + 2.0 * fb * at(2, A, Bq - 1) + fb * (fb - 1.0) * at(0, A, Bq - 2);
+        Mxy[k] = at(5, A, Bq) + fb * at(1, A, Bq - 1) + fa * at(2, A - 1, Bq) + fa * fb * at(0, A - 1, Bq - 1);
       }
     }
   }
@@ -490,90 +414,281 @@ struct RkpmArgs {
   double* dpsi;
   double* ddpsi;
   int8_t* bad;
+  double ir;           // FP64 kernels: 1 / rho
+  const double* fac;   // rho / rho_I per node, or null (single radius)
+  int8_t* tip;         // point in the cap of a crease end (its indicators vary there)
+  double* mom;         // moment sums, [sum][point of the chunk]
+  double* coef;        // shape polynomials, 6 NP per point of the chunk
+  int g0, g1;          // the launch's points
 };
 
-// One Gauss point per thread: GlobalRKPM.h:59-397 for that point.
+// ---- FP64 RKPM -------------------------------------------------------------------------
+//
+// With xi, eta the scaled differences, the six weight jets of a neighbour are w, A xi, A eta, B xi^2,
+// B eta^2 and C xi eta with three radial factors (GlobalRKPM.h:59-84 with its d2x, d2y;
+// f = rho / rho_I):
+//   A = f^2 w'/s,   B = f^4 (w'' + w'/s) / s^2,   C = f^4 (w'' - w'/s) / s^2.
+// Where no crease end caps the point, a crease only scales them (by 0 or 1), and the raw sums of the
+// jets are sums of w, A, B and C against monomials:
+//   S_ab = W(a, b),  S^x_ab = A(a+1, b),  S^y_ab = A(a, b+1),  S^xx_ab = B(a+2, b),
+//   S^yy_ab = B(a, b+2),  S^xy_ab = C(a+1, b+1):
+// 15 + 20 + 24 + 15 sums for the quadratic basis where the six jets take 90, and one division per
+// neighbour. In the cap of a crease end the visibility factors vary with the point
+// (GlobalRKPM.h:87-112) and mix the jets: those points sum the six jets as they come.
+// GB300's FP64 pipe (2 FMA per cycle and SM) bounds all of it, so
+//  - rkpm_moment_kernel takes the sums over a point's neighbours (about 130 FP64 operations each, 150
+//    in a cap) and leaves the pair's w, A, B, C (or its six jets) in the output arrays;
+//  - rkpm_solve_kernel, one point per thread, factors M (point_solve) and leaves the six polynomials
+//    in xi, eta that multiply the jets, derivatives of the basis and powers of rho folded in;
+//  - rkpm_value_kernel, one pair per thread, evaluates them (about 60 operations) over the pair's
+//    jets: reading them back is a tenth of computing them again.
+// Measured on 300,000 points (28 neighbours, quadratic): RKPM 10.7 ms as one kernel of 90 sums and
+// both passes, about 650 operations per neighbour; 3.7 ms so (moments 2.4, solve 0.5, values 0.85).
+// 32,400 points with 113 neighbours, cubic, half of them in a cap: 12.8 -> 3.5 ms.
 template <int ORDER>
-__global__ void __launch_bounds__(kThreads) rkpm_kernel(RkpmArgs a) {
-  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= a.n_gp) return;
-  const int64_t p0 = a.ptr[g], p1 = a.ptr[g + 1];
-  const double gx = a.gp_xy[2 * g], gy = a.gp_xy[2 * g + 1];
-  // The point's crease indicators: a local copy for up to 4 creases, read in place beyond.
-  double gloc[6 * 4];
-  const int nc = a.n_creases;
-  const double* gind = a.gind + static_cast<int64_t>(g) * 6 * nc;
-  if (nc <= 4) {
-    for (int c = 0; c < 6 * nc; ++c) gloc[c] = gind[c];
-    gind = gloc;
+struct MomIdx {
+  static constexpr int D = 2 * ORDER;
+  static constexpr int tri(int d) { return (d + 1) * (d + 2) / 2; }   // monomials of degree <= d
+  static constexpr int NW = tri(D), NA = tri(D + 1) - 1, NB = tri(D + 2) - 4, NC = NW;
+  static constexpr int N = NW + NA + NB + NC;
+  __host__ __device__ static constexpr int r(int a, int b) { return (a + b) * (a + b + 1) / 2 + b; }
+  // Positions in [W | A | B | C]; A starts at degree 1, B at degree 2 without xi eta.
+  __host__ __device__ static constexpr int w(int a, int b) { return r(a, b); }
+  __host__ __device__ static constexpr int ax(int a, int b) { return NW + r(a, b) - 1; }
+  __host__ __device__ static constexpr int bx(int a, int b) {
+    return NW + NA + (r(a, b) == 3 ? 0 : r(a, b) == 5 ? 1 : r(a, b) - 4);
   }
+  __host__ __device__ static constexpr int cx(int a, int b) { return NW + NA + NB + r(a - 1, b - 1); }
+};
 
-  // Raw-moment sums S^g_ab of the six weight jets (see point_solve). Accumulating the
-  // 6 x NR sums per neighbour (90 FMA for ORDER 2) replaces the 6 x NM jets of p_i p_j
-  // (about 6x the FP64 work); M and its jets are formed once per point.
+__global__ void node_fac_kernel(int n_nodes, const double* __restrict__ rho_node, double rho, double* __restrict__ fac) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n_nodes) fac[j] = rho / rho_node[j];
+}
+
+// Radial factors of a neighbour at normalised distance s: w, A, B, C without f.
+__device__ __forceinline__ void radial(int kernel, double s, double& w, double& A, double& B, double& C) {
+  double ds, dd;   // w'/s, w''
+  const double is2 = s == 0.0 ? 0.0 : 1.0 / (s * s);
+  if (kernel == 0) {  // quartic spline, GlobalRKPM.h:15-17
+    w = fma(s * s, fma(s, fma(-3.0, s, 8.0), -6.0), 1.0);
+    ds = fma(s, fma(-12.0, s, 24.0), -12.0);
+    dd = fma(s, fma(-36.0, s, 48.0), -12.0);
+  } else if (s <= 0.5) {  // cubic B-spline (extension)
+    w = fma(s * s, fma(4.0, s, -4.0), 2.0 / 3.0);
+    ds = fma(12.0, s, -8.0);
+    dd = fma(24.0, s, -8.0);
+  } else {
+    const double r = 1.0 - s;
+    w = 4.0 / 3.0 * (r * r * r);
+    ds = -4.0 * (r * r) * (s * is2);
+    dd = 8.0 * r;
+  }
+  if (s >= 1.0) { w = 0.0; ds = 0.0; dd = 0.0; }
+  if (s < 1e-14) ds = 0.0;
+  A = ds;
+  B = (dd + ds) * is2;
+  C = (dd - ds) * is2;
+}
+
+// The sums of one point's neighbours (L lanes share them). PART 0: all; the cubic basis's 132 (168 in
+// a cap) do not fit the registers, so PART 1 takes W and A (the jets w, x, y) and PART 2 B and C (xx,
+// yy, xy). TIP: the points in the cap of a crease end; the others otherwise.
+template <int ORDER, int PART, int L, bool TIP>
+__device__ __forceinline__ void moment_sums(const RkpmArgs& a) {
+  using MI = MomIdx<ORDER>;
   using RI = RawIdx<ORDER>;
-  constexpr int NR = RI::NR;
-  double S0[NR], Sx[NR], Sy[NR], Sxx[NR], Syy[NR], Sxy[NR];
+  constexpr bool P1 = PART != 2, P2 = PART != 1;
+  constexpr int J0 = P1 ? 0 : 3, J1 = P2 ? 6 : 3;   // the jets of a cap's sums
+  constexpr int LO = TIP ? J0 * RI::NR : P1 ? 0 : MI::NW + MI::NA;
+  constexpr int HI = TIP ? J1 * RI::NR : P2 ? MI::N : MI::NW + MI::NA;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = a.g0 + t / L, sub = t % L;
+  const bool here = g < a.g1;
+  const int gc = here ? g : a.g1 - 1;
+  const int nc = a.n_creases;
+  const double* gind = a.gind + static_cast<int64_t>(gc) * 6 * nc;
+  bool tip = false;
+  for (int c = 0; c < nc; ++c)
+    for (int q = 1; q < 6; ++q) tip = tip || gind[6 * c + q] != 0.0;
+  const bool mine = here && tip == TIP;
+  if (!__any_sync(0xffffffffu, mine)) return;
+  if (P1 && mine && sub == 0) a.tip[g] = TIP;
+  const int64_t p0 = a.ptr[gc];
+  const int n = mine ? static_cast<int>(a.ptr[gc + 1] - p0) : 0;
+  const double gx = a.gp_xy[2 * gc], gy = a.gp_xy[2 * gc + 1];
+  double S[HI - LO];
 #pragma unroll
-  for (int k = 0; k < NR; ++k) { S0[k] = 0; Sx[k] = 0; Sy[k] = 0; Sxx[k] = 0; Syy[k] = 0; Sxy[k] = 0; }
-  for (int64_t e = p0; e < p1; ++e) {
+  for (int k = 0; k < HI - LO; ++k) S[k] = 0.0;
+  for (int q = sub; q < n; q += L) {
+    const int64_t e = p0 + q;
     const int j = a.idx[e];
-    const double xi = (gx - a.node_xy[2 * j]) / a.rho;
-    const double eta = (gy - a.node_xy[2 * j + 1]) / a.rho;
-    const double fac = a.rho_node ? a.rho / a.rho_node[j] : 1.0;
-    const Jets J = weight_jets(a.kernel, xi, eta, a.s[e], fac, nc, gind, a.node_side, a.n_nodes, j, a.rho);
-    double xp[RI::D + 1], yp[RI::D + 1];
-    xp[0] = 1.0; yp[0] = 1.0;
+    const double xi = (gx - a.node_xy[2 * j]) * a.ir, eta = (gy - a.node_xy[2 * j + 1]) * a.ir;
+    double w, A, B, C;
+    radial(a.kernel, a.s[e], w, A, B, C);
+    if (a.fac) {
+      const double f = a.fac[j], f2 = f * f, f4 = f2 * f2;
+      A *= f2; B *= f4; C *= f4;
+    }
+    C *= xi * eta;   // the xy jet, and C(a+1, b+1) = sum (C xi eta) xi^a eta^b
+    double J[6];
+    if constexpr (TIP) {
+      J[0] = w; J[1] = A * xi; J[2] = A * eta;
+      J[3] = B * (xi * xi); J[4] = B * (eta * eta); J[5] = C;
+      for (int c = 0; c < nc; ++c) {   // GlobalRKPM.h:87-112
+        const double* I = gind + 6 * c;
+        const double sn = a.node_side[static_cast<int64_t>(c) * a.n_nodes + j] > 0 ? 0.5 : -0.5;
+        const double sr = sn * a.rho, srr = sr * a.rho;
+        const double V = fma(sn, I[0], 0.5), Vx = sr * I[1], Vy = sr * I[2];
+        const double o0 = J[0], o1 = J[1], o2 = J[2];
+        J[0] = o0 * V;
+        J[1] = fma(o1, V, o0 * Vx);
+        J[2] = fma(o2, V, o0 * Vy);
+        J[3] = fma(J[3], V, fma(2.0 * o1, Vx, o0 * (srr * I[3])));
+        J[4] = fma(J[4], V, fma(2.0 * o2, Vy, o0 * (srr * I[4])));
+        J[5] = fma(J[5], V, fma(o1, Vy, fma(o2, Vx, o0 * (srr * I[5]))));
+      }
+      if (P1) { a.psi[e] = J[0]; a.dpsi[2 * e] = J[1]; a.dpsi[2 * e + 1] = J[2]; }
+      if (P2) { a.ddpsi[3 * e] = J[3]; a.ddpsi[3 * e + 1] = J[4]; a.ddpsi[3 * e + 2] = J[5]; }
+    } else {
+      double vis = 1.0;
+      for (int c = 0; c < nc; ++c) {
+        const double f = gind[6 * c];
+        vis *= 0.5 * (1.0 + (a.node_side[static_cast<int64_t>(c) * a.n_nodes + j] > 0 ? f : -f));
+      }
+      if (vis != 1.0) { w *= vis; A *= vis; B *= vis; C *= vis; }
+      if (P1) { a.psi[e] = w; a.dpsi[2 * e] = A; }
+      if (P2) { a.ddpsi[3 * e] = B; a.ddpsi[3 * e + 2] = C; }
+    }
+    // Monomials degree by degree, each from one of the degree before.
+    double m[MI::D + 3];
+    m[0] = 1.0;
 #pragma unroll
-    for (int q = 1; q <= RI::D; ++q) { xp[q] = xp[q - 1] * xi; yp[q] = yp[q - 1] * eta; }
+    for (int d = 0; d <= MI::D + (TIP ? 0 : P2 ? 2 : 1); ++d) {
+      if (d > 0) {
+        m[d] = m[d - 1] * eta;
 #pragma unroll
-    for (int d = 0; d <= RI::D; ++d) {
+        for (int b = d - 1; b >= 0; --b) m[b] *= xi;
+      }
 #pragma unroll
       for (int b = 0; b <= d; ++b) {
-        const int k = RI::r(d - b, b);
-        const double m = xp[d - b] * yp[b];
-        S0[k] += J.w * m; Sx[k] += J.x * m; Sy[k] += J.y * m;
-        Sxx[k] += J.xx * m; Syy[k] += J.yy * m; Sxy[k] += J.xy * m;
+        auto add = [&](int k, double v) { S[k - LO] = fma(v, m[b], S[k - LO]); };
+        if constexpr (TIP) {
+#pragma unroll
+          for (int k = J0; k < J1; ++k) add(k * RI::NR + RI::r(d - b, b), J[k]);
+        } else {
+          if (P1 && d <= MI::D) add(MI::w(d - b, b), w);
+          if (P1 && d >= 1 && d <= MI::D + 1) add(MI::ax(d - b, b), A);
+          if (P2 && d >= 2 && !(d == 2 && b == 1)) add(MI::bx(d - b, b), B);
+          if (P2 && d <= MI::D) add(MI::cx(d - b + 1, b + 1), C);
+        }
       }
     }
   }
-  RowJets<ORDER> R;
-  a.bad[g] = static_cast<int8_t>(point_solve<ORDER>(S0, Sx, Sy, Sxx, Syy, Sxy, R));
-  const double(&c0)[NP] = R.c0;
-  const double(&c0x)[NP] = R.c0x;
-  const double(&c0y)[NP] = R.c0y;
-  const double(&c0xx)[NP] = R.c0xx;
-  const double(&c0yy)[NP] = R.c0yy;
-  const double(&c0xy)[NP] = R.c0xy;
-  // Shape functions (GlobalRKPM.h:363-396).
-  const double rho2 = a.rho * a.rho;
-  for (int64_t e = p0; e < p1; ++e) {
-    const int j = a.idx[e];
-    const double xi = (gx - a.node_xy[2 * j]) / a.rho;
-    const double eta = (gy - a.node_xy[2 * j + 1]) / a.rho;
-    const double fac = a.rho_node ? a.rho / a.rho_node[j] : 1.0;
-    const Jets J = weight_jets(a.kernel, xi, eta, a.s[e], fac, nc, gind, a.node_side, a.n_nodes, j, a.rho);
-    const Basis<ORDER> B(xi, eta);
-    double C = 0.0, Cx = 0.0, Cy = 0.0, Cxx = 0.0, Cyy = 0.0, Cxy = 0.0;
 #pragma unroll
-    for (int jp = 0; jp < NP; ++jp) {
-      C += c0[jp] * B.p[jp];
-      Cx += c0x[jp] * B.p[jp] + c0[jp] * B.px[jp];
-      Cy += c0y[jp] * B.p[jp] + c0[jp] * B.py[jp];
-      Cxx += c0xx[jp] * B.p[jp] + 2.0 * c0x[jp] * B.px[jp] + c0[jp] * B.pxx[jp];
-      Cyy += c0yy[jp] * B.p[jp] + 2.0 * c0y[jp] * B.py[jp] + c0[jp] * B.pyy[jp];
-      Cxy += c0xy[jp] * B.p[jp] + c0x[jp] * B.py[jp] + c0y[jp] * B.px[jp] + c0[jp] * B.pxy[jp];
-    }
-    a.psi[e] = C * J.w;
-    a.dpsi[2 * e] = (Cx * J.w + C * J.x) / a.rho;
-    a.dpsi[2 * e + 1] = (Cy * J.w + C * J.y) / a.rho;
-    a.ddpsi[3 * e] = (Cxx * J.w + 2.0 * Cx * J.x + C * J.xx) / rho2;
-    a.ddpsi[3 * e + 1] = (Cyy * J.w + 2.0 * Cy * J.y + C * J.yy) / rho2;
-    a.ddpsi[3 * e + 2] = (Cxy * J.w + Cx * J.y + Cy * J.x + C * J.xy) / rho2;
+  for (int o = L / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < HI - LO; ++k) S[k] += __shfl_xor_sync(0xffffffffu, S[k], o);
+  if (mine && sub == 0) {
+    const int64_t np = a.g1 - a.g0;
+#pragma unroll
+    for (int k = 0; k < HI - LO; ++k) a.mom[(LO + k) * np + (g - a.g0)] = S[k];
   }
 }
 
+// blockIdx.y: the part (cubic basis), then the kind of points (only launched with creases).
+template <int ORDER, int L>
+__global__ void __launch_bounds__(64) rkpm_moment_kernel(RkpmArgs a) {
+  if constexpr (ORDER < 3) {
+    if (blockIdx.y == 0) moment_sums<ORDER, 0, L, false>(a);
+    else moment_sums<ORDER, 0, L, true>(a);
+  } else {
+    switch (blockIdx.y) {
+      case 0: moment_sums<ORDER, 1, L, false>(a); break;
+      case 1: moment_sums<ORDER, 2, L, false>(a); break;
+      case 2: moment_sums<ORDER, 1, L, true>(a); break;
+      default: moment_sums<ORDER, 2, L, true>(a); break;
+    }
+  }
+}
+
+template <int ORDER>
+__global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
+  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
+  using MI = MomIdx<ORDER>;
+  using RI = RawIdx<ORDER>;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, g = a.g0 + t;
+  if (g >= a.g1) return;
+  const bool tip = a.tip[g];
+  const int64_t np = a.g1 - a.g0;
+  const double* mom = a.mom + t;
+  RowJets<ORDER> R;
+  a.bad[g] = static_cast<int8_t>(point_solve<ORDER>([&](int q, int aa, int bb) {
+    const int k = q == 0 ? MI::w(aa, bb) : q == 1 ? MI::ax(aa + 1, bb) : q == 2 ? MI::ax(aa, bb + 1)
+                : q == 3 ? MI::bx(aa + 2, bb) : q == 4 ? MI::bx(aa, bb + 2) : MI::cx(aa + 1, bb + 1);
+    return mom[(tip ? q * RI::NR + RI::r(aa, bb) : k) * np];
+  }, R));
+  // The polynomials C, C_x / rho, C_y / rho, C_xx / rho^2, C_yy / rho^2, C_xy / rho^2 of
+  // GlobalRKPM.h:363-396: with b = row 0 of M^-1, C = b . p, C_x = b_x . p + b . p_x and so on,
+  // the derivatives of the monomials moved onto the coefficients.
+  double* o = a.coef + static_cast<int64_t>(t) * 6 * NP;
+  const double r1 = a.ir, r2 = a.ir * a.ir;
+  auto co = [&](const double* c, int i, int p, int q) -> double {   // c of xi^(bx+p) eta^(by+q), times its derivative's factor
+    const int x = RI::bx(i) + p, y = RI::by(i) + q;
+    if (x + y > ORDER) return 0.0;
+    double v = c[RI::r(x, y)];
+    for (int k = 0; k < p; ++k) v *= static_cast<double>(x - k);
+    for (int k = 0; k < q; ++k) v *= static_cast<double>(y - k);
+    return v;
+  };
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    o[i] = R.c0[i];
+    o[NP + i] = r1 * (R.c0x[i] + co(R.c0, i, 1, 0));
+    o[2 * NP + i] = r1 * (R.c0y[i] + co(R.c0, i, 0, 1));
+    o[3 * NP + i] = r2 * (R.c0xx[i] + 2.0 * co(R.c0x, i, 1, 0) + co(R.c0, i, 2, 0));
+    o[4 * NP + i] = r2 * (R.c0yy[i] + 2.0 * co(R.c0y, i, 0, 1) + co(R.c0, i, 0, 2));
+    o[5 * NP + i] = r2 * (R.c0xy[i] + co(R.c0y, i, 1, 0) + co(R.c0x, i, 0, 1) + co(R.c0, i, 1, 1));
+  }
+}
+
+constexpr int kValueThreads = 256;
+
+template <int ORDER>
+__global__ void __launch_bounds__(kValueThreads) rkpm_value_kernel(RkpmArgs a) {
+  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
+  using RI = RawIdx<ORDER>;
+  const int64_t e0 = a.ptr[a.g0], e1 = a.ptr[a.g1];
+  const int64_t e = e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + threadIdx.x;
+  if (e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + (threadIdx.x & ~31) >= e1) return;   // the whole warp
+  const int g = point_of(a.ptr, a.g0, a.g1, e, e1);
+  if (e >= e1) return;
+  const int j = a.idx[e];
+  const double x = (a.gp_xy[2 * g] - a.node_xy[2 * j]) * a.ir, y = (a.gp_xy[2 * g + 1] - a.node_xy[2 * j + 1]) * a.ir;
+  const double w = a.psi[e], r2 = a.ir * a.ir;
+  double Jx = a.dpsi[2 * e], Jy = a.dpsi[2 * e + 1], Jxx = a.ddpsi[3 * e], Jyy = a.ddpsi[3 * e + 1], Jxy = a.ddpsi[3 * e + 2];
+  if (!a.tip[g]) { Jy = Jx * y; Jx *= x; Jyy = Jxx * (y * y); Jxx *= x * x; }
+  const double* c = a.coef + static_cast<int64_t>(g - a.g0) * 6 * NP;
+  double m[NP];
+  m[0] = 1.0;
+#pragma unroll
+  for (int i = 1; i < NP; ++i) m[i] = RI::by(i) == 0 ? m[RI::r(RI::bx(i) - 1, 0)] * x : m[RI::r(RI::bx(i), RI::by(i) - 1)] * y;
+  double v[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    v[k] = __ldg(c + k * NP);
+#pragma unroll
+    for (int i = 1; i < NP; ++i) v[k] = fma(__ldg(c + k * NP + i), m[i], v[k]);
+  }
+  const double C2 = v[0] * r2;
+  Jx *= a.ir; Jy *= a.ir;
+  a.psi[e] = v[0] * w;
+  a.dpsi[2 * e] = fma(v[1], w, v[0] * Jx);
+  a.dpsi[2 * e + 1] = fma(v[2], w, v[0] * Jy);
+  a.ddpsi[3 * e] = fma(v[3], w, fma(2.0 * v[1], Jx, C2 * Jxx));
+  a.ddpsi[3 * e + 1] = fma(v[4], w, fma(2.0 * v[2], Jy, C2 * Jyy));
+  a.ddpsi[3 * e + 2] = fma(v[5], w, fma(v[1], Jy, fma(v[2], Jx, C2 * Jxy)));
+}
 
 // ---- mixed precision: the per-neighbour work in FP32 pairs ----------------------------
 //
@@ -847,7 +962,7 @@ __global__ void __launch_bounds__(kThreads, kPairMinBlocks) rkpm_pair_point_kern
     pair_moment_sums<ORDER, 3, 3>(a, P, p0, p1, Sd);
   }
   RowJets<ORDER> R;
-  a.bad[g] = static_cast<int8_t>(point_solve<ORDER>(Sd[0], Sd[1], Sd[2], Sd[3], Sd[4], Sd[5], R));
+  a.bad[g] = static_cast<int8_t>(point_solve<ORDER>([&](int q, int aa, int bb) { return Sd[q][RI::r(aa, bb)]; }, R));
   out[0] = P.gx0; out[1] = P.gx1; out[2] = P.gx2;
   out[3] = P.gy0; out[4] = P.gy1; out[5] = P.gy2;
   float2* cj = reinterpret_cast<float2*>(out + 6 + 12 * P.nc);
@@ -930,6 +1045,42 @@ __global__ void __launch_bounds__(kPairValueThreads) rkpm_pair_value_kernel(Rkpm
 }
 
 inline unsigned blocks_for(int64_t n, int t = kThreads) { return static_cast<unsigned>((n + t - 1) / t); }
+
+// The FP64 RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
+// sums and polynomials of 262,144 points: 260 MB for the quadratic basis, 480 MB for the cubic).
+// Lanes per point of the moment kernel: more while its warps do not fill the SM quarters twice
+// (adding a lane pair's sums costs as many operations as half a neighbour's).
+template <int ORDER>
+void rkpm_fp64(cgb_context* ctx, cgb_shape* out, RkpmArgs ra) {
+  constexpr int kChunk = 1 << 18, NP = (ORDER + 1) * (ORDER + 2) / 2;
+  cudaStream_t st = ctx->stream;
+  const int n_gp = out->n_gp, most = std::min(n_gp, kChunk);
+  constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
+  out->scr_mom.ensure(static_cast<size_t>(most) * kSums);
+  out->scr_coef.ensure(static_cast<size_t>(most) * 6 * NP);
+  ra.mom = out->scr_mom.p;
+  ra.coef = out->scr_coef.p;
+  int sms = 0;
+  CGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  for (int g0 = 0; g0 < n_gp; g0 += kChunk) {
+    ra.g0 = g0;
+    ra.g1 = std::min(n_gp, g0 + kChunk);
+    const int np = ra.g1 - g0;
+    const int64_t full = 2LL * 4 * 32 * sms;   // lanes of two warps per SM quarter
+    auto moments = [&](auto lanes) {
+      constexpr int L = decltype(lanes)::value;
+      const dim3 grid(blocks_for(static_cast<int64_t>(np) * L, 64), (ORDER < 3 ? 1 : 2) * (ra.n_creases > 0 ? 2 : 1));
+      rkpm_moment_kernel<ORDER, L><<<grid, 64, 0, st>>>(ra);
+    };
+    if (np * 8LL <= full) moments(std::integral_constant<int, 8>{});
+    else if (np * 2LL <= full) moments(std::integral_constant<int, 2>{});
+    else moments(std::integral_constant<int, 1>{});
+    rkpm_solve_kernel<ORDER><<<blocks_for(np, 64), 64, 0, st>>>(ra);
+    const int64_t pairs = std::min(out->nnz, static_cast<int64_t>(np) * out->max_n);
+    if (pairs > 0) rkpm_value_kernel<ORDER><<<blocks_for(pairs, kValueThreads), kValueThreads, 0, st>>>(ra);
+  }
+  CGB_CUDA(cudaGetLastError());
+}
 
 }  // namespace
 
@@ -1038,7 +1189,7 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   if (n_gp > 0)
     frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p,
                                                         d_rn, prm.rho, rho2, G, pre,
-                                                        nullptr, d_cnt.p, nullptr, nullptr);
+                                                        nullptr, d_cnt.p, nullptr);
   CGB_CUDA(cudaGetLastError());
   prof_end(ctx, CGB_PHASE_FRNN, n_gp > 0 ? 1 : 0);
   // CSR offsets on the device; only the total and the largest count come back.
@@ -1063,17 +1214,18 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   out->max_n = static_cast<int>(totals[1]);
   out->nbr_idx.alloc(nnz);
   // The mixed RKPM recomputes distances in FP32 pairs and does not read s, so a mixed set
-  // skips the FRNN's rounded square roots and divisions; cgb_shape_download computes s on
-  // demand (shape_distances), bitwise equal.
+  // leaves s out; cgb_shape_download computes it on demand (shape_distances), bitwise equal.
   const bool want_s = prm.precision != CGB_SHAPE_MIXED;
   if (want_s) out->s.alloc(nnz); else out->s.reset();
   prof_begin(ctx, CGB_PHASE_FRNN);
   if (n_gp > 0)
     frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p,
                                                         d_rn, prm.rho, rho2, G, pre,
-                                                        out->nbr_ptr.p, nullptr, out->nbr_idx.p,
-                                                        want_s ? out->s.p : nullptr);
-  prof_end(ctx, CGB_PHASE_FRNN, n_gp > 0 ? 1 : 0);
+                                                        out->nbr_ptr.p, nullptr, out->nbr_idx.p);
+  if (want_s && nnz > 0)
+    distance_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p, d_rn, prm.rho,
+                                                          out->nbr_ptr.p, out->nbr_idx.p, nnz, out->s.p);
+  prof_end(ctx, CGB_PHASE_FRNN, (n_gp > 0 ? 1 : 0) + (want_s && nnz > 0 ? 1 : 0));
   CGB_CUDA(cudaGetLastError());
 
   out->rebuildable = true;
@@ -1132,7 +1284,8 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   };
   RkpmArgs ra{n_gp, n_nodes, out->kernel, nc, out->rho, nullptr, pair_of(1.0 / out->rho),
               pair_of(1.0 / (out->rho * out->rho)), out->gp_xy.p, ctx->node_xy.p, d_rn, out->nbr_ptr.p,
-              out->nbr_idx.p, out->s.p, gind, side, out->psi.p, out->dpsi.p, out->ddpsi.p, bad};
+              out->nbr_idx.p, out->s.p, gind, side, out->psi.p, out->dpsi.p, out->ddpsi.p, bad,
+              0.0, nullptr, nullptr, nullptr, nullptr, 0, n_gp};
   prof_begin(ctx, CGB_PHASE_RKPM);
   if (mixed && n_nodes > 0) {
     out->scr_node_pair.ensure(2 * static_cast<size_t>(n_nodes));
@@ -1161,25 +1314,33 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
           break;
       }
     } else {
+      if (d_rn) {
+        out->scr_fac.ensure(n_nodes);
+        node_fac_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, d_rn, out->rho, out->scr_fac.p);
+        ra.fac = out->scr_fac.p;
+      }
+      out->scr_tip.ensure(n_gp);
+      ra.ir = 1.0 / out->rho;
+      ra.tip = out->scr_tip.p;
       switch (out->order) {
-        case 1: rkpm_kernel<1><<<blocks_for(n_gp), kThreads, 0, st>>>(ra); break;
-        case 2: rkpm_kernel<2><<<blocks_for(n_gp), kThreads, 0, st>>>(ra); break;
-        default: rkpm_kernel<3><<<blocks_for(n_gp), kThreads, 0, st>>>(ra); break;
+        case 1: rkpm_fp64<1>(ctx, out, ra); break;
+        case 2: rkpm_fp64<2>(ctx, out, ra); break;
+        default: rkpm_fp64<3>(ctx, out, ra); break;
       }
     }
   }
   prof_end(ctx, CGB_PHASE_RKPM, (n_gp > 0 ? 1 : 0) + (mixed && n_nodes > 0 ? 1 : 0) + (mixed && nnz > 0 ? 1 : 0));
   CGB_CUDA(cudaGetLastError());
-  std::vector<int8_t> hbad(n_gp);
-  if (n_gp > 0) CGB_CUDA(cudaMemcpyAsync(hbad.data(), bad, n_gp, cudaMemcpyDeviceToHost, st));
-  CGB_CUDA(cudaStreamSynchronize(st));
   // The reference's guards (GlobalRKPM.h:241-257 after the 3x3 block, 347-359 after
   // the bordering): singular first, then pivot collapse.
-  size_t n1 = 0, f1 = 0, n2 = 0, f2 = 0;
-  for (int g = 0; g < n_gp; ++g) {
-    if (hbad[g] == 1) { if (!n1) f1 = g; ++n1; }
-    if (hbad[g] == 2) { if (!n2) f2 = g; ++n2; }
-  }
+  int found[4] = {0, n_gp, 0, n_gp};
+  out->scr_guard.ensure(4);
+  CGB_CUDA(cudaMemcpyAsync(out->scr_guard.p, found, sizeof(found), cudaMemcpyHostToDevice, st));
+  if (n_gp > 0) guard_kernel<<<blocks_for(n_gp, 256), 256, 0, st>>>(n_gp, bad, out->scr_guard.p);
+  CGB_CUDA(cudaGetLastError());
+  CGB_CUDA(cudaMemcpyAsync(found, out->scr_guard.p, sizeof(found), cudaMemcpyDeviceToHost, st));
+  CGB_CUDA(cudaStreamSynchronize(st));
+  const int n1 = found[0], f1 = found[1], n2 = found[2], f2 = found[3];
   auto count_of = [&](size_t g) {
     int64_t pr[2];
     CGB_CUDA(cudaMemcpy(pr, out->nbr_ptr.p + g, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost));
@@ -1213,9 +1374,9 @@ void shape_distances(cgb_shape* sh) {
     throw Error(CGB_ERR_INVALID, "cgb_shape_download: s is computed on demand for mixed-precision sets and the "
                                  "nodes changed since the set was built (cgb_set_nodes)");
   sh->s.alloc(sh->nnz);
-  distance_kernel<<<blocks_for(sh->n_gp), kThreads, 0, ctx->stream>>>(
+  distance_kernel<<<blocks_for(sh->nnz, 256), 256, 0, ctx->stream>>>(
       sh->n_gp, sh->gp_xy.p, ctx->node_xy.p, sh->has_rho_node ? sh->rho_node.p : nullptr, sh->rho, sh->nbr_ptr.p,
-      sh->nbr_idx.p, sh->s.p);
+      sh->nbr_idx.p, sh->nnz, sh->s.p);
   CGB_CUDA(cudaGetLastError());
 }
 
