@@ -173,25 +173,37 @@ __device__ __forceinline__ void point_state(const double s[15], const Material& 
   P.pXY[1] = P.Ci[2] * fa + P.Ci[3] * fb;
 }
 
-// Kinematic sums over the neighbours, lane-strided, reduced across the warp.
-__device__ __forceinline__ void kin_sums(int lane, int64_t p0, int n, const int32_t* idx, const double* dpsi,
-                                         const double* ddpsi, const double* x, double s[15]) {
+// Kinematic sums of one point over its neighbours, the next neighbour's loads in flight while the
+// current one is summed; each(entry, u) sees every neighbour's displacement.
+template <class Each>
+__device__ __forceinline__ void point_sums(int64_t e0, int64_t e1, const int32_t* __restrict__ idx,
+                                           const double* __restrict__ dpsi, const double* __restrict__ ddpsi,
+                                           const double* __restrict__ x, double s[15], Each&& each) {
 #pragma unroll
   for (int k = 0; k < 15; ++k) s[k] = 0.0;
-  for (int a = lane; a < n; a += 32) {
-    const int64_t e = p0 + a;
-    const int64_t j = idx[e];
-    const double u0 = x[3 * j], u1 = x[3 * j + 1], u2 = x[3 * j + 2];
-    const double2 d = reinterpret_cast<const double2*>(dpsi)[e];
-    const double dxx = ddpsi[3 * e], dyy = ddpsi[3 * e + 1], dxy = ddpsi[3 * e + 2];
-    s[0] += u0 * d.x; s[1] += u1 * d.x; s[2] += u2 * d.x;
-    s[3] += u0 * d.y; s[4] += u1 * d.y; s[5] += u2 * d.y;
-    s[6] += u0 * dxx; s[7] += u1 * dxx; s[8] += u2 * dxx;
-    s[9] += u0 * dyy; s[10] += u1 * dyy; s[11] += u2 * dyy;
-    s[12] += u0 * dxy; s[13] += u1 * dxy; s[14] += u2 * dxy;
+  struct Nb { double u0, u1, u2, dx, dy, dxx, dyy, dxy; };
+  auto load = [&](int64_t e, int64_t j) {
+    Nb v{};
+    if (e < e1) {
+      const double2 d = reinterpret_cast<const double2*>(dpsi)[e];
+      v = Nb{x[3 * j], x[3 * j + 1], x[3 * j + 2], d.x, d.y, ddpsi[3 * e], ddpsi[3 * e + 1], ddpsi[3 * e + 2]};
+    }
+    return v;
+  };
+  auto node = [&](int64_t e) -> int64_t { return e < e1 ? idx[e] : 0; };
+  Nb A = load(e0, node(e0));
+  int64_t j = node(e0 + 1);
+  for (int64_t e = e0; e < e1; ++e) {
+    const Nb B = load(e + 1, j);
+    j = node(e + 2);
+    each(e, A.u0, A.u1, A.u2);
+    s[0] += A.u0 * A.dx; s[1] += A.u1 * A.dx; s[2] += A.u2 * A.dx;
+    s[3] += A.u0 * A.dy; s[4] += A.u1 * A.dy; s[5] += A.u2 * A.dy;
+    s[6] += A.u0 * A.dxx; s[7] += A.u1 * A.dxx; s[8] += A.u2 * A.dxx;
+    s[9] += A.u0 * A.dyy; s[10] += A.u1 * A.dyy; s[11] += A.u2 * A.dyy;
+    s[12] += A.u0 * A.dxy; s[13] += A.u1 * A.dxy; s[14] += A.u2 * A.dxy;
+    A = B;
   }
-#pragma unroll
-  for (int k = 0; k < 15; ++k) s[k] = warp_sum(s[k]);
 }
 
 // Scatter of one block into the accumulators. v is row-major in the local (I, J)
@@ -941,27 +953,30 @@ __global__ void det_reduce_F(int n_nodes, const int64_t* __restrict__ lptr, cons
 }
 
 // ---- energies -----------------------------------------------------------------------
-__global__ void __launch_bounds__(128) face_energy_kernel(int n_gp, const int64_t* ptr, const int32_t* idx,
-                                                          const double* dpsi, const double* ddpsi,
-                                                          const double* weight, const double* x, Material m,
-                                                          NatCurv nc, const double* gp_xy, double* out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+// One point per thread: the point's own part (about 150 FP64 operations) on all lanes of a warp
+// with work of their own. A warp per point had issued it, and 75 additions of the lanes' sums, for
+// one point at a time: 57,600 points 560 us.
+__global__ void __launch_bounds__(128) face_energy_kernel(int n_gp, const int64_t* __restrict__ ptr,
+                                                          const int32_t* __restrict__ idx,
+                                                          const double* __restrict__ dpsi,
+                                                          const double* __restrict__ ddpsi,
+                                                          const double* __restrict__ weight,
+                                                          const double* __restrict__ x, Material m,
+                                                          NatCurv nc, const double* __restrict__ gp_xy, double* out) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
   double em = 0.0, eb = 0.0;
-  for (int64_t g = warp; g < n_gp; g += nw) {
-    const int64_t p0 = ptr[g];
-    const int n = static_cast<int>(ptr[g + 1] - p0);
+  if (g < n_gp) {
     double s[15];
-    kin_sums(lane, p0, n, idx, dpsi, ddpsi, x, s);
+    point_sums(ptr[g], ptr[g + 1], idx, dpsi, ddpsi, x, s, [](int64_t, double, double, double) {});
     PointState P;
-    point_state(s, m, P, gp_xy ? natcurv_kappa(nc, gp_xy[2 * g]) : 0.0);
-    if (lane == 0) {   // Meshless.h:204-220, with E1_el (Meshless.h:212)
-      em += 0.5 * weight[g] * (P.e0[0] * P.N[0] + P.e0[1] * P.N[1] + P.e0[2] * P.N[2]);
-      eb += 0.5 * weight[g] * (P.e1el[0] * P.M[0] + P.e1el[1] * P.M[1] + P.e1el[2] * P.M[2]);
-    }
+    point_state(s, m, P, gp_xy ? natcurv_kappa(nc, gp_xy[2 * static_cast<int64_t>(g)]) : 0.0);
+    // Meshless.h:204-220, with E1_el (Meshless.h:212)
+    em = 0.5 * weight[g] * (P.e0[0] * P.N[0] + P.e0[1] * P.N[1] + P.e0[2] * P.N[2]);
+    eb = 0.5 * weight[g] * (P.e1el[0] * P.M[0] + P.e1el[1] * P.M[1] + P.e1el[2] * P.M[2]);
   }
-  if (lane == 0) { atomicAdd(out, em); atomicAdd(out + 1, eb); }
+  em = warp_sum(em);
+  eb = warp_sum(eb);
+  if ((threadIdx.x & 31) == 0) { atomicAdd(out, em); atomicAdd(out + 1, eb); }
 }
 
 // ---- kinematic state of arbitrary points (post-processing) ---------------------------
@@ -981,19 +996,10 @@ __global__ void __launch_bounds__(128) point_state_kernel(int n, const int64_t* 
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n) return;
   double s[15], u[3] = {0.0, 0.0, 0.0};
-  for (int k = 0; k < 15; ++k) s[k] = 0.0;
-  for (int64_t e = ptr[g]; e < ptr[g + 1]; ++e) {
-    const int64_t j = idx[e];
-    const double u0 = x[3 * j], u1 = x[3 * j + 1], u2 = x[3 * j + 2];
-    const double p = psi[e], dx = dpsi[2 * e], dy = dpsi[2 * e + 1];
-    const double dxx = ddpsi[3 * e], dyy = ddpsi[3 * e + 1], dxy = ddpsi[3 * e + 2];
+  point_sums(ptr[g], ptr[g + 1], idx, dpsi, ddpsi, x, s, [&](int64_t e, double u0, double u1, double u2) {
+    const double p = psi[e];
     u[0] += p * u0; u[1] += p * u1; u[2] += p * u2;
-    s[0] += u0 * dx; s[1] += u1 * dx; s[2] += u2 * dx;
-    s[3] += u0 * dy; s[4] += u1 * dy; s[5] += u2 * dy;
-    s[6] += u0 * dxx; s[7] += u1 * dxx; s[8] += u2 * dxx;
-    s[9] += u0 * dyy; s[10] += u1 * dyy; s[11] += u2 * dyy;
-    s[12] += u0 * dxy; s[13] += u1 * dxy; s[14] += u2 * dxy;
-  }
+  });
   PointState P;
   point_state(s, m, P, gp_xy ? natcurv_kappa(nc, gp_xy[2 * static_cast<int64_t>(g)]) : 0.0);
   double* o = out + static_cast<int64_t>(g) * kPointStateCols;
@@ -1008,23 +1014,35 @@ __global__ void __launch_bounds__(128) point_state_kernel(int n, const int64_t* 
   o[24] = P.e1[0]; o[25] = P.e1[1]; o[26] = 0.5 * P.e1[2];
 }
 
-__global__ void hinge_energy_kernel(HingeArgs a, double* out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= a.n_gp) return;
-  if (a.active && a.active[g] == 0) return;
-  double F12[12] = {1, 0, 0, 0, 1, 0, 1, 0, 0, 0, 1, 0};
-  for (int64_t e = a.lptr[g]; e < a.lptr[g + 1]; ++e) {
-    const int64_t j = a.lidx[e];
-    for (int c = 0; c < 3; ++c) { F12[c] += a.x[3 * j + c] * a.ldpsi[2 * e]; F12[3 + c] += a.x[3 * j + c] * a.ldpsi[2 * e + 1]; }
+// One warp per crease point, the neighbours dealt to its lanes.
+__global__ void __launch_bounds__(128) hinge_energy_kernel(HingeArgs a, double* out) {
+  const int lane = threadIdx.x & 31;
+  const int g = static_cast<int>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5);
+  if (g >= a.n_gp || (a.active && a.active[g] == 0)) return;
+  double F12[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    const int64_t* ptr = side ? a.rptr : a.lptr;
+    const int32_t* idx = side ? a.ridx : a.lidx;
+    const double* d = side ? a.rdpsi : a.ldpsi;
+    for (int64_t e = ptr[g] + lane; e < ptr[g + 1]; e += 32) {
+      const int64_t j = idx[e];
+      const double dX = d[2 * e], dY = d[2 * e + 1];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double u = a.x[3 * j + c];
+        F12[6 * side + c] += u * dX;
+        F12[6 * side + 3 + c] += u * dY;
+      }
+    }
   }
-  for (int64_t e = a.rptr[g]; e < a.rptr[g + 1]; ++e) {
-    const int64_t j = a.ridx[e];
-    for (int c = 0; c < 3; ++c) { F12[6 + c] += a.x[3 * j + c] * a.rdpsi[2 * e]; F12[9 + c] += a.x[3 * j + c] * a.rdpsi[2 * e + 1]; }
-  }
+#pragma unroll
+  for (int k = 0; k < 12; ++k) F12[k] = warp_sum(F12[k]);
+  F12[0] += 1.0; F12[4] += 1.0; F12[6] += 1.0; F12[10] += 1.0;
   const double theta = fold_angle(F12, a.tangent[2 * g], a.tangent[2 * g + 1], nullptr);
   const double th0 = a.theta0_gp ? a.theta0_gp[g] : a.theta0;
   const double d = theta - th0;
-  atomicAdd(out, a.weight[g] * (0.5 * a.Kt * (d * d)));
+  if (lane == 0) atomicAdd(out, a.weight[g] * (0.5 * a.Kt * (d * d)));
 }
 
 // ---- bulk-copy (TMA) staging --------------------------------------------------------
@@ -1609,7 +1627,7 @@ void point_state_device(cgb_context* ctx, const cgb_shape* S, const double* d_x,
     throw Error(CGB_ERR_INVALID, "point state: the shape set has no Psi");
   const Material m = make_material(A, B, D);
   const double* xy = natcurv_points(ctx, S, "point state");
-  point_state_kernel<<<nb(S->n_gp, 128), 128, 0, ctx->stream>>>(S->n_gp, S->nbr_ptr.p, S->nbr_idx.p, S->psi.p,
+  point_state_kernel<<<nb(S->n_gp, 64), 64, 0, ctx->stream>>>(S->n_gp, S->nbr_ptr.p, S->nbr_idx.p, S->psi.p,
                                                                 S->dpsi.p, S->ddpsi.p, d_x, m, ctx->natcurv, xy,
                                                                 d_out);
   CGB_CUDA(cudaGetLastError());
@@ -1623,13 +1641,13 @@ void energies_device(cgb_assembler* a, const double* d_x, double* out3) {
   const Material m = make_material(a->A, a->B, a->D);
   const cgb_shape* S = a->faces;
   if (S->n_gp)
-    face_energy_kernel<<<std::max(1u, std::min(nb(S->n_gp, 4), static_cast<unsigned>(sm_count(ctx->device) * 32))), 128, 0, st>>>(
+    face_energy_kernel<<<nb(S->n_gp, 64), 64, 0, st>>>(
         S->n_gp, S->nbr_ptr.p, S->nbr_idx.p, S->dpsi.p, S->ddpsi.p, a->weight.p, d_x, m, ctx->natcurv,
         natcurv_points(ctx, S, "energies"), a->energy.p);
   for (auto& f : a->folds) {
     if (!f.n_gp) continue;
     HingeArgs h = hinge_args(a, f, d_x, 0);
-    hinge_energy_kernel<<<nb(f.n_gp, 128), 128, 0, st>>>(h, a->energy.p + 2);
+    hinge_energy_kernel<<<nb(f.n_gp, 4), 128, 0, st>>>(h, a->energy.p + 2);
   }
   CGB_CUDA(cudaGetLastError());
   CGB_CUDA(cudaMemcpyAsync(out3, a->energy.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));

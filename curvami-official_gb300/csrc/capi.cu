@@ -176,6 +176,8 @@ void ctx_release(cgb_context* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   ctx->node_xy.reset();
   ctx->dev_err.reset();
+  ctx->ws_x.reset();
+  ctx->ws_out.reset();
   for (auto& m : ctx->marks) {
     if (m.start) cudaEventDestroy(m.start);
     if (m.stop) cudaEventDestroy(m.stop);
@@ -657,7 +659,10 @@ int cgb_point_state(cgb_context* ctx, const cgb_shape* pts, const double* x, con
     cudaStream_t st = ctx->stream;
     const size_t nx = 3 * static_cast<size_t>(ctx->n_nodes);
     const size_t no = static_cast<size_t>(pts->n_gp) * CGB_POINT_STATE_COLS;
-    cgb::DevBuf<double> dx(nx), dout(std::max<size_t>(no, 1));
+    // Workspaces of the context, kept between the calls of one step's point sets.
+    cgb::DevBuf<double>&dx = ctx->ws_x, &dout = ctx->ws_out;
+    dx.ensure(nx);
+    dout.ensure(std::max<size_t>(no, 1));
     CGB_CUDA(cudaMemcpyAsync(dx.p, x, nx * sizeof(double), cudaMemcpyHostToDevice, st));
     cgb::point_state_device(ctx, pts, dx.p, A, B, D, dout.p);
     if (no) CGB_CUDA(cudaMemcpyAsync(out, dout.p, no * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -102,6 +102,7 @@ struct cgb_context {
   // Device-side error word written by kernels (bounds checks, capacity).
   cgb::DevBuf<int> dev_err;
   int* h_err = nullptr;  // pinned mirror
+  cgb::DevBuf<double> ws_x, ws_out;  // device copies of cgb_point_state's x and rows
   // Tracing: event pairs per phase, summed when read.
   bool profile = false;
   struct Mark { int phase; cudaEvent_t start, stop; int launches; cudaStream_t stream; };
