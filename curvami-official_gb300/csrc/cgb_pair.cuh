@@ -23,6 +23,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace cgb {
 
 struct fp2 {
@@ -54,9 +56,16 @@ __device__ __forceinline__ fp2 fp2_from_double(double d) {
   return {hi, __double2float_rn(d - static_cast<double>(hi))};
 }
 
-__device__ __forceinline__ double fp2_to_double(fp2 a) {
-  return static_cast<double>(a.hi) + static_cast<double>(a.lo);
+// A float as a double, on the integer pipe: a conversion issues on the FP64 pipe, at 1/62 of the
+// rate. The exponent is rebiased from 127 to 1023; denormals, infinities and NaN convert.
+__device__ __forceinline__ double fp2_widen(float f) {
+  const uint32_t u = __float_as_uint(f), e = u & 0x7f800000u;
+  if (e == 0x7f800000u || (e == 0u && (u << 1) != 0u)) return static_cast<double>(f);
+  const uint32_t hi = (u & 0x80000000u) | (e == 0u ? 0u : ((u & 0x7fffffffu) >> 3) + 0x38000000u);
+  return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
 }
+
+__device__ __forceinline__ double fp2_to_double(fp2 a) { return fp2_widen(a.hi) + fp2_widen(a.lo); }
 
 __device__ __forceinline__ fp2 operator-(fp2 a) { return {-a.hi, -a.lo}; }
 

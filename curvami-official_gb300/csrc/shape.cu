@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(64) rkpm_moment_kernel(RkpmArgs a) {
   }
 }
 
-template <int ORDER>
+template <int ORDER, bool PAIR>
 __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
   constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
   using MI = MomIdx<ORDER>;
@@ -631,7 +631,14 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
   // The polynomials C, C_x / rho, C_y / rho, C_xx / rho^2, C_yy / rho^2, C_xy / rho^2 of
   // GlobalRKPM.h:363-396: with b = row 0 of M^-1, C = b . p, C_x = b_x . p + b . p_x and so on,
   // the derivatives of the monomials moved onto the coefficients.
-  double* o = a.coef + static_cast<int64_t>(t) * 6 * NP;
+  auto put = [&](int i, double v) {   // PAIR: as FP32 pairs, in the same 8 bytes
+    if constexpr (PAIR) {
+      const fp2 p = fp2_from_double(v);
+      reinterpret_cast<float2*>(a.coef)[static_cast<int64_t>(t) * 6 * NP + i] = make_float2(p.hi, p.lo);
+    } else {
+      a.coef[static_cast<int64_t>(t) * 6 * NP + i] = v;
+    }
+  };
   const double r1 = a.ir, r2 = a.ir * a.ir;
   auto co = [&](const double* c, int i, int p, int q) -> double {   // c of xi^(bx+p) eta^(by+q), times its derivative's factor
     const int x = RI::bx(i) + p, y = RI::by(i) + q;
@@ -643,12 +650,12 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
   };
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
-    o[i] = R.c0[i];
-    o[NP + i] = r1 * (R.c0x[i] + co(R.c0, i, 1, 0));
-    o[2 * NP + i] = r1 * (R.c0y[i] + co(R.c0, i, 0, 1));
-    o[3 * NP + i] = r2 * (R.c0xx[i] + 2.0 * co(R.c0x, i, 1, 0) + co(R.c0, i, 2, 0));
-    o[4 * NP + i] = r2 * (R.c0yy[i] + 2.0 * co(R.c0y, i, 0, 1) + co(R.c0, i, 0, 2));
-    o[5 * NP + i] = r2 * (R.c0xy[i] + co(R.c0y, i, 1, 0) + co(R.c0x, i, 0, 1) + co(R.c0, i, 1, 1));
+    put(i, R.c0[i]);
+    put(NP + i, r1 * (R.c0x[i] + co(R.c0, i, 1, 0)));
+    put(2 * NP + i, r1 * (R.c0y[i] + co(R.c0, i, 0, 1)));
+    put(3 * NP + i, r2 * (R.c0xx[i] + 2.0 * co(R.c0x, i, 1, 0) + co(R.c0, i, 2, 0)));
+    put(4 * NP + i, r2 * (R.c0yy[i] + 2.0 * co(R.c0y, i, 0, 1) + co(R.c0, i, 0, 2)));
+    put(5 * NP + i, r2 * (R.c0xy[i] + co(R.c0y, i, 1, 0) + co(R.c0x, i, 0, 1) + co(R.c0, i, 1, 1)));
   }
 }
 
@@ -740,322 +747,290 @@ constexpr float kTwoThirdsLo = static_cast<float>(2.0 / 3.0 - static_cast<double
 constexpr float kFourThirdsHi = static_cast<float>(4.0 / 3.0);
 constexpr float kFourThirdsLo = static_cast<float>(4.0 / 3.0 - static_cast<double>(kFourThirdsHi));
 
-// window() in pairs, same branches and cut-offs, polynomials in Horner form.
-__device__ __forceinline__ void window_pair(int kernel, fp2 s, fp2& w, fp2& dw, fp2& d2w) {
+// radial() in pairs, same branches and cut-offs; z2 = s^2 of the scaled differences.
+__device__ __forceinline__ void radial_pair(int kernel, fp2 z2, fp2& w, fp2& A, fp2& B, fp2& C) {
   const fp2 z{0.0f, 0.0f};
-  if (fp2_ge(s, 1.0f)) { w = z; dw = z; d2w = z; return; }
-  const bool tiny = s.hi < 1e-14f;
+  const fp2 s = fp2_sqrt(z2);
+  if (fp2_ge(s, 1.0f)) { w = z; A = z; B = z; C = z; return; }
+  const bool at_node = fp2_is_zero(s);
+  const fp2 is2 = at_node ? z : fp2_recip(z2);
+  fp2 ds, dd;
   if (kernel == 0) {  // 1 - 6 s^2 + 8 s^3 - 3 s^4
-    const fp2 s2 = fp2_sqr(s);
-    w = 1.0f + s2 * (-6.0f + s * (8.0f - 3.0f * s));
-    dw = tiny ? z : s * (-12.0f + s * (24.0f - 12.0f * s));
-    d2w = -12.0f + s * (48.0f - 36.0f * s);
+    w = 1.0f + z2 * (-6.0f + s * (8.0f - 3.0f * s));
+    ds = -12.0f + s * (24.0f - 12.0f * s);
+    dd = -12.0f + s * (48.0f - 36.0f * s);
   } else if (fp2_le(s, 0.5f)) {  // 2/3 - 4 s^2 + 4 s^3
-    const fp2 s2 = fp2_sqr(s);
-    w = fp2{kTwoThirdsHi, kTwoThirdsLo} + s2 * (-4.0f + 4.0f * s);
-    dw = tiny ? z : s * (-8.0f + 12.0f * s);
-    d2w = -8.0f + 24.0f * s;
+    w = fp2{kTwoThirdsHi, kTwoThirdsLo} + z2 * (-4.0f + 4.0f * s);
+    ds = -8.0f + 12.0f * s;
+    dd = -8.0f + 24.0f * s;
   } else {  // 4/3 (1 - s)^3
     const fp2 r = 1.0f - s;
     const fp2 r2 = fp2_sqr(r);
     w = fp2{kFourThirdsHi, kFourThirdsLo} * (r2 * r);
-    dw = -4.0f * r2;
-    d2w = 8.0f * r;
+    ds = -4.0f * (r2 * (s * is2));
+    dd = 8.0f * r;
   }
+  if (s.hi < 1e-14f) ds = z;
+  A = ds;
+  B = (dd + ds) * is2;
+  C = (dd - ds) * is2;
 }
 
-// weight_jets() in pairs: jets v = {w, x, y, xx, yy, xy}. gc holds per crease
-// 0.5 I_f, 0.5 I_gx rho, 0.5 I_gy rho, 0.5 I_hxx rho^2, 0.5 I_hyy rho^2, 0.5 I_hxy rho^2.
-struct JetsP {
-  fp2 v[6];
-};
-__device__ __forceinline__ JetsP weight_jets_pair(int kernel, fp2 xi, fp2 eta, fp2 fac, bool scaled, int nc,
-                                                  const fp2* gc, const int8_t* __restrict__ node_side,
-                                                  int n_nodes, int j) {
-  const fp2 zx = scaled ? xi * fac : xi, zy = scaled ? eta * fac : eta;
-  const fp2 si = fp2_sqrt(fp2_sqr(zx) + fp2_sqr(zy));
-  fp2 wi, d, dd;
-  window_pair(kernel, si, wi, d, dd);
-  JetsP J;
-  J.v[0] = wi;
-  if (fp2_is_zero(si)) {  // s == 0: dx = dy = 0, d2x = d2y = d2w, no cross term
-    const fp2 z{0.0f, 0.0f};
-    J.v[1] = z; J.v[2] = z;
-    J.v[3] = d * dd; J.v[4] = d * dd; J.v[5] = z;
-  } else {
-    const fp2 is = fp2_recip(si);
-    const fp2 dx = zx * is, dy = zy * is;
-    const fp2 is3 = fp2_sqr(is) * is;
-    J.v[1] = d * dx;
-    J.v[2] = d * dy;
-    J.v[3] = dd * fp2_sqr(dx) + d * (fp2_sqr(zx) * is3);  // the reference's d2x = xi^2 / s^3
-    J.v[4] = dd * fp2_sqr(dy) + d * (fp2_sqr(zy) * is3);  // and d2y = eta^2 / s^3
-    J.v[5] = dd * (dx * dy) - d * ((zx * zy) * is3);
-  }
-  if (scaled) {
-    const fp2 f2 = fp2_sqr(fac);
-    J.v[1] = J.v[1] * fac; J.v[2] = J.v[2] * fac;
-    J.v[3] = J.v[3] * f2; J.v[4] = J.v[4] * f2; J.v[5] = J.v[5] * f2;
-  }
-  for (int c = 0; c < nc; ++c) {
-    const fp2* G = gc + 6 * c;
-    const float sn = node_side[static_cast<int64_t>(c) * n_nodes + j] > 0 ? 1.0f : -1.0f;
-    const fp2 W = G[0] * sn + 0.5f;
-    const fp2 dWx = G[1] * sn, dWy = G[2] * sn;
-    const fp2 ddWxx = G[3] * sn, ddWyy = G[4] * sn, ddWxy = G[5] * sn;
-    const JetsP o = J;
-    J.v[0] = o.v[0] * W;
-    J.v[1] = o.v[1] * W + o.v[0] * dWx;
-    J.v[2] = o.v[2] * W + o.v[0] * dWy;
-    J.v[3] = o.v[3] * W + 2.0f * (o.v[1] * dWx) + o.v[0] * ddWxx;
-    J.v[4] = o.v[4] * W + 2.0f * (o.v[2] * dWy) + o.v[0] * ddWyy;
-    J.v[5] = o.v[5] * W + o.v[1] * dWy + o.v[2] * dWx + o.v[0] * ddWxy;
-  }
-  return J;
-}
+// Point records of the mixed kernels: the coordinates split in three floats each (two float4), then
+// per crease the six indicators scaled for the visibility product, as pairs: 0.5 I_f, 0.5 I_gx rho,
+// 0.5 I_gy rho, 0.5 I_hxx rho^2, 0.5 I_hyy rho^2, 0.5 I_hxy rho^2. They are made once per point: the
+// splits and roundings of doubles issue on the FP64 pipe.
+__host__ __device__ constexpr int pair_record_floats(int n_creases) { return 8 + 12 * n_creases; }
 
-// Monomial basis jets in pairs (Basis<ORDER> above).
-template <int ORDER>
-struct BasisPair {
-  static constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  fp2 p[NP], px[NP], py[NP], pxx[NP], pyy[NP], pxy[NP];
-  __device__ __forceinline__ static fp2 mono(const fp2* xp, const fp2* yp, int a, int b) {
-    return a == 0 ? yp[b] : (b == 0 ? xp[a] : xp[a] * yp[b]);
-  }
-  __device__ __forceinline__ explicit BasisPair(fp2 x, fp2 y) {
-    fp2 xp[ORDER + 1], yp[ORDER + 1];
-    xp[0] = fp2{1.0f, 0.0f}; yp[0] = fp2{1.0f, 0.0f};
-#pragma unroll
-    for (int q = 1; q <= ORDER; ++q) { xp[q] = q == 1 ? x : xp[q - 1] * x; yp[q] = q == 1 ? y : yp[q - 1] * y; }
-    const fp2 z{0.0f, 0.0f};
-    int idx = 0;
-#pragma unroll
-    for (int d = 0; d <= ORDER; ++d) {
-#pragma unroll
-      for (int qy = 0; qy <= d; ++qy) {
-        const int qx = d - qy;
-        p[idx] = mono(xp, yp, qx, qy);
-        px[idx] = qx > 0 ? static_cast<float>(qx) * mono(xp, yp, qx - 1, qy) : z;
-        py[idx] = qy > 0 ? static_cast<float>(qy) * mono(xp, yp, qx, qy - 1) : z;
-        pxx[idx] = qx > 1 ? static_cast<float>(qx * (qx - 1)) * mono(xp, yp, qx - 2, qy) : z;
-        pyy[idx] = qy > 1 ? static_cast<float>(qy * (qy - 1)) * mono(xp, yp, qx, qy - 2) : z;
-        pxy[idx] = (qx > 0 && qy > 0) ? static_cast<float>(qx * qy) * mono(xp, yp, qx - 1, qy - 1) : z;
-        ++idx;
-      }
-    }
-  }
-};
-
-// Per-point inputs of the pair passes.
-struct PairPoint {
-  float gx0, gx1, gx2, gy0, gy1, gy2;
-  int nc;
-  bool scaled;
-  fp2 gc[6 * 4];    // scaled crease indicators, up to 4 creases
-  const fp2* gcp;   // gc, or the point record's copy when there are more creases
-};
-
-__device__ __forceinline__ void pair_xi(const RkpmArgs& a, const PairPoint& P, int j, fp2& xi, fp2& eta, fp2& fac) {
-  const float4 n0 = __ldg(a.node_pair + 2 * j), n1 = __ldg(a.node_pair + 2 * j + 1);
-  xi = diff3(P.gx0, P.gx1, P.gx2, n0.x, n0.y, n0.z) * a.irho;
-  eta = diff3(P.gy0, P.gy1, P.gy2, n0.w, n1.x, n1.y) * a.irho;
-  fac = fp2{n1.z, n1.w};
-}
-
-// Raw-moment sums of weight jets J0 .. J0 + NJ - 1 over the point's neighbours, in pairs
-// (Dot2 accumulation), rounded to FP64 into Sd[J0 + jj][k].
-template <int ORDER, int J0, int NJ>
-__device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const PairPoint& P, int64_t p0, int64_t p1,
-                                                 double (&Sd)[6][RawIdx<ORDER>::NR]) {
-  using RI = RawIdx<ORDER>;
-  constexpr int NR = RI::NR;
-  fp2 S[NJ][NR];
-#pragma unroll
-  for (int q = 0; q < NJ; ++q)
-#pragma unroll
-    for (int k = 0; k < NR; ++k) S[q][k] = fp2{0.0f, 0.0f};
-  for (int64_t e = p0; e < p1; ++e) {
-    const int j = a.idx[e];
-    fp2 xi, eta, fac;
-    pair_xi(a, P, j, xi, eta, fac);
-    const JetsP J = weight_jets_pair(a.kernel, xi, eta, fac, P.scaled, P.nc, P.gcp, a.node_side, a.n_nodes, j);
-    fp2 xp[RI::D + 1], yp[RI::D + 1];
-    xp[0] = fp2{1.0f, 0.0f}; yp[0] = fp2{1.0f, 0.0f};
-#pragma unroll
-    for (int q = 1; q <= RI::D; ++q) { xp[q] = q == 1 ? xi : xp[q - 1] * xi; yp[q] = q == 1 ? eta : yp[q - 1] * eta; }
-#pragma unroll
-    for (int d = 0; d <= RI::D; ++d) {
-#pragma unroll
-      for (int b = 0; b <= d; ++b) {
-        const int k = RI::r(d - b, b);
-        const fp2 m = BasisPair<ORDER>::mono(xp, yp, d - b, b);
-#pragma unroll
-        for (int q = 0; q < NJ; ++q) fp2_fma_acc(S[q][k], J.v[J0 + q], m);
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < NJ; ++q)
-#pragma unroll
-    for (int k = 0; k < NR; ++k) Sd[J0 + q][k] = fp2_to_double(S[q][k]);
-}
-
-// The mixed RKPM runs as two kernels:
-//  - rkpm_pair_point_kernel, one Gauss point per thread: the raw-moment sums in pairs over
-//    the point's neighbours, the per-point FP64 solve, and a point record for the second
-//    kernel (the point's coordinates split in three floats, its crease indicators scaled
-//    for the visibility product, and row 0 of M^-1 with its five jets, all as pairs);
-//  - rkpm_pair_value_kernel, one (point, neighbour) pair per thread: the weight and basis
-//    jets of that neighbour and Phi, grad Phi, Hessian Phi from the point record.
-// Split this way the per-pair half runs at full occupancy instead of inside a thread
-// that holds 90 pair accumulators, and each kernel's code fits the instruction cache.
-//
-// Launch shape of the point kernel, measured on the 1,000,000-point stage (order 2; RKPM
-// phase of both kernels): 2 blocks per SM (255 registers) 8.24 ms, 3 blocks (168 registers,
-// more spills) 8.80 ms; the jets summed in two passes of three (half the accumulators, the
-// weight jets computed twice) 9.4 ms at 3 and 9.2 ms at 4 blocks per SM; before the split,
-// one kernel doing both passes took 11.3 ms. Order 3 (28 raw moments) needs the two passes
-// to keep the accumulators in registers.
-constexpr int kPairMinBlocks = 2;
-constexpr int kPairSplitOrder = 3;
-constexpr int kPairValueThreads = 256;
-
-// Floats per point record: 6 coordinate parts, 12 per crease (6 pairs), 12 per basis
-// function (6 jets x 1 pair), rounded up to 4 so every record starts on 16 bytes.
-__host__ __device__ constexpr int pair_record_floats(int order, int n_creases) {
-  return (6 + 12 * n_creases + 6 * (order + 1) * (order + 2) + 3) & ~3;
-}
-
-template <int ORDER>
-__global__ void __launch_bounds__(kThreads, kPairMinBlocks) rkpm_pair_point_kernel(RkpmArgs a, float* __restrict__ rec,
-                                                                                   int RS) {
-  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  using RI = RawIdx<ORDER>;
+__global__ void point_pair_kernel(RkpmArgs a, float* __restrict__ rec) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.n_gp) return;
-  const int64_t p0 = a.ptr[g], p1 = a.ptr[g + 1];
-  PairPoint P;
-  split3(a.gp_xy[2 * g], P.gx0, P.gx1, P.gx2);
-  split3(a.gp_xy[2 * g + 1], P.gy0, P.gy1, P.gy2);
-  P.nc = a.n_creases;
-  P.scaled = a.rho_node != nullptr;
-  const double r1 = 0.5 * a.rho, r2 = 0.5 * a.rho * a.rho;
-  float* out = rec + static_cast<int64_t>(g) * RS;
-  // The scaled indicators go to the point record first; with more than 4 creases the
-  // moment sums read them back from there (this thread's own writes).
-  for (int c = 0; c < P.nc; ++c) {
+  float x0, x1, x2, y0, y1, y2;
+  split3(a.gp_xy[2 * g], x0, x1, x2);
+  split3(a.gp_xy[2 * g + 1], y0, y1, y2);
+  float* o = rec + static_cast<int64_t>(g) * pair_record_floats(a.n_creases);
+  reinterpret_cast<float4*>(o)[0] = make_float4(x0, x1, x2, y0);
+  reinterpret_cast<float4*>(o)[1] = make_float4(y1, y2, 0.0f, 0.0f);
+  bool tip = false;
+  for (int c = 0; c < a.n_creases; ++c) {
     const double* I = a.gind + (static_cast<int64_t>(g) * a.n_creases + c) * 6;
-    const fp2 v[6] = {fp2_from_double(0.5 * I[0]), fp2_from_double(r1 * I[1]), fp2_from_double(r1 * I[2]),
-                      fp2_from_double(r2 * I[3]), fp2_from_double(r2 * I[4]), fp2_from_double(r2 * I[5])};
+    const double r1 = 0.5 * a.rho, r2 = r1 * a.rho;
     for (int q = 0; q < 6; ++q) {
-      if (c < 4) P.gc[6 * c + q] = v[q];
-      out[6 + 2 * (6 * c + q)] = v[q].hi;
-      out[7 + 2 * (6 * c + q)] = v[q].lo;
+      const fp2 v = fp2_from_double((q == 0 ? 0.5 : q < 3 ? r1 : r2) * I[q]);
+      o[8 + 12 * c + 2 * q] = v.hi;
+      o[9 + 12 * c + 2 * q] = v.lo;
+      tip = tip || (q > 0 && I[q] != 0.0);
     }
   }
-  P.gcp = P.nc <= 4 ? P.gc : reinterpret_cast<const fp2*>(out + 6);
-  double Sd[6][RI::NR];
-  if constexpr (ORDER < kPairSplitOrder) {
-    pair_moment_sums<ORDER, 0, 6>(a, P, p0, p1, Sd);
+  a.tip[g] = tip;
+}
+
+// Scaled differences of a pair from the split coordinates: accurate relative to themselves.
+__device__ __forceinline__ void pair_xi(const RkpmArgs& a, float4 p0, float4 p1, float4 n0, float4 n1, fp2& xi, fp2& eta) {
+  xi = diff3(p0.x, p0.y, p0.z, n0.x, n0.y, n0.z) * a.irho;
+  eta = diff3(p0.w, p1.x, p1.y, n0.w, n1.x, n1.y) * a.irho;
+}
+
+__device__ __forceinline__ float2 as_float2(fp2 v) { return make_float2(v.hi, v.lo); }
+__device__ __forceinline__ fp2 as_fp2(float2 v) { return fp2{v.x, v.y}; }
+
+// The jets of every pair of the chunk, one pair per thread, left in the output arrays as FP32 pairs:
+// w, A, -, B, -, C xi eta, or in a cap the six jets.
+__global__ void __launch_bounds__(kValueThreads) rkpm_pair_jet_kernel(RkpmArgs a, const float* __restrict__ rec) {
+  const int64_t e0 = a.ptr[a.g0], e1 = a.ptr[a.g1];
+  const int64_t e = e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + threadIdx.x;
+  if (e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + (threadIdx.x & ~31) >= e1) return;   // the whole warp
+  const int g = point_of(a.ptr, a.g0, a.g1, e, e1);
+  if (e >= e1) return;
+  const int nc = a.n_creases;
+  const float* R = rec + static_cast<int64_t>(g) * pair_record_floats(nc);
+  const int j = a.idx[e];
+  const float4 n0 = __ldg(a.node_pair + 2 * j), n1 = __ldg(a.node_pair + 2 * j + 1);
+  fp2 xi, eta;
+  pair_xi(a, *reinterpret_cast<const float4*>(R), *reinterpret_cast<const float4*>(R + 4), n0, n1, xi, eta);
+  fp2 z2;
+  const fp2 fac{n1.z, n1.w};
+  const bool scaled = a.rho_node != nullptr;
+  if (scaled) {
+    const fp2 zx = xi * fac, zy = eta * fac;
+    z2 = fp2_sqr(zx) + fp2_sqr(zy);
   } else {
-    pair_moment_sums<ORDER, 0, 3>(a, P, p0, p1, Sd);
-    pair_moment_sums<ORDER, 3, 3>(a, P, p0, p1, Sd);
+    z2 = fp2_sqr(xi) + fp2_sqr(eta);
   }
-  RowJets<ORDER> R;
-  a.bad[g] = static_cast<int8_t>(point_solve<ORDER>([&](int q, int aa, int bb) { return Sd[q][RI::r(aa, bb)]; }, R));
-  out[0] = P.gx0; out[1] = P.gx1; out[2] = P.gx2;
-  out[3] = P.gy0; out[4] = P.gy1; out[5] = P.gy2;
-  float2* cj = reinterpret_cast<float2*>(out + 6 + 12 * P.nc);
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    fp2 v = fp2_from_double(R.c0[i]);   cj[i] = make_float2(v.hi, v.lo);
-    v = fp2_from_double(R.c0x[i]);      cj[NP + i] = make_float2(v.hi, v.lo);
-    v = fp2_from_double(R.c0y[i]);      cj[2 * NP + i] = make_float2(v.hi, v.lo);
-    v = fp2_from_double(R.c0xx[i]);     cj[3 * NP + i] = make_float2(v.hi, v.lo);
-    v = fp2_from_double(R.c0yy[i]);     cj[4 * NP + i] = make_float2(v.hi, v.lo);
-    v = fp2_from_double(R.c0xy[i]);     cj[5 * NP + i] = make_float2(v.hi, v.lo);
+  fp2 w, A, B, C;
+  radial_pair(a.kernel, z2, w, A, B, C);
+  if (scaled) {
+    const fp2 f2 = fp2_sqr(fac), f4 = fp2_sqr(f2);
+    A = A * f2; B = B * f4; C = C * f4;
+  }
+  C = C * (xi * eta);
+  float2* o0 = reinterpret_cast<float2*>(a.psi) + e;
+  float2* o1 = reinterpret_cast<float2*>(a.dpsi) + 2 * e;
+  float2* o2 = reinterpret_cast<float2*>(a.ddpsi) + 3 * e;
+  if (a.tip[g]) {
+    fp2 J[6] = {w, A * xi, A * eta, B * fp2_sqr(xi), B * fp2_sqr(eta), C};
+    for (int c = 0; c < nc; ++c) {   // GlobalRKPM.h:87-112
+      const fp2* G = reinterpret_cast<const fp2*>(R + 8 + 12 * c);
+      const float sn = a.node_side[static_cast<int64_t>(c) * a.n_nodes + j] > 0 ? 1.0f : -1.0f;
+      const fp2 V = G[0] * sn + 0.5f, Vx = G[1] * sn, Vy = G[2] * sn;
+      const fp2 o0j = J[0], o1j = J[1], o2j = J[2];
+      J[0] = o0j * V;
+      J[1] = o1j * V + o0j * Vx;
+      J[2] = o2j * V + o0j * Vy;
+      J[3] = J[3] * V + 2.0f * (o1j * Vx) + o0j * (G[3] * sn);
+      J[4] = J[4] * V + 2.0f * (o2j * Vy) + o0j * (G[4] * sn);
+      J[5] = J[5] * V + o1j * Vy + o2j * Vx + o0j * (G[5] * sn);
+    }
+    o0[0] = as_float2(J[0]); o1[0] = as_float2(J[1]); o1[1] = as_float2(J[2]);
+    o2[0] = as_float2(J[3]); o2[1] = as_float2(J[4]); o2[2] = as_float2(J[5]);
+  } else {
+    float vis = 1.0f;   // exact: the indicator is 1, -1 or (on the crease) 0
+    for (int c = 0; c < nc; ++c) {
+      const float h = R[8 + 12 * c];
+      vis *= 0.5f + (a.node_side[static_cast<int64_t>(c) * a.n_nodes + j] > 0 ? h : -h);
+    }
+    o0[0] = as_float2(w * vis); o1[0] = as_float2(A * vis);
+    o2[0] = as_float2(B * vis); o2[2] = as_float2(C * vis);
   }
 }
 
-// Shape functions (GlobalRKPM.h:363-396) of one (point, neighbour) pair per thread. The
-// point of pair e is the last g with ptr[g] <= e: lane 0 of each warp finds it for the
-// warp's first pair by bisection, the other lanes step forward from there.
-template <int ORDER>
-__global__ void __launch_bounds__(kPairValueThreads) rkpm_pair_value_kernel(RkpmArgs a, const float* __restrict__ rec,
-                                                                            int RS, int64_t nnz) {
-  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  int g0 = 0;
-  if (lane == 0) {
-    const int64_t ef = e < nnz ? e : nnz - 1;
-    int lo = 0, hi = a.n_gp;             // ptr[lo] <= ef < ptr[hi]
-    while (hi - lo > 1) {
-      const int mid = lo + (hi - lo) / 2;
-      if (__ldg(a.ptr + mid) <= ef) lo = mid; else hi = mid;
-    }
-    g0 = lo;
-  }
-  g0 = __shfl_sync(0xffffffffu, g0, 0);
-  if (e >= nnz) return;
-  int g = g0;
-  while (__ldg(a.ptr + g + 1) <= e) ++g;
-  const float* R = rec + static_cast<int64_t>(g) * RS;
-  const int nc = a.n_creases;
-  const fp2* gc = reinterpret_cast<const fp2*>(R + 6);
-  const fp2* cj = reinterpret_cast<const fp2*>(R + 6 + 12 * nc);
-  const int j = a.idx[e];
-  const float4 n0 = __ldg(a.node_pair + 2 * j), n1 = __ldg(a.node_pair + 2 * j + 1);
-  const fp2 xi = diff3(__ldg(R), __ldg(R + 1), __ldg(R + 2), n0.x, n0.y, n0.z) * a.irho;
-  const fp2 eta = diff3(__ldg(R + 3), __ldg(R + 4), __ldg(R + 5), n0.w, n1.x, n1.y) * a.irho;
-  const fp2 fac{n1.z, n1.w};
-  const JetsP J = weight_jets_pair(a.kernel, xi, eta, fac, a.rho_node != nullptr, nc, gc, a.node_side, a.n_nodes, j);
-  const BasisPair<ORDER> B(xi, eta);
-  const fp2 z{0.0f, 0.0f};
-  fp2 C = z, Cx = z, Cy = z, Cxx = z, Cyy = z, Cxy = z;
+// The sums of moment_sums from the pairs' jets, accumulated in pairs (Dot2) and rounded to FP64.
+template <int ORDER, int PART, int L, bool TIP>
+__device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float* __restrict__ rec) {
+  using MI = MomIdx<ORDER>;
+  using RI = RawIdx<ORDER>;
+  constexpr bool P1 = PART == 1;
+  constexpr int LO = TIP ? (P1 ? 0 : 3 * RI::NR) : P1 ? 0 : MI::NW + MI::NA;
+  constexpr int HI = TIP ? (P1 ? 3 * RI::NR : 6 * RI::NR) : P1 ? MI::NW + MI::NA : MI::N;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = a.g0 + t / L, sub = t % L;
+  const bool here = g < a.g1;
+  const int gc = here ? g : a.g1 - 1;
+  const bool mine = here && (a.tip[gc] != 0) == TIP;
+  if (!__any_sync(0xffffffffu, mine)) return;
+  const int64_t p0 = a.ptr[gc];
+  const int n = mine ? static_cast<int>(a.ptr[gc + 1] - p0) : 0;
+  const float* R = rec + static_cast<int64_t>(gc) * pair_record_floats(a.n_creases);
+  const float4 r0 = *reinterpret_cast<const float4*>(R), r1 = *reinterpret_cast<const float4*>(R + 4);
+  const float2* i0 = reinterpret_cast<const float2*>(a.psi);
+  const float2* i1 = reinterpret_cast<const float2*>(a.dpsi);
+  const float2* i2 = reinterpret_cast<const float2*>(a.ddpsi);
+  fp2 S[HI - LO];
 #pragma unroll
-  for (int jp = 0; jp < NP; ++jp) {
-    const fp2 c0 = cj[jp], c0x = cj[NP + jp], c0y = cj[2 * NP + jp];
-    const fp2 c0xx = cj[3 * NP + jp], c0yy = cj[4 * NP + jp], c0xy = cj[5 * NP + jp];
-    const fp2 c0x2 = c0x * 2.0f, c0y2 = c0y * 2.0f;
-    fp2_fma_acc(C, c0, B.p[jp]);
-    fp2_fma_acc(Cx, c0x, B.p[jp]); fp2_fma_acc(Cx, c0, B.px[jp]);
-    fp2_fma_acc(Cy, c0y, B.p[jp]); fp2_fma_acc(Cy, c0, B.py[jp]);
-    fp2_fma_acc(Cxx, c0xx, B.p[jp]); fp2_fma_acc(Cxx, c0x2, B.px[jp]); fp2_fma_acc(Cxx, c0, B.pxx[jp]);
-    fp2_fma_acc(Cyy, c0yy, B.p[jp]); fp2_fma_acc(Cyy, c0y2, B.py[jp]); fp2_fma_acc(Cyy, c0, B.pyy[jp]);
-    fp2_fma_acc(Cxy, c0xy, B.p[jp]); fp2_fma_acc(Cxy, c0x, B.py[jp]);
-    fp2_fma_acc(Cxy, c0y, B.px[jp]); fp2_fma_acc(Cxy, c0, B.pxy[jp]);
+  for (int k = 0; k < HI - LO; ++k) S[k] = fp2{0.0f, 0.0f};
+  for (int q = sub; q < n; q += L) {
+    const int64_t e = p0 + q;
+    const int j = a.idx[e];
+    fp2 xi, eta;
+    pair_xi(a, r0, r1, __ldg(a.node_pair + 2 * j), __ldg(a.node_pair + 2 * j + 1), xi, eta);
+    fp2 J[3];   // w, x, y or xx, yy, xy in a cap; w, A or B, C xi eta otherwise
+    if (P1) { J[0] = as_fp2(i0[e]); J[1] = as_fp2(i1[2 * e]); if (TIP) J[2] = as_fp2(i1[2 * e + 1]); }
+    else { J[0] = as_fp2(i2[3 * e]); J[2] = as_fp2(i2[3 * e + 2]); if (TIP) J[1] = as_fp2(i2[3 * e + 1]); }
+    fp2 m[MI::D + 3];
+    m[0] = fp2{1.0f, 0.0f};
+#pragma unroll
+    for (int d = 0; d <= MI::D + (TIP ? 0 : P1 ? 1 : 2); ++d) {
+      if (d == 1) { m[1] = eta; m[0] = xi; }
+      if (d > 1) {
+        m[d] = m[d - 1] * eta;
+#pragma unroll
+        for (int b = d - 1; b >= 0; --b) m[b] = m[b] * xi;
+      }
+#pragma unroll
+      for (int b = 0; b <= d; ++b) {
+        auto add = [&](int k, fp2 v) { fp2_fma_acc(S[k - LO], v, m[b]); };
+        if constexpr (TIP) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) add((P1 ? k : k + 3) * RI::NR + RI::r(d - b, b), J[k]);
+        } else {
+          if (P1 && d <= MI::D) add(MI::w(d - b, b), J[0]);
+          if (P1 && d >= 1) add(MI::ax(d - b, b), J[1]);
+          if (!P1 && d >= 2 && !(d == 2 && b == 1)) add(MI::bx(d - b, b), J[0]);
+          if (!P1 && d <= MI::D) add(MI::cx(d - b + 1, b + 1), J[2]);
+        }
+      }
+    }
   }
-  C = fp2_norm(C); Cx = fp2_norm(Cx); Cy = fp2_norm(Cy);
-  Cxx = fp2_norm(Cxx); Cyy = fp2_norm(Cyy); Cxy = fp2_norm(Cxy);
-  const fp2* w = J.v;
-  fp2 gx = z, gy = z, hxx = z, hyy = z, hxy = z;
-  fp2_fma_acc(gx, Cx, w[0]); fp2_fma_acc(gx, C, w[1]);
-  fp2_fma_acc(gy, Cy, w[0]); fp2_fma_acc(gy, C, w[2]);
-  const fp2 Cx2 = Cx * 2.0f, Cy2 = Cy * 2.0f;
-  fp2_fma_acc(hxx, Cxx, w[0]); fp2_fma_acc(hxx, Cx2, w[1]); fp2_fma_acc(hxx, C, w[3]);
-  fp2_fma_acc(hyy, Cyy, w[0]); fp2_fma_acc(hyy, Cy2, w[2]); fp2_fma_acc(hyy, C, w[4]);
-  fp2_fma_acc(hxy, Cxy, w[0]); fp2_fma_acc(hxy, Cx, w[2]); fp2_fma_acc(hxy, Cy, w[1]); fp2_fma_acc(hxy, C, w[5]);
-  a.psi[e] = fp2_to_double(C * w[0]);
-  a.dpsi[2 * e] = fp2_to_double(fp2_norm(gx) * a.irho);
-  a.dpsi[2 * e + 1] = fp2_to_double(fp2_norm(gy) * a.irho);
-  a.ddpsi[3 * e] = fp2_to_double(fp2_norm(hxx) * a.irho2);
-  a.ddpsi[3 * e + 1] = fp2_to_double(fp2_norm(hyy) * a.irho2);
-  a.ddpsi[3 * e + 2] = fp2_to_double(fp2_norm(hxy) * a.irho2);
+  const int64_t np = a.g1 - a.g0;
+#pragma unroll
+  for (int k = 0; k < HI - LO; ++k) {
+    double v = fp2_to_double(S[k]);
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (mine && sub == 0) a.mom[(LO + k) * np + (g - a.g0)] = v;
+  }
+}
+
+// blockIdx.y: the part, then the kind of points (only launched with creases).
+template <int ORDER, int L>
+__global__ void __launch_bounds__(64) rkpm_pair_moment_kernel(RkpmArgs a, const float* __restrict__ rec) {
+  switch (blockIdx.y) {
+    case 0: pair_moment_sums<ORDER, 1, L, false>(a, rec); break;
+    case 1: pair_moment_sums<ORDER, 2, L, false>(a, rec); break;
+    case 2: pair_moment_sums<ORDER, 1, L, true>(a, rec); break;
+    default: pair_moment_sums<ORDER, 2, L, true>(a, rec); break;
+  }
+}
+
+// rkpm_value_kernel in pairs; the polynomials come as pairs too.
+template <int ORDER>
+__global__ void __launch_bounds__(kValueThreads) rkpm_pair_value_kernel(RkpmArgs a, const float* __restrict__ rec) {
+  constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
+  using RI = RawIdx<ORDER>;
+  const int64_t e0 = a.ptr[a.g0], e1 = a.ptr[a.g1];
+  const int64_t e = e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + threadIdx.x;
+  if (e0 + static_cast<int64_t>(blockIdx.x) * kValueThreads + (threadIdx.x & ~31) >= e1) return;   // the whole warp
+  const int g = point_of(a.ptr, a.g0, a.g1, e, e1);
+  if (e >= e1) return;
+  const float* R = rec + static_cast<int64_t>(g) * pair_record_floats(a.n_creases);
+  const int j = a.idx[e];
+  fp2 x, y;
+  pair_xi(a, *reinterpret_cast<const float4*>(R), *reinterpret_cast<const float4*>(R + 4),
+          __ldg(a.node_pair + 2 * j), __ldg(a.node_pair + 2 * j + 1), x, y);
+  const float2* i1 = reinterpret_cast<const float2*>(a.dpsi) + 2 * e;
+  const float2* i2 = reinterpret_cast<const float2*>(a.ddpsi) + 3 * e;
+  const fp2 w = as_fp2(reinterpret_cast<const float2*>(a.psi)[e]);
+  fp2 Jx = as_fp2(i1[0]), Jxx = as_fp2(i2[0]), Jy, Jyy;
+  const fp2 Jxy = as_fp2(i2[2]);
+  if (a.tip[g]) {
+    Jy = as_fp2(i1[1]);
+    Jyy = as_fp2(i2[1]);
+  } else {
+    Jy = Jx * y; Jx = Jx * x;
+    Jyy = Jxx * fp2_sqr(y); Jxx = Jxx * fp2_sqr(x);
+  }
+  Jx = Jx * a.irho;
+  Jy = Jy * a.irho;
+  fp2 m[NP];
+#pragma unroll
+  for (int i = 1; i < NP; ++i) {
+    if (i == 1) m[i] = x;
+    else if (i == 2) m[i] = y;
+    else m[i] = RI::by(i) == 0 ? m[RI::r(RI::bx(i) - 1, 0)] * x : m[RI::r(RI::bx(i), RI::by(i) - 1)] * y;
+  }
+  const float2* c = reinterpret_cast<const float2*>(a.coef) + static_cast<int64_t>(g - a.g0) * 6 * NP;
+  fp2 v[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    v[k] = as_fp2(__ldg(c + k * NP));
+#pragma unroll
+    for (int i = 1; i < NP; ++i) fp2_fma_acc(v[k], as_fp2(__ldg(c + k * NP + i)), m[i]);
+    v[k] = fp2_norm(v[k]);
+  }
+  const fp2 C2 = v[0] * a.irho2, vx2 = v[1] * 2.0f, vy2 = v[2] * 2.0f;
+  a.psi[e] = fp2_to_double(v[0] * w);
+  fp2 r = v[1] * w;
+  fp2_fma_acc(r, v[0], Jx);
+  a.dpsi[2 * e] = fp2_to_double(r);
+  r = v[2] * w;
+  fp2_fma_acc(r, v[0], Jy);
+  a.dpsi[2 * e + 1] = fp2_to_double(r);
+  r = v[3] * w;
+  fp2_fma_acc(r, vx2, Jx); fp2_fma_acc(r, C2, Jxx);
+  a.ddpsi[3 * e] = fp2_to_double(r);
+  r = v[4] * w;
+  fp2_fma_acc(r, vy2, Jy); fp2_fma_acc(r, C2, Jyy);
+  a.ddpsi[3 * e + 1] = fp2_to_double(r);
+  r = v[5] * w;
+  fp2_fma_acc(r, v[1], Jy); fp2_fma_acc(r, v[2], Jx); fp2_fma_acc(r, C2, Jxy);
+  a.ddpsi[3 * e + 2] = fp2_to_double(r);
 }
 
 inline unsigned blocks_for(int64_t n, int t = kThreads) { return static_cast<unsigned>((n + t - 1) / t); }
 
-// The FP64 RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
+// The RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
 // sums and polynomials of 262,144 points: 260 MB for the quadratic basis, 480 MB for the cubic).
 // Lanes per point of the moment kernel: more while its warps do not fill the SM quarters twice
 // (adding a lane pair's sums costs as many operations as half a neighbour's).
-template <int ORDER>
-void rkpm_fp64(cgb_context* ctx, cgb_shape* out, RkpmArgs ra) {
+// Returns the kernels launched.
+template <int ORDER, bool PAIR>
+int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
   constexpr int kChunk = 1 << 18, NP = (ORDER + 1) * (ORDER + 2) / 2;
+  constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
+  constexpr int kParts = PAIR || ORDER == 3 ? 2 : 1;
   cudaStream_t st = ctx->stream;
   const int n_gp = out->n_gp, most = std::min(n_gp, kChunk);
-  constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
+  int launches = 0;
   out->scr_mom.ensure(static_cast<size_t>(most) * kSums);
   out->scr_coef.ensure(static_cast<size_t>(most) * 6 * NP);
   ra.mom = out->scr_mom.p;
@@ -1066,20 +1041,26 @@ void rkpm_fp64(cgb_context* ctx, cgb_shape* out, RkpmArgs ra) {
     ra.g0 = g0;
     ra.g1 = std::min(n_gp, g0 + kChunk);
     const int np = ra.g1 - g0;
+    const int64_t pairs = std::min(out->nnz, static_cast<int64_t>(np) * out->max_n);
+    const unsigned vb = blocks_for(std::max<int64_t>(pairs, 1), kValueThreads);
+    if constexpr (PAIR) rkpm_pair_jet_kernel<<<vb, kValueThreads, 0, st>>>(ra, rec);
     const int64_t full = 2LL * 4 * 32 * sms;   // lanes of two warps per SM quarter
     auto moments = [&](auto lanes) {
       constexpr int L = decltype(lanes)::value;
-      const dim3 grid(blocks_for(static_cast<int64_t>(np) * L, 64), (ORDER < 3 ? 1 : 2) * (ra.n_creases > 0 ? 2 : 1));
-      rkpm_moment_kernel<ORDER, L><<<grid, 64, 0, st>>>(ra);
+      const dim3 grid(blocks_for(static_cast<int64_t>(np) * L, 64), kParts * (ra.n_creases > 0 ? 2 : 1));
+      if constexpr (PAIR) rkpm_pair_moment_kernel<ORDER, L><<<grid, 64, 0, st>>>(ra, rec);
+      else rkpm_moment_kernel<ORDER, L><<<grid, 64, 0, st>>>(ra);
     };
     if (np * 8LL <= full) moments(std::integral_constant<int, 8>{});
     else if (np * 2LL <= full) moments(std::integral_constant<int, 2>{});
     else moments(std::integral_constant<int, 1>{});
-    rkpm_solve_kernel<ORDER><<<blocks_for(np, 64), 64, 0, st>>>(ra);
-    const int64_t pairs = std::min(out->nnz, static_cast<int64_t>(np) * out->max_n);
-    if (pairs > 0) rkpm_value_kernel<ORDER><<<blocks_for(pairs, kValueThreads), kValueThreads, 0, st>>>(ra);
+    rkpm_solve_kernel<ORDER, PAIR><<<blocks_for(np, 64), 64, 0, st>>>(ra);
+    if constexpr (PAIR) rkpm_pair_value_kernel<ORDER><<<vb, kValueThreads, 0, st>>>(ra, rec);
+    else rkpm_value_kernel<ORDER><<<vb, kValueThreads, 0, st>>>(ra);
+    launches += PAIR ? 4 : 3;
   }
   CGB_CUDA(cudaGetLastError());
+  return launches;
 }
 
 }  // namespace
@@ -1293,43 +1274,29 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
                                                                  out->scr_node_pair.p);
     ra.node_pair = out->scr_node_pair.p;
   }
+  int nl = mixed && n_nodes > 0 ? 1 : 0;
   if (n_gp > 0) {
+    nl += mixed || d_rn ? 1 : 0;
+    out->scr_tip.ensure(n_gp);
+    ra.ir = 1.0 / out->rho;
+    ra.tip = out->scr_tip.p;
+    const float* rec = nullptr;
     if (mixed) {
-      const int RS = pair_record_floats(out->order, nc);
-      out->scr_point_rec.ensure(static_cast<size_t>(n_gp) * RS);
-      float* rec = out->scr_point_rec.p;
-      const unsigned vb = blocks_for(std::max<int64_t>(nnz, 1), kPairValueThreads);
-      switch (out->order) {
-        case 1:
-          rkpm_pair_point_kernel<1><<<blocks_for(n_gp), kThreads, 0, st>>>(ra, rec, RS);
-          if (nnz > 0) rkpm_pair_value_kernel<1><<<vb, kPairValueThreads, 0, st>>>(ra, rec, RS, nnz);
-          break;
-        case 2:
-          rkpm_pair_point_kernel<2><<<blocks_for(n_gp), kThreads, 0, st>>>(ra, rec, RS);
-          if (nnz > 0) rkpm_pair_value_kernel<2><<<vb, kPairValueThreads, 0, st>>>(ra, rec, RS, nnz);
-          break;
-        default:
-          rkpm_pair_point_kernel<3><<<blocks_for(n_gp), kThreads, 0, st>>>(ra, rec, RS);
-          if (nnz > 0) rkpm_pair_value_kernel<3><<<vb, kPairValueThreads, 0, st>>>(ra, rec, RS, nnz);
-          break;
-      }
-    } else {
-      if (d_rn) {
-        out->scr_fac.ensure(n_nodes);
-        node_fac_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, d_rn, out->rho, out->scr_fac.p);
-        ra.fac = out->scr_fac.p;
-      }
-      out->scr_tip.ensure(n_gp);
-      ra.ir = 1.0 / out->rho;
-      ra.tip = out->scr_tip.p;
-      switch (out->order) {
-        case 1: rkpm_fp64<1>(ctx, out, ra); break;
-        case 2: rkpm_fp64<2>(ctx, out, ra); break;
-        default: rkpm_fp64<3>(ctx, out, ra); break;
-      }
+      out->scr_point_rec.ensure(static_cast<size_t>(n_gp) * pair_record_floats(nc));
+      point_pair_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(ra, out->scr_point_rec.p);
+      rec = out->scr_point_rec.p;
+    } else if (d_rn) {
+      out->scr_fac.ensure(n_nodes);
+      node_fac_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, d_rn, out->rho, out->scr_fac.p);
+      ra.fac = out->scr_fac.p;
+    }
+    switch (out->order) {
+      case 1: nl += mixed ? rkpm<1, true>(ctx, out, ra, rec) : rkpm<1, false>(ctx, out, ra, rec); break;
+      case 2: nl += mixed ? rkpm<2, true>(ctx, out, ra, rec) : rkpm<2, false>(ctx, out, ra, rec); break;
+      default: nl += mixed ? rkpm<3, true>(ctx, out, ra, rec) : rkpm<3, false>(ctx, out, ra, rec); break;
     }
   }
-  prof_end(ctx, CGB_PHASE_RKPM, (n_gp > 0 ? 1 : 0) + (mixed && n_nodes > 0 ? 1 : 0) + (mixed && nnz > 0 ? 1 : 0));
+  prof_end(ctx, CGB_PHASE_RKPM, nl);
   CGB_CUDA(cudaGetLastError());
   // The reference's guards (GlobalRKPM.h:241-257 after the 3x3 block, 347-359 after
   // the bordering): singular first, then pivot collapse.
