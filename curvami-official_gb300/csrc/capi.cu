@@ -178,6 +178,7 @@ void ctx_release(cgb_context* ctx) {
   ctx->dev_err.reset();
   ctx->ws_x.reset();
   ctx->ws_out.reset();
+  ctx->scratch = cgb::ShapeScratch{};
   for (auto& m : ctx->marks) {
     if (m.start) cudaEventDestroy(m.start);
     if (m.stop) cudaEventDestroy(m.stop);
@@ -252,6 +253,11 @@ int cgb_set_nodes(cgb_context* ctx, const double* node_xy, int n_nodes) {
     if (ctx->n_nodes != n_nodes || !std::equal(node_xy, node_xy + m, ctx->h_node_xy.begin())) ++ctx->node_gen;
     ctx->n_nodes = n_nodes;
     ctx->h_node_xy.assign(node_xy, node_xy + m);
+    for (int c = 0; c < 2; ++c) ctx->node_min[c] = ctx->node_max[c] = node_xy[c];
+    for (size_t i = 0; i < m; ++i) {
+      ctx->node_min[i & 1] = std::min(ctx->node_min[i & 1], node_xy[i]);
+      ctx->node_max[i & 1] = std::max(ctx->node_max[i & 1], node_xy[i]);
+    }
     cgb::upload(ctx->node_xy, node_xy, 2 * static_cast<size_t>(n_nodes), ctx->stream);
     CGB_CUDA(cudaStreamSynchronize(ctx->stream));
   });

@@ -81,6 +81,29 @@ struct TileCell {
   int32_t n_ent, n_items, U, pad;
 };
 
+// Scratch of the shape stage, kept by the context between builds and rebuilds (a set holds only its
+// results): each such call runs on the context's stream and waits for it before it returns, and a
+// context is used by one thread at a time. Grows to the largest call's need, freed with the context.
+struct ShapeScratch {
+  // Node cell grid and neighbour search.
+  DevBuf<int64_t> cell_start, totals, bsum;
+  DevBuf<unsigned long long> cell_cursor;
+  DevBuf<int32_t> cell_count, node_key, node_list, cell_nodes, gp_count, bmax;
+  DevBuf<float2> cell32;
+  DevBuf<float> r2c32;
+  DevBuf<uint32_t> gp_mask;
+  // Creases and RKPM.
+  DevBuf<double> cxy;        // crease vertices, all creases
+  DevBuf<int8_t> side;       // n_creases * n_nodes
+  DevBuf<double> gind;       // n_creases * 6 * n_gp
+  DevBuf<int8_t> bad, tip;   // n_gp
+  DevBuf<int> guard;         // 4: flagged points
+  DevBuf<double> fac;        // n_nodes, FP64 with per-node radius
+  DevBuf<double> mom, coef;  // moment sums and polynomials of a chunk of points
+  DevBuf<float4> node_pair;  // 2 * n_nodes, mixed precision
+  DevBuf<float> point_rec;   // point records, mixed precision
+};
+
 }  // namespace cgb
 
 // Opaque handles of the C ABI.
@@ -102,6 +125,8 @@ struct cgb_context {
   // Device-side error word written by kernels (bounds checks, capacity).
   cgb::DevBuf<int> dev_err;
   int* h_err = nullptr;  // pinned mirror
+  double node_min[2] = {0.0, 0.0}, node_max[2] = {0.0, 0.0};  // bounds of the nodes
+  cgb::ShapeScratch scratch;
   cgb::DevBuf<double> ws_x, ws_out;  // device copies of cgb_point_state's x and rows
   // Tracing: event pairs per phase, summed when read.
   bool profile = false;
@@ -135,17 +160,6 @@ struct cgb_shape {
   cgb::DevBuf<double> rho_node;   // n_nodes (per-node radius) when has_rho_node
   uint64_t node_gen = 0;
   uint64_t version = 0;           // bumped by every rebuild (derived copies go stale)
-  // Scratch of the crease / RKPM stage, kept for the next rebuild (no allocation per step).
-  cgb::DevBuf<double> scr_cxy;    // crease vertices, all creases
-  cgb::DevBuf<int8_t> scr_side;   // n_creases * n_nodes
-  cgb::DevBuf<double> scr_gind;   // n_creases * 6 * n_gp
-  cgb::DevBuf<int8_t> scr_bad;    // n_gp
-  cgb::DevBuf<int> scr_guard;     // 4: flagged points
-  cgb::DevBuf<int8_t> scr_tip;        // n_gp, FP64
-  cgb::DevBuf<double> scr_fac;        // n_nodes, FP64 with per-node radius
-  cgb::DevBuf<double> scr_mom, scr_coef;  // FP64: moment sums and polynomials of a chunk of points
-  cgb::DevBuf<float4> scr_node_pair;  // 2 * n_nodes, mixed precision only
-  cgb::DevBuf<float> scr_point_rec;   // point records of the mixed RKPM, n_gp x record floats
 };
 
 // Per-fold data kept by the assembler (plate/PlateData.h: Fold; Constraints.h:341).

@@ -4,7 +4,7 @@
 // Reference: core/include/curvami/FRNN.h:23-78, core/include/curvami/Enrichment.h:23-92,
 // core/include/curvami/GlobalRKPM.h:15-397.
 //
-// Design: the node cell grid is a dense array over the reference's flattened cell key
+// Design: the node cell grid, made on the device, is a dense array over the reference's flattened cell key
 // (y * cols + x, so keys that wrap across a row resolve to the same cells as the
 // reference's hash map). One thread per Gauss point gathers its neighbours in the
 // reference's order (dx outer, dy inner, node index ascending in a cell) with an FP64
@@ -29,70 +29,136 @@ namespace {
 
 constexpr int kThreads = 128;
 
+inline unsigned blocks_for(int64_t n, int t = kThreads) { return static_cast<unsigned>((n + t - 1) / t); }
+
+// The node cell grid (FRNN.h:33-44): the nodes of every cell in ascending order, with their float
+// coordinates beside them.
 struct GridDev {
   double minx, miny, cell;
   int cols;
   long long ncells;
-  const int32_t* cell_start;  // ncells + 1
+  const int64_t* cell_start;  // ncells + 1
   const int32_t* cell_nodes;
 };
 
 // FP32 pre-test of the FRNN distance test. Coordinates relative to the grid's lower corner
-// are rounded to float (node32, per node; the point's in the kernel), the squared distance
-// is formed in float, and `margin` bounds its difference from the exact squared distance
+// are rounded to float (cell32, per node in cell order; the point's in the kernel), the squared
+// distance is formed in float, and `margin` bounds its difference from the exact squared distance
 // (coordinate rounding, float arithmetic, the float radius; computed on the host from the
 // extent of the nodes and points). A candidate beyond r^2 + margin is outside and one
 // below r^2 - margin inside whatever FP64 gives; only those within the margin take the
 // exact FP64 test, so every decision is the FP64 one.
 struct FrnnPre {
-  const float2* node32;   // per node, (x - minx, y - miny) in float
-  const float* r2n32;     // per node r^2 in float, or nullptr for the single radius
+  const float2* cell32;   // per node in cell order, (x - minx, y - miny) in float
+  const float* r2c32;     // per node in cell order r^2 in float, or nullptr for the single radius
   float r2f;              // the single radius squared, in float
   float margin;
 };
 
-// Thread per Gauss point: count (out_idx == nullptr) or fill the neighbour list.
+// Cell key of every node, and the nodes per cell.
+__global__ void cell_count_kernel(int n_nodes, const double* __restrict__ node_xy, GridDev G, int32_t* __restrict__ key,
+                                  int32_t* __restrict__ count) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n_nodes) return;
+  const int cx = static_cast<int>(floor(__ddiv_rn(__dsub_rn(node_xy[2 * j], G.minx), G.cell)));
+  const int cy = static_cast<int>(floor(__ddiv_rn(__dsub_rn(node_xy[2 * j + 1], G.miny), G.cell)));
+  const long long at = static_cast<long long>(cy) * G.cols + cx;
+  const int k = at >= 0 && at < G.ncells ? static_cast<int>(at) : 0;   // (a coordinate that is not a number)
+  key[j] = k;
+  atomicAdd(&count[k], 1);
+}
+
+// The nodes into their cells, in any order (cursor: a copy of cell_start).
+__global__ void cell_fill_kernel(int n_nodes, const int32_t* __restrict__ key, unsigned long long* __restrict__ cursor,
+                                 int32_t* __restrict__ list) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n_nodes) list[atomicAdd(&cursor[key[j]], 1ULL)] = j;
+}
+
+// Ascending node index per cell: every node's rank among its cell's, and its float coordinates
+// and radius at that place.
+__global__ void cell_sort_kernel(int n_nodes, const double* __restrict__ node_xy, const double* __restrict__ rho_node,
+                                 GridDev G, const int32_t* __restrict__ key, const int32_t* __restrict__ list,
+                                 int32_t* __restrict__ sorted, float2* __restrict__ cell32, float* __restrict__ r2c32) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n_nodes) return;
+  const int64_t k0 = G.cell_start[key[j]], k1 = G.cell_start[key[j] + 1];
+  int64_t at = k0;
+  for (int64_t k = k0; k < k1; ++k) at += list[k] < j;
+  sorted[at] = j;
+  cell32[at] = make_float2(__double2float_rn(__dsub_rn(node_xy[2 * j], G.minx)),
+                           __double2float_rn(__dsub_rn(node_xy[2 * j + 1], G.miny)));
+  if (rho_node) r2c32[at] = __double2float_rn(__dmul_rn(rho_node[j], rho_node[j]));
+}
+
+// Thread per Gauss point. The counting pass (out_idx == nullptr) leaves the decisions of the first
+// kMaskWords * 32 candidates as bits, [word][point]; the filling pass reads them back and tests only
+// candidates beyond. Candidates of a cell are consecutive, so the counting pass makes one 8-byte
+// load per candidate. 1,000,000 scattered points: both passes 2.1 ms when each tested every
+// candidate through its node index.
+constexpr int kMaskWords = 8;
+
 __global__ void frnn_kernel(int n_gp, const double* __restrict__ gp_xy,
                             const double* __restrict__ node_xy, const double* __restrict__ rho_node,
-                            double rho, double rho2, GridDev G, FrnnPre pre, const int64_t* __restrict__ ptr,
-                            int32_t* __restrict__ count, int32_t* __restrict__ out_idx) {
+                            double rho2, GridDev G, FrnnPre pre, const int64_t* __restrict__ ptr,
+                            int32_t* __restrict__ count, uint32_t* __restrict__ mask, int32_t* __restrict__ out_idx) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n_gp) return;
   const double gx = gp_xy[2 * g], gy = gp_xy[2 * g + 1];
   const float gxf = __double2float_rn(gx - G.minx), gyf = __double2float_rn(gy - G.miny);
   const int qx = static_cast<int>(floor(__ddiv_rn(__dsub_rn(gx, G.minx), G.cell)));
   const int qy = static_cast<int>(floor(__ddiv_rn(__dsub_rn(gy, G.miny), G.cell)));
-  int64_t pos = out_idx ? ptr[g] : 0;
-  int cnt = 0;
+  auto test = [&](int64_t k) {
+    const float2 nf = pre.cell32[k];
+    const float fdx = nf.x - gxf, fdy = nf.y - gyf;
+    const float d2f = fdx * fdx + fdy * fdy;
+    const float r2f = pre.r2c32 ? pre.r2c32[k] : pre.r2f;
+    if (d2f > r2f + pre.margin) return false;      // outside, whatever FP64 gives
+    if (d2f < r2f - pre.margin) return true;       // inside, whatever FP64 gives
+    const int j = G.cell_nodes[k];
+    const double ddx = __dsub_rn(node_xy[2 * j], gx);
+    const double ddy = __dsub_rn(node_xy[2 * j + 1], gy);
+    const double dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
+    return dist2 <= (rho_node ? __dmul_rn(rho_node[j], rho_node[j]) : rho2);
+  };
+  const bool fill = out_idx != nullptr;
+  int64_t pos = fill ? ptr[g] : 0;
+  int cnt = 0, o = 0;           // neighbours; candidates so far
+  uint32_t word = fill ? mask[g] : 0u;
   for (int dx = -1; dx <= 1; ++dx) {
     for (int dy = -1; dy <= 1; ++dy) {
       const long long key = static_cast<long long>(qy + dy) * G.cols + (qx + dx);
       if (key < 0 || key >= G.ncells) continue;
-      const int k0 = G.cell_start[key], k1 = G.cell_start[key + 1];
-      for (int k = k0; k < k1; ++k) {
-        const int j = G.cell_nodes[k];
-        const float2 nf = pre.node32[j];
-        const float fdx = nf.x - gxf, fdy = nf.y - gyf;
-        const float d2f = fdx * fdx + fdy * fdy;
-        const float r2f = pre.r2n32 ? pre.r2n32[j] : pre.r2f;
-        if (d2f > r2f + pre.margin) continue;          // outside, whatever FP64 gives
-        bool inside = d2f < r2f - pre.margin;          // inside, whatever FP64 gives
-        if (!inside) {
-          const double ddx = __dsub_rn(node_xy[2 * j], gx);
-          const double ddy = __dsub_rn(node_xy[2 * j + 1], gy);
-          const double dist2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
-          double r2 = rho2;
-          if (rho_node) { const double r = rho_node[j]; r2 = __dmul_rn(r, r); }
-          inside = dist2 <= r2;
+      int64_t k = G.cell_start[key];
+      const int64_t k1 = G.cell_start[key + 1];
+      if (!fill) {
+        for (; k < k1; ++k, ++o) {
+          const bool in = test(k);
+          cnt += in;
+          if (o < 32 * kMaskWords) {
+            word |= static_cast<uint32_t>(in) << (o & 31);
+            if ((o & 31) == 31) { mask[static_cast<int64_t>(o >> 5) * n_gp + g] = word; word = 0u; }
+          }
         }
-        if (inside) {
-          if (out_idx) out_idx[pos++] = j;
-          ++cnt;
+      } else {
+        while (k < k1 && o < 32 * kMaskWords) {   // the set bits of this cell's candidates, word by word
+          const int bit = o & 31, len = static_cast<int>(min(static_cast<int64_t>(32 - bit), k1 - k));
+          uint32_t b = word >> bit;
+          if (len < 32) b &= (1u << len) - 1u;
+          for (; b; b &= b - 1u) out_idx[pos++] = G.cell_nodes[k + __ffs(b) - 1];
+          k += len;
+          o += len;
+          if ((o & 31) == 0 && o < 32 * kMaskWords) word = mask[static_cast<int64_t>(o >> 5) * n_gp + g];
         }
+        for (; k < k1; ++k)
+          if (test(k)) out_idx[pos++] = G.cell_nodes[k];
       }
     }
   }
-  if (!out_idx) count[g] = cnt;
+  if (!fill) {
+    count[g] = cnt;
+    if (o < 32 * kMaskWords) mask[static_cast<int64_t>(o >> 5) * n_gp + g] = word;   // the last, part-filled word
+  }
 }
 
 // The point of entry e of the points [g0, g1): lane 0 of each warp finds it for the warp's first
@@ -145,7 +211,7 @@ __global__ void guard_kernel(int n, const int8_t* __restrict__ bad, int* __restr
 // total and the largest count for the host (two numbers instead of the whole array).
 constexpr int kScanThreads = 1024;
 
-__global__ void scan_local_kernel(int n, const int32_t* __restrict__ cnt, int64_t* __restrict__ ptr,
+__global__ void scan_local_kernel(int64_t n, const int32_t* __restrict__ cnt, int64_t* __restrict__ ptr,
                                   int64_t* __restrict__ block_sum, int32_t* __restrict__ block_max) {
   __shared__ int64_t sv[kScanThreads];
   __shared__ int32_t mv[kScanThreads];
@@ -170,26 +236,46 @@ __global__ void scan_local_kernel(int n, const int32_t* __restrict__ cnt, int64_
   }
 }
 
-// One thread: block totals -> exclusive block offsets (in place); totals[0] = nnz, [1] = max.
+// One warp: block totals -> exclusive block offsets (in place); totals[0] = sum, [1] = max.
 __global__ void scan_blocks_kernel(int nb, int64_t* __restrict__ block_sum, const int32_t* __restrict__ block_max,
                                    int64_t* __restrict__ totals) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  const int lane = threadIdx.x;
   int64_t run = 0;
   int32_t mx = 0;
-  for (int b = 0; b < nb; ++b) {
-    const int64_t v = block_sum[b];
-    block_sum[b] = run;
-    run += v;
-    mx = max(mx, block_max[b]);
+  for (int b0 = 0; b0 < nb; b0 += 32) {
+    const int b = b0 + lane;
+    const int64_t v = b < nb ? block_sum[b] : 0;
+    mx = max(mx, b < nb ? block_max[b] : 0);
+    int64_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (b < nb) block_sum[b] = run + incl - v;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  totals[0] = run;
-  totals[1] = mx;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) { totals[0] = run; totals[1] = mx; }
 }
 
-__global__ void scan_add_kernel(int n, int64_t* __restrict__ ptr, const int64_t* __restrict__ block_off) {
+__global__ void scan_add_kernel(int64_t n, int64_t* __restrict__ ptr, const int64_t* __restrict__ block_off) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * kScanThreads + threadIdx.x;
   if (i < n) ptr[i + 1] += block_off[blockIdx.x];
   if (i == 0) ptr[0] = 0;
+}
+
+// ptr[i + 1] = cnt[0] + .. + cnt[i] (n > 0); tot: the sum and the largest count, on the device.
+void scan_counts(cgb_context* ctx, int64_t n, const int32_t* cnt, int64_t* ptr, int64_t* tot) {
+  cudaStream_t st = ctx->stream;
+  const int nb = static_cast<int>((n + kScanThreads - 1) / kScanThreads);
+  ShapeScratch& w = ctx->scratch;
+  w.bsum.ensure(nb);
+  w.bmax.ensure(nb);
+  scan_local_kernel<<<nb, kScanThreads, 0, st>>>(n, cnt, ptr, w.bsum.p, w.bmax.p);
+  scan_blocks_kernel<<<1, 32, 0, st>>>(nb, w.bsum.p, w.bmax.p, tot);
+  scan_add_kernel<<<nb, kScanThreads, 0, st>>>(n, ptr, w.bsum.p);
+  CGB_CUDA(cudaGetLastError());
 }
 
 // Per-node crease side sn = (f >= 0 ? +1 : -1) (GlobalRKPM.h:92-93).
@@ -874,14 +960,19 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_pair_jet_kernel(RkpmArgs a
   }
 }
 
-// The sums of moment_sums from the pairs' jets, accumulated in pairs (Dot2) and rounded to FP64.
+// The sums of moment_sums from the pairs' jets, accumulated in pairs (Dot2) and rounded to FP64, in
+// three parts: W and C, A, B; in a cap two of the six jets each. All sums of a point in one thread (74
+// pairs, 206 registers in two parts) left two warps per scheduler to hide the long chains of pair
+// arithmetic; forming the monomials three times costs a tenth more instructions.
 template <int ORDER, int PART, int L, bool TIP>
 __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float* __restrict__ rec) {
   using MI = MomIdx<ORDER>;
   using RI = RawIdx<ORDER>;
-  constexpr bool P1 = PART == 1;
-  constexpr int LO = TIP ? (P1 ? 0 : 3 * RI::NR) : P1 ? 0 : MI::NW + MI::NA;
-  constexpr int HI = TIP ? (P1 ? 3 * RI::NR : 6 * RI::NR) : P1 ? MI::NW + MI::NA : MI::N;
+  constexpr int N0 = TIP ? RI::NR : PART == 0 ? MI::NW : PART == 1 ? MI::NA : MI::NB;   // sums of the first factor
+  constexpr int N1 = TIP ? RI::NR : PART == 0 ? MI::NC : 0;
+  constexpr int AT0 = TIP ? 2 * PART * RI::NR : PART == 0 ? 0 : PART == 1 ? MI::NW : MI::NW + MI::NA;
+  constexpr int AT1 = TIP ? (2 * PART + 1) * RI::NR : MI::NW + MI::NA + MI::NB;
+  constexpr int DEG = MI::D + (TIP ? 0 : PART);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int g = a.g0 + t / L, sub = t % L;
   const bool here = g < a.g1;
@@ -892,24 +983,28 @@ __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float*
   const int n = mine ? static_cast<int>(a.ptr[gc + 1] - p0) : 0;
   const float* R = rec + static_cast<int64_t>(gc) * pair_record_floats(a.n_creases);
   const float4 r0 = *reinterpret_cast<const float4*>(R), r1 = *reinterpret_cast<const float4*>(R + 4);
-  const float2* i0 = reinterpret_cast<const float2*>(a.psi);
-  const float2* i1 = reinterpret_cast<const float2*>(a.dpsi);
-  const float2* i2 = reinterpret_cast<const float2*>(a.ddpsi);
-  fp2 S[HI - LO];
+  // The array of a pair's jet k: psi, dpsi (2), ddpsi (3); w, A, B and C xi eta are jets 0, 1, 3, 5.
+  auto jet = [&](int k, int64_t e) {
+    const double* p = k == 0 ? a.psi + e : k < 3 ? a.dpsi + 2 * e + (k - 1) : a.ddpsi + 3 * e + (k - 3);
+    return as_fp2(*reinterpret_cast<const float2*>(p));
+  };
+  constexpr int K0 = TIP ? 2 * PART : PART == 0 ? 0 : PART == 1 ? 1 : 3;
+  constexpr int K1 = TIP ? 2 * PART + 1 : 5;
+  fp2 S0[N0], S1[N1 > 0 ? N1 : 1];
 #pragma unroll
-  for (int k = 0; k < HI - LO; ++k) S[k] = fp2{0.0f, 0.0f};
+  for (int k = 0; k < N0; ++k) S0[k] = fp2{0.0f, 0.0f};
+#pragma unroll
+  for (int k = 0; k < N1; ++k) S1[k] = fp2{0.0f, 0.0f};
   for (int q = sub; q < n; q += L) {
     const int64_t e = p0 + q;
     const int j = a.idx[e];
     fp2 xi, eta;
     pair_xi(a, r0, r1, __ldg(a.node_pair + 2 * j), __ldg(a.node_pair + 2 * j + 1), xi, eta);
-    fp2 J[3];   // w, x, y or xx, yy, xy in a cap; w, A or B, C xi eta otherwise
-    if (P1) { J[0] = as_fp2(i0[e]); J[1] = as_fp2(i1[2 * e]); if (TIP) J[2] = as_fp2(i1[2 * e + 1]); }
-    else { J[0] = as_fp2(i2[3 * e]); J[2] = as_fp2(i2[3 * e + 2]); if (TIP) J[1] = as_fp2(i2[3 * e + 1]); }
-    fp2 m[MI::D + 3];
+    const fp2 J0 = jet(K0, e), J1 = N1 > 0 ? jet(K1, e) : fp2{0.0f, 0.0f};
+    fp2 m[DEG + 1];
     m[0] = fp2{1.0f, 0.0f};
 #pragma unroll
-    for (int d = 0; d <= MI::D + (TIP ? 0 : P1 ? 1 : 2); ++d) {
+    for (int d = 0; d <= DEG; ++d) {
       if (d == 1) { m[1] = eta; m[0] = xi; }
       if (d > 1) {
         m[d] = m[d - 1] * eta;
@@ -918,36 +1013,40 @@ __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float*
       }
 #pragma unroll
       for (int b = 0; b <= d; ++b) {
-        auto add = [&](int k, fp2 v) { fp2_fma_acc(S[k - LO], v, m[b]); };
-        if constexpr (TIP) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) add((P1 ? k : k + 3) * RI::NR + RI::r(d - b, b), J[k]);
-        } else {
-          if (P1 && d <= MI::D) add(MI::w(d - b, b), J[0]);
-          if (P1 && d >= 1) add(MI::ax(d - b, b), J[1]);
-          if (!P1 && d >= 2 && !(d == 2 && b == 1)) add(MI::bx(d - b, b), J[0]);
-          if (!P1 && d <= MI::D) add(MI::cx(d - b + 1, b + 1), J[2]);
+        const int x = d - b;
+        if (TIP || PART == 0) {
+          fp2_fma_acc(S0[RI::r(x, b)], J0, m[b]);
+          if (N1 > 0) fp2_fma_acc(S1[RI::r(x, b)], J1, m[b]);
+        } else if (PART == 1) {
+          if (d >= 1) fp2_fma_acc(S0[MI::ax(x, b) - AT0], J0, m[b]);
+        } else if (d >= 2 && !(d == 2 && b == 1)) {
+          fp2_fma_acc(S0[MI::bx(x, b) - AT0], J0, m[b]);
         }
       }
     }
   }
   const int64_t np = a.g1 - a.g0;
-#pragma unroll
-  for (int k = 0; k < HI - LO; ++k) {
-    double v = fp2_to_double(S[k]);
+  auto put = [&](int k, fp2 sum) {
+    double v = fp2_to_double(sum);
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (mine && sub == 0) a.mom[(LO + k) * np + (g - a.g0)] = v;
-  }
+    if (mine && sub == 0) a.mom[k * np + (g - a.g0)] = v;
+  };
+#pragma unroll
+  for (int k = 0; k < N0; ++k) put(AT0 + k, S0[k]);
+#pragma unroll
+  for (int k = 0; k < N1; ++k) put(AT1 + k, S1[k]);
 }
 
 // blockIdx.y: the part, then the kind of points (only launched with creases).
 template <int ORDER, int L>
-__global__ void __launch_bounds__(64) rkpm_pair_moment_kernel(RkpmArgs a, const float* __restrict__ rec) {
+__global__ void __launch_bounds__(64, ORDER < 3 ? 8 : 4) rkpm_pair_moment_kernel(RkpmArgs a, const float* __restrict__ rec) {
   switch (blockIdx.y) {
-    case 0: pair_moment_sums<ORDER, 1, L, false>(a, rec); break;
-    case 1: pair_moment_sums<ORDER, 2, L, false>(a, rec); break;
-    case 2: pair_moment_sums<ORDER, 1, L, true>(a, rec); break;
+    case 0: pair_moment_sums<ORDER, 0, L, false>(a, rec); break;
+    case 1: pair_moment_sums<ORDER, 1, L, false>(a, rec); break;
+    case 2: pair_moment_sums<ORDER, 2, L, false>(a, rec); break;
+    case 3: pair_moment_sums<ORDER, 0, L, true>(a, rec); break;
+    case 4: pair_moment_sums<ORDER, 1, L, true>(a, rec); break;
     default: pair_moment_sums<ORDER, 2, L, true>(a, rec); break;
   }
 }
@@ -1016,8 +1115,6 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_pair_value_kernel(RkpmArgs
   a.ddpsi[3 * e + 2] = fp2_to_double(r);
 }
 
-inline unsigned blocks_for(int64_t n, int t = kThreads) { return static_cast<unsigned>((n + t - 1) / t); }
-
 // The RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
 // sums and polynomials of 262,144 points: 260 MB for the quadratic basis, 480 MB for the cubic).
 // Lanes per point of the moment kernel: more while its warps do not fill the SM quarters twice
@@ -1027,14 +1124,14 @@ template <int ORDER, bool PAIR>
 int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
   constexpr int kChunk = 1 << 18, NP = (ORDER + 1) * (ORDER + 2) / 2;
   constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
-  constexpr int kParts = PAIR || ORDER == 3 ? 2 : 1;
+  constexpr int kParts = PAIR ? 3 : ORDER == 3 ? 2 : 1;
   cudaStream_t st = ctx->stream;
   const int n_gp = out->n_gp, most = std::min(n_gp, kChunk);
   int launches = 0;
-  out->scr_mom.ensure(static_cast<size_t>(most) * kSums);
-  out->scr_coef.ensure(static_cast<size_t>(most) * 6 * NP);
-  ra.mom = out->scr_mom.p;
-  ra.coef = out->scr_coef.p;
+  ctx->scratch.mom.ensure(static_cast<size_t>(most) * kSums);
+  ctx->scratch.coef.ensure(static_cast<size_t>(most) * 6 * NP);
+  ra.mom = ctx->scratch.mom.p;
+  ra.coef = ctx->scratch.coef.p;
   int sms = 0;
   CGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   for (int g0 = 0; g0 < n_gp; g0 += kChunk) {
@@ -1086,50 +1183,59 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   out->precision = prm.precision;
   out->node_gen = ctx->node_gen;
 
-  // ---- node cell grid (FRNN.h:33-44), host side, O(n_nodes) ----
-  const double* nxy = ctx->h_node_xy.data();
+  // ---- node cell grid (FRNN.h:33-44) ----
+  ShapeScratch& w = ctx->scratch;
   double cell = prm.rho;
-  std::vector<double> rn;
   if (prm.rho_node) {
-    rn.assign(prm.rho_node, prm.rho_node + n_nodes);
     cell = 0.0;
-    for (double r : rn) {
-      if (!(r > 0.0)) throw Error(CGB_ERR_INVALID, "cgb_shape_build: rho_node must be > 0");
-      cell = std::max(cell, r);
+    for (int i = 0; i < n_nodes; ++i) {
+      if (!(prm.rho_node[i] > 0.0)) throw Error(CGB_ERR_INVALID, "cgb_shape_build: rho_node must be > 0");
+      cell = std::max(cell, prm.rho_node[i]);
     }
   }
-  double minx = nxy[0], miny = nxy[1], maxx = nxy[0];
-  for (int i = 0; i < n_nodes; ++i) {
-    minx = std::min(minx, nxy[2 * i]);
-    miny = std::min(miny, nxy[2 * i + 1]);
-    maxx = std::max(maxx, nxy[2 * i]);
+  const double minx = ctx->node_min[0], miny = ctx->node_min[1], maxx = ctx->node_max[0], maxy = ctx->node_max[1];
+  const double cells_x = std::ceil((maxx - minx) / cell), cells_y = std::floor((maxy - miny) / cell);
+  // The grid ends with the largest key; a bound on it decides except beside the limit itself.
+  constexpr double kMostCells = static_cast<double>(1LL << 28);
+  bool fits = cells_x < kMostCells && cells_y < kMostCells && cells_y * (cells_x + 1.0) + 1.0 <= kMostCells;
+  const int cols = fits ? static_cast<int>(cells_x) + 1 : 1;
+  long long ncells = fits ? (static_cast<long long>(cells_y) + 1) * cols : 0;
+  if (ncells > (1LL << 28)) {
+    ncells = 0;
+    for (int i = 0; i < n_nodes; ++i) {
+      const double* q = ctx->h_node_xy.data() + 2 * static_cast<size_t>(i);
+      ncells = std::max(ncells, static_cast<long long>(std::floor((q[1] - miny) / cell)) * cols +
+                                    static_cast<long long>(std::floor((q[0] - minx) / cell)) + 1);
+    }
+    fits = ncells <= (1LL << 28);
   }
-  const int cols = static_cast<int>(std::ceil((maxx - minx) / cell)) + 1;
-  std::vector<long long> key(n_nodes);
-  long long kmax = 0;
-  for (int i = 0; i < n_nodes; ++i) {
-    const int cx = static_cast<int>(std::floor((nxy[2 * i] - minx) / cell));
-    const int cy = static_cast<int>(std::floor((nxy[2 * i + 1] - miny) / cell));
-    key[i] = static_cast<long long>(cy) * cols + cx;
-    kmax = std::max(kmax, key[i]);
-  }
-  const long long ncells = kmax + 1;
-  if (ncells > (1LL << 28))
+  if (!fits)
     throw Error(CGB_ERR_CAPACITY, "cgb_shape_build: the node cell grid exceeds 2^28 cells (rho too small for the node extent)");
-  std::vector<int32_t> cstart(ncells + 1, 0), cnodes(n_nodes);
-  for (int i = 0; i < n_nodes; ++i) cstart[key[i] + 1]++;
-  for (long long c = 0; c < ncells; ++c) cstart[c + 1] += cstart[c];
-  {
-    std::vector<int32_t> cur(cstart.begin(), cstart.end() - 1);
-    for (int i = 0; i < n_nodes; ++i) cnodes[cur[key[i]]++] = i;  // ascending node index per cell
-  }
-  DevBuf<int32_t> d_cstart, d_cnodes;
-  upload(d_cstart, cstart.data(), cstart.size(), st);
-  upload(d_cnodes, cnodes.data(), cnodes.size(), st);
   out->has_rho_node = prm.rho_node != nullptr;
-  if (prm.rho_node) upload(out->rho_node, rn.data(), rn.size(), st);
+  if (prm.rho_node) upload(out->rho_node, prm.rho_node, n_nodes, st);
   const double* d_rn = prm.rho_node ? out->rho_node.p : nullptr;
-  GridDev G{minx, miny, cell, cols, ncells, d_cstart.p, d_cnodes.p};
+  w.cell_start.ensure(static_cast<size_t>(ncells) + 1);
+  w.cell_cursor.ensure(static_cast<size_t>(ncells) + 1);
+  w.cell_count.ensure(static_cast<size_t>(ncells));
+  w.node_key.ensure(n_nodes);
+  w.node_list.ensure(n_nodes);
+  w.cell_nodes.ensure(n_nodes);
+  w.cell32.ensure(n_nodes);
+  w.totals.ensure(4);
+  if (d_rn) w.r2c32.ensure(n_nodes);
+  const GridDev G{minx, miny, cell, cols, ncells, w.cell_start.p, w.cell_nodes.p};
+  prof_begin(ctx, CGB_PHASE_FRNN);
+  CGB_CUDA(cudaMemsetAsync(w.cell_count.p, 0, static_cast<size_t>(ncells) * sizeof(int32_t), st));
+  cell_count_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, ctx->node_xy.p, G, w.node_key.p, w.cell_count.p);
+  scan_counts(ctx, ncells, w.cell_count.p, w.cell_start.p, w.totals.p + 2);
+  CGB_CUDA(cudaMemcpyAsync(w.cell_cursor.p, w.cell_start.p, static_cast<size_t>(ncells) * sizeof(int64_t),
+                           cudaMemcpyDeviceToDevice, st));
+  cell_fill_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, w.node_key.p, w.cell_cursor.p, w.node_list.p);
+  cell_sort_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, ctx->node_xy.p, d_rn, G, w.node_key.p,
+                                                               w.node_list.p, w.cell_nodes.p, w.cell32.p,
+                                                               d_rn ? w.r2c32.p : nullptr);
+  CGB_CUDA(cudaGetLastError());
+  prof_end(ctx, CGB_PHASE_FRNN, 6);
 
   upload(out->gp_xy, gp_xy, 2 * static_cast<size_t>(n_gp), st);
   out->has_xy = true;
@@ -1146,50 +1252,34 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   // X may be taken over the node box widened by two cells: a point farther out is more than
   // 2c from every node, truly outside, and its float distance (off by a relative 2^-23) stays
   // above 4 c^2 (1 - 2^-22)^2 > r^2 + margin, so it is classified outside too.
-  double maxy = miny;
-  for (int i = 0; i < n_nodes; ++i) maxy = std::max(maxy, nxy[2 * i + 1]);
   const double ext = std::max(maxx - minx, maxy - miny) + 2.0 * cell;
   const double e = std::ldexp(ext, -23), fu = std::ldexp(1.0, -24);
   const double margin = 16.0 * cell * e + 8.0 * e * e + 64.0 * fu * cell * cell;
-  std::vector<float> n32(2 * static_cast<size_t>(n_nodes)), r32;
-  for (int i = 0; i < n_nodes; ++i) {
-    n32[2 * i] = static_cast<float>(nxy[2 * i] - minx);
-    n32[2 * i + 1] = static_cast<float>(nxy[2 * i + 1] - miny);
-  }
-  DevBuf<float> d_n32, d_r32;
-  upload(d_n32, n32.data(), n32.size(), st);
-  if (prm.rho_node) {
-    r32.resize(n_nodes);
-    for (int i = 0; i < n_nodes; ++i) r32[i] = static_cast<float>(rn[i] * rn[i]);
-    upload(d_r32, r32.data(), r32.size(), st);
-  }
-  const FrnnPre pre{reinterpret_cast<const float2*>(d_n32.p), prm.rho_node ? d_r32.p : nullptr,
-                    static_cast<float>(rho2), static_cast<float>(margin)};
-  DevBuf<int32_t> d_cnt(n_gp);
-  prof_begin(ctx, CGB_PHASE_FRNN);
-  if (n_gp > 0)
-    frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p,
-                                                        d_rn, prm.rho, rho2, G, pre,
-                                                        nullptr, d_cnt.p, nullptr);
-  CGB_CUDA(cudaGetLastError());
-  prof_end(ctx, CGB_PHASE_FRNN, n_gp > 0 ? 1 : 0);
-  // CSR offsets on the device; only the total and the largest count come back.
+  const FrnnPre pre{w.cell32.p, d_rn ? w.r2c32.p : nullptr, static_cast<float>(rho2), static_cast<float>(margin)};
   out->nbr_ptr.alloc(static_cast<size_t>(n_gp) + 1);
   int64_t totals[2] = {0, 0};
   if (n_gp > 0) {
-    const int nb = static_cast<int>((static_cast<int64_t>(n_gp) + kScanThreads - 1) / kScanThreads);
-    DevBuf<int64_t> bsum(nb), tot(2);
-    DevBuf<int32_t> bmax(nb);
-    scan_local_kernel<<<nb, kScanThreads, 0, st>>>(n_gp, d_cnt.p, out->nbr_ptr.p, bsum.p, bmax.p);
-    scan_blocks_kernel<<<1, 1, 0, st>>>(nb, bsum.p, bmax.p, tot.p);
-    scan_add_kernel<<<nb, kScanThreads, 0, st>>>(n_gp, out->nbr_ptr.p, bsum.p);
-    CGB_CUDA(cudaGetLastError());
-    CGB_CUDA(cudaMemcpyAsync(totals, tot.p, sizeof(totals), cudaMemcpyDeviceToHost, st));
+    w.gp_count.ensure(n_gp);
+    w.gp_mask.ensure(static_cast<size_t>(n_gp) * kMaskWords);
+    prof_begin(ctx, CGB_PHASE_FRNN);
+    frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p, d_rn, rho2, G, pre,
+                                                        nullptr, w.gp_count.p, w.gp_mask.p, nullptr);
+    // CSR offsets on the device; only the total and the largest count come back.
+    scan_counts(ctx, n_gp, w.gp_count.p, out->nbr_ptr.p, w.totals.p);
+    prof_end(ctx, CGB_PHASE_FRNN, 4);
+    CGB_CUDA(cudaMemcpyAsync(totals, w.totals.p, sizeof(totals), cudaMemcpyDeviceToHost, st));
     CGB_CUDA(cudaStreamSynchronize(st));
   } else {
     CGB_CUDA(cudaMemsetAsync(out->nbr_ptr.p, 0, sizeof(int64_t), st));
   }
   const int64_t nnz = totals[0];
+  auto drop_grid = [&] {   // a sparse grid of many cells is not kept
+    if (ncells <= (1LL << 24)) return;
+    CGB_CUDA(cudaStreamSynchronize(st));
+    w.cell_start.reset();
+    w.cell_cursor.reset();
+    w.cell_count.reset();
+  };
   if (nnz >= (1LL << 31)) throw Error(CGB_ERR_CAPACITY, "cgb_shape_build: more than 2^31 neighbour entries");
   out->nnz = nnz;
   out->max_n = static_cast<int>(totals[1]);
@@ -1200,15 +1290,15 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   if (want_s) out->s.alloc(nnz); else out->s.reset();
   prof_begin(ctx, CGB_PHASE_FRNN);
   if (n_gp > 0)
-    frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p,
-                                                        d_rn, prm.rho, rho2, G, pre,
-                                                        out->nbr_ptr.p, nullptr, out->nbr_idx.p);
+    frnn_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p, d_rn, rho2, G, pre,
+                                                        out->nbr_ptr.p, nullptr, w.gp_mask.p, out->nbr_idx.p);
   if (want_s && nnz > 0)
     distance_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(n_gp, out->gp_xy.p, ctx->node_xy.p, d_rn, prm.rho,
                                                           out->nbr_ptr.p, out->nbr_idx.p, nnz, out->s.p);
   prof_end(ctx, CGB_PHASE_FRNN, (n_gp > 0 ? 1 : 0) + (want_s && nnz > 0 ? 1 : 0));
   CGB_CUDA(cudaGetLastError());
 
+  drop_grid();
   out->rebuildable = true;
   shape_values(ctx, out, creases);
 }
@@ -1229,18 +1319,18 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
     all_xy.insert(all_xy.end(), creases[c].xy.begin(), creases[c].xy.end());
     off[c + 1] = all_xy.size();
   }
-  out->scr_cxy.ensure(std::max<size_t>(all_xy.size(), 1));
-  out->scr_side.ensure(static_cast<size_t>(std::max(nc, 1)) * n_nodes);
-  out->scr_gind.ensure(static_cast<size_t>(std::max(nc, 1)) * 6 * std::max(n_gp, 1));
-  out->scr_bad.ensure(std::max(n_gp, 1));
+  ctx->scratch.cxy.ensure(std::max<size_t>(all_xy.size(), 1));
+  ctx->scratch.side.ensure(static_cast<size_t>(std::max(nc, 1)) * n_nodes);
+  ctx->scratch.gind.ensure(static_cast<size_t>(std::max(nc, 1)) * 6 * std::max(n_gp, 1));
+  ctx->scratch.bad.ensure(std::max(n_gp, 1));
   if (!all_xy.empty())
-    CGB_CUDA(cudaMemcpyAsync(out->scr_cxy.p, all_xy.data(), all_xy.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-  int8_t* side = out->scr_side.p;
-  double* gind = out->scr_gind.p;
+    CGB_CUDA(cudaMemcpyAsync(ctx->scratch.cxy.p, all_xy.data(), all_xy.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  int8_t* side = ctx->scratch.side.p;
+  double* gind = ctx->scratch.gind.p;
   std::vector<DevCrease> dcr(nc);
   prof_begin(ctx, CGB_PHASE_CREASE);
   for (int c = 0; c < nc; ++c) {
-    dcr[c] = DevCrease{out->scr_cxy.p + off[c], static_cast<int>(creases[c].xy.size() / 2), creases[c].extend_start,
+    dcr[c] = DevCrease{ctx->scratch.cxy.p + off[c], static_cast<int>(creases[c].xy.size() / 2), creases[c].extend_start,
                        creases[c].extend_end, creases[c].is_closed};
     node_side_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, ctx->node_xy.p, dcr[c],
                                                                  side + static_cast<int64_t>(c) * n_nodes);
@@ -1256,7 +1346,7 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   if (out->psi.n < static_cast<size_t>(std::max<int64_t>(nnz, 1))) out->psi.alloc(nnz);
   if (out->dpsi.n < static_cast<size_t>(std::max<int64_t>(2 * nnz, 1))) out->dpsi.alloc(2 * nnz);
   if (out->ddpsi.n < static_cast<size_t>(std::max<int64_t>(3 * nnz, 1))) out->ddpsi.alloc(3 * nnz);
-  int8_t* bad = out->scr_bad.p;
+  int8_t* bad = ctx->scratch.bad.p;
   const double* d_rn = out->has_rho_node ? out->rho_node.p : nullptr;
   const bool mixed = out->precision == CGB_SHAPE_MIXED;
   auto pair_of = [](double v) {
@@ -1269,26 +1359,26 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
               0.0, nullptr, nullptr, nullptr, nullptr, 0, n_gp};
   prof_begin(ctx, CGB_PHASE_RKPM);
   if (mixed && n_nodes > 0) {
-    out->scr_node_pair.ensure(2 * static_cast<size_t>(n_nodes));
+    ctx->scratch.node_pair.ensure(2 * static_cast<size_t>(n_nodes));
     node_pair_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, ctx->node_xy.p, d_rn, out->rho,
-                                                                 out->scr_node_pair.p);
-    ra.node_pair = out->scr_node_pair.p;
+                                                                 ctx->scratch.node_pair.p);
+    ra.node_pair = ctx->scratch.node_pair.p;
   }
   int nl = mixed && n_nodes > 0 ? 1 : 0;
   if (n_gp > 0) {
     nl += mixed || d_rn ? 1 : 0;
-    out->scr_tip.ensure(n_gp);
+    ctx->scratch.tip.ensure(n_gp);
     ra.ir = 1.0 / out->rho;
-    ra.tip = out->scr_tip.p;
+    ra.tip = ctx->scratch.tip.p;
     const float* rec = nullptr;
     if (mixed) {
-      out->scr_point_rec.ensure(static_cast<size_t>(n_gp) * pair_record_floats(nc));
-      point_pair_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(ra, out->scr_point_rec.p);
-      rec = out->scr_point_rec.p;
+      ctx->scratch.point_rec.ensure(static_cast<size_t>(n_gp) * pair_record_floats(nc));
+      point_pair_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(ra, ctx->scratch.point_rec.p);
+      rec = ctx->scratch.point_rec.p;
     } else if (d_rn) {
-      out->scr_fac.ensure(n_nodes);
-      node_fac_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, d_rn, out->rho, out->scr_fac.p);
-      ra.fac = out->scr_fac.p;
+      ctx->scratch.fac.ensure(n_nodes);
+      node_fac_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, d_rn, out->rho, ctx->scratch.fac.p);
+      ra.fac = ctx->scratch.fac.p;
     }
     switch (out->order) {
       case 1: nl += mixed ? rkpm<1, true>(ctx, out, ra, rec) : rkpm<1, false>(ctx, out, ra, rec); break;
@@ -1301,11 +1391,11 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   // The reference's guards (GlobalRKPM.h:241-257 after the 3x3 block, 347-359 after
   // the bordering): singular first, then pivot collapse.
   int found[4] = {0, n_gp, 0, n_gp};
-  out->scr_guard.ensure(4);
-  CGB_CUDA(cudaMemcpyAsync(out->scr_guard.p, found, sizeof(found), cudaMemcpyHostToDevice, st));
-  if (n_gp > 0) guard_kernel<<<blocks_for(n_gp, 256), 256, 0, st>>>(n_gp, bad, out->scr_guard.p);
+  ctx->scratch.guard.ensure(4);
+  CGB_CUDA(cudaMemcpyAsync(ctx->scratch.guard.p, found, sizeof(found), cudaMemcpyHostToDevice, st));
+  if (n_gp > 0) guard_kernel<<<blocks_for(n_gp, 256), 256, 0, st>>>(n_gp, bad, ctx->scratch.guard.p);
   CGB_CUDA(cudaGetLastError());
-  CGB_CUDA(cudaMemcpyAsync(found, out->scr_guard.p, sizeof(found), cudaMemcpyDeviceToHost, st));
+  CGB_CUDA(cudaMemcpyAsync(found, ctx->scratch.guard.p, sizeof(found), cudaMemcpyDeviceToHost, st));
   CGB_CUDA(cudaStreamSynchronize(st));
   const int n1 = found[0], f1 = found[1], n2 = found[2], f2 = found[3];
   auto count_of = [&](size_t g) {
