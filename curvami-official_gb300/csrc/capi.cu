@@ -253,11 +253,13 @@ int cgb_set_nodes(cgb_context* ctx, const double* node_xy, int n_nodes) {
     if (ctx->n_nodes != n_nodes || !std::equal(node_xy, node_xy + m, ctx->h_node_xy.begin())) ++ctx->node_gen;
     ctx->n_nodes = n_nodes;
     ctx->h_node_xy.assign(node_xy, node_xy + m);
-    for (int c = 0; c < 2; ++c) ctx->node_min[c] = ctx->node_max[c] = node_xy[c];
-    for (size_t i = 0; i < m; ++i) {
-      ctx->node_min[i & 1] = std::min(ctx->node_min[i & 1], node_xy[i]);
-      ctx->node_max[i & 1] = std::max(ctx->node_max[i & 1], node_xy[i]);
+    double x0 = node_xy[0], x1 = x0, y0 = node_xy[1], y1 = y0;
+    for (size_t i = 0; i < m; i += 2) {
+      x0 = std::min(x0, node_xy[i]); x1 = std::max(x1, node_xy[i]);
+      y0 = std::min(y0, node_xy[i + 1]); y1 = std::max(y1, node_xy[i + 1]);
     }
+    ctx->node_min[0] = x0; ctx->node_min[1] = y0;
+    ctx->node_max[0] = x1; ctx->node_max[1] = y1;
     cgb::upload(ctx->node_xy, node_xy, 2 * static_cast<size_t>(n_nodes), ctx->stream);
     CGB_CUDA(cudaStreamSynchronize(ctx->stream));
   });

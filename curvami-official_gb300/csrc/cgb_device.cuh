@@ -27,13 +27,34 @@ struct DevCrease {
   const double* xy;  // 2 * n_vertices
   int n_vertices;
   int extend_start, extend_end, is_closed;
+  const float2* xyf;  // the vertices relative to the first, in float
+  float extent;       // their largest coordinate
 };
+
+// Squared distance in float of a point (relative to the crease's first vertex) to segment i.
+__device__ __forceinline__ float segment_dist2f(const DevCrease& c, int i, float px, float py) {
+  const float2 A = c.xyf[i], B = c.xyf[i + 1];
+  const float vx = B.x - A.x, vy = B.y - A.y, wx = px - A.x, wy = py - A.y;
+  const float v2 = vx * vx + vy * vy;
+  float t = v2 > 0.0f ? __fdividef(wx * vx + wy * vy, v2) : 0.0f;
+  if (!(i == 0 && c.extend_start)) t = fmaxf(t, 0.0f);
+  if (!(i == c.n_vertices - 2 && c.extend_end)) t = fminf(t, 1.0f);
+  const float ex = wx - t * vx, ey = wy - t * vy;
+  return ex * ex + ey * ey;
+}
 
 // Enrichment::evaluateIndicator (core/include/curvami/Enrichment.h:23-92). The
 // geometric decisions (closest segment with a strict '<', clamping of t, the 1e-12
 // validity distance, the end caps, the side test) are evaluated with explicitly
 // rounded operations, so they are taken exactly as a non-contracted FP64 CPU run
 // takes them.
+// Segments that cannot be the closest are left out by a float pass. With X a bound on the relative
+// coordinates, rounding them (2^-24 X each) and the float arithmetic move a segment's distance by
+// less than eps = 2^-18 X (the foot's error along the segment, 2^-20 X, is the largest part); a
+// segment more than 4 eps beyond the closest one's float distance is therefore farther than it by
+// 2 eps, far more than the FP64 comparison resolves, and the walk over the others in their order
+// ends where the walk over all would. The FP64 work of a point, some 45 operations a segment with a
+// division, falls from all segments to a few (a point that all are equally far from keeps all).
 struct DevIndicator {
   double f, gx, gy, hxx, hyy, hxy;
 };
@@ -46,7 +67,19 @@ __device__ __forceinline__ DevIndicator eval_indicator(double px, double py, con
   double d = inf;
   double Cx = 0, Cy = 0, t_best = 0, snx = 0, sny = 0;
   int idx_best = 0;
+  const bool sift = N > 4;
+  float fx = 0.0f, fy = 0.0f, limit = 0.0f;
+  if (sift) {
+    fx = __double2float_rn(px - c.xy[0]);
+    fy = __double2float_rn(py - c.xy[1]);
+    float least = __int_as_float(0x7f800000);
+    for (int i = 0; i < N - 1; ++i) least = fminf(least, segment_dist2f(c, i, fx, fy));
+    const float eps = fmaxf(fmaxf(fabsf(fx), fabsf(fy)), c.extent) * (1.0f / 262144.0f);
+    limit = sqrtf(least) + 4.0f * eps;
+    limit *= limit;
+  }
   for (int i = 0; i < N - 1; ++i) {
+    if (sift && segment_dist2f(c, i, fx, fy) > limit) continue;
     const double Ax = c.xy[2 * i], Ay = c.xy[2 * i + 1];
     const double Bx = c.xy[2 * i + 2], By = c.xy[2 * i + 3];
     const double vx = __dsub_rn(Bx, Ax), vy = __dsub_rn(By, Ay);

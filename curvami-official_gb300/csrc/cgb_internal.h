@@ -94,6 +94,7 @@ struct ShapeScratch {
   DevBuf<uint32_t> gp_mask;
   // Creases and RKPM.
   DevBuf<double> cxy;        // crease vertices, all creases
+  DevBuf<float2> cxyf;       // the same relative to each crease's first, in float
   DevBuf<int8_t> side;       // n_creases * n_nodes
   DevBuf<double> gind;       // n_creases * 6 * n_gp
   DevBuf<int8_t> bad, tip;   // n_gp

@@ -1320,25 +1320,37 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
     off[c + 1] = all_xy.size();
   }
   ctx->scratch.cxy.ensure(std::max<size_t>(all_xy.size(), 1));
+  ctx->scratch.cxyf.ensure(std::max<size_t>(all_xy.size() / 2, 1));
+  std::vector<float2> all_f(all_xy.size() / 2);
+  std::vector<float> extent(nc, 0.0f);
+  for (int c = 0; c < nc; ++c)
+    for (size_t v = off[c]; v < off[c + 1]; v += 2) {
+      const float2 f = make_float2(static_cast<float>(all_xy[v] - all_xy[off[c]]),
+                                   static_cast<float>(all_xy[v + 1] - all_xy[off[c] + 1]));
+      all_f[v / 2] = f;
+      extent[c] = std::max(extent[c], std::max(std::fabs(f.x), std::fabs(f.y)));
+    }
   ctx->scratch.side.ensure(static_cast<size_t>(std::max(nc, 1)) * n_nodes);
   ctx->scratch.gind.ensure(static_cast<size_t>(std::max(nc, 1)) * 6 * std::max(n_gp, 1));
   ctx->scratch.bad.ensure(std::max(n_gp, 1));
   if (!all_xy.empty())
     CGB_CUDA(cudaMemcpyAsync(ctx->scratch.cxy.p, all_xy.data(), all_xy.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  if (!all_f.empty())
+    CGB_CUDA(cudaMemcpyAsync(ctx->scratch.cxyf.p, all_f.data(), all_f.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
   int8_t* side = ctx->scratch.side.p;
   double* gind = ctx->scratch.gind.p;
   std::vector<DevCrease> dcr(nc);
   prof_begin(ctx, CGB_PHASE_CREASE);
   for (int c = 0; c < nc; ++c) {
     dcr[c] = DevCrease{ctx->scratch.cxy.p + off[c], static_cast<int>(creases[c].xy.size() / 2), creases[c].extend_start,
-                       creases[c].extend_end, creases[c].is_closed};
-    node_side_kernel<<<blocks_for(n_nodes), kThreads, 0, st>>>(n_nodes, ctx->node_xy.p, dcr[c],
+                       creases[c].extend_end, creases[c].is_closed, ctx->scratch.cxyf.p + off[c] / 2, extent[c]};
+    node_side_kernel<<<blocks_for(n_nodes, 32), 32, 0, st>>>(n_nodes, ctx->node_xy.p, dcr[c],
                                                                  side + static_cast<int64_t>(c) * n_nodes);
   }
   // Gauss-point indicators laid out [g][c][6].
   if (nc > 0 && n_gp > 0)
     for (int c = 0; c < nc; ++c)
-      gp_indicator_kernel<<<blocks_for(n_gp), kThreads, 0, st>>>(n_gp, out->gp_xy.p, dcr[c], c, nc, gind);
+      gp_indicator_kernel<<<blocks_for(n_gp, 64), 64, 0, st>>>(n_gp, out->gp_xy.p, dcr[c], c, nc, gind);
   prof_end(ctx, CGB_PHASE_CREASE, nc * (1 + (n_gp > 0 ? 1 : 0)));
   CGB_CUDA(cudaGetLastError());
 
