@@ -123,7 +123,7 @@ int cgb_shape_concat(cgb_context* ctx, const cgb_shape* const* sets, const int32
                      cgb_shape** out) {
   if (!ctx || !out) return CGB_ERR_INVALID;
   *out = nullptr;
-  auto* sh = new cgb_shape();
+  auto* sh = new cgb_shape(&ctx->shape_pool);
   const int rc = guarded_ctx(ctx, [&] {
     if (n_sets < 1 || !sets || !node_offset) throw Error(CGB_ERR_INVALID, "cgb_shape_concat: empty set list");
     CGB_CUDA(cudaSetDevice(ctx->device));

@@ -145,6 +145,7 @@ int cgb_create(int device, cgb_context** out) {
     bind_device(ctx);
     CGB_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = true;
+    ctx->shape_pool.create(device);
     ctx->dev_err.alloc(1);
     CGB_CUDA(cudaMemsetAsync(ctx->dev_err.p, 0, sizeof(int), ctx->stream));
     CGB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -152,6 +153,7 @@ int cgb_create(int device, cgb_context** out) {
   if (rc != CGB_OK) {
     static thread_local std::string msg;
     msg = ctx->last_error;
+    ctx->shape_pool.destroy();
     delete ctx;
     return rc;
   }
@@ -179,6 +181,7 @@ void ctx_release(cgb_context* ctx) {
   ctx->ws_x.reset();
   ctx->ws_out.reset();
   ctx->scratch = cgb::ShapeScratch{};
+  ctx->shape_pool.destroy();
   for (auto& m : ctx->marks) {
     if (m.start) cudaEventDestroy(m.start);
     if (m.stop) cudaEventDestroy(m.stop);
@@ -285,7 +288,7 @@ int cgb_shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_s
                     const cgb_crease* creases, int n_creases, cgb_shape** out) {
   if (!ctx || !out) return CGB_ERR_INVALID;
   *out = nullptr;
-  auto* sh = new cgb_shape();
+  auto* sh = new cgb_shape(&ctx->shape_pool);
   const int rc = guarded(ctx, [&] {
     need(params != nullptr, "cgb_shape_build: params is NULL");
     need(n_gp == 0 || gp_xy, "cgb_shape_build: gp_xy is NULL");
@@ -319,7 +322,7 @@ int cgb_shape_from_host(cgb_context* ctx, int n_gp, const int64_t* nbr_ptr, cons
                         const double* psi, const double* dpsi, const double* ddpsi, cgb_shape** out) {
   if (!ctx || !out) return CGB_ERR_INVALID;
   *out = nullptr;
-  auto* sh = new cgb_shape();
+  auto* sh = new cgb_shape(&ctx->shape_pool);
   const int rc = guarded(ctx, [&] {
     need(n_gp >= 0 && nbr_ptr, "cgb_shape_from_host: nbr_ptr is NULL");
     bind_device(ctx);
@@ -399,8 +402,11 @@ int cgb_shape_destroy(cgb_shape* sh) {
   if (!sh) return CGB_OK;
   cgb_context* ctx = sh->ctx;
   if (ctx) {
+    // The blocks go back to the context's pool for the next set: work on any stream that reads them
+    // is waited for, as cudaFree does.
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    cudaDeviceSynchronize();
   }
   delete sh;
   if (ctx) cgb::ctx_release(ctx);
