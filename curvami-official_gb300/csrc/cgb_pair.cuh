@@ -50,22 +50,74 @@ __device__ __forceinline__ fp2 fp2_two_prod(float a, float b) {
 
 __device__ __forceinline__ fp2 fp2_of(float a) { return {a, 0.0f}; }
 
-// Split of a double into a pair (per point or per node only: uses the FP64 pipe).
-__device__ __forceinline__ fp2 fp2_from_double(double d) {
-  const float hi = __double2float_rn(d);
-  return {hi, __double2float_rn(d - static_cast<double>(hi))};
-}
-
-// A float as a double, on the integer pipe: a conversion issues on the FP64 pipe, at 1/62 of the
-// rate. The exponent is rebiased from 127 to 1023; denormals, infinities and NaN convert.
+// Conversions between doubles and floats. Like an addition of doubles, the instructions for them
+// issue on the FP64 pipe, at 1/62 of the FP32 rate, so they are done on the bits; only exponents near
+// the ends of the float range, infinities and NaN in a pair take the instructions, in volatile asm so
+// that they are not executed beside the common path and selected. (Under a predicate they would still
+// take their turn on the pipe: fp2_to_double therefore converts several pairs at a time, behind one
+// branch.)
 __device__ __forceinline__ double fp2_widen(float f) {
-  const uint32_t u = __float_as_uint(f), e = u & 0x7f800000u;
-  if (e == 0x7f800000u || (e == 0u && (u << 1) != 0u)) return static_cast<double>(f);
-  const uint32_t hi = (u & 0x80000000u) | (e == 0u ? 0u : ((u & 0x7fffffffu) >> 3) + 0x38000000u);
-  return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
+  const uint32_t sign = __float_as_uint(f) & 0x80000000u;
+  uint32_t m = __float_as_uint(f) & 0x7fffffffu, bias = 0x38000000u;   // exponent from 127 to 1023
+  if (m >= 0x7f800000u) bias = 0x70000000u;                            // infinity, NaN: from 255 to 2047
+  if (m < 0x00800000u) {                                               // zero; denormals times 2^64
+    m = __float_as_uint(__fmul_rn(__uint_as_float(m), 0x1p64f));
+    bias = m == 0u ? 0u : 0x34000000u;
+  }
+  return __hiloint2double(static_cast<int>(((m >> 3) + bias) | sign), static_cast<int>(m << 29));
 }
 
-__device__ __forceinline__ double fp2_to_double(fp2 a) { return fp2_widen(a.hi) + fp2_widen(a.lo); }
+// hi = the double rounded to 24 bits, lo = the other 29 bits rounded to 24.
+__device__ __forceinline__ fp2 fp2_from_double(double d) {
+  const uint32_t h = static_cast<uint32_t>(__double2hiint(d)), l = static_cast<uint32_t>(__double2loint(d));
+  const uint32_t e = (h >> 20) & 0x7ffu, sign = h & 0x80000000u;
+  const uint32_t low = l & 0x1fffffffu, up = low >> 28;
+  const uint32_t hi = __funnelshift_l(l, h & 0x7fffffffu, 3) - 0xc0000000u + up;   // exponent - 896
+  const float lo = __int2float_rn(static_cast<int>(low) - static_cast<int>(up << 29)) * __uint_as_float((e - 948u) << 23);
+  fp2 r = {__uint_as_float(hi | sign), __uint_as_float(__float_as_uint(lo) ^ sign)};
+  if (((h << 1) | l) == 0u) {
+    r = {__uint_as_float(sign), 0.0f};
+  } else if (e < 949u || e > 1149u) {   // lo would be denormal, or hi may round to infinity
+    asm volatile("{\n\t.reg .f64 a;\n\tcvt.rn.f32.f64 %0, %2;\n\tcvt.f64.f32 a, %0;\n\tsub.rn.f64 a, %2, a;\n\t"
+                 "cvt.rn.f32.f64 %1, a;\n\t}" : "=&f"(r.hi), "=f"(r.lo) : "d"(d));
+  }
+  return r;
+}
+
+// hi + lo rounded to double, normalised or not. Normalised, lo in units of the last place of hi as a
+// double is rounded to an integer and added to its bits; below a power of two those units are half
+// as large.
+template <int N>
+__device__ __forceinline__ void fp2_to_double(const fp2 (&b)[N], double (&d)[N]) {
+  bool rest = false;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const fp2 a = fp2_two_sum(b[k].hi, b[k].lo);
+    const uint32_t u = __float_as_uint(a.hi), sign = u & 0x80000000u, m = u & 0x7fffffffu, e = m >> 23;
+    float t = __fmul_rn(a.lo, __uint_as_float((306u - e) << 23));   // lo 2^(52 - exponent)
+    t = __uint_as_float(__float_as_uint(t) ^ sign);
+    if ((u & 0x7fffffu) == 0u && t < 0.0f) t = __fadd_rn(t, t);
+    const bool zero = (m | (__float_as_uint(a.lo) << 1)) == 0u;
+    const long long bits = __double_as_longlong(__hiloint2double(static_cast<int>((m >> 3) + 0x38000000u), static_cast<int>(m << 29)))
+                           + __float2int_rn(t);
+    d[k] = __longlong_as_double(bits | static_cast<long long>(static_cast<unsigned long long>(sign) << 32));
+    if (zero) d[k] = __hiloint2double(static_cast<int>(__float_as_uint(b[k].hi) & __float_as_uint(b[k].lo) & 0x80000000u), 0);
+    rest = rest || (!zero && (e < 52u || e == 255u || !(fabsf(t) <= 268435456.0f)));   // 2^28: half a unit of hi
+  }
+  if (rest) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      asm volatile("{\n\t.reg .f64 a, b;\n\tcvt.f64.f32 a, %1;\n\tcvt.f64.f32 b, %2;\n\tadd.rn.f64 %0, a, b;\n\t}"
+                   : "=d"(d[k]) : "f"(b[k].hi), "f"(b[k].lo));
+  }
+}
+
+__device__ __forceinline__ double fp2_to_double(fp2 a) {
+  const fp2 b[1] = {a};
+  double d[1];
+  fp2_to_double(b, d);
+  return d[0];
+}
 
 __device__ __forceinline__ fp2 operator-(fp2 a) { return {-a.hi, -a.lo}; }
 

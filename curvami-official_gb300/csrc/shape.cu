@@ -161,19 +161,22 @@ __global__ void frnn_kernel(int n_gp, const double* __restrict__ gp_xy,
   }
 }
 
-// The point of entry e of the points [g0, g1): lane 0 of each warp finds it for the warp's first
-// entry by bisection, the other lanes step forward from there. Every lane of the warp calls it.
+// The point of entry e of the points [g0, g1): the warp finds it for its first entry, 32 probes at a
+// time (four dependent loads for 262,144 points, where a bisection takes 18), and the lanes step
+// forward from there. Every lane of the warp calls it.
 __device__ __forceinline__ int point_of(const int64_t* __restrict__ ptr, int g0, int g1, int64_t e, int64_t e_end) {
-  int lo = g0;
-  if ((threadIdx.x & 31) == 0) {
-    const int64_t ef = e < e_end ? e : e_end - 1;
-    int hi = g1;                       // ptr[lo] <= ef < ptr[hi]
-    while (hi - lo > 1) {
-      const int mid = lo + (hi - lo) / 2;
-      if (__ldg(ptr + mid) <= ef) lo = mid; else hi = mid;
-    }
+  const int lane = threadIdx.x & 31;
+  const int64_t ef = __shfl_sync(0xffffffffu, e < e_end ? e : e_end - 1, 0);
+  int lo = g0, n = g1 - g0;            // the point is one of [lo, lo + n): ptr[lo] <= ef < ptr[lo + n]
+  while (n > 1) {
+    const int step = (n - 1) / 32 + 1;
+    const int at = lo + lane * step;
+    const bool below = lane * step < n && __ldg(ptr + at) <= ef;
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, below));   // lane 0 is always below
+    lo += last * step;
+    n = min(step, n - last * step);
   }
-  int g = __shfl_sync(0xffffffffu, lo, 0);
+  int g = lo;
   if (e < e_end)
     while (__ldg(ptr + g + 1) <= e) ++g;
   return g;
@@ -299,15 +302,6 @@ __global__ void gp_indicator_kernel(int n_gp, const double* __restrict__ gp_xy, 
   o[0] = I.f; o[1] = I.gx; o[2] = I.gy; o[3] = I.hxx; o[4] = I.hyy; o[5] = I.hxy;
 }
 
-template <int NP>
-struct PackedIdx {
-  // K[i][j] of GlobalRKPM.h:29-36, row-major over i <= j.
-  __device__ __forceinline__ static int k(int i, int j) {
-    const int a = i < j ? i : j, b = i < j ? j : i;
-    return a * NP - a * (a - 1) / 2 + (b - a);
-  }
-};
-
 __device__ __forceinline__ void inv3(const double m[3][3], double r[3][3]) {
   const double c00 = m[1][1] * m[2][2] - m[1][2] * m[2][1];
   const double c10 = m[1][2] * m[2][0] - m[1][0] * m[2][2];
@@ -346,97 +340,82 @@ struct RawIdx {
   __host__ __device__ static constexpr int bx(int i) { return deg(i) - by(i); }
 };
 
-// Row 0 of M^-1 and its five jets at one point.
+// The polynomials of one point, scaled by their powers of rho: C, C_x, C_y, C_xx, C_yy, C_xy of
+// GlobalRKPM.h:363-396, coefficients of the monomials of xi, eta.
 template <int ORDER>
 struct RowJets {
   static constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
   double c0[NP], c0x[NP], c0y[NP], c0xx[NP], c0yy[NP], c0xy[NP];
 };
 
-// The per-point part of GlobalRKPM::solve (GlobalRKPM.h:161-359) from the raw-moment sums
-// S^g_ab of the six weight jets (FP64): M and its jets, the reference's guards, and row 0
-// of M^-1 with its jets. Returns the guard code (0 fine, 1 singular, 2 pivot collapse).
+// The per-point part of GlobalRKPM::solve (GlobalRKPM.h:161-396) from the raw-moment sums of the six
+// weight jets (FP64): M, the reference's guards, and the polynomials that multiply the jets. Returns
+// the guard code (0 fine, 1 singular, 2 pivot collapse).
 //
-// Moments (GlobalRKPM.h:161-189): M, dMx, dMy, d2Mxx, d2Myy, d2Mxy. Every entry of
-// M = sum_I w_I p_I p_I^T is a raw moment mu_ab = sum_I w_I xi^a eta^b with
-// a + b <= 2 ORDER, and the jets follow from the weight jets by the product rule,
-//   D_x mu_ab = S^x_ab + a S_{a-1,b},   D_xx mu_ab = S^xx_ab + 2a S^x_{a-1,b} + a(a-1) S_{a-2,b},
-//   D_xy mu_ab = S^xy_ab + b S^x_{a,b-1} + a S^y_{a-1,b} + ab S_{a-1,b-1}   (y alike),
-// with S^g_ab = sum_I (D^g w_I) xi^a eta^b.
-// at(g, a, b): S^g_ab for g = 0 (w), 1 (x), 2 (y), 3 (xx), 4 (yy), 5 (xy).
+// Every entry of M = sum_I w_I p_I p_I^T is a raw moment, and so is every entry of the S^g =
+// sum_I (D^g w_I) p_I p_I^T. With p_x = D p (a constant matrix) M_x = S^x + D M + M D^T. The
+// reference's C = b . p, b = M^-1 e0, has the derivative C_x = (b_x + D^T b) . p; written for
+// c = b_x + D^T b the terms D M and M D^T of M_x b_x = -M^-1 M_x b become constants:
+//   M b = e0,   M c_x = -S^x b - D_x e0,
+//   M c_xx = -S^xx b - 2 S^x c_x + D_x D_x e0,   M c_xy = -S^xy b - S^x c_y - S^y c_x + D_x D_y e0
+// (y alike), with D_x e0 the unit vector of xi, D_x D_x e0 twice that of xi^2, D_x D_y e0 that of
+// xi eta. So neither the jets of M (135 of 1,050 FP64 operations for the quadratic basis) nor the
+// derivatives of the basis on the coefficients (40) are formed. 262,144 points,
+// quadratic: 485 -> 373 us, with the coefficients left as pairs 560 -> 385 us.
+// at(g, a, b): S^g_ab = sum_I (D^g w_I) xi^a eta^b for g = 0 (w), 1 (x), 2 (y), 3 (xx), 4 (yy), 5 (xy).
 template <int ORDER, class Sums>
-__device__ __forceinline__ int point_solve(const Sums& sums, RowJets<ORDER>& R) {
+__device__ __forceinline__ int point_solve(const Sums& at, RowJets<ORDER>& R) {
   constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
-  constexpr int NM = NP * (NP + 1) / 2;
-  using PI = PackedIdx<NP>;
   using RI = RawIdx<ORDER>;
-  double M[NM], Mx[NM], My[NM], Mxx[NM], Myy[NM], Mxy[NM];
-  {
-    auto at = [&](int g, int aa, int bb) { return (aa < 0 || bb < 0) ? 0.0 : sums(g, aa, bb); };
-#pragma unroll
-    for (int ip = 0; ip < NP; ++ip) {
-#pragma unroll
-      for (int jp = ip; jp < NP; ++jp) {
-        const int k = PI::k(ip, jp);
-        const int A = RI::bx(ip) + RI::bx(jp), Bq = RI::by(ip) + RI::by(jp);
-        const double fa = static_cast<double>(A), fb = static_cast<double>(Bq);
-        M[k] = at(0, A, Bq);
-        Mx[k] = at(1, A, Bq) + fa * at(0, A - 1, Bq);
-        My[k] = at(2, A, Bq) + fb * at(0, A, Bq - 1);
-        Mxx[k] = at(3, A, Bq) + 2.0 * fa * at(1, A - 1, Bq) + fa * (fa - 1.0) * at(0, A - 2, Bq);
-        Myy[k] = at(4, A, Bq) + 2.0 * fb * at(2, A, Bq - 1) + fb * (fb - 1.0) * at(0, A, Bq - 2);
-        Mxy[k] = at(5, A, Bq) + fb * at(1, A, Bq - 1) + fa * at(2, A - 1, Bq) + fa * fb * at(0, A - 1, Bq - 1);
-      }
-    }
-  }
+  auto entry = [&](int g, int i, int j) { return at(g, RI::bx(i) + RI::bx(j), RI::by(i) + RI::by(j)); };
 
   // The reference inverts M by blocks (GlobalRKPM.h:197-345): the leading 3x3 block with
   // a residual guard, then one bordering step per further basis function with a Schur-pivot
-  // guard, carrying the five derivative jets of the whole inverse along. The shape
-  // functions only use row 0 of M^-1 and its jets, i.e. b = M^-1 e0 and
-  //   b_x = -M^-1 (M_x b),  b_xx = -M^-1 (M_xx b + 2 M_x b_x),
-  //   b_xy = -M^-1 (M_xy b + M_x b_y + M_y b_x)   (y alike),
-  // so M is factored once (LDL^T, no pivoting: M is symmetric positive semi-definite) and
-  // six solves give b and its jets - about a quarter of the FP64 work of the full inverse
-  // jets. The guards are evaluated as the reference does: the 3x3 residual test on the
-  // leading block, and the pivot test on the Schur complements, which are the LDL^T pivots
-  // d_k for k >= 3.
+  // guard, carrying the five derivative jets of the whole inverse along. Here M is factored once
+  // (LDL^T, no pivoting: M is symmetric positive semi-definite). The guards are evaluated as the
+  // reference does: the 3x3 residual test on the leading block, and the pivot test on the Schur
+  // complements, which are the LDL^T pivots d_k for k >= 3.
   int bad = 0;
   {
     double m3[3][3];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) m3[r][c] = M[PI::k(r, c)];
+      for (int c = 0; c < 3; ++c) m3[r][c] = entry(0, r, c);
     double inv[3][3], chk[3][3];
     inv3(m3, inv);
     mm3(m3, inv, chk);
-    bool finite = true;
-    double res = 0.0;
+    // |chk - I| <= 1e-8 on the bits: a comparison of doubles issues on the FP64 pipe. NaN passes,
+    // as it does through fmax.
+    const long long mag = 0x7fffffffffffffffll, inf = 0x7ff0000000000000ll;
+    const long long lim = __double_as_longlong(1e-8);
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        if (!isfinite(inv[r][c])) finite = false;
-        res = fmax(res, fabs(chk[r][c] - (r == c ? 1.0 : 0.0)));
+        const long long res = __double_as_longlong(chk[r][c] - (r == c ? 1.0 : 0.0)) & mag;
+        if (!isfinite(inv[r][c]) || (res > lim && res <= inf)) bad = 1;
       }
-    if (!finite || res > 1e-8) bad = 1;
   }
-  // LDL^T of M: L unit lower (packed like M, strictly lower part used), D diagonal.
+  // LDL^T of M: L unit lower, iD the reciprocal pivots.
   double Lf[NP][NP], Dg[NP], iD[NP];
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
-    double d = M[PI::k(j, j)];
+    const double mjj = entry(0, j, j);
+    double d = mjj, LD[NP];
 #pragma unroll
-    for (int q = 0; q < j; ++q) d -= Lf[j][q] * Lf[j][q] * Dg[q];
+    for (int q = 0; q < j; ++q) {
+      LD[q] = Lf[j][q] * Dg[q];
+      d -= Lf[j][q] * LD[q];
+    }
     Dg[j] = d;
     iD[j] = 1.0 / d;
-    if (j >= 3 && !(fabs(d) > 1e-12 * fmax(fabs(M[PI::k(j, j)]), 1.0)) && bad == 0) bad = 2;
+    if (j >= 3 && !(fabs(d) > 1e-12 * fmax(fabs(mjj), 1.0)) && bad == 0) bad = 2;
 #pragma unroll
     for (int i = j + 1; i < NP; ++i) {
-      double v = M[PI::k(i, j)];
+      double v = entry(0, i, j);
 #pragma unroll
-      for (int q = 0; q < j; ++q) v -= Lf[i][q] * Lf[j][q] * Dg[q];
+      for (int q = 0; q < j; ++q) v -= Lf[i][q] * LD[q];
       Lf[i][j] = v * iD[j];
     }
   }
@@ -453,33 +432,29 @@ __device__ __forceinline__ int point_solve(const Sums& sums, RowJets<ORDER>& R) 
 #pragma unroll
       for (int q = i + 1; q < NP; ++q) x[i] -= Lf[q][i] * x[q];
   };
-  // y += alpha * S x for a packed symmetric S.
-  auto symv = [&](const double* S, const double* x, double alpha, double* y) {
+  // y -= S^g x.
+  auto symv = [&](int g, const double* x, double* y) {
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      double t = 0.0;
+    for (int i = 0; i < NP; ++i)
 #pragma unroll
-      for (int q = 0; q < NP; ++q) t += S[PI::k(i, q)] * x[q];
-      y[i] += alpha * t;
-    }
+      for (int q = 0; q < NP; ++q) y[i] -= entry(g, i, q) * x[q];
   };
-  double(&c0)[NP] = R.c0;
-  double(&c0x)[NP] = R.c0x;
-  double(&c0y)[NP] = R.c0y;
-  double(&c0xx)[NP] = R.c0xx;
-  double(&c0yy)[NP] = R.c0yy;
-  double(&c0xy)[NP] = R.c0xy;
+  // y <- the value v at the monomial xi^a eta^b.
+  auto unit = [&](double* y, int a, int b, double v) {
 #pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    c0[i] = i == 0 ? 1.0 : 0.0;
-    c0x[i] = 0.0; c0y[i] = 0.0; c0xx[i] = 0.0; c0yy[i] = 0.0; c0xy[i] = 0.0;
-  }
-  solve(c0);
-  symv(Mx, c0, -1.0, c0x); solve(c0x);
-  symv(My, c0, -1.0, c0y); solve(c0y);
-  symv(Mxx, c0, -1.0, c0xx); symv(Mx, c0x, -2.0, c0xx); solve(c0xx);
-  symv(Myy, c0, -1.0, c0yy); symv(My, c0y, -2.0, c0yy); solve(c0yy);
-  symv(Mxy, c0, -1.0, c0xy); symv(Mx, c0y, -1.0, c0xy); symv(My, c0x, -1.0, c0xy); solve(c0xy);
+    for (int i = 0; i < NP; ++i) y[i] = a + b <= ORDER && i == RI::r(a, b) ? v : 0.0;
+  };
+  auto twice = [&](const double* x, double* y) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) y[i] = x[i] + x[i];
+  };
+  double t[NP];
+  unit(R.c0, 0, 0, 1.0); solve(R.c0);
+  unit(R.c0x, 1, 0, -1.0); symv(1, R.c0, R.c0x); solve(R.c0x);
+  unit(R.c0y, 0, 1, -1.0); symv(2, R.c0, R.c0y); solve(R.c0y);
+  unit(R.c0xx, 2, 0, 2.0); symv(3, R.c0, R.c0xx); twice(R.c0x, t); symv(1, t, R.c0xx); solve(R.c0xx);
+  unit(R.c0yy, 0, 2, 2.0); symv(4, R.c0, R.c0yy); twice(R.c0y, t); symv(2, t, R.c0yy); solve(R.c0yy);
+  unit(R.c0xy, 1, 1, 1.0); symv(5, R.c0, R.c0xy); symv(1, R.c0y, R.c0xy); symv(2, R.c0x, R.c0xy); solve(R.c0xy);
   return bad;
 }
 
@@ -529,8 +504,8 @@ struct RkpmArgs {
 //  - rkpm_value_kernel, one pair per thread, evaluates them (about 60 operations) over the pair's
 //    jets: reading them back is a tenth of computing them again.
 // Measured on 300,000 points (28 neighbours, quadratic): RKPM 10.7 ms as one kernel of 90 sums and
-// both passes, about 650 operations per neighbour; 3.7 ms so (moments 2.4, solve 0.5, values 0.85).
-// 32,400 points with 113 neighbours, cubic, half of them in a cap: 12.8 -> 3.5 ms.
+// both passes, about 650 operations per neighbour; 4.15 ms so (moments 2.7, solve 0.45, values 1.0).
+// 32,400 points with 113 neighbours, cubic, half of them in a cap: 12.8 -> 3.45 ms.
 template <int ORDER>
 struct MomIdx {
   static constexpr int D = 2 * ORDER;
@@ -714,9 +689,6 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
                 : q == 3 ? MI::bx(aa + 2, bb) : q == 4 ? MI::bx(aa, bb + 2) : MI::cx(aa + 1, bb + 1);
     return mom[(tip ? q * RI::NR + RI::r(aa, bb) : k) * np];
   }, R));
-  // The polynomials C, C_x / rho, C_y / rho, C_xx / rho^2, C_yy / rho^2, C_xy / rho^2 of
-  // GlobalRKPM.h:363-396: with b = row 0 of M^-1, C = b . p, C_x = b_x . p + b . p_x and so on,
-  // the derivatives of the monomials moved onto the coefficients.
   auto put = [&](int i, double v) {   // PAIR: as FP32 pairs, in the same 8 bytes
     if constexpr (PAIR) {
       const fp2 p = fp2_from_double(v);
@@ -726,22 +698,14 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
     }
   };
   const double r1 = a.ir, r2 = a.ir * a.ir;
-  auto co = [&](const double* c, int i, int p, int q) -> double {   // c of xi^(bx+p) eta^(by+q), times its derivative's factor
-    const int x = RI::bx(i) + p, y = RI::by(i) + q;
-    if (x + y > ORDER) return 0.0;
-    double v = c[RI::r(x, y)];
-    for (int k = 0; k < p; ++k) v *= static_cast<double>(x - k);
-    for (int k = 0; k < q; ++k) v *= static_cast<double>(y - k);
-    return v;
-  };
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     put(i, R.c0[i]);
-    put(NP + i, r1 * (R.c0x[i] + co(R.c0, i, 1, 0)));
-    put(2 * NP + i, r1 * (R.c0y[i] + co(R.c0, i, 0, 1)));
-    put(3 * NP + i, r2 * (R.c0xx[i] + 2.0 * co(R.c0x, i, 1, 0) + co(R.c0, i, 2, 0)));
-    put(4 * NP + i, r2 * (R.c0yy[i] + 2.0 * co(R.c0y, i, 0, 1) + co(R.c0, i, 0, 2)));
-    put(5 * NP + i, r2 * (R.c0xy[i] + co(R.c0y, i, 1, 0) + co(R.c0x, i, 0, 1) + co(R.c0, i, 1, 1)));
+    put(NP + i, r1 * R.c0x[i]);
+    put(2 * NP + i, r1 * R.c0y[i]);
+    put(3 * NP + i, r2 * R.c0xx[i]);
+    put(4 * NP + i, r2 * R.c0yy[i]);
+    put(5 * NP + i, r2 * R.c0xy[i]);
   }
 }
 
@@ -785,16 +749,13 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_value_kernel(RkpmArgs a) {
 
 // ---- mixed precision: the per-neighbour work in FP32 pairs ----------------------------
 //
-// The FP64 kernel spends about 650 FP64 operations per neighbour (differences and
-// divisions by rho, the window jets with their divisions by s, the crease product, the
-// 90 moment FMAs, then the jets again and the shape-function sums), and GB300 issues FP64
-// at 1/62 of the FP32 rate. The mixed kernels do all of that per-neighbour arithmetic in
-// FP32 pairs (cgb_pair.cuh, about 48 significant bits) on the FP32 pipe, and keep FP64
-// for the per-point part: the raw-moment sums are rounded to FP64 and point_solve forms
-// M and its jets, applies the reference's guards, factors M (LDL^T) and solves for row 0
-// of M^-1 and its jets exactly as the FP64 kernel does. Only the per-point factorisation
-// is FP64, which is 1/n of the work; the shape functions are then summed in pairs from the
-// FP64 row jets and rounded to FP64 once.
+// The FP64 kernels spend about 200 FP64 operations per neighbour, and GB300 issues FP64 at 1/62 of
+// the FP32 rate. The mixed kernels do that per-neighbour arithmetic in FP32 pairs (cgb_pair.cuh,
+// about 48 significant bits) on the FP32 pipe, conversions to and from doubles on the bits; only
+// point_solve, 1/n of the work, is FP64, as in the FP64 path. 1,000,000 points of 28 neighbours,
+// quadratic: RKPM 5.9 ms (jets 0.8, moments 2.4, solve 1.5, values 1.25); 7.1 ms with the FP64
+// pipe's conversions, the jets of M in the solve and a bisection in each warp of the pair
+// kernels.
 //
 // Coordinates: node and point coordinates are split into three floats each (72 bits, so
 // the split of a double is exact) and differenced in pairs, so xi = (x - x_I) / rho is
@@ -1026,16 +987,19 @@ __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float*
     }
   }
   const int64_t np = a.g1 - a.g0;
-  auto put = [&](int k, fp2 sum) {
-    double v = fp2_to_double(sum);
+  auto put = [&](int at, const auto& S) {
+    constexpr int N = sizeof(S) / sizeof(S[0]);
+    double v[N];
+    fp2_to_double(S, v);
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (mine && sub == 0) a.mom[k * np + (g - a.g0)] = v;
+    for (int k = 0; k < N; ++k) {
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+      if (mine && sub == 0) a.mom[(at + k) * np + (g - a.g0)] = v[k];
+    }
   };
-#pragma unroll
-  for (int k = 0; k < N0; ++k) put(AT0 + k, S0[k]);
-#pragma unroll
-  for (int k = 0; k < N1; ++k) put(AT1 + k, S1[k]);
+  put(AT0, S0);
+  if constexpr (N1 > 0) put(AT1, S1);
 }
 
 // blockIdx.y: the part, then the kind of points (only launched with creases).
@@ -1097,22 +1061,19 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_pair_value_kernel(RkpmArgs
     v[k] = fp2_norm(v[k]);
   }
   const fp2 C2 = v[0] * a.irho2, vx2 = v[1] * 2.0f, vy2 = v[2] * 2.0f;
-  a.psi[e] = fp2_to_double(v[0] * w);
-  fp2 r = v[1] * w;
-  fp2_fma_acc(r, v[0], Jx);
-  a.dpsi[2 * e] = fp2_to_double(r);
-  r = v[2] * w;
-  fp2_fma_acc(r, v[0], Jy);
-  a.dpsi[2 * e + 1] = fp2_to_double(r);
-  r = v[3] * w;
-  fp2_fma_acc(r, vx2, Jx); fp2_fma_acc(r, C2, Jxx);
-  a.ddpsi[3 * e] = fp2_to_double(r);
-  r = v[4] * w;
-  fp2_fma_acc(r, vy2, Jy); fp2_fma_acc(r, C2, Jyy);
-  a.ddpsi[3 * e + 1] = fp2_to_double(r);
-  r = v[5] * w;
-  fp2_fma_acc(r, v[1], Jy); fp2_fma_acc(r, v[2], Jx); fp2_fma_acc(r, C2, Jxy);
-  a.ddpsi[3 * e + 2] = fp2_to_double(r);
+  fp2 r[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) r[k] = v[k] * w;
+  fp2_fma_acc(r[1], v[0], Jx);
+  fp2_fma_acc(r[2], v[0], Jy);
+  fp2_fma_acc(r[3], vx2, Jx); fp2_fma_acc(r[3], C2, Jxx);
+  fp2_fma_acc(r[4], vy2, Jy); fp2_fma_acc(r[4], C2, Jyy);
+  fp2_fma_acc(r[5], v[1], Jy); fp2_fma_acc(r[5], v[2], Jx); fp2_fma_acc(r[5], C2, Jxy);
+  double out[6];
+  fp2_to_double(r, out);
+  a.psi[e] = out[0];
+  a.dpsi[2 * e] = out[1]; a.dpsi[2 * e + 1] = out[2];
+  a.ddpsi[3 * e] = out[3]; a.ddpsi[3 * e + 1] = out[4]; a.ddpsi[3 * e + 2] = out[5];
 }
 
 // The RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
