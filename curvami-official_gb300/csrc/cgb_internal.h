@@ -134,6 +134,7 @@ struct ShapeScratch {
   DevBuf<int8_t> side;       // n_creases * n_nodes
   DevBuf<double> gind;       // n_creases * 6 * n_gp
   DevBuf<int8_t> bad, tip;   // n_gp
+  DevBuf<int32_t> order;     // n_gp, the moment kernels' order
   DevBuf<int> guard;         // 4: flagged points
   DevBuf<double> fac;        // n_nodes, FP64 with per-node radius
   DevBuf<double> mom, coef;  // moment sums and polynomials of a chunk of points

@@ -478,6 +478,7 @@ struct RkpmArgs {
   double ir;           // FP64 kernels: 1 / rho
   const double* fac;   // rho / rho_I per node, or null (single radius)
   int8_t* tip;         // point in the cap of a crease end (its indicators vary there)
+  int32_t* order;      // the points in the order the moment kernels take them (point_order_kernel)
   double* mom;         // moment sums, [sum][point of the chunk]
   double* coef;        // shape polynomials, 6 NP per point of the chunk
   int g0, g1;          // the launch's points
@@ -504,8 +505,8 @@ struct RkpmArgs {
 //  - rkpm_value_kernel, one pair per thread, evaluates them (about 60 operations) over the pair's
 //    jets: reading them back is a tenth of computing them again.
 // Measured on 300,000 points (28 neighbours, quadratic): RKPM 10.7 ms as one kernel of 90 sums and
-// both passes, about 650 operations per neighbour; 4.15 ms so (moments 2.7, solve 0.45, values 1.0).
-// 32,400 points with 113 neighbours, cubic, half of them in a cap: 12.8 -> 3.45 ms.
+// both passes, about 650 operations per neighbour; 3.9 ms so (moments 2.5, solve 0.45, values 1.0).
+// 32,400 points with 113 neighbours, cubic, half of them in a cap: 12.8 -> 3.3 ms.
 template <int ORDER>
 struct MomIdx {
   static constexpr int D = 2 * ORDER;
@@ -521,6 +522,47 @@ struct MomIdx {
   }
   __host__ __device__ static constexpr int cx(int a, int b) { return NW + NA + NB + r(a - 1, b - 1); }
 };
+
+// The order in which the moment kernels take the points: within windows of kSortPoints, those outside
+// the caps first, then by falling neighbour counts. The lanes of a warp wait for the one with the most
+// neighbours, and a warp with points of both kinds is walked twice.
+// RKPM of 300,000 scattered points of 28 neighbours 4.15 -> 3.94 ms, 32,400 cubic Gauss points of 113,
+// half of them in a cap, 3.47 -> 3.31 ms, 1,000,000 mixed points 5.88 -> 5.79 ms.
+constexpr int kSortPoints = 1024;
+__global__ void __launch_bounds__(kSortPoints) point_order_kernel(RkpmArgs a) {
+  constexpr int kBins = 512;
+  __shared__ int s_bin[kBins];
+  const int t = threadIdx.x, w0 = blockIdx.x * kSortPoints, g = w0 + t;
+  if (t < kBins) s_bin[t] = 0;
+  __syncthreads();
+  int bin = 0, rank = 0;
+  if (g < a.n_gp) {
+    const double* I = a.gind + static_cast<int64_t>(g) * 6 * a.n_creases;
+    bool tip = false;
+    for (int c = 0; c < a.n_creases; ++c)
+      for (int q = 1; q < 6; ++q) tip = tip || I[6 * c + q] != 0.0;
+    a.tip[g] = tip;
+    const int64_t n = a.ptr[g + 1] - a.ptr[g];
+    bin = (tip ? kBins / 2 : 0) + kBins / 2 - 1 - static_cast<int>(min(n, static_cast<int64_t>(kBins / 2 - 1)));
+    rank = atomicAdd(&s_bin[bin], 1);
+  }
+  __syncthreads();
+  if (t < 32) {   // exclusive sums of the bins, 16 per lane
+    int v[kBins / 32], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kBins / 32; ++k) { v[k] = sum; sum += s_bin[t * (kBins / 32) + k]; }
+    int before = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int up = __shfl_up_sync(0xffffffffu, before, o);
+      if (t >= o) before += up;
+    }
+#pragma unroll
+    for (int k = 0; k < kBins / 32; ++k) s_bin[t * (kBins / 32) + k] = before - sum + v[k];
+  }
+  __syncthreads();
+  if (g < a.n_gp) a.order[w0 + s_bin[bin] + rank] = g;
+}
 
 __global__ void node_fac_kernel(int n_nodes, const double* __restrict__ rho_node, double rho, double* __restrict__ fac) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -564,17 +606,13 @@ __device__ __forceinline__ void moment_sums(const RkpmArgs& a) {
   constexpr int LO = TIP ? J0 * RI::NR : P1 ? 0 : MI::NW + MI::NA;
   constexpr int HI = TIP ? J1 * RI::NR : P2 ? MI::N : MI::NW + MI::NA;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int g = a.g0 + t / L, sub = t % L;
-  const bool here = g < a.g1;
-  const int gc = here ? g : a.g1 - 1;
+  const int slot = t / L, sub = t % L;
+  const bool here = slot < a.g1 - a.g0;
+  const int gc = a.order[here ? a.g0 + slot : a.g1 - 1];
   const int nc = a.n_creases;
   const double* gind = a.gind + static_cast<int64_t>(gc) * 6 * nc;
-  bool tip = false;
-  for (int c = 0; c < nc; ++c)
-    for (int q = 1; q < 6; ++q) tip = tip || gind[6 * c + q] != 0.0;
-  const bool mine = here && tip == TIP;
+  const bool mine = here && (a.tip[gc] != 0) == TIP;
   if (!__any_sync(0xffffffffu, mine)) return;
-  if (P1 && mine && sub == 0) a.tip[g] = TIP;
   const int64_t p0 = a.ptr[gc];
   const int n = mine ? static_cast<int>(a.ptr[gc + 1] - p0) : 0;
   const double gx = a.gp_xy[2 * gc], gy = a.gp_xy[2 * gc + 1];
@@ -653,7 +691,7 @@ __device__ __forceinline__ void moment_sums(const RkpmArgs& a) {
   if (mine && sub == 0) {
     const int64_t np = a.g1 - a.g0;
 #pragma unroll
-    for (int k = 0; k < HI - LO; ++k) a.mom[(LO + k) * np + (g - a.g0)] = S[k];
+    for (int k = 0; k < HI - LO; ++k) a.mom[(LO + k) * np + slot] = S[k];
   }
 }
 
@@ -678,8 +716,9 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
   constexpr int NP = (ORDER + 1) * (ORDER + 2) / 2;
   using MI = MomIdx<ORDER>;
   using RI = RawIdx<ORDER>;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, g = a.g0 + t;
-  if (g >= a.g1) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.g1 - a.g0) return;
+  const int g = a.order[a.g0 + t], at = g - a.g0;
   const bool tip = a.tip[g];
   const int64_t np = a.g1 - a.g0;
   const double* mom = a.mom + t;
@@ -692,9 +731,9 @@ __global__ void __launch_bounds__(64) rkpm_solve_kernel(RkpmArgs a) {
   auto put = [&](int i, double v) {   // PAIR: as FP32 pairs, in the same 8 bytes
     if constexpr (PAIR) {
       const fp2 p = fp2_from_double(v);
-      reinterpret_cast<float2*>(a.coef)[static_cast<int64_t>(t) * 6 * NP + i] = make_float2(p.hi, p.lo);
+      reinterpret_cast<float2*>(a.coef)[static_cast<int64_t>(at) * 6 * NP + i] = make_float2(p.hi, p.lo);
     } else {
-      a.coef[static_cast<int64_t>(t) * 6 * NP + i] = v;
+      a.coef[static_cast<int64_t>(at) * 6 * NP + i] = v;
     }
   };
   const double r1 = a.ir, r2 = a.ir * a.ir;
@@ -753,7 +792,7 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_value_kernel(RkpmArgs a) {
 // the FP32 rate. The mixed kernels do that per-neighbour arithmetic in FP32 pairs (cgb_pair.cuh,
 // about 48 significant bits) on the FP32 pipe, conversions to and from doubles on the bits; only
 // point_solve, 1/n of the work, is FP64, as in the FP64 path. 1,000,000 points of 28 neighbours,
-// quadratic: RKPM 5.9 ms (jets 0.8, moments 2.4, solve 1.5, values 1.25); 7.1 ms with the FP64
+// quadratic: RKPM 5.8 ms (jets 0.8, moments 2.3, solve 1.5, values 1.2); 7.1 ms with the FP64
 // pipe's conversions, the jets of M in the solve and a bisection in each warp of the pair
 // kernels.
 //
@@ -838,7 +877,6 @@ __global__ void point_pair_kernel(RkpmArgs a, float* __restrict__ rec) {
   float* o = rec + static_cast<int64_t>(g) * pair_record_floats(a.n_creases);
   reinterpret_cast<float4*>(o)[0] = make_float4(x0, x1, x2, y0);
   reinterpret_cast<float4*>(o)[1] = make_float4(y1, y2, 0.0f, 0.0f);
-  bool tip = false;
   for (int c = 0; c < a.n_creases; ++c) {
     const double* I = a.gind + (static_cast<int64_t>(g) * a.n_creases + c) * 6;
     const double r1 = 0.5 * a.rho, r2 = r1 * a.rho;
@@ -846,10 +884,8 @@ __global__ void point_pair_kernel(RkpmArgs a, float* __restrict__ rec) {
       const fp2 v = fp2_from_double((q == 0 ? 0.5 : q < 3 ? r1 : r2) * I[q]);
       o[8 + 12 * c + 2 * q] = v.hi;
       o[9 + 12 * c + 2 * q] = v.lo;
-      tip = tip || (q > 0 && I[q] != 0.0);
     }
   }
-  a.tip[g] = tip;
 }
 
 // Scaled differences of a pair from the split coordinates: accurate relative to themselves.
@@ -935,9 +971,9 @@ __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float*
   constexpr int AT1 = TIP ? (2 * PART + 1) * RI::NR : MI::NW + MI::NA + MI::NB;
   constexpr int DEG = MI::D + (TIP ? 0 : PART);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int g = a.g0 + t / L, sub = t % L;
-  const bool here = g < a.g1;
-  const int gc = here ? g : a.g1 - 1;
+  const int slot = t / L, sub = t % L;
+  const bool here = slot < a.g1 - a.g0;
+  const int gc = a.order[here ? a.g0 + slot : a.g1 - 1];
   const bool mine = here && (a.tip[gc] != 0) == TIP;
   if (!__any_sync(0xffffffffu, mine)) return;
   const int64_t p0 = a.ptr[gc];
@@ -995,7 +1031,7 @@ __device__ __forceinline__ void pair_moment_sums(const RkpmArgs& a, const float*
     for (int k = 0; k < N; ++k) {
 #pragma unroll
       for (int o = L / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-      if (mine && sub == 0) a.mom[(at + k) * np + (g - a.g0)] = v[k];
+      if (mine && sub == 0) a.mom[(at + k) * np + slot] = v[k];
     }
   };
   put(AT0, S0);
@@ -1088,7 +1124,12 @@ int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
   constexpr int kParts = PAIR ? 3 : ORDER == 3 ? 2 : 1;
   cudaStream_t st = ctx->stream;
   const int n_gp = out->n_gp, most = std::min(n_gp, kChunk);
-  int launches = 0;
+  int launches = 1;
+  ctx->scratch.tip.ensure(n_gp);
+  ctx->scratch.order.ensure(n_gp);
+  ra.tip = ctx->scratch.tip.p;
+  ra.order = ctx->scratch.order.p;
+  point_order_kernel<<<blocks_for(n_gp, kSortPoints), kSortPoints, 0, st>>>(ra);
   ctx->scratch.mom.ensure(static_cast<size_t>(most) * kSums);
   ctx->scratch.coef.ensure(static_cast<size_t>(most) * 6 * NP);
   ra.mom = ctx->scratch.mom.p;
@@ -1329,7 +1370,7 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   RkpmArgs ra{n_gp, n_nodes, out->kernel, nc, out->rho, nullptr, pair_of(1.0 / out->rho),
               pair_of(1.0 / (out->rho * out->rho)), out->gp_xy.p, ctx->node_xy.p, d_rn, out->nbr_ptr.p,
               out->nbr_idx.p, out->s.p, gind, side, out->psi.p, out->dpsi.p, out->ddpsi.p, bad,
-              0.0, nullptr, nullptr, nullptr, nullptr, 0, n_gp};
+              0.0, nullptr, nullptr, nullptr, nullptr, nullptr, 0, n_gp};
   prof_begin(ctx, CGB_PHASE_RKPM);
   if (mixed && n_nodes > 0) {
     ctx->scratch.node_pair.ensure(2 * static_cast<size_t>(n_nodes));
@@ -1340,9 +1381,7 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   int nl = mixed && n_nodes > 0 ? 1 : 0;
   if (n_gp > 0) {
     nl += mixed || d_rn ? 1 : 0;
-    ctx->scratch.tip.ensure(n_gp);
     ra.ir = 1.0 / out->rho;
-    ra.tip = ctx->scratch.tip.p;
     const float* rec = nullptr;
     if (mixed) {
       ctx->scratch.point_rec.ensure(static_cast<size_t>(n_gp) * pair_record_floats(nc));
