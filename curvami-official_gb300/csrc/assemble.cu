@@ -106,6 +106,8 @@ struct FaceArgs {
   double* Fc;        // deterministic F contributions (3 per entry)
   void* Kacc;        // atomic block accumulator
   void* Kc;          // deterministic contributions (9 per pair)
+  double2* zero;     // the block accumulator, cleared by the launch's residual (null: not)
+  int64_t n_zero;
 };
 
 // Per-point kinematics and resultants (Kinematics.h:61-120, Constitutive.h:57-70).
@@ -624,6 +626,13 @@ template <typename TK, bool DET, bool STORE, int LANES>
 __global__ void __launch_bounds__(256) face_residual_kernel(FaceArgs a, TK* gstate, int* __restrict__ work) {
   constexpr int PTS = 32 / LANES;
   const int lane = threadIdx.x & 31;
+  // The first residual of a step clears the block accumulator that the tangent and the hinge add
+  // into after it: stores beside FP64 work, and a launch less (15 x 15 nodes: step 166.8 -> 162.6 us).
+  // Cleared on the tangent's stream instead, a captured step of 600,000 points took 5.66 ms, not 4.56.
+  if (STORE && !DET && a.zero)
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < a.n_zero;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+      a.zero[i] = make_double2(0.0, 0.0);
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(work, 1);
@@ -1357,14 +1366,14 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   // Accumulators.
   prof_begin(ctx, CGB_PHASE_ZERO);
   if (!det) CGB_CUDA(cudaMemsetAsync(d_F, 0, ndof * sizeof(double), st));
+  void* zero = nullptr;   // the block accumulator: whole 16-byte words, cleared by the first residual
+  size_t zero_bytes = 0;
   if (want_K && !det) {
-    if (mixed) {
-      a->kacc32.ensure(12 * a->n_blocks);
-      CGB_CUDA(cudaMemsetAsync(a->kacc32.p, 0, 12 * a->n_blocks * sizeof(float), st));
-    } else {
-      a->kacc64.ensure(9 * a->n_blocks);
-      CGB_CUDA(cudaMemsetAsync(a->kacc64.p, 0, 9 * a->n_blocks * sizeof(double), st));
-    }
+    zero_bytes = (static_cast<size_t>(a->n_blocks) * (mixed ? 12 * sizeof(float) : 9 * sizeof(double)) + 15) / 16 * 16;
+    if (mixed) a->kacc32.ensure(zero_bytes / sizeof(float));
+    else a->kacc64.ensure(zero_bytes / sizeof(double));
+    zero = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
+    if (S->n_gp == 0 && zero_bytes > 0) CGB_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, st));
   }
   const int64_t n_contrib = k_face_units + [&] { int64_t s = 0; for (auto& f : a->folds) s += f.n_pairs; return s; }();
   if (det) {
@@ -1490,6 +1499,8 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     fa.g_end = cb(c + 1);
     if (fa.g_begin >= fa.g_end) break;
     const int ncg = fa.g_end - fa.g_begin;
+    fa.zero = c == 0 ? static_cast<double2*>(zero) : nullptr;
+    fa.n_zero = static_cast<int64_t>(zero_bytes / sizeof(double2));
     prof_begin(ctx, CGB_PHASE_FACE);
     auto rl = [&](auto lanes, auto* stp) {
       constexpr int L = decltype(lanes)::value;
