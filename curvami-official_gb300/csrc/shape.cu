@@ -361,7 +361,8 @@ struct RowJets {
 // (y alike), with D_x e0 the unit vector of xi, D_x D_x e0 twice that of xi^2, D_x D_y e0 that of
 // xi eta. So neither the jets of M (135 of 1,050 FP64 operations for the quadratic basis) nor the
 // derivatives of the basis on the coefficients (40) are formed. 262,144 points,
-// quadratic: 485 -> 373 us, with the coefficients left as pairs 560 -> 385 us.
+// quadratic: 485 -> 373 us, with the coefficients left as pairs 560 -> 385 us. Against extended
+// precision the coefficients' errors are the same (quadratic) or a quarter smaller (cubic).
 // at(g, a, b): S^g_ab = sum_I (D^g w_I) xi^a eta^b for g = 0 (w), 1 (x), 2 (y), 3 (xx), 4 (yy), 5 (xy).
 template <int ORDER, class Sums>
 __device__ __forceinline__ int point_solve(const Sums& at, RowJets<ORDER>& R) {
@@ -1113,13 +1114,15 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_pair_value_kernel(RkpmArgs
 }
 
 // The RKPM of a set: moments, solve, values over chunks of points that bound the scratch (the
-// sums and polynomials of 262,144 points: 260 MB for the quadratic basis, 480 MB for the cubic).
+// sums and polynomials of 1,048,576 points: 1.1 GB for the quadratic basis, 1.9 GB for the cubic).
+// A chunk's kernels each end in a part-filled wave: with 262,144 points to a chunk 1,000,000 mixed
+// points take 7.18 ms, not 6.87, and 300,000 FP64 points 4.94, not 4.85.
 // Lanes per point of the moment kernel: more while its warps do not fill the SM quarters twice
 // (adding a lane pair's sums costs as many operations as half a neighbour's).
 // Returns the kernels launched.
 template <int ORDER, bool PAIR>
 int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
-  constexpr int kChunk = 1 << 18, NP = (ORDER + 1) * (ORDER + 2) / 2;
+  constexpr int kChunk = 1 << 20, NP = (ORDER + 1) * (ORDER + 2) / 2;
   constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
   constexpr int kParts = PAIR ? 3 : ORDER == 3 ? 2 : 1;
   cudaStream_t st = ctx->stream;

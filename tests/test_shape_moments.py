@@ -58,15 +58,15 @@ def test_against_oracle(ctx, n_gp, order, rho, kernel, cut):
 
 
 def test_more_points_than_a_chunk(ctx):
-    """262,144 points share the scratch: a larger set equals, bitwise, its parts built alone."""
+    """1,048,576 points share the scratch: a larger set equals, bitwise, its parts built alone."""
     rng = np.random.default_rng(8)
-    xy, pts = nodes(101), rng.uniform(0.0, 50.0, (262144 + 40000, 2))
+    xy, pts = nodes(101), rng.uniform(0.0, 50.0, (2**20 + 40000, 2))
     cuts = [inner_cut(25.2, 15.0, 33.0)]
     ctx.set_nodes(xy)
-    whole = cg.shape_functions(ctx, pts, 1.6, 2, cuts).download()
-    at = 262144
+    whole = cg.shape_functions(ctx, pts, 0.9, 1, cuts).download()
+    at = 2**20
     for part, g in ((pts[:at], slice(0, at)), (pts[at:], slice(at, len(pts)))):
-        sh = cg.shape_functions(ctx, part, 1.6, 2, cuts).download()
+        sh = cg.shape_functions(ctx, part, 0.9, 1, cuts).download()
         e = slice(whole["ptr"][g.start], whole["ptr"][g.stop])
         for k in ("idx", "s", "psi", "dpsi", "ddpsi"):
             assert np.array_equal(sh[k], whole[k][e]), k
