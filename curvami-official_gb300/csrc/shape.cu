@@ -282,24 +282,34 @@ void scan_counts(cgb_context* ctx, int64_t n, const int32_t* cnt, int64_t* ptr, 
 }
 
 // Per-node crease side sn = (f >= 0 ? +1 : -1) (GlobalRKPM.h:92-93).
+template <int L>
 __global__ void node_side_kernel(int n_nodes, const double* __restrict__ node_xy, DevCrease cr,
                                  int8_t* __restrict__ side) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_nodes) return;
-  const DevIndicator I = eval_indicator(node_xy[2 * j], node_xy[2 * j + 1], cr);
-  side[j] = (I.f >= 0.0) ? 1 : -1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = min(t / L, n_nodes - 1);
+  const DevIndicator I = eval_indicator<L>(node_xy[2 * j], node_xy[2 * j + 1], cr);
+  if (t / L < n_nodes && t % L == 0) side[j] = (I.f >= 0.0) ? 1 : -1;
 }
 
-// Gauss-point indicators, 6 doubles per point per crease.
 // Crease c's indicator at every Gauss point, written in place into the [g][crease][6]
 // layout the RKPM kernel reads (n_creases values per point).
+template <int L>
 __global__ void gp_indicator_kernel(int n_gp, const double* __restrict__ gp_xy, DevCrease cr, int c, int n_creases,
                                     double* __restrict__ out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_gp) return;
-  const DevIndicator I = eval_indicator(gp_xy[2 * g], gp_xy[2 * g + 1], cr);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, g = min(t / L, n_gp - 1);
+  const DevIndicator I = eval_indicator<L>(gp_xy[2 * g], gp_xy[2 * g + 1], cr);
+  if (t / L >= n_gp || t % L != 0) return;
   double* o = out + 6 * (static_cast<int64_t>(g) * n_creases + c);
   o[0] = I.f; o[1] = I.gx; o[2] = I.gy; o[3] = I.hxx; o[4] = I.hyy; o[5] = I.hxy;
+}
+
+// Lanes per point of the indicator kernels: a warp's FP64 part takes as long for one point as for 32,
+// so more lanes only while every warp has an SM quarter of its own.
+template <class F>
+void indicator_lanes(int n, int sms, F&& launch) {
+  const int64_t lanes = 32LL * 4 * sms;
+  if (n * 32LL <= lanes) launch(std::integral_constant<int, 32>{});
+  else if (n * 4LL <= lanes) launch(std::integral_constant<int, 4>{});
+  else launch(std::integral_constant<int, 1>{});
 }
 
 __device__ __forceinline__ void inv3(const double m[3][3], double r[3][3]) {
@@ -1345,17 +1355,26 @@ void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& c
   int8_t* side = ctx->scratch.side.p;
   double* gind = ctx->scratch.gind.p;
   std::vector<DevCrease> dcr(nc);
+  int sms = 0;
+  CGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   prof_begin(ctx, CGB_PHASE_CREASE);
   for (int c = 0; c < nc; ++c) {
     dcr[c] = DevCrease{ctx->scratch.cxy.p + off[c], static_cast<int>(creases[c].xy.size() / 2), creases[c].extend_start,
                        creases[c].extend_end, creases[c].is_closed, ctx->scratch.cxyf.p + off[c] / 2, extent[c]};
-    node_side_kernel<<<blocks_for(n_nodes, 32), 32, 0, st>>>(n_nodes, ctx->node_xy.p, dcr[c],
-                                                                 side + static_cast<int64_t>(c) * n_nodes);
+    indicator_lanes(n_nodes, sms, [&](auto lanes) {
+      constexpr int L = decltype(lanes)::value;
+      node_side_kernel<L><<<blocks_for(static_cast<int64_t>(n_nodes) * L, 32), 32, 0, st>>>(
+          n_nodes, ctx->node_xy.p, dcr[c], side + static_cast<int64_t>(c) * n_nodes);
+    });
   }
   // Gauss-point indicators laid out [g][c][6].
   if (nc > 0 && n_gp > 0)
     for (int c = 0; c < nc; ++c)
-      gp_indicator_kernel<<<blocks_for(n_gp, 64), 64, 0, st>>>(n_gp, out->gp_xy.p, dcr[c], c, nc, gind);
+      indicator_lanes(n_gp, sms, [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        gp_indicator_kernel<L><<<blocks_for(static_cast<int64_t>(n_gp) * L, 64), 64, 0, st>>>(n_gp, out->gp_xy.p, dcr[c],
+                                                                                             c, nc, gind);
+      });
   prof_end(ctx, CGB_PHASE_CREASE, nc * (1 + (n_gp > 0 ? 1 : 0)));
   CGB_CUDA(cudaGetLastError());
 

@@ -49,3 +49,24 @@ def test_against_oracle(name, extend, shift):
     sh = cg.shape_functions(ctx, pts, 2.6, 1, [cut]).download()
     for k, ref in (("psi", psi), ("dpsi", dpsi), ("ddpsi", ddpsi)):
         assert np.abs(sh[k] - ref).max() <= 1e-8 * np.abs(ref).max(), k
+
+
+@pytest.mark.parametrize("n", [3, 608, 609, 4865])
+@pytest.mark.parametrize("name", ["arc", "zigzag"])
+def test_lanes_per_point(name, n):
+    """32, 4 or one lane per point, by the set's size."""
+    import __graft_entry__ as ge
+
+    ge.build()
+    rng = np.random.default_rng(n)
+    v = polylines()[name][::7]                       # 26 vertices: the last group of segments is part-filled
+    xy, pts = synth.grid_nodes(41, 41, 0.5, 0.1, rng), rng.uniform(3.0, 17.0, (n, 2))
+    cut = {"vertices": v, "extend_start": True, "extend_end": True, "is_closed": False}
+    ctx, o = cg.Context(0), Oracle()
+    ctx.set_nodes(xy)
+    ptr, idx, s = o.frnn(xy, pts, 2.6)
+    psi, dpsi, ddpsi, bad, rc = o.rkpm(xy, pts, ptr, idx, s, 2.6, 1, [cut])
+    assert rc == 0
+    sh = cg.shape_functions(ctx, pts, 2.6, 1, [cut]).download()
+    for k, ref in (("psi", psi), ("dpsi", dpsi), ("ddpsi", ddpsi)):
+        assert np.abs(sh[k] - ref).max() <= 1e-8 * np.abs(ref).max(), k
