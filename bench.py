@@ -38,12 +38,12 @@ for _p in (ROOT, PKG_DIR):
 METRIC = "Gauss-pt residual+tangent evals/s, mixed vs FP64 GPU at stated error"
 UNIT = "GP evals/s"
 SEED = 1003
-# DRAM bytes (read + write) per Gauss point of the merged FP32 tangent, from one ncu capture
-# of the whole 101 x 101 plate in one launch (160,000 points: 318.7 MB read + 20.9 MB
+# DRAM bytes (read + write) per Gauss point of the FP32 tangent, from one ncu capture
+# of the whole 101 x 101 plate in one launch (160,000 points: 179.0 MB read + 14.9 MB
 # written); the traffic per point does not depend on the plate size, so it scales to the
 # full launch by its points.
-TANGENT_DRAM_BYTES_PER_GP = 2122.0
-TANGENT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of face_tangent_merged_kernel over "
+TANGENT_DRAM_BYTES_PER_GP = 1212.0
+TANGENT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of face_tangent_tile_kernel over "
                           "the 101 x 101 plate in one launch (bench.py --n-side 101 --profile-mixed 1,128,0,0), "
                           "per Gauss point, times the points of one launch")
 WORKLOAD = ("single-plate assembly at scale: 201x201 jittered nodes, 4x4 Gauss rule (640,000 "
@@ -437,7 +437,7 @@ def run_gpu(args):
     barrier()
 
     # Roofline. The step runs two kernels per chunk: the FP64 residual kernel ("face") and,
-    # on a second stream, the FP32 tangent ("tangent", the merged CUDA-core kernel, which
+    # on a second stream, the FP32 tangent ("tangent", the CUDA-core kernel by cells, which
     # dominates). Its compute roof is the FP32 pipe; HBM is the secondary figure. Times are
     # sums over the step's chunk launches (events on each kernel's own stream).
     ptr = model.faces.download()["ptr"]
@@ -451,9 +451,9 @@ def run_gpu(args):
     flops_total = float((181 * n * (n + 1) / 2 + 364 * n + 200).sum())
     flops_fp32 = flops_total - flops_fp64                       # the tangent's share of F_B(n)
     # Compulsory bytes of the tangent per step: per-point state (32 floats), per neighbour
-    # the FP32 grad / Hessian Phi (20 B), per pair its 2-byte code, per merged entry its block
-    # slot and contribution range (8 B), and the FP32 block accumulator once (48 B per block).
-    alg_bytes = float((128 + 20 * n + n * (n + 1)).sum() + 8.0 * work["entries"] + 48.0 * work["blocks"])
+    # the FP32 grad / Hessian Phi and the place in the cell's nodes (21 B), per block of a cell its
+    # share of an item's code and slots (5 B), and the FP32 block accumulator once (48 B per block).
+    alg_bytes = float((128 + 21 * n).sum() + 5.0 * work["entries"] + 48.0 * work["blocks"])
     peaks, peak_kind = measured_peaks()
     p64, p32 = fma_peaks(local)
     tf32_peak = peaks["bf16_tflops"] / 2.0
@@ -468,10 +468,10 @@ def run_gpu(args):
         "traffic_source": TANGENT_TRAFFIC_SOURCE,
         "peak_source": "measured live on this GPU (cgb_measure_fma_peaks: dependent FP32 FMA chains on "
                        "every SM); MEASURED_PEAKS.json has no CUDA-core FP32 figure",
-        "kernel": "face_tangent_merged_kernel (FP32 CUDA cores, merged contributions)",
-        "binding_unit": ("the L1 / shared-memory data pipe: 90 % of its peak in ncu with the kernel alone "
-                         "(1.44 shared wavefronts per pair contribution), FMA pipe 42 %; in the step the FP64 "
-                         "residual's loads share that pipe"),
+        "kernel": "face_tangent_tile_kernel (FP32 CUDA cores, a cell's contributions to a block added first)",
+        "binding_unit": ("the shared-memory data pipe and latency at two CTAs per SM: data pipe 73 %, issue 50 %, "
+                         "FMA pipe 38 % in ncu with the kernel alone; in the step the FP64 residual shares the "
+                         "register file and that pipe"),
         "achieved_what": "the reference's hand-counted tangent flops, F_B(n) - F_R(n) per Gauss point, per second",
         "launch_ms": tan_ms / tan_launches, "launches_per_step": tan_launches, "step_ms": tan_ms,
         "algorithmic_flops_per_step": flops_fp32, "work": work,
@@ -480,7 +480,7 @@ def run_gpu(args):
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"},
         "tensor_core_tangent": {
             "kernel": "face_tangent_tc_kernel (tcgen05.mma kind::tf32, 3xTF32, A in tensor memory, accumulator "
-                      "in tensor memory) + face_tangent_merged_kernel for the cells it does not take",
+                      "in tensor memory) + face_tangent_tile_kernel for the cells it does not take",
             "step_ms": tan_tc_ms, "launches_per_step": max(int(ph_tc_n["tangent"]) // steps, 1),
             "achieved_tflops": flops_fp32 / (tan_tc_ms * 1e-3) / 1e12,
             "tensor_pipe": {"executed_tflops": tensor_flops / (tan_tc_ms * 1e-3) / 1e12, "peak": tf32_peak,

@@ -170,7 +170,7 @@ int cgb_graph_create(cgb_assembler* a, const double* d_x, double* d_K, double* d
     if ((flags & CGB_TANGENT) && !d_K) throw Error(CGB_ERR_INVALID, "cgb_graph_create: d_K is NULL with CGB_TANGENT");
     if (!ctx->stream) throw Error(CGB_ERR_INVALID, "cgb_graph_create: the context's stream is the legacy default stream");
     CGB_CUDA(cudaSetDevice(ctx->device));
-    // One direct call first: it builds every table and buffer the call needs (merge tables,
+    // One direct call first: it builds every table and buffer the call needs (cell tables,
     // deterministic lists, FP32 copies, the second stream), none of which may be created
     // while a stream is being captured.
     const bool prof = ctx->profile;

@@ -558,7 +558,7 @@ void tile_prepare(cgb_assembler* a) {
 
 // Ordered lists for the deterministic scatter. F contribution ids: face entries
 // [0, nnz_face), then hinge merged-node entries fold by fold. K unit ids: the face units
-// (pairs, or merged entries), then hinge pairs fold by fold. Each K block and each node sums
+// (pairs, or four blocks per item of the cells), then hinge pairs fold by fold. Each K block and each node sums
 // its units in ascending id order, i.e. Gauss point (or group of Gauss points) by Gauss
 // point in the reference's loop order.
 namespace {

@@ -265,7 +265,7 @@ class NonLinearAssembler:
 
     def tensor_stats(self):
         """{"tensor_groups", "core_groups", "point_cols", "ctas_per_sm"}: the tensor-core
-        tangent's share (groups of 16 points as one tensor-core product, groups left to the
+        tangent's share (cells of 16 points as one tensor-core product, cells left to the
         CUDA cores, the sum of points x MMA columns, i.e. 10,240 x point_cols TF32 flops per
         assembly) and the CTAs per SM of its last launch."""
         out = np.zeros(4, np.int64)

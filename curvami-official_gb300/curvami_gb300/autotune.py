@@ -2,7 +2,7 @@
 
 The knobs: the number of Gauss-point chunks whose FP64 residual and FP32-class tangent
 kernels overlap on two streams, the residual kernel's block size, the resident CTAs per SM
-of the CUDA-core merged tangent, and which tangent forms the cells (tensor cores or CUDA
+of the CUDA-core tangent by cells, and which tangent forms the cells (tensor cores or CUDA
 cores). The best setting depends on the problem's size and neighbour counts
 (a batch of small plates wants fewer, larger chunks than one big plate). ``autotune``
 times every candidate on the caller's own problem and device buffers, keeps the fastest,

@@ -182,14 +182,14 @@ int cgb_assembler_download_pattern(const cgb_assembler* a, int32_t* outer, int32
  * block rows of column max(ni, nj). */
 int cgb_assembler_download_map(const cgb_assembler* a, int32_t* map, int64_t n_entries);
 /* Sizes of the assembler's work (no reference counterpart; for measurement): out[0] local
- * pairs over all face Gauss points (sum n(n+1)/2), out[1] 3x3 blocks of K, out[2] merged
- * entries of the FP32 tangent (distinct blocks per group of 16 consecutive Gauss points),
- * out[3] groups too large to merge. The first call builds the merge tables. */
+ * pairs over all face Gauss points (sum n(n+1)/2), out[1] 3x3 blocks of K, out[2] the blocks
+ * that the FP32 tangent adds per cell (distinct blocks per cell of 16 consecutive Gauss points),
+ * out[3] cells too large for that. The first call builds the cell tables. */
 int cgb_assembler_stats(cgb_assembler* a, int64_t out[4]);
 /* The tensor-core tangent's share of the work (no reference counterpart; for measurement):
- * out[0] groups of 16 points formed as one tensor-core product, out[1] groups left to the
- * CUDA cores (node union above 42 nodes, or too large to merge), out[2] the sum over the
- * tensor groups of points x MMA columns N (each point is five 128 x N x 8 TF32 MMAs, so
+ * out[0] cells of 16 points formed as one tensor-core product, out[1] cells left to the
+ * CUDA cores (node union above 42 nodes, or too large for a cell), out[2] the sum over the
+ * tensor cells of points x MMA columns N (each point is five 128 x N x 8 TF32 MMAs, so
  * the tensor pipe executes 10,240 x out[2] flops per assembly), out[3] the CTAs per SM of
  * the last tensor-core launch (0 before the first). The first call builds the tables. */
 int cgb_assembler_tensor_stats(cgb_assembler* a, int64_t out[4]);
@@ -294,10 +294,10 @@ int cgb_shape_concat(cgb_context* ctx, const cgb_shape* const* sets, const int32
 /* Launch shape of an assembly; 0 keeps the library's choice. n_chunks (1..16): Gauss-point
  * chunks whose residual and tangent kernels overlap on two streams (default 4 for the mixed
  * step from 98,304 points, else 1); residual_threads (64, 128, 256): block size of the residual kernel
- * (default by size; small launches split points over lanes instead); tangent_ctas_per_sm (1..4): resident CTAs per SM of the merged FP32
- * tangent (default: as many as fit); tangent_kind, the mixed-precision tangent:
- * CGB_TANGENT_CORES (the default) every cell on the CUDA cores (FP32, merged
- * contributions); CGB_TANGENT_TENSOR forms each quadrature cell's blocks as one
+ * (default by size; small launches split points over lanes instead); tangent_ctas_per_sm
+ * (1..4): resident CTAs per SM of the FP32 tangent by cells (default: as many as fit);
+ * tangent_kind, the mixed-precision tangent: CGB_TANGENT_CORES (the default) every cell on
+ * the CUDA cores (FP32, a cell's contributions to a block added first); CGB_TANGENT_TENSOR forms each quadrature cell's blocks as one
  * tensor-core product (tcgen05, 3xTF32, FP32 accumulation) where the cell's neighbour union
  * has at most 42 nodes, the rest on the CUDA cores. With the quadratic basis's 20-45
  * neighbours per point the CUDA-core form is both faster (0.54 against 0.82 ms for
