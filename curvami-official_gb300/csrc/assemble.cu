@@ -11,7 +11,7 @@
 // resultants, nodal forces, and the point's state for the tangent) and the tangent, which forms
 // the n(n+1)/2 blocks of every point: per cell of 16 points with the contributions to
 // a block summed first (tangent_tile.cuh, FP32), or per (point, neighbour) entry (tangent_entry.cuh:
-// FP64, and FP32 supports too wide for a cell). They form each block of
+// FP64, and FP32 supports too wide for a cell). The blocks follow from
 //
 //     K_IJ = a1 (x) Y1 + a2 (x) Y2 + b (x) Y3 + geo I,
 // which follows from Bm_I = a1 (x) (dx, 0, dy) + a2 (x) (0, dy, dx) in strain space,
@@ -20,8 +20,10 @@
 //     Y2 = dy_I P_J1 + dx_I P_J2 - Tu_I c_J1 b
 //     Y3 = beta_I . Q_J - Tu_J (a1 c_I0 + a2 c_I1) + bv (dPhi_I . c_J) b
 //     geo = dPhi_I . N dPhi_J,
-// the same terms as K_mat + K_geo_m + T12 + T3 of Assembly.h:290-300 (70 FMA per block
-// against the reference's ~90), with the Gauss weight folded into the J-side factors.
+// the same terms as K_mat + K_geo_m + T12 + T3 of Assembly.h:290-300. Both kernels sort them by the
+// five derivatives of Phi_I, K_IJ = sum_a phi_I[a] T_J[a] (tangent_entry.cuh: 36 FMA per block, 54 with
+// B, against the reference's ~90), with the Gauss weight folded into T_J; the entry point on
+// caller-owned arrays uses the form above (70 FMA).
 //
 // Precision modes: FP64 throughout, or "mixed" (FP64 kinematics, resultants and
 // residual; the per-neighbour factors and the pair loop in FP32, accumulated into an
@@ -1544,7 +1546,11 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       const int per_cell = glist ? static_cast<int>(nb(static_cast<int64_t>(kMG) * fa.nmax, kEntryThreads)) : 0;
       const unsigned egrid = glist ? static_cast<unsigned>(gcount) * per_cell
                                    : std::max(1u, nb(std::min(S->nnz, static_cast<int64_t>(ncg) * fa.nmax), kEntryThreads));
-      kern<<<egrid, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p, glist, per_cell);
+      int mix = 0;   // FP32 sums: the blocks in a mixed order (face_tangent_entry_kernel)
+      if (mixed && !det && !glist)
+        while (mix < 16 && (1u << mix) < egrid) ++mix;
+      const unsigned window = 1u << mix;
+      kern<<<(egrid + window - 1) / window * window, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p, glist, per_cell, mix);
     };
     int ntan = 1;
     if (merged) {

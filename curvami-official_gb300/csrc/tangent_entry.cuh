@@ -1,5 +1,5 @@
 // tangent_entry.cuh — the tangent of the face Gauss points with one thread per (point,
-// neighbour) entry: FP64 mode, and the FP32 tangent of supports too wide to merge.
+// neighbour) entry: FP64 mode, and the FP32 tangent of supports too wide for a cell.
 // Included by assemble.cu.
 //
 // The variations of the strains are linear in the five derivatives phi = (dx, dy, dxx, dyy,
@@ -184,7 +184,8 @@ constexpr int kEntryThreads = 128;
 template <typename TK, bool DET, bool BZERO>
 __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceArgs a, const TK* __restrict__ gstate,
                                                                          const int32_t* __restrict__ ent_point,
-                                                                         const int32_t* __restrict__ glist, int per_cell) {
+                                                                         const int32_t* __restrict__ glist, int per_cell,
+                                                                         int mix_bits) {
   __shared__ TK s_val[kEntryThreads / 32][32 * 9];
   __shared__ int64_t s_at[kEntryThreads / 32][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -193,6 +194,19 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
     gb = kMG * glist[blockIdx.x / per_cell];
     ge = min(gb + kMG, a.g_end);
     blk = blockIdx.x % per_cell;
+  } else if (mix_bits > 0) {
+    // FP32 sums by atomics: the blocks of a window of 2^mix_bits are taken in a mixed order (odd factors
+    // and shifts right, each a permutation of the window). In ascending order a block's contributions
+    // come point by point; on a regular mesh the sums of all its translates then round alike and
+    // the errors add up over smooth displacements: the path of a 61 x 61 cubic sheet took steps of
+    // 0.007 where it takes 0.1 so. No slower: 2,405 us a step there.
+    const unsigned mask = (1u << mix_bits) - 1u, half = (mix_bits + 1) / 2;
+    unsigned m = static_cast<unsigned>(blk) & mask;
+    m = (m * 0x9e3779b1u) & mask;
+    m ^= m >> half;
+    m = (m * 0x85ebca6bu) & mask;
+    m ^= m >> half;
+    blk = static_cast<int>((static_cast<unsigned>(blk) & ~mask) | m);
   }
   const int64_t e_end = a.ptr[ge];
   const int64_t ew = a.ptr[gb] + static_cast<int64_t>(blk) * kEntryThreads + 32 * w;  // the warp's first
