@@ -679,9 +679,8 @@ struct HingeArgs {
   int exact;
   int want_K;
   int parts;         // warps per crease point
-  int tk_float;      // accumulator type
-  double* F; void* Kacc;              // atomic mode
-  double* Fc; void* Kc;               // deterministic mode
+  double* F; double* Kacc;            // atomic mode: Kacc by pair_slot
+  double* Fc; double* Kc;             // deterministic mode
   int64_t f_base, k_base;             // contribution id offsets of this fold
 };
 
@@ -866,14 +865,8 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
             }
             v[3 * dk + dm] = val;
           }
-        if (a.Kc) {
-          if (a.tk_float) { float t[9]; for (int k = 0; k < 9; ++k) t[k] = static_cast<float>(v[k]); store_contrib<float>(a.Kc, a.k_base + q0 + p, false, t); }
-          else store_contrib<double>(a.Kc, a.k_base + q0 + p, false, v);
-        } else {
-          const int32_t slot = a.pair_slot[q0 + p];
-          if (a.tk_float) { float t[9]; for (int k = 0; k < 9; ++k) t[k] = static_cast<float>(v[k]); scatter_atomic<float>(a.Kacc, slot, false, t); }
-          else scatter_atomic<double>(a.Kacc, slot, false, v);
-        }
+        if (a.Kc) store_contrib<double>(a.Kc, a.k_base + q0 + p, false, v);
+        else scatter_atomic<double>(a.Kacc, a.pair_slot[q0 + p], false, v);
         off += 32 * a.parts;
         while (P < mu && off >= mu - P) { off -= mu - P; ++P; }
       }
@@ -886,11 +879,21 @@ __global__ void __launch_bounds__(32 * kHingeWarps) hinge_kernel(HingeArgs a) {
 __device__ __forceinline__ double widen(float v) { return fp2_widen(v); }
 __device__ __forceinline__ double widen(double v) { return v; }
 
+// The hinge's blocks of the mixed mode, in FP64 apart from the FP32 accumulator: those of column
+// j are [ptr[j], ptr[j + 1]), each at block row pos of the column. In the FP32 accumulator they
+// would round whatever is added after them at their own size: on a plate of 41 x 41 nodes a
+// hinge entry is a hundred times the plate's bending entries beside the crease.
+struct HingeBlocks {
+  const int64_t* ptr;    // null: none
+  const int32_t* pos;
+  const double* acc;     // 9 per block
+};
+
 // Column node j holds len_j block rows; scalar column 3j+c starts at 9 col_ptr[j] +
 // 3 c len_j and lists rows 3i+r for the block rows i ascending (Assembly.h:103-107).
 template <typename TA, int STRIDE>
 __global__ void blocks_to_csc(int n_nodes, const int64_t* __restrict__ col_ptr, const TA* __restrict__ acc,
-                              double* __restrict__ K) {
+                              HingeBlocks hinge, double* K) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -902,6 +905,14 @@ __global__ void blocks_to_csc(int n_nodes, const int64_t* __restrict__ col_ptr, 
       // t enumerates the column's output in storage order: c major, then (pos, r).
       const int c = t / (3 * len), rem = t - c * 3 * len, pos = rem / 3, r = rem - 3 * pos;
       col[t] = widen(acc[(b0 + pos) * STRIDE + 3 * r + c]);
+    }
+    if (!hinge.ptr) continue;
+    const int64_t h0 = hinge.ptr[j];
+    const int nh = 9 * static_cast<int>(hinge.ptr[j + 1] - h0);
+    __syncwarp();   // the column's other lanes have stored it
+    for (int t = lane; t < nh; t += 32) {
+      const int q = t / 9, k = t - 9 * q, r = k / 3, c = k - 3 * r;
+      col[3 * c * len + 3 * hinge.pos[h0 + q] + r] += hinge.acc[9 * h0 + t];
     }
   }
 }
@@ -937,13 +948,16 @@ __global__ void blocks_to_csc_outer(int n_nodes, int64_t n_blocks, const int32_t
 // column. 430,000 FP32 blocks of 9 contributions (87 x 87 nodes) with det_reduce_F: 202 -> 108 us;
 // a lane per block had nine separate loads for each contribution, 36 bytes apart between the lanes.
 // 12 or 16 contributions ahead, or the next block's range fetched early: 115-120 us.
+// FP32 contributions: the units from n_face on are the hinge's, in FP64 in an array of their own
+// (hinge), and are summed apart.
 constexpr int kReduceThreads = 128;   // 14 blocks at a time
 constexpr int kReduceAhead = 8;
 template <typename TC>
 __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes, const int64_t* __restrict__ col_ptr,
                                                                     const int64_t* __restrict__ lptr,
                                                                     const int64_t* __restrict__ list,
-                                                                    const TC* __restrict__ contrib,
+                                                                    const TC* __restrict__ contrib, int64_t n_face,
+                                                                    const double* __restrict__ hinge,
                                                                     double* __restrict__ K) {
   constexpr int kGroups = kReduceThreads / 9;
   const int group = threadIdx.x / 9, k = threadIdx.x - 9 * group;
@@ -956,15 +970,28 @@ __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes,
     for (int pos = group; pos < len; pos += kGroups) {
       const int64_t end = lptr[b0 + pos + 1];
       TC s = TC(0);
+      double h = 0.0;
       for (int64_t q = lptr[b0 + pos]; q < end; q += kReduceAhead) {
+        int64_t id[kReduceAhead];
         TC v[kReduceAhead];
+        bool apart = false;
 #pragma unroll
-        for (int i = 0; i < kReduceAhead; ++i) v[i] = q + i < end ? contrib[9 * list[q + i] + k] : TC(0);
+        for (int i = 0; i < kReduceAhead; ++i) {
+          id[i] = q + i < end ? list[q + i] : -1;
+          const bool face = sizeof(TC) == 8 ? id[i] >= 0 : id[i] >= 0 && id[i] < n_face;
+          apart = apart || (id[i] >= 0 && !face);
+          v[i] = face ? contrib[9 * id[i] + k] : TC(0);
+        }
+        if (apart) {
+#pragma unroll
+          for (int i = 0; i < kReduceAhead; ++i)
+            if (id[i] >= n_face) h += hinge[9 * (id[i] - n_face) + k];
+        }
 #pragma unroll
         for (int i = 0; i < kReduceAhead; ++i)
           if (q + i < end) s += v[i];
       }
-      col[3 * c * len + 3 * pos + r] = widen(s);
+      col[3 * c * len + 3 * pos + r] = h != 0.0 ? widen(s) + h : widen(s);
     }
   }
 }
@@ -1195,11 +1222,11 @@ HingeArgs hinge_args(cgb_assembler* a, cgb_fold_dev& f, const double* d_x, int f
   h.theta0_gp = f.has_theta0_gp ? f.theta0_gp.p : nullptr;
   h.active = f.has_active ? f.active.p : nullptr;
   h.u_ptr = f.u_ptr.p; h.u_node = f.u_node.p; h.l_pos = f.l_pos.p; h.r_pos = f.r_pos.p;
-  h.pair_ptr = f.pair_ptr.p; h.pair_slot = f.pair_slot.p;
+  h.pair_ptr = f.pair_ptr.p;
+  h.pair_slot = (flags & CGB_MIXED) ? f.pair_hslot.p : f.pair_slot.p;
   h.x = d_x;
   h.exact = (flags & CGB_HINGE_EXACT) ? 1 : 0;
   h.want_K = (flags & CGB_TANGENT) ? 1 : 0;
-  h.tk_float = (flags & CGB_MIXED) ? 1 : 0;
   (void)a;
   return h;
 }
@@ -1370,27 +1397,38 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   if (!det) CGB_CUDA(cudaMemsetAsync(d_F, 0, ndof * sizeof(double), st));
   void* zero = nullptr;   // the block accumulator: whole 16-byte words, cleared by the first residual
   size_t zero_bytes = 0;
+  HingeBlocks hinge_blocks{};
   if (want_K && !det) {
-    zero_bytes = (static_cast<size_t>(a->n_blocks) * (mixed ? 12 * sizeof(float) : 9 * sizeof(double)) + 15) / 16 * 16;
-    if (mixed) a->kacc32.ensure(zero_bytes / sizeof(float));
-    else a->kacc64.ensure(zero_bytes / sizeof(double));
+    auto words = [](size_t bytes) { return (bytes + 15) / 16 * 16; };
+    if (mixed) {   // the hinge's FP64 blocks follow the FP32 ones (12 floats each)
+      const size_t face = static_cast<size_t>(a->n_blocks) * 12 * sizeof(float);
+      const size_t both = words(face + static_cast<size_t>(a->n_hinge_blocks) * 9 * sizeof(double));
+      a->kacc32.ensure(both / sizeof(float));
+      zero_bytes = hinge ? both : face;
+      if (hinge && a->n_hinge_blocks > 0)
+        hinge_blocks = {a->hinge_col.p, a->hinge_pos.p, reinterpret_cast<double*>(a->kacc32.p + 12 * a->n_blocks)};
+    } else {
+      zero_bytes = words(static_cast<size_t>(a->n_blocks) * 9 * sizeof(double));
+      a->kacc64.ensure(zero_bytes / sizeof(double));
+    }
     zero = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
     if (S->n_gp == 0 && zero_bytes > 0) CGB_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, st));
   }
-  const int64_t n_contrib = k_face_units + [&] { int64_t s = 0; for (auto& f : a->folds) s += f.n_pairs; return s; }();
+  int64_t n_hinge = 0;
+  for (auto& f : a->folds) n_hinge += f.n_pairs;
   if (det) {
     a->fcontrib.ensure(3 * std::max<int64_t>(a->n_fcontrib, 1));
     if (want_K) {
-      if (mixed) a->contrib32.ensure(9 * std::max<int64_t>(n_contrib, 1));
-      else a->contrib64.ensure(9 * std::max<int64_t>(n_contrib, 1));
+      if (mixed) a->contrib32.ensure(9 * std::max<int64_t>(k_face_units, 1));
+      else a->contrib64.ensure(9 * std::max<int64_t>(k_face_units + n_hinge, 1));
+      if (mixed) a->hinge_contrib.ensure(9 * std::max<int64_t>(n_hinge, 1));
     }
     // Hinge entries of inactive crease points contribute zero.
     if (a->n_fcontrib > S->nnz)
       CGB_CUDA(cudaMemsetAsync(a->fcontrib.p + 3 * S->nnz, 0, 3 * (a->n_fcontrib - S->nnz) * sizeof(double), st));
-    if (want_K && n_contrib > k_face_units) {
-      if (mixed) CGB_CUDA(cudaMemsetAsync(a->contrib32.p + 9 * k_face_units, 0, 9 * (n_contrib - k_face_units) * sizeof(float), st));
-      else CGB_CUDA(cudaMemsetAsync(a->contrib64.p + 9 * k_face_units, 0, 9 * (n_contrib - k_face_units) * sizeof(double), st));
-    }
+    if (want_K && n_hinge > 0)
+      CGB_CUDA(cudaMemsetAsync(mixed ? a->hinge_contrib.p : a->contrib64.p + 9 * k_face_units, 0,
+                               9 * n_hinge * sizeof(double), st));
   }
 
   prof_end(ctx, CGB_PHASE_ZERO, 0);
@@ -1457,22 +1495,22 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   a->work_ctr.ensure(kMaxChunks);
   CGB_CUDA(cudaMemsetAsync(a->work_ctr.p, 0, kMaxChunks * sizeof(int), st));
   // Hinge: it reads x, its shape sets and the fold state and adds into F and the block
-  // accumulator with atomics (or into its own contribution slots in deterministic mode), none
+  // accumulator (mixed: its own FP64 blocks) with atomics (or into its own contribution slots in deterministic mode), none
   // of which the face kernels read, so it runs beside them: on the side stream when the residual
   // is all there is (a hinge launch is mostly the latency of one warp), else on the context
   // stream beside the last tangent chunks.
   auto launch_hinge = [&](cudaStream_t hst) {
     prof_begin(ctx, CGB_PHASE_HINGE, hst);
     int nl = 0;
-    int64_t kb = k_face_units, fb = a->hinge_f_base;
+    int64_t kb = mixed ? 0 : k_face_units, fb = a->hinge_f_base;
     for (auto& f : a->folds) {
       if (f.n_gp == 0) continue;
       HingeArgs h = hinge_args(a, f, d_x, flags);
       h.F = d_F;
-      h.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
+      h.Kacc = mixed ? const_cast<double*>(hinge_blocks.acc) : a->kacc64.p;
       if (det) {
         h.Fc = a->fcontrib.p;
-        h.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
+        h.Kc = mixed ? a->hinge_contrib.p : a->contrib64.p;
         h.f_base = fb; h.k_base = kb;
       }
       // Warps per point: two per SM quarter over the launch, each with at least 4 rounds of pairs.
@@ -1635,14 +1673,15 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     det_reduce_F<<<nb(a->n_nodes, kReduceNodes), 32 * kReduceNodes, 0, st>>>(a->n_nodes, a->node_list_ptr.p, a->node_list.p, a->fcontrib.p, d_F);
     if (want_K) {
       const unsigned dg = static_cast<unsigned>(std::max(a->n_nodes, 1));
-      if (merged) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, d_K);
-      else if (mixed) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, d_K);
-      else det_reduce_blocks<double><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, d_K);
+      const double* hc = n_hinge > 0 ? a->hinge_contrib.p : nullptr;
+      if (merged) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, k_face_units, hc, d_K);
+      else if (mixed) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, k_face_units, hc, d_K);
+      else det_reduce_blocks<double><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, k_face_units, nullptr, d_K);
     }
   } else if (want_K) {
     nred = 1;
-    if (mixed) blocks_to_csc<float, 12><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc32.p, d_K);
-    else blocks_to_csc<double, 9><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc64.p, d_K);
+    if (mixed) blocks_to_csc<float, 12><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc32.p, hinge_blocks, d_K);
+    else blocks_to_csc<double, 9><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc64.p, hinge_blocks, d_K);
   }
   prof_end(ctx, CGB_PHASE_REDUCE, nred);
   CGB_CUDA(cudaGetLastError());

@@ -222,6 +222,7 @@ struct cgb_fold_dev {
   cgb::DevBuf<int32_t> l_pos, r_pos;
   cgb::DevBuf<int64_t> pair_ptr;    // n_gp + 1, pairs P <= Q over the merged list
   cgb::DevBuf<int32_t> pair_slot;   // block slot of each pair in the union pattern
+  cgb::DevBuf<int32_t> pair_hslot;  // the same among the blocks that any hinge pair touches
   int max_u = 0;
   int64_t n_u = 0;      // merged-node entries over all crease points (u_ptr[n_gp])
   int64_t n_pairs = 0;
@@ -249,7 +250,13 @@ struct cgb_assembler {
   bool have_material = false;
   // Accumulators.
   cgb::DevBuf<double> kacc64;       // 9 * n_blocks
-  cgb::DevBuf<float> kacc32;        // 12 * n_blocks (padded for 16-byte vector atomics)
+  cgb::DevBuf<float> kacc32;        // 12 * n_blocks (padded for 16-byte vector atomics), then the
+                                    // hinge's blocks in FP64 (9 * n_hinge_blocks)
+  // The blocks that hinge pairs touch, ascending by slot: the first of each column, and each one's
+  // block row within its column.
+  int64_t n_hinge_blocks = 0;
+  cgb::DevBuf<int64_t> hinge_col;   // n_nodes + 1
+  cgb::DevBuf<int32_t> hinge_pos;
   cgb::DevBuf<double> F;            // 3 n_nodes (device scratch for host-buffer calls)
   cgb::DevBuf<double> K;            // 9 n_blocks (device scratch for host-buffer calls)
   cgb::DevBuf<double> x;            // 3 n_nodes
@@ -303,6 +310,7 @@ struct cgb_assembler {
   cgb::DevBuf<int64_t> node_list;     // F contribution ids, ascending
   cgb::DevBuf<double> contrib64;      // 9 per contribution
   cgb::DevBuf<float> contrib32;
+  cgb::DevBuf<double> hinge_contrib;  // the hinge pairs' in mixed mode
   cgb::DevBuf<double> fcontrib;       // 3 per F contribution
   int64_t n_fcontrib = 0;
   int64_t hinge_f_base = 0;

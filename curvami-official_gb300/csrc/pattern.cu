@@ -466,9 +466,11 @@ void pattern_build(cgb_assembler* a) {
     CGB_CUDA(cudaMemcpyAsync(hcn.data(), a->col_nodes.p, hcn.size() * 4, cudaMemcpyDeviceToHost, st));
     CGB_CUDA(cudaStreamSynchronize(st));
     int64_t hoff = 0;
-    for (auto& f : a->folds) {
+    std::vector<std::vector<int32_t>> slots(a->folds.size());
+    for (size_t k = 0; k < a->folds.size(); ++k) {
+      auto& f = a->folds[k];
       std::vector<int64_t> pp(f.n_gp + 1, 0);
-      std::vector<int32_t> ps;
+      std::vector<int32_t>& ps = slots[k];
       for (int g = 0; g < f.n_gp; ++g) {
         const int64_t u0 = hptr[hoff + g], u1 = hptr[hoff + g + 1];
         for (int64_t P = u0; P < u1; ++P)
@@ -488,6 +490,27 @@ void pattern_build(cgb_assembler* a) {
       upload(f.pair_slot, ps.data(), ps.size(), st);
       CGB_CUDA(cudaStreamSynchronize(st));
     }
+    // The touched blocks numbered by slot (the mixed mode adds the hinge into FP64 blocks of its own).
+    std::vector<int32_t> at(a->n_blocks, -1), pos;
+    for (const auto& ps : slots)
+      for (int32_t q : ps) at[q] = 0;
+    std::vector<int64_t> hcol(n_nodes + 1, 0);
+    for (int j = 0; j < n_nodes; ++j) {
+      for (int64_t b = cptr[j]; b < cptr[j + 1]; ++b)
+        if (at[b] == 0) {
+          at[b] = static_cast<int32_t>(pos.size());
+          pos.push_back(static_cast<int32_t>(b - cptr[j]));
+        }
+      hcol[j + 1] = static_cast<int64_t>(pos.size());
+    }
+    a->n_hinge_blocks = hcol[n_nodes];
+    upload(a->hinge_col, hcol.data(), hcol.size(), st);
+    upload(a->hinge_pos, pos.data(), pos.size(), st);
+    for (size_t k = 0; k < a->folds.size(); ++k) {
+      for (int32_t& q : slots[k]) q = at[q];
+      upload(a->folds[k].pair_hslot, slots[k].data(), slots[k].size(), st);
+    }
+    CGB_CUDA(cudaStreamSynchronize(st));
   }
   CGB_CUDA(cudaStreamSynchronize(st));
 }
