@@ -31,14 +31,13 @@ struct DevCrease {
   float extent;       // their largest coordinate
 };
 
-// Squared distance in float of a point (relative to the crease's first vertex) to segment i.
+// Squared distance in float of a point (relative to the crease's first vertex) to segment i, its ends
+// not extended.
 __device__ __forceinline__ float segment_dist2f(const DevCrease& c, int i, float px, float py) {
   const float2 A = c.xyf[i], B = c.xyf[i + 1];
   const float vx = B.x - A.x, vy = B.y - A.y, wx = px - A.x, wy = py - A.y;
   const float v2 = vx * vx + vy * vy;
-  float t = v2 > 0.0f ? __fdividef(wx * vx + wy * vy, v2) : 0.0f;
-  if (!(i == 0 && c.extend_start)) t = fmaxf(t, 0.0f);
-  if (!(i == c.n_vertices - 2 && c.extend_end)) t = fminf(t, 1.0f);
+  const float t = v2 > 0.0f ? __saturatef(__fdividef(wx * vx + wy * vy, v2)) : 0.0f;
   const float ex = wx - t * vx, ey = wy - t * vy;
   return ex * ex + ey * ey;
 }
@@ -53,7 +52,9 @@ __device__ __forceinline__ float segment_dist2f(const DevCrease& c, int i, float
 // less than eps = 2^-18 X (the foot's error along the segment, 2^-20 X, is the largest part); a
 // segment more than 4 eps beyond the closest one's float distance is therefore farther than it by
 // 2 eps, far more than the FP64 comparison resolves, and the walk over the others in their order
-// ends where the walk over all would. The FP64 work of a point, some 45 operations a segment with a
+// ends where the walk over all would. That holds for feet within the segment: on an extended end the
+// rounding of the segment's direction grows with the distance along it, without bound, so extended
+// segments take no part in the float pass and are always walked. The FP64 work of a point, some 45 operations a segment with a
 // division, falls from all segments to a few (a point that all are equally far from keeps all).
 // L lanes (an aligned group of the warp, all with the same point) share the float pass: on 152 SMs 32
 // for up to 608 points, 4 for up to 4,864, else one (indicator_lanes in shape.cu). The three sets and
@@ -74,13 +75,14 @@ __device__ __forceinline__ DevIndicator eval_indicator(double px, double py, con
   double Cx = 0, Cy = 0, t_best = 0, snx = 0, sny = 0;
   int idx_best = 0;
   const bool sift = N > 4;
+  const int s0 = c.extend_start ? 1 : 0, s1 = N - 1 - (c.extend_end ? 1 : 0);   // the segments of the float pass
   float fx = 0.0f, fy = 0.0f, limit = 0.0f;
   if (sift) {
     fx = __double2float_rn(px - c.xy[0]);
     fy = __double2float_rn(py - c.xy[1]);
     float least = __int_as_float(0x7f800000);
 #pragma unroll 4
-    for (int i = sub; i < N - 1; i += L) least = fminf(least, segment_dist2f(c, i, fx, fy));
+    for (int i = s0 + sub; i < s1; i += L) least = fminf(least, segment_dist2f(c, i, fx, fy));
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(group, least, o));
     const float eps = fmaxf(fmaxf(fabsf(fx), fabsf(fy)), c.extent) * (1.0f / 262144.0f);
@@ -111,6 +113,7 @@ __device__ __forceinline__ DevIndicator eval_indicator(double px, double py, con
       sny = __ddiv_rn(vx, len);
     }
   };
+  auto left_out = [&](int i) { return sift && i >= s0 && i < s1 && segment_dist2f(c, i, fx, fy) > limit; };
   // The segments that are left, in their order: kStep decisions, then the walk over those that stay.
   constexpr int kStep = L == 1 ? 8 : L;
   for (int base = 0; base < N - 1; base += kStep) {
@@ -118,10 +121,10 @@ __device__ __forceinline__ DevIndicator eval_indicator(double px, double py, con
     if constexpr (L == 1) {
 #pragma unroll
       for (int k = 0; k < kStep; ++k)
-        if (base + k < N - 1 && !(sift && segment_dist2f(c, base + k, fx, fy) > limit)) keep |= 1u << k;
+        if (base + k < N - 1 && !left_out(base + k)) keep |= 1u << k;
     } else {
       const int i = base + sub;
-      keep = __ballot_sync(group, i < N - 1 && !(sift && segment_dist2f(c, i, fx, fy) > limit)) >> (lane - sub);
+      keep = __ballot_sync(group, i < N - 1 && !left_out(i)) >> (lane - sub);
     }
     for (; keep; keep &= keep - 1u) closer(base + __ffs(keep) - 1);
   }
