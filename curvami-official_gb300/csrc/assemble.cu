@@ -948,15 +948,16 @@ __global__ void blocks_to_csc_outer(int n_nodes, int64_t n_blocks, const int32_t
 // column. 430,000 FP32 blocks of 9 contributions (87 x 87 nodes) with det_reduce_F: 202 -> 108 us;
 // a lane per block had nine separate loads for each contribution, 36 bytes apart between the lanes.
 // 12 or 16 contributions ahead, or the next block's range fetched early: 115-120 us.
-// FP32 contributions: the units from n_face on are the hinge's, in FP64 in an array of their own
-// (hinge), and are summed apart.
+// With face_end the units from there on are the hinge's (from n_face on), in FP64 in an array of their
+// own, and are summed apart.
 constexpr int kReduceThreads = 128;   // 14 blocks at a time
 constexpr int kReduceAhead = 8;
 template <typename TC>
 __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes, const int64_t* __restrict__ col_ptr,
                                                                     const int64_t* __restrict__ lptr,
                                                                     const int64_t* __restrict__ list,
-                                                                    const TC* __restrict__ contrib, int64_t n_face,
+                                                                    const TC* __restrict__ contrib,
+                                                                    const int64_t* __restrict__ face_end, int64_t n_face,
                                                                     const double* __restrict__ hinge,
                                                                     double* __restrict__ K) {
   constexpr int kGroups = kReduceThreads / 9;
@@ -968,30 +969,25 @@ __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes,
     const int len = static_cast<int>(col_ptr[j + 1] - b0);
     double* col = K + 9 * b0;
     for (int pos = group; pos < len; pos += kGroups) {
-      const int64_t end = lptr[b0 + pos + 1];
+      const int64_t end = face_end ? face_end[b0 + pos] : lptr[b0 + pos + 1];
       TC s = TC(0);
-      double h = 0.0;
       for (int64_t q = lptr[b0 + pos]; q < end; q += kReduceAhead) {
-        int64_t id[kReduceAhead];
         TC v[kReduceAhead];
-        bool apart = false;
 #pragma unroll
-        for (int i = 0; i < kReduceAhead; ++i) {
-          id[i] = q + i < end ? list[q + i] : -1;
-          const bool face = sizeof(TC) == 8 ? id[i] >= 0 : id[i] >= 0 && id[i] < n_face;
-          apart = apart || (id[i] >= 0 && !face);
-          v[i] = face ? contrib[9 * id[i] + k] : TC(0);
-        }
-        if (apart) {
-#pragma unroll
-          for (int i = 0; i < kReduceAhead; ++i)
-            if (id[i] >= n_face) h += hinge[9 * (id[i] - n_face) + k];
-        }
+        for (int i = 0; i < kReduceAhead; ++i) v[i] = q + i < end ? contrib[9 * list[q + i] + k] : TC(0);
 #pragma unroll
         for (int i = 0; i < kReduceAhead; ++i)
           if (q + i < end) s += v[i];
       }
-      col[3 * c * len + 3 * pos + r] = h != 0.0 ? widen(s) + h : widen(s);
+      double sum = widen(s);
+      if (face_end) {
+        double h = 0.0;
+        const int64_t last = lptr[b0 + pos + 1];
+#pragma unroll 4
+        for (int64_t q = end; q < last; ++q) h += hinge[9 * (list[q] - n_face) + k];
+        if (end < last) sum += h;
+      }
+      col[3 * c * len + 3 * pos + r] = sum;
     }
   }
 }
@@ -1426,7 +1422,9 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     // Hinge entries of inactive crease points contribute zero.
     if (a->n_fcontrib > S->nnz)
       CGB_CUDA(cudaMemsetAsync(a->fcontrib.p + 3 * S->nnz, 0, 3 * (a->n_fcontrib - S->nnz) * sizeof(double), st));
-    if (want_K && n_hinge > 0)
+    bool all = hinge;   // every hinge pair is written
+    for (auto& f : a->folds) all = all && !f.has_active;
+    if (want_K && n_hinge > 0 && !all)
       CGB_CUDA(cudaMemsetAsync(mixed ? a->hinge_contrib.p : a->contrib64.p + 9 * k_face_units, 0,
                                9 * n_hinge * sizeof(double), st));
   }
@@ -1673,10 +1671,11 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     det_reduce_F<<<nb(a->n_nodes, kReduceNodes), 32 * kReduceNodes, 0, st>>>(a->n_nodes, a->node_list_ptr.p, a->node_list.p, a->fcontrib.p, d_F);
     if (want_K) {
       const unsigned dg = static_cast<unsigned>(std::max(a->n_nodes, 1));
-      const double* hc = n_hinge > 0 ? a->hinge_contrib.p : nullptr;
-      if (merged) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, k_face_units, hc, d_K);
-      else if (mixed) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, k_face_units, hc, d_K);
-      else det_reduce_blocks<double><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, k_face_units, nullptr, d_K);
+      const double* hc = a->hinge_contrib.p;
+      const int64_t* fe = n_hinge > 0 ? (merged ? a->ent_face_end.p : a->blk_face_end.p) : nullptr;
+      if (merged) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
+      else if (mixed) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
+      else det_reduce_blocks<double><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, nullptr, 0, nullptr, d_K);
     }
   } else if (want_K) {
     nred = 1;

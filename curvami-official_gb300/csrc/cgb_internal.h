@@ -304,6 +304,7 @@ struct cgb_assembler {
   bool det_entries_ready = false;     // K lists over the items' slots
   cgb::DevBuf<int64_t> blk_list_ptr;  // n_blocks + 1 (pair units)
   cgb::DevBuf<int64_t> blk_list;      // pair unit ids, ascending
+  cgb::DevBuf<int64_t> blk_face_end, ent_face_end;  // per block, the first hinge pair in its list
   cgb::DevBuf<int64_t> ent_list_ptr;  // n_blocks + 1 (entry units)
   cgb::DevBuf<int64_t> ent_list;      // entry unit ids, ascending
   cgb::DevBuf<int64_t> node_list_ptr; // n_nodes + 1

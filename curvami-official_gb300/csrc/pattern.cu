@@ -176,6 +176,19 @@ __global__ void sort_lists(int64_t n, const int64_t* __restrict__ lptr, int64_t*
   }
 }
 
+// The first unit of each (sorted) list that is n_face or more.
+__global__ void face_ends(int64_t n, const int64_t* __restrict__ lptr, const int64_t* __restrict__ list, int64_t n_face,
+                          int64_t* __restrict__ end) {
+  const int64_t b = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (b >= n) return;
+  int64_t lo = lptr[b], hi = lptr[b + 1];
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (list[mid] < n_face) lo = mid + 1; else hi = mid;
+  }
+  end[b] = lo;
+}
+
 // ---- tables of the FP32 tangent ---------------------------------------------------------
 // A cell is kMergeGroup consecutive face Gauss points (one quadrature cell with a 4x4 rule). Its
 // node union, ascending, numbers the cell's nodes u; a block (I, J), I <= J, of the cell is then in
@@ -589,7 +602,7 @@ namespace {
 // Per-block ascending lists of K units: n_face face units whose block slots are face_slot,
 // then every fold's pairs.
 void block_lists(cgb_assembler* a, int64_t n_face, const int32_t* face_slot, DevBuf<int64_t>& ptr,
-                 DevBuf<int64_t>& list) {
+                 DevBuf<int64_t>& list, DevBuf<int64_t>& face_end) {
   cudaStream_t st = a->ctx->stream;
   int64_t nq = n_face;
   for (auto& f : a->folds) nq += f.n_pairs;
@@ -614,6 +627,8 @@ void block_lists(cgb_assembler* a, int64_t n_face, const int32_t* face_slot, Dev
     base += f.n_pairs;
   }
   sort_lists<<<nb(a->n_blocks, 128), 128, 0, st>>>(a->n_blocks, ptr.p, list.p);
+  face_end.alloc(a->n_blocks);
+  face_ends<<<nb(a->n_blocks, 128), 128, 0, st>>>(a->n_blocks, ptr.p, list.p, n_face, face_end.p);
   CGB_CUDA(cudaGetLastError());
   CGB_CUDA(cudaStreamSynchronize(st));
 }
@@ -622,7 +637,7 @@ void block_lists(cgb_assembler* a, int64_t n_face, const int32_t* face_slot, Dev
 
 void deterministic_pair_lists(cgb_assembler* a) {
   if (a->det_pairs_ready) return;
-  block_lists(a, a->n_pairs, a->map_slot.p, a->blk_list_ptr, a->blk_list);
+  block_lists(a, a->n_pairs, a->map_slot.p, a->blk_list_ptr, a->blk_list, a->blk_face_end);
   a->det_pairs_ready = true;
 }
 
@@ -630,7 +645,7 @@ void deterministic_entry_lists(cgb_assembler* a) {
   if (a->det_entries_ready) return;
   tile_prepare(a);
   if (!a->direct_h.empty()) throw Error(CGB_ERR_INVALID, "deterministic entry lists need every group merged");
-  block_lists(a, 4 * a->n_items, a->item_slot.p, a->ent_list_ptr, a->ent_list);
+  block_lists(a, 4 * a->n_items, a->item_slot.p, a->ent_list_ptr, a->ent_list, a->ent_face_end);
   a->det_entries_ready = true;
 }
 
