@@ -952,7 +952,12 @@ __global__ void blocks_to_csc_outer(int n_nodes, int64_t n_blocks, const int32_t
 // own, and are summed apart.
 constexpr int kReduceThreads = 128;   // 14 blocks at a time
 constexpr int kReduceAhead = 8;
-template <typename TC>
+// TWO (FP32 pair units): the sum in two floats. A node's block is the sum of as many units as points
+// share it, 1,000 for the cubic basis at rho = 6h; added in one float in the same order at every node
+// of a regular mesh their rounding errors are alike, and a mixed path of 61 x 61 nodes stalled on it.
+// K's error there 8.5e-7 -> 2.3e-8 of its largest entry, first steps in 4 and 5 iterations like FP64's.
+// The units of cells are a tenth as many: 87 x 87 nodes 562 us a step, with two floats 588.
+template <typename TC, bool TWO>
 __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes, const int64_t* __restrict__ col_ptr,
                                                                     const int64_t* __restrict__ lptr,
                                                                     const int64_t* __restrict__ list,
@@ -970,16 +975,25 @@ __global__ void __launch_bounds__(kReduceThreads) det_reduce_blocks(int n_nodes,
     double* col = K + 9 * b0;
     for (int pos = group; pos < len; pos += kGroups) {
       const int64_t end = face_end ? face_end[b0 + pos] : lptr[b0 + pos + 1];
-      TC s = TC(0);
+      TC s = TC(0), lo = TC(0);
       for (int64_t q = lptr[b0 + pos]; q < end; q += kReduceAhead) {
         TC v[kReduceAhead];
 #pragma unroll
         for (int i = 0; i < kReduceAhead; ++i) v[i] = q + i < end ? contrib[9 * list[q + i] + k] : TC(0);
 #pragma unroll
         for (int i = 0; i < kReduceAhead; ++i)
-          if (q + i < end) s += v[i];
+          if (q + i < end) {
+            if constexpr (TWO) {   // what the sum rounds off, in lo
+              const TC t = __fadd_rn(s, v[i]), d = __fsub_rn(t, s);
+              lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(s, __fsub_rn(t, d)), __fsub_rn(v[i], d)));
+              s = t;
+            } else {
+              s += v[i];
+            }
+          }
       }
       double sum = widen(s);
+      if (TWO) sum += widen(lo);
       if (face_end) {
         double h = 0.0;
         const int64_t last = lptr[b0 + pos + 1];
@@ -1673,9 +1687,9 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       const unsigned dg = static_cast<unsigned>(std::max(a->n_nodes, 1));
       const double* hc = a->hinge_contrib.p;
       const int64_t* fe = n_hinge > 0 ? (merged ? a->ent_face_end.p : a->blk_face_end.p) : nullptr;
-      if (merged) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
-      else if (mixed) det_reduce_blocks<float><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
-      else det_reduce_blocks<double><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, nullptr, 0, nullptr, d_K);
+      if (merged) det_reduce_blocks<float, false><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->ent_list_ptr.p, a->ent_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
+      else if (mixed) det_reduce_blocks<float, true><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib32.p, fe, k_face_units, hc, d_K);
+      else det_reduce_blocks<double, false><<<dg, kReduceThreads, 0, st>>>(a->n_nodes, a->col_ptr.p, a->blk_list_ptr.p, a->blk_list.p, a->contrib64.p, nullptr, 0, nullptr, d_K);
     }
   } else if (want_K) {
     nred = 1;
