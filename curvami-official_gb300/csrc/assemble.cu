@@ -1436,9 +1436,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     // Hinge entries of inactive crease points contribute zero.
     if (a->n_fcontrib > S->nnz)
       CGB_CUDA(cudaMemsetAsync(a->fcontrib.p + 3 * S->nnz, 0, 3 * (a->n_fcontrib - S->nnz) * sizeof(double), st));
-    bool all = hinge;   // every hinge pair is written
-    for (auto& f : a->folds) all = all && !f.has_active;
-    if (want_K && n_hinge > 0 && !all)
+    if (want_K && n_hinge > 0)
       CGB_CUDA(cudaMemsetAsync(mixed ? a->hinge_contrib.p : a->contrib64.p + 9 * k_face_units, 0,
                                9 * n_hinge * sizeof(double), st));
   }
