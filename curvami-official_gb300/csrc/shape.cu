@@ -844,7 +844,8 @@ constexpr float kTwoThirdsLo = static_cast<float>(2.0 / 3.0 - static_cast<double
 constexpr float kFourThirdsHi = static_cast<float>(4.0 / 3.0);
 constexpr float kFourThirdsLo = static_cast<float>(4.0 / 3.0 - static_cast<double>(kFourThirdsHi));
 
-// radial() in pairs, same branches and cut-offs; z2 = s^2 of the scaled differences.
+// radial() in pairs, same branches and cut-offs; z2 = s^2 of the scaled differences. The window takes
+// s^2 from s: near s = 1 its terms cancel, and so do the errors of s in them when s^2 has the same.
 __device__ __forceinline__ void radial_pair(int kernel, fp2 z2, fp2& w, fp2& A, fp2& B, fp2& C) {
   const fp2 z{0.0f, 0.0f};
   const fp2 s = fp2_sqrt(z2);
@@ -853,11 +854,11 @@ __device__ __forceinline__ void radial_pair(int kernel, fp2 z2, fp2& w, fp2& A, 
   const fp2 is2 = at_node ? z : fp2_recip(z2);
   fp2 ds, dd;
   if (kernel == 0) {  // 1 - 6 s^2 + 8 s^3 - 3 s^4
-    w = 1.0f + z2 * (-6.0f + s * (8.0f - 3.0f * s));
+    w = 1.0f + fp2_sqr(s) * (-6.0f + s * (8.0f - 3.0f * s));
     ds = -12.0f + s * (24.0f - 12.0f * s);
     dd = -12.0f + s * (48.0f - 36.0f * s);
   } else if (fp2_le(s, 0.5f)) {  // 2/3 - 4 s^2 + 4 s^3
-    w = fp2{kTwoThirdsHi, kTwoThirdsLo} + z2 * (-4.0f + 4.0f * s);
+    w = fp2{kTwoThirdsHi, kTwoThirdsLo} + fp2_sqr(s) * (-4.0f + 4.0f * s);
     ds = -8.0f + 12.0f * s;
     dd = -8.0f + 24.0f * s;
   } else {  // 4/3 (1 - s)^3
