@@ -405,8 +405,7 @@ int cgb_shape_destroy(cgb_shape* sh) {
     // The blocks go back to the context's pool for the next set: work on any stream that reads them
     // is waited for, as cudaFree does.
     cudaSetDevice(ctx->device);
-    cudaStreamSynchronize(ctx->stream);
-    cudaDeviceSynchronize();
+    ctx->shape_pool.wait();
   }
   delete sh;
   if (ctx) cgb::ctx_release(ctx);

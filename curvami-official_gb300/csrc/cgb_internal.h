@@ -29,12 +29,13 @@ inline void cuda_check(cudaError_t e, const char* what) {
 // Device memory of one context's shape sets. A set is several arrays of up to a gigabyte, and mapping
 // and unmapping that with cudaMalloc and cudaFree cost 1.2 ms of a 6 ms build and its destruction.
 // Freed blocks stay with the pool, up to kKeep bytes, for the next set. Blocks are taken and given
-// back on a stream of the pool's own: take() waits for it (nothing else runs there), and a set is given
-// back only after its context's stream is idle (cgb_shape_destroy). The context destroys the pool.
+// back on a stream of the pool's own: a taker waits for it (nothing else runs there), and a set's blocks
+// are given back only after wait(). The context destroys the pool.
 struct ShapePool {
   static constexpr uint64_t kKeep = 4ULL << 30;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  mutable char* token = nullptr;   // what wait() frees
   void create(int device) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -44,8 +45,25 @@ struct ShapePool {
     uint64_t keep = kKeep;
     CGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
     CGB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    CGB_CUDA(cudaMalloc(&token, 1));
+  }
+  // Waits for the device's work as cudaFree of a set's arrays would. Not cudaDeviceSynchronize: that
+  // is an error while another thread captures a stream, and breaks the capture. 3 us when idle.
+  void wait() const {
+    if (!token && cudaMalloc(&token, 1) != cudaSuccess) {
+      cudaGetLastError();
+      cudaDeviceSynchronize();
+      return;
+    }
+    cudaFree(token);
+    if (cudaMalloc(&token, 1) != cudaSuccess) {
+      cudaGetLastError();
+      token = nullptr;
+    }
   }
   void destroy() {
+    if (token) cudaFree(token);
+    token = nullptr;
     if (stream) { cudaStreamSynchronize(stream); cudaStreamDestroy(stream); }
     if (pool) cudaMemPoolDestroy(pool);
     stream = nullptr;

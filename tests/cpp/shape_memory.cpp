@@ -1,0 +1,53 @@
+// The memory of shape sets over fake_cudart.cpp: what the library's C entries do to the device's memory and in
+// which order. Prints "ok" or what went wrong.
+#include <algorithm>
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "../../include/curvami_gb300.h"
+
+namespace fake {
+extern std::vector<std::string> log;
+extern size_t limit, held, idle;
+}  // namespace fake
+
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s (%s)\n", __LINE__, #x, cgb_last_error(ctx)); return 1; } } while (0)
+
+// A wait for all work on the device.
+static bool waits(const std::string& s) { return s == "cudaFree" || s == "cudaDeviceSynchronize"; }
+
+int main(int argc, char** argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  cgb_context* ctx = nullptr;
+  if (cgb_create(0, &ctx) != CGB_OK) return 2;
+  std::vector<double> xy;
+  for (int i = 0; i < 400; ++i) { xy.push_back(i % 20); xy.push_back(i / 20); }
+  CHECK(cgb_set_nodes(ctx, xy.data(), 400) == CGB_OK);
+  const int n = 1000;
+  std::vector<int64_t> ptr(n + 1);
+  std::vector<int32_t> idx(4 * n, 7);
+  std::vector<double> v(12 * n, 1.0);
+  for (int g = 0; g <= n; ++g) ptr[g] = 4 * g;
+  cgb_shape* sh = nullptr;
+  auto first_after = [](size_t at, auto&& is) {
+    return std::find_if(fake::log.begin() + at, fake::log.end(), is) - fake::log.begin();
+  };
+  auto given = [](const std::string& s) { return s == "cudaFreeAsync"; };
+
+  if (what == "destroy") {   // waits, but not with a call that another thread's capture forbids
+    CHECK(cgb_shape_from_host(ctx, n, ptr.data(), idx.data(), v.data(), v.data(), v.data(), &sh) == CGB_OK);
+    fake::log.clear();
+    CHECK(cgb_shape_destroy(sh) == CGB_OK);
+    CHECK(std::find(fake::log.begin(), fake::log.end(), "cudaDeviceSynchronize") == fake::log.end());
+    CHECK(first_after(0, waits) < first_after(0, given));
+  } else {
+    std::printf("unknown\n");
+    return 2;
+  }
+  cgb_destroy(ctx);
+  CHECK(fake::held == 0);
+  std::printf("ok\n");
+  return 0;
+}
