@@ -401,13 +401,8 @@ int cgb_shape_device(const cgb_shape* sh, const int64_t** nbr_ptr, const int32_t
 int cgb_shape_destroy(cgb_shape* sh) {
   if (!sh) return CGB_OK;
   cgb_context* ctx = sh->ctx;
-  if (ctx) {
-    // The blocks go back to the context's pool for the next set: work on any stream that reads them
-    // is waited for, as cudaFree does.
-    cudaSetDevice(ctx->device);
-    ctx->shape_pool.wait();
-  }
-  delete sh;
+  if (ctx) cudaSetDevice(ctx->device);
+  delete sh;   // its destructor waits for the work that reads it, on any stream
   if (ctx) cgb::ctx_release(ctx);
   return CGB_OK;
 }

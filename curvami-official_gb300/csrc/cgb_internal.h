@@ -195,11 +195,16 @@ struct cgb_context {
 };
 
 struct cgb_shape {
-  explicit cgb_shape(const cgb::ShapePool* pool) {
+  explicit cgb_shape(const cgb::ShapePool* from_pool) : pool(from_pool) {
     gp_xy.from = s.from = psi.from = dpsi.from = ddpsi.from = rho_node.from = pool;
     nbr_ptr.from = pool;
     nbr_idx.from = pool;
   }
+  // Also of a set whose making failed half way: kernels may still write its arrays.
+  ~cgb_shape() {
+    if (nbr_ptr.p || gp_xy.p || rho_node.p) pool->wait();
+  }
+  const cgb::ShapePool* pool;
   cgb_context* ctx = nullptr;
   int n_gp = 0;
   int64_t nnz = 0;

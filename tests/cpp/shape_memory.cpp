@@ -36,7 +36,17 @@ int main(int argc, char** argv) {
   };
   auto given = [](const std::string& s) { return s == "cudaFreeAsync"; };
 
-  if (what == "destroy") {   // waits, but not with a call that another thread's capture forbids
+  if (what == "failed_set") {   // no room for the last array: the copies into the others may be in flight
+    const size_t all = 8 * (n + 1) + 4 * 4 * n + 8 * 4 * n * 6;
+    fake::limit = fake::held + all - 8;
+    fake::log.clear();
+    CHECK(cgb_shape_from_host(ctx, n, ptr.data(), idx.data(), v.data(), v.data(), v.data(), &sh) == CGB_ERR_CUDA);
+    size_t copy = 0;
+    for (size_t k = 0; k < fake::log.size(); ++k) if (fake::log[k] == "cudaMemcpyAsync") copy = k;
+    const size_t wait = first_after(copy, waits), free_at = first_after(copy, given);
+    CHECK(free_at < fake::log.size());
+    CHECK(wait < free_at);
+  } else if (what == "destroy") {   // waits, but not with a call that another thread's capture forbids
     CHECK(cgb_shape_from_host(ctx, n, ptr.data(), idx.data(), v.data(), v.data(), v.data(), &sh) == CGB_OK);
     fake::log.clear();
     CHECK(cgb_shape_destroy(sh) == CGB_OK);
