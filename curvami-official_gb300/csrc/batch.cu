@@ -102,6 +102,7 @@ namespace {
 
 template <class F>
 int guarded_ctx(cgb_context* ctx, F&& body) {
+  const cgb::Active active(ctx);
   try {
     body();
     if (ctx) ctx->last_error.clear();

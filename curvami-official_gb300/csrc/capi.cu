@@ -15,6 +15,7 @@ namespace {
 
 template <class F>
 int guarded(cgb_context* ctx, F&& body) {
+  const cgb::Active active(ctx);
   try {
     body();
     if (ctx) ctx->last_error.clear();
@@ -86,6 +87,13 @@ void collect_marks(cgb_context* ctx) {
 }  // namespace
 
 namespace cgb {
+void reclaim() {
+  ShapePool::trim_all();
+  cgb_context* ctx = cgb_context::active;
+  if (!ctx || ctx->scratch.busy) return;
+  cudaStreamSynchronize(ctx->stream);
+  ctx->scratch = ShapeScratch{};
+}
 void prof_begin(cgb_context* ctx, int phase, cudaStream_t stream) {
   if (!ctx->profile) return;
   if (!stream) stream = ctx->stream;
@@ -227,6 +235,19 @@ int cgb_synchronize(cgb_context* ctx) {
     CGB_CUDA(cudaMemcpyAsync(&dev_err, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CGB_CUDA(cudaStreamSynchronize(ctx->stream));
     check_device_word(ctx, dev_err);
+  });
+}
+
+int cgb_trim(cgb_context* ctx) {
+  if (!ctx) return CGB_ERR_INVALID;
+  return guarded(ctx, [&] {
+    bind_device(ctx);
+    CGB_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->ws_x.reset();
+    ctx->ws_out.reset();
+    ctx->scratch = cgb::ShapeScratch{};
+    CGB_CUDA(cudaStreamSynchronize(ctx->shape_pool.stream));
+    CGB_CUDA(cudaMemPoolTrimTo(ctx->shape_pool.pool, 0));
   });
 }
 
@@ -667,7 +688,7 @@ int cgb_point_state(cgb_context* ctx, const cgb_shape* pts, const double* x, con
     cudaStream_t st = ctx->stream;
     const size_t nx = 3 * static_cast<size_t>(ctx->n_nodes);
     const size_t no = static_cast<size_t>(pts->n_gp) * CGB_POINT_STATE_COLS;
-    // Workspaces of the context, kept between the calls of one step's point sets.
+    // Workspaces of the context, kept between the calls of one step's point sets (large rows are not).
     cgb::DevBuf<double>&dx = ctx->ws_x, &dout = ctx->ws_out;
     dx.ensure(nx);
     dout.ensure(std::max<size_t>(no, 1));
@@ -675,6 +696,7 @@ int cgb_point_state(cgb_context* ctx, const cgb_shape* pts, const double* x, con
     cgb::point_state_device(ctx, pts, dx.p, A, B, D, dout.p);
     if (no) CGB_CUDA(cudaMemcpyAsync(out, dout.p, no * sizeof(double), cudaMemcpyDeviceToHost, st));
     CGB_CUDA(cudaStreamSynchronize(st));
+    if (dout.bytes() > cgb::ShapeScratch::kKeep) dout.reset();
   });
 }
 

@@ -1133,26 +1133,38 @@ __global__ void __launch_bounds__(kValueThreads) rkpm_pair_value_kernel(RkpmArgs
 // Returns the kernels launched.
 template <int ORDER, bool PAIR>
 int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
-  constexpr int kChunk = 1 << 20, NP = (ORDER + 1) * (ORDER + 2) / 2;
+  constexpr int kChunk = 1 << 20, kLeastChunk = 1 << 15, NP = (ORDER + 1) * (ORDER + 2) / 2;
   constexpr int kSums = std::max(MomIdx<ORDER>::N, 6 * RawIdx<ORDER>::NR);
   constexpr int kParts = PAIR ? 3 : ORDER == 3 ? 2 : 1;
   cudaStream_t st = ctx->stream;
-  const int n_gp = out->n_gp, most = std::min(n_gp, kChunk);
+  const int n_gp = out->n_gp;
+  int chunk = kChunk;
   int launches = 1;
   ctx->scratch.tip.ensure(n_gp);
   ctx->scratch.order.ensure(n_gp);
   ra.tip = ctx->scratch.tip.p;
   ra.order = ctx->scratch.order.p;
   point_order_kernel<<<blocks_for(n_gp, kSortPoints), kSortPoints, 0, st>>>(ra);
-  ctx->scratch.mom.ensure(static_cast<size_t>(most) * kSums);
-  ctx->scratch.coef.ensure(static_cast<size_t>(most) * 6 * NP);
+  for (;;) {   // half the points at a time where the scratch finds no room
+    const size_t most = std::min(n_gp, chunk);
+    try {
+      ctx->scratch.mom.ensure(most * kSums);
+      ctx->scratch.coef.ensure(most * 6 * NP);
+      break;
+    } catch (const OutOfMemory&) {
+      if (most <= kLeastChunk) throw;
+      while (chunk >= static_cast<int>(most)) chunk /= 2;
+      ctx->scratch.mom.reset();
+      ctx->scratch.coef.reset();
+    }
+  }
   ra.mom = ctx->scratch.mom.p;
   ra.coef = ctx->scratch.coef.p;
   int sms = 0;
   CGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  for (int g0 = 0; g0 < n_gp; g0 += kChunk) {
+  for (int g0 = 0; g0 < n_gp; g0 += chunk) {
     ra.g0 = g0;
-    ra.g1 = std::min(n_gp, g0 + kChunk);
+    ra.g1 = std::min(n_gp, g0 + chunk);
     const int np = ra.g1 - g0;
     const int64_t pairs = std::min(out->nnz, static_cast<int64_t>(np) * out->max_n);
     const unsigned vb = blocks_for(std::max<int64_t>(pairs, 1), kValueThreads);
@@ -1180,6 +1192,19 @@ int rkpm(cgb_context* ctx, cgb_shape* out, RkpmArgs ra, const float* rec) {
 
 void shape_values(cgb_context* ctx, cgb_shape* out, const std::vector<Crease>& creases);
 
+namespace {
+// A build's or rebuild's hold on the context's scratch, until its kernels have ended (however the call ends).
+struct ScratchUse {
+  cgb_context* ctx;
+  explicit ScratchUse(cgb_context* c) : ctx(c) { ctx->scratch.busy = true; }
+  ~ScratchUse() {
+    cudaStreamSynchronize(ctx->stream);
+    ctx->scratch.busy = false;
+    ctx->scratch.drop_large();
+  }
+};
+}  // namespace
+
 void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shape_params& prm,
                  const std::vector<Crease>& creases, cgb_shape* out) {
   cudaStream_t st = ctx->stream;
@@ -1200,6 +1225,7 @@ void shape_build(cgb_context* ctx, const double* gp_xy, int n_gp, const cgb_shap
   out->node_gen = ctx->node_gen;
 
   // ---- node cell grid (FRNN.h:33-44) ----
+  const ScratchUse use(ctx);
   ShapeScratch& w = ctx->scratch;
   double cell = prm.rho;
   if (prm.rho_node) {
@@ -1480,6 +1506,7 @@ void shape_rebuild(cgb_shape* sh, const std::vector<Crease>& creases) {
     throw Error(CGB_ERR_INVALID, "cgb_shape_rebuild: the nodes changed since the set was built (cgb_set_nodes)");
   // The new values stand even when a guard fires, as the reference's arrays do.
   ++sh->version;
+  const ScratchUse use(ctx);
   shape_values(ctx, sh, creases);
 }
 

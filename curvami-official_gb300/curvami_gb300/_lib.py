@@ -34,6 +34,7 @@ SIGNATURES = {
     "cgb_last_error": (cp, [vp]),
     "cgb_set_stream": (i32, [vp, vp]),
     "cgb_synchronize": (i32, [vp]),
+    "cgb_trim": (i32, [vp]),
     "cgb_set_nodes": (i32, [vp, vp, i32]),
     "cgb_set_natural_curvature": (i32, [vp, vp]),
     "cgb_shape_build": (i32, [vp, vp, i32, vp, vp, i32, C.POINTER(vp)]),

@@ -73,6 +73,10 @@ class Context:
         """Launch on the caller's cudaStream_t (e.g. torch.cuda.current_stream().cuda_stream)."""
         self.check(self.lib.cgb_set_stream(self.h, C.c_void_p(stream_ptr)))
 
+    def trim(self):
+        """Gives back the device memory kept for the context's next calls (cgb_trim)."""
+        self.check(self.lib.cgb_trim(self.h))
+
     def profile(self, on: bool):
         self.check(self.lib.cgb_profile_enable(self.h, int(bool(on))))
 

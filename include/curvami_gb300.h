@@ -107,6 +107,11 @@ const char* cgb_last_error(const cgb_context* ctx);
 /* Use the caller's cudaStream_t (passed as void*) for every launch and copy. */
 int cgb_set_stream(cgb_context* ctx, void* stream);
 int cgb_synchronize(cgb_context* ctx);
+/* Gives the device memory back that the context keeps for its next calls (scratch of the shape stage, up to
+ * 4 GiB of the arrays of destroyed shape sets); the next builds take it anew. An allocation of the
+ * context that finds no room does so by itself; a build with no room for its scratch takes fewer
+ * points at a time. */
+int cgb_trim(cgb_context* ctx);
 
 /* Reference node coordinates (Node::X_ref, core/include/curvami/MeshfreeData.h:7-14). */
 int cgb_set_nodes(cgb_context* ctx, const double* node_xy, int n_nodes);

@@ -11,7 +11,7 @@
 
 namespace fake {
 std::vector<std::string> log;
-size_t limit = ~size_t(0), held = 0, idle = 0;   // idle: of held, kept by the pool
+size_t limit = ~size_t(0), held = 0, idle = 0, peak = 0;   // idle: of held, kept by the pool
 std::map<void*, size_t> blocks;
 int launches = 0;
 
@@ -21,6 +21,7 @@ cudaError_t take(void** p, size_t n, bool pool) {
   if (held - reuse + n > limit) return cudaErrorMemoryAllocation;
   if (pool) idle -= reuse;
   held += n - reuse;
+  if (held > peak) peak = held;
   *p = std::calloc(n ? n : 1, 1);
   blocks[*p] = n;
   return cudaSuccess;

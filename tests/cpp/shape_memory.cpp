@@ -10,7 +10,7 @@
 
 namespace fake {
 extern std::vector<std::string> log;
-extern size_t limit, held, idle;
+extern size_t limit, held, idle, peak;
 }  // namespace fake
 
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s (%s)\n", __LINE__, #x, cgb_last_error(ctx)); return 1; } } while (0)
@@ -52,6 +52,31 @@ int main(int argc, char** argv) {
     CHECK(cgb_shape_destroy(sh) == CGB_OK);
     CHECK(std::find(fake::log.begin(), fake::log.end(), "cudaDeviceSynchronize") == fake::log.end());
     CHECK(first_after(0, waits) < first_after(0, given));
+  } else if (what == "room" || what == "scratch" || what == "trim") {
+    const int np = 200000;
+    std::vector<double> pts(2 * np, 5.5);
+    cgb_shape_params prm;
+    std::memset(&prm, 0, sizeof(prm));
+    prm.rho = 3.0;
+    prm.order = 2;
+    const size_t small = fake::held, scratch = size_t(np) * (90 + 36) * 8;   // moment sums and polynomials
+    CHECK(cgb_shape_build(ctx, pts.data(), np, &prm, nullptr, 0, &sh) == CGB_OK);
+    const size_t peak = fake::peak;
+    CHECK(peak > small + scratch);
+    CHECK(cgb_shape_destroy(sh) == CGB_OK);
+    if (what == "room") {   // other arrays find the room that destroyed sets and the scratch had
+      fake::limit = fake::held;
+      std::vector<double> more(2000000, 1.0);
+      CHECK(cgb_set_nodes(ctx, more.data(), 1000000) == CGB_OK);
+    } else {
+      CHECK(cgb_trim(ctx) == CGB_OK);
+      CHECK(fake::idle == 0 && fake::held < small + (8u << 20));
+      if (what == "scratch") {    // fewer points at a time
+        fake::limit = peak - scratch / 3;
+        CHECK(cgb_shape_build(ctx, pts.data(), np, &prm, nullptr, 0, &sh) == CGB_OK);
+        CHECK(cgb_shape_destroy(sh) == CGB_OK);
+      }
+    }
   } else {
     std::printf("unknown\n");
     return 2;

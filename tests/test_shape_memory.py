@@ -24,7 +24,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["failed_set", "destroy"])
+@pytest.mark.parametrize("what", ["failed_set", "destroy", "room", "scratch", "trim"])
 def test_memory(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
