@@ -344,8 +344,8 @@ struct cgb_assembler {
   uint64_t faces_version = 0;       // faces->version the copies (FP32, sliced-ELL) were made from
   // Tables of the FP32 tangent (tile_prepare): per face entry the index of its node in its
   // cell's sorted node union (a cell: 16 consecutive Gauss points), per cell the union's size,
-  // and the cell's items, each a node J and four nodes I <= J: the mask of the points they
-  // share | tile << 16 | J << 24, and the four block slots (-1: none). Cells with too many pairs
+  // and the cell's items, each a node J and four nodes I <= J that share a point with it: the mask of
+  // J's points | tile << 16 | J << 24, and the four block slots (-1: none). Cells with too many pairs
   // or nodes are "direct" (the per-entry tangent); tc_rest: the others that the tensor-core
   // tangent does not take (union above 42 nodes).
   bool tile_ready = false;

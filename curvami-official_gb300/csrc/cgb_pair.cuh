@@ -48,8 +48,6 @@ __device__ __forceinline__ fp2 fp2_two_prod(float a, float b) {
   return {p, __fmaf_rn(a, b, -p)};
 }
 
-__device__ __forceinline__ fp2 fp2_of(float a) { return {a, 0.0f}; }
-
 // Conversions between doubles and floats. Like an addition of doubles, the instructions for them
 // issue on the FP64 pipe, at 1/62 of the FP32 rate, so they are done on the bits; only exponents near
 // the ends of the float range, infinities and NaN in a pair take the instructions, in volatile asm so

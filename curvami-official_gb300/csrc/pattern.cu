@@ -193,8 +193,8 @@ __global__ void face_ends(int64_t n, const int64_t* __restrict__ lptr, const int
 // A cell is kMergeGroup consecutive face Gauss points (one quadrature cell with a 4x4 rule). Its
 // node union, ascending, numbers the cell's nodes u; a block (I, J), I <= J, of the cell is then in
 // its stored orientation (row: the lower node). The tangent's work item is a node J and a tile of
-// four consecutive nodes I <= J, with the mask of the points that have J and at least one of them
-// as neighbours: one CTA per cell finds the union, every entry's index in it, and the items, their
+// four consecutive nodes I <= J, with the mask of J's points (the derivatives of a node that a point does
+// not have are zeros; a tile that shares no point with J is no item): one CTA per cell finds the union, every entry's index in it, and the items, their
 // block slots (-1 where no point has both nodes) and their order: most points first, so the lanes
 // of a warp have loops of about one length, then by J, so that they share J's records.
 // A cell with more than kMergePairs pairs, a list above 64 or with a node twice, or a union above

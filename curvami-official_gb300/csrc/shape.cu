@@ -1,5 +1,5 @@
 // shape.cu — stage A on sm_103a: neighbour gather (GlobalFRNN) and RKPM shape
-// functions with crease visibility (GlobalRKPM), FP64.
+// functions with crease visibility (GlobalRKPM), FP64 or with the per-neighbour part in FP32 pairs.
 //
 // Reference: core/include/curvami/FRNN.h:23-78, core/include/curvami/Enrichment.h:23-92,
 // core/include/curvami/GlobalRKPM.h:15-397.
@@ -9,10 +9,13 @@
 // reference's hash map). One thread per Gauss point gathers its neighbours in the
 // reference's order (dx outer, dy inner, node index ascending in a cell) with an FP64
 // distance test written without FMA contraction, so the neighbour sets and their order
-// are bit-exact. The RKPM solve is FP64-pipe bound on GB300 (the FP64 rate is 1/62 of
-// the FP32 rate), so it also runs one Gauss point per thread: two passes over the
-// neighbours (moments, then shape functions) recompute the per-neighbour jets instead
-// of storing them, and per-node crease sides are hoisted into a per-node array.
+// are bit-exact. The RKPM runs as three kernels (four in pairs) over chunks of points, each
+// with the parallelism its part has: moments, one or a few threads per point, which leave the
+// weights' jets of every neighbour in the output arrays (in pairs a kernel of one thread
+// per neighbour makes them first); the solve, a thread per point; the values, a thread per
+// neighbour, from the jets and the point's polynomials. GB300's FP64 rate is 1/62 of the FP32 rate, so
+// the FP64 pipe bounds the first form throughout and the solve alone in the second. Per-node
+// crease sides are hoisted into a per-node array.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -4,7 +4,7 @@
 // One CTA per cell. The block of a pair is sum_a phi_i[a] T_j[a] (tangent_entry.cuh), so over the
 // cell's node union the blocks of a node J are products of T_J, one record per point that has J as
 // a neighbour, with the derivatives phi of the nodes I <= J. A thread takes J and a tile of four
-// consecutive I (an item of tile_prepare) and walks the points they share: it reads T_J (27
+// consecutive I (an item of tile_prepare) and walks the points of J: it reads T_J (27
 // values) and the normal once and phi of the four nodes, zero where a point does not have one of
 // them, and adds 4 x 36 FMA to 36 sums in registers, then scatters its blocks with three 16-byte
 // FP32 vector atomics each (a scattered block costs three L2 atomics and the chip sustains about
