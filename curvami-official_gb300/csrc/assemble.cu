@@ -27,7 +27,8 @@
 //
 // Precision modes: FP64 throughout, or "mixed" (FP64 kinematics, resultants and
 // residual; the per-neighbour factors and the pair loop in FP32, accumulated into an
-// FP32 block array that is widened to FP64 on output).
+// FP32 block array that is widened to FP64 on output, the hinge beside it in FP64; into an FP64 one
+// where the supports are too wide for cells).
 // Scatter modes: atomics into a block array (BSR, one 3x3 block per pattern slot), or
 // deterministic: every block value goes to a contribution array and a second kernel
 // sums each block's contributions in ascending Gauss-point order.
@@ -1233,7 +1234,6 @@ HingeArgs hinge_args(cgb_assembler* a, cgb_fold_dev& f, const double* d_x, int f
   h.active = f.has_active ? f.active.p : nullptr;
   h.u_ptr = f.u_ptr.p; h.u_node = f.u_node.p; h.l_pos = f.l_pos.p; h.r_pos = f.r_pos.p;
   h.pair_ptr = f.pair_ptr.p;
-  h.pair_slot = (flags & CGB_MIXED) ? f.pair_hslot.p : f.pair_slot.p;
   h.x = d_x;
   h.exact = (flags & CGB_HINGE_EXACT) ? 1 : 0;
   h.want_K = (flags & CGB_TANGENT) ? 1 : 0;
@@ -1400,6 +1400,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     else deterministic_pair_lists(a);
   }
   const int64_t k_face_units = merged ? 4 * a->n_items : a->n_pairs;
+  const bool acc32 = merged;   // the block accumulator: FP32 with the cells' tangent, else FP64
 
   const int64_t ndof = 3 * static_cast<int64_t>(a->n_nodes);
   // Accumulators.
@@ -1410,7 +1411,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   HingeBlocks hinge_blocks{};
   if (want_K && !det) {
     auto words = [](size_t bytes) { return (bytes + 15) / 16 * 16; };
-    if (mixed) {   // the hinge's FP64 blocks follow the FP32 ones (12 floats each)
+    if (acc32) {   // the hinge's FP64 blocks follow the FP32 ones (12 floats each)
       const size_t face = static_cast<size_t>(a->n_blocks) * 12 * sizeof(float);
       const size_t both = words(face + static_cast<size_t>(a->n_hinge_blocks) * 9 * sizeof(double));
       a->kacc32.ensure(both / sizeof(float));
@@ -1421,7 +1422,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       zero_bytes = words(static_cast<size_t>(a->n_blocks) * 9 * sizeof(double));
       a->kacc64.ensure(zero_bytes / sizeof(double));
     }
-    zero = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
+    zero = acc32 ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
     if (S->n_gp == 0 && zero_bytes > 0) CGB_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, st));
   }
   int64_t n_hinge = 0;
@@ -1459,7 +1460,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
   fa.gp_xy = natcurv_points(ctx, S, "assemble");
   fa.F = d_F;
   fa.Fc = a->fcontrib.p;
-  fa.Kacc = mixed ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
+  fa.Kacc = acc32 ? static_cast<void*>(a->kacc32.p) : static_cast<void*>(a->kacc64.p);
   fa.Kc = mixed ? static_cast<void*>(a->contrib32.p) : static_cast<void*>(a->contrib64.p);
   if (want_K && (!merged || !a->direct_h.empty())) ensure_entry_points(a);
   if (mixed && want_K) {
@@ -1517,7 +1518,8 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       if (f.n_gp == 0) continue;
       HingeArgs h = hinge_args(a, f, d_x, flags);
       h.F = d_F;
-      h.Kacc = mixed ? const_cast<double*>(hinge_blocks.acc) : a->kacc64.p;
+      h.Kacc = acc32 ? const_cast<double*>(hinge_blocks.acc) : a->kacc64.p;
+      h.pair_slot = acc32 ? f.pair_hslot.p : f.pair_slot.p;
       if (det) {
         h.Fc = a->fcontrib.p;
         h.Kc = mixed ? a->hinge_contrib.p : a->contrib64.p;
@@ -1594,11 +1596,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       const int per_cell = glist ? static_cast<int>(nb(static_cast<int64_t>(kMG) * fa.nmax, kEntryThreads)) : 0;
       const unsigned egrid = glist ? static_cast<unsigned>(gcount) * per_cell
                                    : std::max(1u, nb(std::min(S->nnz, static_cast<int64_t>(ncg) * fa.nmax), kEntryThreads));
-      int mix = 0;   // FP32 sums: the blocks in a mixed order (face_tangent_entry_kernel)
-      if (mixed && !det && !glist)
-        while (mix < 16 && (1u << mix) < egrid) ++mix;
-      const unsigned window = 1u << mix;
-      kern<<<(egrid + window - 1) / window * window, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p, glist, per_cell, mix);
+      kern<<<egrid, kEntryThreads, 0, a->side>>>(fa, stp, a->ent_point.p, glist, per_cell);
     };
     int ntan = 1;
     if (merged) {
@@ -1651,16 +1649,16 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
       }
       const auto [at, count] = part(a->direct_h);
       if (count > 0) {
-        if (bzero) tl(face_tangent_entry_kernel<float, false, true>, st32, a->direct.p + at, count);
-        else tl(face_tangent_entry_kernel<float, false, false>, st32, a->direct.p + at, count);
+        if (bzero) tl(face_tangent_entry_kernel<float, float, false, true>, st32, a->direct.p + at, count);
+        else tl(face_tangent_entry_kernel<float, float, false, false>, st32, a->direct.p + at, count);
         ++ntan;
       }
     } else if (mixed) {
-      if (det) { if (bzero) tl(face_tangent_entry_kernel<float, true, true>, st32); else tl(face_tangent_entry_kernel<float, true, false>, st32); }
-      else { if (bzero) tl(face_tangent_entry_kernel<float, false, true>, st32); else tl(face_tangent_entry_kernel<float, false, false>, st32); }
+      if (det) { if (bzero) tl(face_tangent_entry_kernel<float, float, true, true>, st32); else tl(face_tangent_entry_kernel<float, float, true, false>, st32); }
+      else { if (bzero) tl(face_tangent_entry_kernel<float, double, false, true>, st32); else tl(face_tangent_entry_kernel<float, double, false, false>, st32); }
     } else {
-      if (det) { if (bzero) tl(face_tangent_entry_kernel<double, true, true>, st64); else tl(face_tangent_entry_kernel<double, true, false>, st64); }
-      else { if (bzero) tl(face_tangent_entry_kernel<double, false, true>, st64); else tl(face_tangent_entry_kernel<double, false, false>, st64); }
+      if (det) { if (bzero) tl(face_tangent_entry_kernel<double, double, true, true>, st64); else tl(face_tangent_entry_kernel<double, double, true, false>, st64); }
+      else { if (bzero) tl(face_tangent_entry_kernel<double, double, false, true>, st64); else tl(face_tangent_entry_kernel<double, double, false, false>, st64); }
     }
     ++nface;
     prof_end(ctx, CGB_PHASE_TANGENT, ntan, a->side);
@@ -1691,7 +1689,7 @@ void assemble_device(cgb_assembler* a, const double* d_x, double* d_K, double* d
     }
   } else if (want_K) {
     nred = 1;
-    if (mixed) blocks_to_csc<float, 12><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc32.p, hinge_blocks, d_K);
+    if (acc32) blocks_to_csc<float, 12><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc32.p, hinge_blocks, d_K);
     else blocks_to_csc<double, 9><<<cg, 128, 0, st>>>(a->n_nodes, a->col_ptr.p, a->kacc64.p, hinge_blocks, d_K);
   }
   prof_end(ctx, CGB_PHASE_REDUCE, nred);

@@ -330,7 +330,7 @@ struct cgb_assembler {
   bool have_material = false;
   // Accumulators.
   cgb::DevBuf<double> kacc64;       // 9 * n_blocks
-  cgb::DevBuf<float> kacc32;        // 12 * n_blocks (padded for 16-byte vector atomics), then the
+  cgb::DevBuf<float> kacc32;        // cells' tangent: 12 * n_blocks (padded for 16-byte vector atomics), then the
                                     // hinge's blocks in FP64 (9 * n_hinge_blocks)
   // The blocks that hinge pairs touch, ascending by slot: the first of each column, and each one's
   // block row within its column.

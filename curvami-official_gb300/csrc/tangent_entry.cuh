@@ -181,11 +181,17 @@ constexpr int kEntryThreads = 128;
 // every entry. A warp's 32 blocks of one step are turned through shared memory, so that a
 // block's nine values leave on neighbouring lanes (72 consecutive bytes: 3 sectors instead of
 // the 9 of one value per lane and instruction).
-template <typename TK, bool DET, bool BZERO>
+// TA: the type of the block accumulator (DET: of the contributions). FP32 blocks go into FP64 sums where every
+// entry of the plate comes here. A node's block is the sum of up to 1,000 of them, and added in FP32
+// the sums round alike at all nodes of a regular mesh, which adds up over smooth displacements: the
+// first steps of a 61 x 61 cubic sheet (rho = 6h) took 10, 14 and 16 corrector iterations, and stalled where the
+// points came in ascending order; with FP64 sums 4, 5 and 5, as with an FP64 tangent. K's error
+// there 8.3e-7 -> 2.3e-8 of its largest entry, a step 2.55 -> 3.44 ms. Cells too large for a tile
+// add to the FP32 sums of the others.
+template <typename TK, typename TA, bool DET, bool BZERO>
 __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceArgs a, const TK* __restrict__ gstate,
                                                                          const int32_t* __restrict__ ent_point,
-                                                                         const int32_t* __restrict__ glist, int per_cell,
-                                                                         int mix_bits) {
+                                                                         const int32_t* __restrict__ glist, int per_cell) {
   __shared__ TK s_val[kEntryThreads / 32][32 * 9];
   __shared__ int64_t s_at[kEntryThreads / 32][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -194,21 +200,6 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
     gb = kMG * glist[blockIdx.x / per_cell];
     ge = min(gb + kMG, a.g_end);
     blk = blockIdx.x % per_cell;
-  } else if (mix_bits > 0) {
-    // FP32 sums by atomics: the blocks of a window of 2^mix_bits are taken in a mixed order (odd factors
-    // and shifts right, each a permutation of the window). In ascending order a block's contributions
-    // come point by point; on a regular mesh the sums of all its translates then round alike and
-    // the errors add up over smooth displacements: for w = 1 on a flat 61 x 61 cubic plate dK is off by 9.2e-8 so
-    // and by 2.7e-8 in the mixed order (the hinge, in FP64 apart, has no part in it), and such a sheet's path
-    // stalled in ascending order. No slower: 2,405 us a step there. Cells left to this kernel (glist) are taken
-    // as they come: at rho = 5h, with most cells left to it, the errors are those of the mixed order.
-    const unsigned mask = (1u << mix_bits) - 1u, half = (mix_bits + 1) / 2;
-    unsigned m = static_cast<unsigned>(blk) & mask;
-    m = (m * 0x9e3779b1u) & mask;
-    m ^= m >> half;
-    m = (m * 0x85ebca6bu) & mask;
-    m ^= m >> half;
-    blk = static_cast<int>((static_cast<unsigned>(blk) & ~mask) | m);
   }
   const int64_t e_end = a.ptr[ge];
   const int64_t ew = a.ptr[gb] + static_cast<int64_t>(blk) * kEntryThreads + 32 * w;  // the warp's first
@@ -234,8 +225,8 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
   const int64_t m0 = a.map_ptr[g];
   const int steps = live ? n / 2 + 1 : 0;
   const int wsteps = __reduce_max_sync(0xffffffffu, steps);
-  TK* acc = static_cast<TK*>(DET ? a.Kc : a.Kacc);
-  constexpr int64_t kStride = (DET || sizeof(TK) == 8) ? 9 : 12;
+  TA* acc = static_cast<TA*>(DET ? a.Kc : a.Kacc);
+  constexpr int64_t kStride = (DET || sizeof(TA) == 8) ? 9 : 12;
   TK* sv = s_val[w];
   int64_t* sa = s_at[w];
   for (int d = 0; d < wsteps; ++d) {
@@ -266,6 +257,7 @@ __global__ void __launch_bounds__(kEntryThreads) face_tangent_entry_kernel(FaceA
       const int64_t to = sa[l];
       if (to >= 0) {
         if constexpr (DET) acc[to + (t - 9 * l)] = sv[t];
+        else if constexpr (sizeof(TA) > sizeof(TK)) atomicAdd(acc + to + (t - 9 * l), fp2_widen(sv[t]));
         else atomicAdd(acc + to + (t - 9 * l), sv[t]);
       }
     }

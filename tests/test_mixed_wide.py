@@ -1,4 +1,5 @@
-"""The deterministic FP32 tangent of wide supports (lists above 110, the per-entry tangent) against FP64.
+"""The FP32 tangent of wide supports (lists above 110, the per-entry tangent), atomic and deterministic, against
+FP64.
 
 A block of K is the sum of m contributions of size t, m up to 9 * 113 here; FP32 forms each with a dozen
 roundings, u = 2^-24, independent within a block: an error of 12 u t sqrt(m), 12 u / sqrt(m) = 0.4 u of the
@@ -14,7 +15,8 @@ from curvami_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 
-def test_wide_supports_sum():
+@pytest.mark.parametrize("mode", [cg.MIXED, cg.MIXED | cg.DETERMINISTIC])
+def test_wide_supports_sum(mode):
     import __graft_entry__ as ge
 
     ge.build()
@@ -22,5 +24,5 @@ def test_wide_supports_sum():
     asm = cg.PlateModel(p, cg.Context(0)).asm
     x = np.zeros(3 * len(p.node_xy))
     K = asm.assemble(x, cg.TANGENT | cg.DETERMINISTIC)[0].copy()
-    K32 = asm.assemble(x, cg.TANGENT | cg.MIXED | cg.DETERMINISTIC)[0]
+    K32 = asm.assemble(x, cg.TANGENT | mode)[0]
     assert np.abs(K32 - K).max() <= 4.0 * 2.0 ** -24 * np.abs(K).max()
