@@ -874,8 +874,8 @@ def four_creases_assembly(cg, ctx, stream):
 def arc_length_path(cg, ctx, n_side=41, target_deg=150.0, kmax=80):
     """The full arc-length path at reduced size: NonLinearSolver::KinematicArcLength restated
     (curvami_gb300/arclength.py) over the GPU's FP64 assembly with the exact hinge tangent
-    (the predictor of this thin plate, t / L = 2.5e-3, needs the FP64 tangent: with the FP32
-    one the run reversed its first steps). Four creases from the centre, sectors
+    (on this thin plate, t / L = 2.5e-3, the FP32 tangent takes about twice the corrector
+    iterations). Four creases from the centre, sectors
     90 +/- 15 deg (seeded);
     creases 0 and 2 are the drivers (stiff hinges, Kt = 0.1, whose rest angle goes from 0 to
     150 deg with the deployment parameter mu), 1 and 3 passive elastic hinges (Kt = 1e-3);
